@@ -2,23 +2,22 @@
 // step (C-ABI in include/shoc_tr_gpu.h).
 //
 // Per step, on the handle's stream:
-//   k_reset     clears the per-step reductions
-//   k_lateral   set_lateral_BC_tr (tracers.c:5574) into both tracer buffers
-//   k_set_dz    one thread per column: set_dz (tracers.c:5731-5848), the
+//   k_lateral   set_lateral_BC_tr (tracers.c:5574) into both tracer buffers,
+//               and the per-step reductions cleared (k_reset where it is not run)
+//   k_set_dz    one block per tile of 32 columns: set_dz (tracers.c:5731-5848), the
 //               scheme work arrays w5/w9 (:561-567) and their 2/(w9+w9)
 //               factors, the sub-step search (:591-668) as a min-reduction,
 //               and the tracer-independent tridiagonal LU factors of
 //               vert_diffuse_3d / implicit_vdiff_tr (:3841-3889, :4185-4195)
 //   per sub-step:
-//     k_courant   w6/w7/w8 (:726-737) of the general-path columns
 //     k_adv32 + k_vd32 (FP32-mixed, shoc_tr_tile.cuh; or the one fused
 //                 k_step32 of shoc_tr_fused.cuh, SHOC_TR_GPU_KERNELS=fused)
 //                 or k_adv64 + k_vd64 (FP64, shoc_tr_tile64.cuh): the
 //                 columns whose surface cell stays in its layer, one thread
 //                 per cell, then one per (column, tracer)
-//     k_serial    the other columns (surface crossing a layer face, thin-
+//     k_general   the other columns (surface crossing a layer face, thin-
 //                 surface fix coupling tracers, degenerate solve range), one
-//                 thread per column looping over tracers: column_pass
+//                 thread per (column, tracer): column_pass
 // Tracers ping-pong between two buffers; a step is captured in a CUDA graph
 // once its sub-step schedule is known.
 #include <cuda_runtime.h>
@@ -46,7 +45,7 @@ using namespace shoc;
 namespace {
 
 constexpr int kItermax = 20;  // tracers.c:430
-constexpr int kSerialBlocks = 148 * 2;  // general-path kernel: one thread per listed column
+constexpr int kGeneralBlocks = 148 * 8;  // general-path kernel: most blocks of one launch
 
 struct Sched {
   double dtm = 0.0;
@@ -140,7 +139,7 @@ struct shoc_tr_gpu {
   cudaStream_t s_up = nullptr, s_dn = nullptr;  // host -> device, device -> host
   std::vector<cudaEvent_t> pev;     // [0] flow sent, then per chunk: sent, stepped
   double *xout = nullptr;           // FP32-mixed: one tracer of FP64 for the way back
-  uint8_t *c3s = nullptr;           // [kItermax + 2][ncol] k_serial cursors between chunks
+  uint8_t *c3s = nullptr;           // [kItermax + 2][ncol] k_general cursors between chunks
 };
 
 namespace {
@@ -191,23 +190,26 @@ int dupload(shoc_tr_gpu *h, T **p, const T *src, size_t n) {
 // ---------------------------------------------------------------------------
 // kernels
 
+__device__ __forceinline__ void reset_reductions(const Work &W, int *counts) {
+  *W.dtm_bits = 0x7ff0000000000000ull;  // +inf
+  *W.serial_count = 0;
+  counts[0] = 0;
+  counts[1] = 0;
+}
 __global__ void k_reset(Work W, int *counts) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    *W.dtm_bits = 0x7ff0000000000000ull;  // +inf
-    *W.serial_count = 0;
-    counts[0] = 0;
-    counts[1] = 0;
-  }
+  if (threadIdx.x == 0 && blockIdx.x == 0) reset_reductions(W, counts);
 }
 
 // Lateral ghosts take their interior value (set_lateral_BC_tr): written into
 // both tracer buffers so the value read during every sub-step, and the value
 // left in the returned array, is the start-of-step one.  la / lb (FP32_COMP):
-// the buffers' compensations, copied alike.
+// the buffers' compensations, copied alike.  counts (or null): also clears
+// the step's reductions, which saves a launch.
 template <class TR>
 __global__ void k_lateral(int nbpt, const int *bpt, const int *bin, const int *slot_tr,
-                          int nslot, int S, TR *tra, TR *trb, int16_t *la = nullptr,
-                          int16_t *lb = nullptr) {
+                          int nslot, int S, TR *tra, TR *trb, int16_t *la, int16_t *lb, Work W,
+                          int *counts) {
+  if (counts && threadIdx.x == 0 && blockIdx.x == 0) reset_reductions(W, counts);
   long long tot = (long long)nbpt * nslot;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < tot;
        i += (long long)gridDim.x * blockDim.x) {
@@ -228,274 +230,315 @@ __device__ __forceinline__ void atomic_min_pos(unsigned long long *p, double v) 
   atomicMin(p, (unsigned long long)__double_as_longlong(v));
 }
 
-// One thread per column: the surface cells, set_dz (tracers.c:5731-5848), the
-// scheme work arrays w5/w9 (:561-567) and their 2/(w9+w9) factors, the
-// sub-step search (:591-668) as a min-reduction, the column flags and the
-// tracer-independent LU factors of vert_diffuse_3d / implicit_vdiff_tr
-// (:3841-3889, :4185-4195).  Layer j of the column (j = 0 the sediment cell,
-// j = 1..nk the wet layers from the bottom up) comes from the layer-by-column
-// table; the thickness of a layer is a function of the surface cells and two
-// layer faces, so the column is streamed twice without per-layer arrays: top
-// down for the thicknesses, work arrays and sub-step search (a window of the
-// layers around j in registers), bottom up for the LU recurrence.  Every
-// value is the reference's expression on the reference's operands, and the
-// sub-step minimum does not depend on the order the cells are visited in.
+// The step's set-up, a block of kSetDzWarps warps per tile of 32 columns (lane =
+// column): set_dz (tracers.c:5731-5848), the scheme work arrays w5/w9 (:561-567)
+// and their 2/(w9+w9) factors, the sub-step search (:591-668) as a
+// min-reduction, the column flags and the tracer-independent LU factors of
+// vert_diffuse_3d / implicit_vdiff_tr (:3841-3889, :4185-4195).
+//
+// What bounds it: one thread per column walked its column twice through
+// dependent loads (cell, face, thickness, divisions): 31 us at 64 x 64 x 20,
+// 0.60 ms at 1024 x 512 x 50, however few columns there were.  Here
+// only the LU recurrence is serial.  Layer j of a column (j = 0 the sediment
+// cell, j = 1..nk the wet layers from the bottom up) is a function of the
+// surface cells and of the layer faces around it, so the warps of the block
+// share the layers: (0) cells and bottom faces into shared memory; (1) per
+// layer the thicknesses, the work arrays, the sub-step search and the rows of
+// the tridiagonal matrix (their divisions included); (2) one warp runs the
+// recurrence div(j) = C(j) - cm1(j) cp1(j-1) / div(j-1) from shared memory;
+// (3) all warps write the factors.  Every value is the reference's expression
+// on the reference's operands; the sub-step minimum does not depend on the
+// order the cells are visited in.
+//
 // list_all: put every column the tile kernels do not handle on the
 // general-path list (else only the tracer-coupled thin-surface columns).
-// fp32: also write the FP32 thickness and LU factors.
-// own (or null): 1 for the columns whose cells count in the sub-step minimum
-// (a strip of a decomposed basin counts its own columns, not its halo).
-// probe: compute the minimum only and leave the surface vectors as they are.
-// Reads of arrays no kernel of the step writes go through the read-only
-// path (__ldg), so the compiler may issue them ahead of this thread's stores
-// to the work arrays.  The walk down a column waits on dependent loads, so
-// the kernel is held to 64 registers for 8 blocks (32 warps) per SM: 2.26
-// against 2.67 ms outside the transport kernels at stiff2048 (80 registers,
-// 6 blocks); tighter bounds spill.
-__global__ void __launch_bounds__(128, 8) k_set_dz(Geo G, Flow F, Work W, Opt O, Tile Tl,
-                                                int any_vdiff, int *counts, int list_all,
-                                                int fp32, const int *own, int probe) {
-  int col = blockIdx.x * blockDim.x + threadIdx.x;
-  double dtmin = __longlong_as_double(0x7ff0000000000000ll);
-  int nwetcol = 0, ncells = 0;  // this column's share of counts[0], counts[1]
-  if (col < G.ncol) {
-    const int top = G.col_top[col], bot = G.col_bot[col], kb = G.col_kb[col];
-    const int nk = G.nz - kb;  // wet layers of the column
-    const int sed = G.zm1[bot];
-    // cell of layer j and the layer of a cell of this column
-    auto cell = [&](int j) {
-      return j == 0 ? sed : __ldg(&Tl.cellk[(size_t)(kb + j - 1) * Tl.ncolp + col]);
-    };
-    auto jof = [&](int c) { return c == sed ? 0 : __ldg(&G.kof[c]) - kb + 1; };
+// what: SD_* flags.  own (or null): 1 for the columns whose cells count in the
+// sub-step minimum (a strip of a decomposed basin counts its own columns, not
+// its halo).  Without SD_SEARCH there is no sub-step search: a step whose
+// schedule is known does not read its result.
+constexpr int SD_PROBE = 1;   // leave the surface vectors as they are
+constexpr int SD_SEARCH = 2;  // the sub-step minimum into W.dtm_bits
+constexpr int SD_F32 = 4;     // also the FP32 thickness and LU factors
+constexpr int SD_WORK = 8;    // w5, w9, dbz, dfz of the tile kernels' columns
+constexpr int SD_LU64 = 16;   // FP64 LU factors of the tile kernels' columns
+                              // (the general path's columns get all of them)
+constexpr int kSetDzWarps = 8;
+// bytes: FP64 faces (then ud), rows cm1 and dz/dt (then div) and the cells of
+// nz layers of 32 columns
+inline size_t set_dz_smem(int nz) { return (size_t)nz * 32 * (3 * 8 + 4); }
 
-    // new and old surface cells (tracers.c:5739-5755): down from the top
-    // while the cell's bottom is at or above eta, at most to the sediment
-    int sur = W.nsur_t[col];
-    int jn = nk;
-    const double etat = F.eta[top];
-    while (jn > 0 && __ldg(&G.gridz[cell(jn)]) >= etat) --jn;
-    int nsur = cell(jn);
-    if (!probe) {
-      W.sur_t[col] = sur;
-      W.nsur_t[col] = nsur;
+__global__ void __launch_bounds__(kSetDzWarps * 32, 4)
+    k_set_dz(Geo G, Flow F, Work W, Opt O, Tile Tl, int any_vdiff, int *counts, int list_all,
+             int what, const int *own) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  constexpr unsigned FULL = 0xffffffffu;
+  const int nz = G.nz, lane = threadIdx.x, wy = threadIdx.y;
+  double *const sZ = reinterpret_cast<double *>(smem) + lane;  // bottom face z, then ud
+  double *const sCm = sZ + nz * 32;                            // cm1
+  double *const sDv = sCm + nz * 32;                           // dz / dt, then div
+  int *const sC = reinterpret_cast<int *>(reinterpret_cast<double *>(smem) + 3 * nz * 32) + lane;
+  __shared__ int sJa[32];        // highest layer <= jn of zero thickness
+  __shared__ double sMin[kSetDzWarps];
+  const int col = blockIdx.x * 32 + lane;
+  const bool on = col < G.ncol;
+  const int4 rec = Tl.colrec[col];  // {bottom cell, top cell, bottom layer}
+  const int bot = rec.x, top = rec.y, kb = rec.z, nk = on ? nz - kb : 0;
+
+  // (0) cells and faces; the surface before the step
+  if (wy == 0) sJa[lane] = 0;
+  const int sur = on ? W.nsur_t[col] : 0;
+  const int sed = on ? __ldg(&G.zm1[bot]) : 0;
+  for (int k = wy; k < nz; k += kSetDzWarps)
+    if (on && k >= kb) {
+      const int c = __ldg(&Tl.cellk[(size_t)k * Tl.ncolp + col]);
+      sC[k * 32] = c;
+      sZ[k * 32] = __ldg(&G.gridz[c]);
     }
-    const bool counts_min = !own || own[col];
-    const int js0 = jof(sur);
-    // cells-to-process membership (:5778-5800): s is the lower of the two
-    int s = sur > nsur ? sur : nsur;
-    const int js = js0 < jn ? js0 : jn;
-    int c2 = G.m2d[s];
-    double tz = F.eta[c2] < F.oldeta[c2] ? F.eta[c2] : F.oldeta[c2];
-    double bz = SHOC_TR_DRY_FRAC * O.hmin + G.botz[c2];
-    bool wet = (tz > bz && js > 0);
-    // thickness of layer j (:5824-5846): from the old surface down to the
-    // bottom, the layers above the old surface copy the old surface cell's
-    // (with the old surface in the sediment, every layer copies the
-    // sediment's)
-    const int t2 = G.m2d[sur];
-    const double oet = F.oldeta[t2], bott = G.botz[t2], dzsed = W.dz[sed];
-    auto dzof = [&](int j) -> double {
-      const int jj = j < js0 ? j : js0;
-      if (jj == 0) return dzsed;
-      const double tp = (jj == js0) ? oet : __ldg(&G.gridz[cell(jj + 1)]);
-      return tp - ((jj > 1) ? __ldg(&G.gridz[cell(jj)]) : bott);
-    };
-    // top-down pass: dz, dz32, w5, w9, dbz, dfz (:530-567), the sub-step
-    // search over the cells to process (:591-661) and what the flags need
-    const bool substep = O.substep != 0, quick = O.trasc == SHOC_TR_QUICKEST;
-    int nc = 0;
-    int ja = -1;             // highest layer <= jn of zero thickness
-    double dz_js0 = dzsed, dz_jn = 0.0, dz_jn1 = 0.0;
-    double dzc = dzof(nk);                         // dz(j)
-    double dzm = nk >= 1 ? dzof(nk - 1) : dzsed;   // dz(j - 1)
-    double w9c = 0.5 * (dzc + dzm), w9p = w9c;     // w9(j), w9(j + 1)
-    for (int j = nk; j >= 1; --j) {
-      const int cc = cell(j);
-      const double dzmm = j >= 2 ? dzof(j - 2) : 0.0;
-      const double w9m = j >= 2 ? 0.5 * (dzm + dzmm) : 0.0;  // w9(j - 1)
-      W.dz[cc] = dzc;
-      if (fp32) W.dz32[cc] = (float)dzc;
+  __syncthreads();
+
+  // the column: new and old surface cells (tracers.c:5739-5755), down from the
+  // top while the cell's bottom is at or above eta, at most to the sediment;
+  // membership (:5778-5800): s is the lower of the two
+  int jn = nk, nsur = 0, js0 = 0, js = 0, s = 0, c2 = 0;
+  bool wet = false, pre_staged = false;
+  double oet = 0.0, bott = 0.0, dzsed = 0.0;
+  if (on) {
+    const double etat = F.eta[top];
+    while (jn > 0 && sZ[(kb + jn - 1) * 32] >= etat) --jn;
+    nsur = jn ? sC[(kb + jn - 1) * 32] : sed;
+    js0 = sur == sed ? 0 : max(0, __ldg(&G.kof[sur]) - kb + 1);
+    js = js0 < jn ? js0 : jn;
+    s = sur > nsur ? sur : nsur;
+    c2 = __ldg(&G.m2d[s]);
+    const int t2 = __ldg(&G.m2d[sur]);
+    oet = F.oldeta[t2];
+    bott = __ldg(&G.botz[t2]);
+    dzsed = W.dz[sed];
+    const double tz = F.eta[c2] < F.oldeta[c2] ? F.eta[c2] : F.oldeta[c2];
+    const double bz = SHOC_TR_DRY_FRAC * O.hmin + __ldg(&G.botz[c2]);
+    wet = (tz > bz && js > 0);
+    pre_staged = O.tiled && wet && s == sur && s == nsur;
+  }
+  // thickness of layer j (:5824-5846): from the old surface down to the
+  // bottom, the layers above the old surface copy the old surface cell's
+  // (with the old surface in the sediment, every layer copies the sediment's)
+  auto dzof = [&](int j) -> double {
+    const int jj = j < js0 ? j : js0;
+    if (jj == 0) return dzsed;
+    const double tp = (jj == js0) ? oet : sZ[(kb + jj) * 32];
+    return tp - ((jj > 1) ? sZ[(kb + jj - 1) * 32] : bott);
+  };
+  const bool quick = O.trasc == SHOC_TR_QUICKEST;
+  const double dt = F.dt;
+  // w5, w9 and their factors of layer j (:530-567)
+  auto work_arrays = [&](int j, int cc) {
+    const double dzc = dzof(j), dzm = dzof(j - 1);
+    const double w9c = 0.5 * (dzc + dzm);
+    const double w9m = j >= 2 ? 0.5 * (dzm + dzof(j - 2)) : 0.0;
+    const double w9p = j < nk ? 0.5 * (dzof(j + 1) + dzc) : w9c;
+    if (quick || O.trasc == SHOC_TR_ORDER2) W.w5[cc] = dzm / (dzm + dzc);
+    W.w9[cc] = w9c;
+    W.dbz[cc] = 2.0 / (w9m + w9c);
+    W.dfz[cc] = 2.0 / (w9c + w9p);
+  };
+
+  // (1) every layer
+  double dtmin = __longlong_as_double(0x7ff0000000000000ll);
+  const bool search = (what & SD_SEARCH) && O.substep != 0 && wet && (!own || own[col]);
+  const bool all_work = (what & SD_WORK) || !pre_staged;
+  for (int k = nz - 1 - wy; k >= 0; k -= kSetDzWarps) {
+    if (!on || k < kb) continue;
+    const int j = k - kb + 1, cc = sC[k * 32];
+    const double dzc = dzof(j), dzm = dzof(j - 1);
+    W.dz[cc] = dzc;
+    if (what & SD_F32) W.dz32[cc] = (float)dzc;
+    if (all_work) work_arrays(j, cc);
+    if (j <= jn && !dzc) atomicMax(&sJa[lane], j);
+    if (any_vdiff) {  // rows of the implicit solve (:3841-3889)
+      sDv[k * 32] = dzc / dt;
+      sCm[k * 32] = -__ldg(&F.Kz[cc]) / (0.5 * (dzm + dzc));
+    }
+    if (search && j <= js) {
+      const int xp = __ldg(&G.xp1[cc]), yp = __ldg(&G.yp1[cc]);
+      double d4 = 0.5 * (__ldg(&F.u1[cc]) + __ldg(&F.u1[xp]));
+      if (fabs(d4) < kMinVal) d4 = kMinVal;
+      const double d1 = kSF * fabs(__ldg(&G.h1acell[c2]) / d4);
+      if (d1 < dtmin) dtmin = d1;
+      d4 = 0.5 * (__ldg(&F.u2[cc]) + __ldg(&F.u2[yp]));
+      if (fabs(d4) < kMinVal) d4 = kMinVal;
+      const double d2 = kSF * fabs(__ldg(&G.h2acell[c2]) / d4);
+      if (d2 < dtmin) dtmin = d2;
+      if (j != js) {
+        d4 = 0.5 * (__ldg(&F.w[cc]) + __ldg(&F.w[j < nk ? sC[(k + 1) * 32] : cc]));
+        if (fabs(d4) < kMinVal) d4 = kMinVal;
+        const double d3 = kSF * fabs(dzc * 1.0 / d4);
+        if (d3 > 0.0 && d3 < dtmin) dtmin = d3;
+      }
+    }
+  }
+  // what the flags need, before the faces' shared memory is used again
+  const double dz_js0 = on ? dzof(js0) : 0.0;
+  const double dz_jn = on ? dzof(jn) : 0.0, dz_jn1 = (on && jn > 0) ? dzof(jn - 1) : 0.0;
+  for (int o = 16; o > 0; o >>= 1) dtmin = fmin(dtmin, __shfl_xor_sync(FULL, dtmin, o));
+  if (lane == 0) sMin[wy] = dtmin;
+  __syncthreads();
+
+  // (2) flags and the solve's range, in every warp alike; warp 0 runs the LU
+  int flags = 0, cbs = 0, jb = 0, stat = 0;
+  bool solve = false;
+  if (on && wet) {
+    flags |= COL_WET;
+    // tr_bounds thin-surface test (:3250-3252)
+    if (js > 1 && dz_js0 < O.hmin) {
+      flags |= COL_THIN;
+      if (s != top) flags |= COL_SERIAL;
+    }
+    if (jn <= 1 || !dz_jn1) {
+      flags |= COL_SINGLE;
+    } else if (any_vdiff && !dz_jn) {
+      // zero-thickness surface cell: the reference solves over an empty
+      // range and reads stale work memory; report instead of guessing
+      flags |= COL_NOSOLVE;
+      stat |= ST_GEOM;
+    } else if (any_vdiff) {
+      jb = sJa[lane] + 1;  // bottom of the solve
+      cbs = sC[(kb + jb - 1) * 32];
+      solve = true;
+    }
+  } else if (on && col == G.v2col) {
+    stat |= ST_LASTDRY;
+  }
+  ColInfo ci;
+  ci.s = wet ? s : 0;
+  ci.co = sur;
+  ci.cs = nsur;
+  ci.cbs = cbs;
+  ci.flags = flags;
+  ci.ks = kb + js - 1;
+  const bool staged = on && O.tiled && staged_column(ci, bot);
+  if (staged) ci.flags |= COL_STAGED;
+  if (wy == 0) {
+    if (solve) {
+      // LU (:4185-4195), bottom up from the lowest layer of the solve; the
+      // upper diagonal of a row is the lower one of the row above it
+      int k = kb + jb - 1;
+      double bp1 = sCm[(k + 1) * 32];
+      double div = sDv[k * 32] - bp1;
+      sCm[k * 32] = 0.0;
+      sDv[k * 32] = div;
+      sZ[k * 32] = 0.0;
+      const int kt = kb + jn - 1;
+#pragma unroll 2
+      for (++k; k <= kt; ++k) {
+        const double cm1 = sCm[k * 32], cp1 = k < kt ? sCm[(k + 1) * 32] : 0.0;
+        double C = sDv[k * 32] - cm1;
+        if (k < kt) C = C - cp1;
+        const double ud = bp1 / div;
+        div = C - cm1 * ud;
+        if (div == 0.0) stat |= ST_PIVOT;
+        sDv[k * 32] = div;
+        sZ[k * 32] = ud;
+        bp1 = cp1;
+      }
+    }
+    if (stat) atomicOr(W.status, stat);
+    if (on) {
+      if (!(what & SD_PROBE)) {
+        W.sur_t[col] = sur;
+        W.nsur_t[col] = nsur;
+      }
+      W.col[col] = ci;
+      if ((flags & COL_SERIAL) || (list_all && !staged)) {
+        const int i = atomicAdd(W.serial_count, 1);
+        W.serial_list[i] = col;
+      }
+    }
+    const int wc = __reduce_add_sync(FULL, (on && wet) ? 1 : 0);
+    const int wn = __reduce_add_sync(FULL, (on && wet) ? js : 0);
+    if (lane == 0) {
+      if (wc) atomicAdd(&counts[0], wc);
+      if (wn) atomicAdd(&counts[1], wn);
+      double v = sMin[0];
+      for (int i = 1; i < kSetDzWarps; ++i) v = fmin(v, sMin[i]);
+      if (v < __longlong_as_double(0x7ff0000000000000ll)) atomic_min_pos(W.dtm_bits, v);
+    }
+  }
+  __syncthreads();
+
+  // (3) the factors (and the work arrays of a column the tile kernels turned
+  // out not to handle, whose faces the ud have overwritten: from W.dz)
+  const bool lu64 = (what & SD_LU64) || !staged;
+  const bool late = on && pre_staged && !staged && !(what & SD_WORK);
+  if (!solve && !late) return;
+  for (int k = wy; k < nz; k += kSetDzWarps) {
+    if (k < kb) continue;
+    const int j = k - kb + 1, cc = sC[k * 32];
+    const double dzc = W.dz[cc];
+    if (solve && j >= jb && j <= jn) {
+      const double dzdt = dzc / dt, cm1 = sCm[k * 32], div = sDv[k * 32], ud = sZ[k * 32];
+      if (lu64) {
+        W.vd_cm1[cc] = cm1;
+        W.vd_div[cc] = div;
+        W.vd_ud[cc] = ud;
+        W.vd_dzdt[cc] = dzdt;
+      }
+      if (what & SD_F32)
+        W.lu32[cc] = make_float4((float)dzdt, (float)cm1, (float)(1.0 / div), (float)ud);
+    }
+    if (late) {
+      const double dzm = j > 1 ? W.dz[sC[(k - 1) * 32]] : dzsed;
+      const double w9c = 0.5 * (dzc + dzm);
+      const double dzmm = j > 2 ? W.dz[sC[(k - 2) * 32]] : dzsed;
+      const double w9m = j >= 2 ? 0.5 * (dzm + dzmm) : 0.0;
+      const double w9p = j < nk ? 0.5 * (W.dz[sC[(k + 1) * 32]] + dzc) : w9c;
       if (quick || O.trasc == SHOC_TR_ORDER2) W.w5[cc] = dzm / (dzm + dzc);
       W.w9[cc] = w9c;
       W.dbz[cc] = 2.0 / (w9m + w9c);
       W.dfz[cc] = 2.0 / (w9c + w9p);
-      if (j == js0) dz_js0 = dzc;
-      if (j == jn) dz_jn = dzc;
-      if (j == jn - 1) dz_jn1 = dzc;
-      if (j <= jn && ja < 0 && !dzc) ja = j;
-      if (wet && j <= js) {
-        nc++;
-        if (substep && counts_min) {
-          const int xp = __ldg(&G.xp1[cc]), yp = __ldg(&G.yp1[cc]), zp = cell(j < nk ? j + 1 : nk);
-          double d4 = 0.5 * (__ldg(&F.u1[cc]) + __ldg(&F.u1[xp]));
-          if (fabs(d4) < kMinVal) d4 = kMinVal;
-          double d1 = kSF * fabs(G.h1acell[c2] / d4);
-          if (d1 < dtmin) dtmin = d1;
-          d4 = 0.5 * (__ldg(&F.u2[cc]) + __ldg(&F.u2[yp]));
-          if (fabs(d4) < kMinVal) d4 = kMinVal;
-          double d2 = kSF * fabs(G.h2acell[c2] / d4);
-          if (d2 < dtmin) dtmin = d2;
-          if (j != js) {
-            d4 = 0.5 * (__ldg(&F.w[cc]) + __ldg(&F.w[zp]));
-            if (fabs(d4) < kMinVal) d4 = kMinVal;
-            double d3 = kSF * fabs(dzc * 1.0 / d4);
-            if (d3 > 0.0 && d3 < dtmin) dtmin = d3;
-          }
-        }
-      }
-      w9p = w9c;
-      w9c = w9m;
-      dzc = dzm;
-      dzm = dzmm;
     }
-    if (jn == 0) dz_jn = dzsed;
-    if (ja < 0) ja = 0;
-    int flags = 0;
-    int cbs = 0;
-    if (wet) {
-      flags |= COL_WET;
-      nwetcol = 1;
-      ncells = nc;
-      // tr_bounds thin-surface test (:3250-3252)
-      if (js > 1 && dz_js0 < O.hmin) {
-        flags |= COL_THIN;
-        if (s != top) flags |= COL_SERIAL;
-      }
-      // implicit vertical diffusion set-up (:3841-3889) and LU (:4185-4195),
-      // bottom up from the lowest layer of the solve
-      int cs = nsur;
-      if (jn <= 1 || !dz_jn1) {
-        flags |= COL_SINGLE;
-      } else if (any_vdiff && !dz_jn) {
-        // zero-thickness surface cell: the reference solves over an empty
-        // range and reads stale work memory; report instead of guessing
-        flags |= COL_NOSOLVE;
-        atomicOr(W.status, ST_GEOM);
-      } else if (any_vdiff) {
-        const int jb = ja + 1;  // bottom of the solve
-        cbs = cell(jb);
-        // dzface(c) = 0.5 (dz[zm1] + dz[c]) for c in [cbs, cs]
-        double dt = F.dt;
-        int cb = cbs;
-        int zpb = cell(jb + 1);
-        double dzj = W.dz[cb], dzj1 = W.dz[zpb];
-        double dzf_p = 0.5 * (dzj + dzj1);
-        double dzdt = dzj / dt;
-        double cp1 = -__ldg(&F.Kz[zpb]) / dzf_p;
-        double C = dzdt - cp1;
-        double div = C;
-        W.vd_cm1[cb] = 0.0;
-        W.vd_div[cb] = div;
-        W.vd_ud[cb] = 0.0;
-        W.vd_dzdt[cb] = dzdt;
-        if (fp32) W.lu32[cb] = make_float4((float)dzdt, 0.f, (float)(1.0 / div), 0.f);
-        double bp1 = cp1;
-        int cc2 = zpb;
-        for (int j = jb + 1; j < jn; ++j) {
-          const int zp = cell(j + 1);
-          const double dzn = W.dz[zp];
-          double dzf_c = dzf_p;
-          dzf_p = 0.5 * (dzj1 + dzn);
-          dzdt = dzj1 / dt;
-          double cm1 = -__ldg(&F.Kz[cc2]) / dzf_c;
-          cp1 = -__ldg(&F.Kz[zp]) / dzf_p;
-          C = dzdt - cm1 - cp1;
-          double ud = bp1 / div;
-          div = C - cm1 * ud;
-          if (div == 0.0) atomicOr(W.status, ST_PIVOT);
-          W.vd_cm1[cc2] = cm1;
-          W.vd_div[cc2] = div;
-          W.vd_ud[cc2] = ud;
-          W.vd_dzdt[cc2] = dzdt;
-          if (fp32)
-            W.lu32[cc2] = make_float4((float)dzdt, (float)cm1, (float)(1.0 / div), (float)ud);
-          bp1 = cp1;
-          cc2 = zp;
-          dzj1 = dzn;
-        }
-        {
-          double dzf_c = dzf_p;
-          dzdt = dz_jn / dt;
-          double cm1 = -__ldg(&F.Kz[cs]) / dzf_c;
-          C = dzdt - cm1;
-          double ud = bp1 / div;
-          div = C - cm1 * ud;
-          if (div == 0.0) atomicOr(W.status, ST_PIVOT);
-          W.vd_cm1[cs] = cm1;
-          W.vd_div[cs] = div;
-          W.vd_ud[cs] = ud;
-          W.vd_dzdt[cs] = dzdt;
-          if (fp32)
-            W.lu32[cs] = make_float4((float)dzdt, (float)cm1, (float)(1.0 / div), (float)ud);
-        }
-      }
-    } else if (col == G.v2col) {
-      atomicOr(W.status, ST_LASTDRY);
-    }
-    ColInfo ci;
-    ci.s = wet ? s : 0;
-    ci.co = sur;
-    ci.cs = nsur;
-    ci.cbs = cbs;
-    ci.flags = flags;
-    ci.ks = kb + js - 1;
-    if (O.tiled && staged_column(ci, bot)) ci.flags |= COL_STAGED;
-    W.col[col] = ci;
-    if ((flags & COL_SERIAL) || (list_all && !(ci.flags & COL_STAGED))) {
-      int i = atomicAdd(W.serial_count, 1);
-      W.serial_list[i] = col;
-    }
-  }
-  // warp-reduce the counts and the sub-step minimum: one atomic per warp
-  const int wc = __reduce_add_sync(0xffffffffu, nwetcol);
-  const int wn = __reduce_add_sync(0xffffffffu, ncells);
-  double v = dtmin;
-  for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-  if ((threadIdx.x & 31) == 0) {
-    if (wc) atomicAdd(&counts[0], wc);
-    if (wn) atomicAdd(&counts[1], wn);
-    if (v < __longlong_as_double(0x7ff0000000000000ll)) atomic_min_pos(W.dtm_bits, v);
   }
 }
 
-// Courant numbers of one sub-step over every wet cell (tracers.c:730-736).
-// only_listed: skip when the general-path list is empty (the staged kernels
-// compute their own Courant numbers).
-__global__ void k_courant(Geo G, Flow F, Work W, double dtu, int only_listed) {
-  if (only_listed && *W.serial_count == 0) return;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < G.S; c += gridDim.x * blockDim.x) {
-    if (!(G.cflag[c] & CF_WET)) continue;
-    int c2 = G.m2d[c];
-    W.w6[c] = F.u1[c] * dtu / G.h1au1[c2];
-    W.w7[c] = F.u2[c] * dtu / G.h2au2[c2];
-    W.w8[c] = F.w[c] * dtu / (W.w9[c] * 1.0);
-  }
-}
-
-// Columns where tr_bounds' thin-surface cursor can move between tracers:
-// one thread per column, tracers in tbdy order, as the reference loops.
+// The general path: the columns the tile kernels do not handle, one thread per
+// (listed column, tracer), a warp holding 32 listed columns of one tracer (the
+// list keeps neighbouring columns together, so most of a warp's loads
+// coalesce).  Only where tr_bounds' thin-surface cursor can move between
+// tracers (COL_SERIAL) one thread steps a column's tracers in tbdy order, as
+// the reference loops.  One thread per column for every column left the chip
+// idle: at 200 x 180 x 30 with 6 tracers (every column listed) a sub-step took
+// 2.52 ms, at 192 x 160 x 24 with 800 listed columns 0.69 ms.
 // When the tracers go through in chunks of slots (the drop-in step's
 // pipeline), c3s holds each listed column's cursor state between the chunks
 // of one sub-step: read when c3_load, written back always.  lo_out
 // (FP32_COMP): these columns step their FP32 values as stored, and their
 // compensations, from the sediment ghost to the top cell, are set to 0.
+constexpr int kGeneralThreads = 128;
 template <bool LAST, class TR>
-__global__ void k_serial(Geo G, Flow F, Work W, Opt O, TrSet T, SubStep ss,
-                         const TR *__restrict__ tr_in, TR *__restrict__ tr_out,
-                         uint8_t *__restrict__ c3s, int c3_load,
-                         int16_t *__restrict__ lo_out = nullptr) {
-  int cnt = *W.serial_count;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
-    int col = W.serial_list[i];
+__global__ void __launch_bounds__(kGeneralThreads)
+    k_general(Geo G, Flow F, Work W, Opt O, TrSet T, SubStep ss, Tile Tl,
+              const TR *__restrict__ tr_in, TR *__restrict__ tr_out, uint8_t *__restrict__ c3s,
+              int c3_load, int16_t *__restrict__ lo_out = nullptr) {
+  const int cnt = *W.serial_count;
+  const int cntp = (cnt + 31) & ~31;
+  const long long tot = (long long)cntp * T.nslot;
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < tot;
+       q += (long long)gridDim.x * blockDim.x) {
+    const int i = (int)(q % cntp);
+    int sl = (int)(q / cntp);
+    if (i >= cnt) continue;
+    const int col = W.serial_list[i];
+    const bool coupled = (W.col[col].flags & COL_SERIAL) != 0;
+    if (coupled && sl > 0) continue;
+    const int sl1 = coupled ? T.nslot : sl + 1;
     LocalSol sol;
-    bool c3 = (c3s && c3_load) ? c3s[i] != 0 : false;
+    bool c3 = (coupled && c3s && c3_load) ? c3s[i] != 0 : false;
     unsigned long long warn = 0;
     int stat = 0;
-    for (int sl = 0; sl < T.nslot; ++sl) {
-      int n = T.slot_tr[sl];
+    for (; sl < sl1; ++sl) {
+      const int n = T.slot_tr[sl];
       if (n >= G.colntr[col]) continue;  // not carried in this column
-      column_pass<LAST>(G, F, W, O, T, ss, tr_in + (size_t)n * G.S, tr_out + (size_t)n * G.S,
-                        col, n, G.col_kb[col], true, sol, c3, warn, stat);
+      column_pass<LAST>(G, F, W, O, T, ss, Tl, tr_in + (size_t)n * G.S,
+                        tr_out + (size_t)n * G.S, col, n, sol, c3, warn, stat);
       if (lo_out) {
         int16_t *lo = lo_out + (size_t)n * G.S;
         int c = G.zm1[G.col_bot[col]];
@@ -506,7 +549,7 @@ __global__ void k_serial(Geo G, Flow F, Work W, Opt O, TrSet T, SubStep ss,
         } while (c != G.col_top[col]);
       }
     }
-    if (c3s) c3s[i] = c3 ? 1 : 0;
+    if (coupled && c3s) c3s[i] = c3 ? 1 : 0;
     if (warn) atomicAdd(W.nwarn, warn);
     if (stat) atomicOr(W.status, stat);
   }
@@ -1154,7 +1197,7 @@ int check_geom(const shoc_tr_geom *g, const shoc_tr_opts *o, int ntr) {
   }
   if (g->v3_t != g->b3_t || g->b3_t != g->a3_t) return SHOC_TR_EUNSUPPORTED;  // OBC / aux cells
   if (g->v2_t != g->b2_t || g->b2_t != g->a2_t) return SHOC_TR_EUNSUPPORTED;
-  if (g->nz < 1 || g->nz > kSerialMaxLayers) return SHOC_TR_EUNSUPPORTED;
+  if (g->nz < 1 || g->nz > kMaxLayers) return SHOC_TR_EUNSUPPORTED;
   if (o->ntr2d) {  // per-column tracer counts: the advected tracers in ascending order
     for (int i = 1; i < o->ntbdy; i++)
       if (o->tbdy[i] <= o->tbdy[i - 1]) return SHOC_TR_EARG;
@@ -1454,9 +1497,6 @@ int shoc_tr_gpu_create(const shoc_tr_geom *g, const shoc_tr_opts *o, int ntr, in
   TRY(dupload<double>(h, &W.w9, nullptr, S));
   TRY(dupload<double>(h, &W.dbz, nullptr, S));
   TRY(dupload<double>(h, &W.dfz, nullptr, S));
-  TRY(dupload<double>(h, &W.w6, nullptr, S));
-  TRY(dupload<double>(h, &W.w7, nullptr, S));
-  TRY(dupload<double>(h, &W.w8, nullptr, S));
   TRY(dupload<double>(h, &W.vd_cm1, nullptr, S));
   TRY(dupload<double>(h, &W.vd_div, nullptr, S));
   TRY(dupload<double>(h, &W.vd_ud, nullptr, S));
@@ -1599,7 +1639,9 @@ int shoc_tr_gpu_create(const shoc_tr_geom *g, const shoc_tr_opts *o, int ntr, in
   h->h_status = (int *)((char *)pin + 8);
   h->h_nwarn = (unsigned long long *)((char *)pin + 16);
   h->h_counts = (int *)((char *)pin + 24);
-  if (cudaFuncSetAttribute(k_vd64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  if (cudaFuncSetAttribute(k_set_dz, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)set_dz_smem(kMaxLayers)) != cudaSuccess ||
+      cudaFuncSetAttribute(k_vd64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            227 * 1024) != cudaSuccess ||
       cudaFuncSetAttribute(k_vd64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            227 * 1024) != cudaSuccess ||
@@ -1646,21 +1688,43 @@ int make_schedule(shoc_tr_gpu *h, double dmin, Sched &s) {
 }
 
 // set_lateral_BC_tr for the tracers of T (every tracer, or one chunk of the
-// drop-in step's pipeline) into both buffers
-void launch_lateral(shoc_tr_gpu *h, int cur, const TrSet &T) {
-  if (h->nbpt <= 0 || T.nslot <= 0) return;
+// drop-in step's pipeline) into both buffers; reset: clear the step's
+// reductions too
+void launch_lateral(shoc_tr_gpu *h, int cur, const TrSet &T, bool reset) {
   cudaStream_t st = h->stream;
+  if (h->nbpt <= 0 || T.nslot <= 0) {
+    if (reset) {
+      k_reset<<<1, 32, 0, st>>>(h->W, h->d_counts);
+      h->launches++;
+    }
+    return;
+  }
+  int *counts = reset ? h->d_counts : nullptr;
   long long tot = (long long)h->nbpt * T.nslot;
   int blocks = (int)std::min<long long>((tot + 255) / 256, 148 * 16);
   if (h->esize == sizeof(float))
     k_lateral<float><<<blocks, 256, 0, st>>>(h->nbpt, h->bpt, h->bin, T.slot_tr, T.nslot, h->S,
                                              (float *)h->tr[cur], (float *)h->tr[cur ^ 1],
                                              h->comp ? h->lo[cur] : nullptr,
-                                             h->comp ? h->lo[cur ^ 1] : nullptr);
+                                             h->comp ? h->lo[cur ^ 1] : nullptr, h->W, counts);
   else
     k_lateral<double><<<blocks, 256, 0, st>>>(h->nbpt, h->bpt, h->bin, T.slot_tr, T.nslot,
                                               h->S, (double *)h->tr[cur],
-                                              (double *)h->tr[cur ^ 1]);
+                                              (double *)h->tr[cur ^ 1], nullptr, nullptr, h->W,
+                                              counts);
+  h->launches++;
+}
+
+// k_set_dz over every column; what: SD_PROBE / SD_SEARCH (the arrays to write
+// follow from the precision)
+void launch_set_dz(shoc_tr_gpu *h, int what) {
+  if (h->esize == sizeof(float))
+    what |= SD_F32 | (h->comp ? SD_WORK : 0);
+  else
+    what |= SD_WORK | SD_LU64;
+  k_set_dz<<<h->tl.ncolp / 32, dim3(32, kSetDzWarps), set_dz_smem(h->nz), h->stream>>>(
+      h->G, h->F, h->W, h->O, h->tl, h->any_vdiff ? 1 : 0, h->d_counts, h->staged ? 1 : 0, what,
+      h->colown);
   h->launches++;
 }
 
@@ -1694,24 +1758,42 @@ int launch_preamble(shoc_tr_gpu *h) {
 }
 
 // Step set-up: counters, lateral boundaries (when `lateral`), the flow
-// preamble (when on) and k_set_dz.  k_set_dz reads no tracer, so the lateral
-// copies may follow it instead.
-int launch_part_a(shoc_tr_gpu *h, int cur, bool lateral = true) {
+// preamble (when on) and k_set_dz (with the sub-step search when `search`:
+// a step whose schedule is known does not need it).  k_set_dz reads no tracer,
+// so the lateral copies may follow it instead.
+int launch_part_a(shoc_tr_gpu *h, int cur, bool lateral, bool search) {
   cudaStream_t st = h->stream;
-  k_reset<<<1, 32, 0, st>>>(h->W, h->d_counts);
-  h->launches++;
-  if (lateral) launch_lateral(h, cur, h->T);
+  if (lateral) {
+    launch_lateral(h, cur, h->T, true);
+  } else {
+    k_reset<<<1, 32, 0, st>>>(h->W, h->d_counts);
+    h->launches++;
+  }
   if (h->pre.on) {
     const int rc = launch_preamble(h);
     if (rc) return rc;
   }
-  int nb = (h->ncol + 127) / 128;
-  k_set_dz<<<nb, 128, 0, st>>>(h->G, h->F, h->W, h->O, h->tl, h->any_vdiff ? 1 : 0, h->d_counts,
-                               h->staged ? 1 : 0, h->esize == sizeof(float) ? 1 : 0, h->colown,
-                               0);
-  h->launches++;
+  launch_set_dz(h, search ? SD_SEARCH : 0);
   CK(cudaGetLastError());
   return 0;
+}
+
+// One sub-step of the general-path columns for the tracers of T
+template <class TR>
+void launch_general(shoc_tr_gpu *h, bool last, const TrSet &T, const SubStep &ss, const TR *tin,
+                    TR *tout, uint8_t *c3row, bool c3_load, int16_t *lo_out) {
+  // as many threads as the longest list has (column, tracer) pairs, at most
+  // eight blocks per SM
+  const long long tot = (long long)(h->ncol + 31) / 32 * 32 * T.nslot;
+  const int blocks = (int)std::min<long long>((tot + kGeneralThreads - 1) / kGeneralThreads,
+                                              kGeneralBlocks);
+  if (last)
+    k_general<true, TR><<<blocks, kGeneralThreads, 0, h->stream>>>(
+        h->G, h->F, h->W, h->O, T, ss, h->tl, tin, tout, c3row, c3_load, lo_out);
+  else
+    k_general<false, TR><<<blocks, kGeneralThreads, 0, h->stream>>>(
+        h->G, h->F, h->W, h->O, T, ss, h->tl, tin, tout, c3row, c3_load, lo_out);
+  h->launches++;
 }
 
 // One FP64 transport sub-step over the staged columns: k_adv64, then one
@@ -1797,7 +1879,7 @@ Tile vd_classes(const shoc_tr_gpu *h, int nw) {
 }
 
 // The transport sub-steps of one step for the tracers of T (every tracer, or
-// one chunk of the drop-in step's pipeline; c3s/c3_load as k_serial takes
+// one chunk of the drop-in step's pipeline; c3s/c3_load as k_general takes
 // them, one row of ncol bytes per sub-step).
 int launch_part_b(shoc_tr_gpu *h, const Sched &s, int cur0, const TrSet &T,
                   uint8_t *c3s = nullptr, bool c3_load = false) {
@@ -1805,13 +1887,10 @@ int launch_part_b(shoc_tr_gpu *h, const Sched &s, int cur0, const TrSet &T,
   int cur = cur0;
   const int nsub = (int)s.sub.size();
   const int tw = std::max(1, std::min(h->tw, T.nslot));  // no idle tracer rows
-  int cblocks = std::min((h->S + 255) / 256, 148 * 32);
   for (int i = 0; i < nsub; i++) {
     const SubStep &ss = s.sub[i];
     bool last = (i == nsub - 1);
     uint8_t *c3row = c3s ? c3s + (size_t)i * h->ncol : nullptr;
-    k_courant<<<cblocks, 256, 0, st>>>(h->G, h->F, h->W, ss.dtu, h->staged ? 1 : 0);
-    h->launches++;
     if (h->esize == sizeof(float) && T.nslot > 0) {  // FP32-mixed
       const float *tin = (const float *)h->tr[cur];
       float *tout = (float *)h->tr[cur ^ 1];
@@ -1847,13 +1926,7 @@ int launch_part_b(shoc_tr_gpu *h, const Sched &s, int cur0, const TrSet &T,
         for (int k = 0; k < tl.nclass; k++) h->launches += tl.ctile[k + 1] > tl.ctile[k] ? 1 : 0;
       }
       int16_t *lo_out = h->comp ? h->lo[cur ^ 1] : nullptr;
-      if (last)
-        k_serial<true, float><<<kSerialBlocks, 64, 0, st>>>(h->G, h->F, h->W, h->O, T, ss,
-                                                            tin, tout, c3row, c3_load, lo_out);
-      else
-        k_serial<false, float><<<kSerialBlocks, 64, 0, st>>>(h->G, h->F, h->W, h->O, T, ss,
-                                                             tin, tout, c3row, c3_load, lo_out);
-      h->launches++;
+      launch_general<float>(h, last, T, ss, tin, tout, c3row, c3_load, lo_out);
       cur ^= 1;
       continue;
     }
@@ -1872,13 +1945,7 @@ int launch_part_b(shoc_tr_gpu *h, const Sched &s, int cur0, const TrSet &T,
         h->ev.push_back({2, ev[1], ev[2]});
       }
       h->launches += nl;
-      if (last)
-        k_serial<true, double><<<kSerialBlocks, 64, 0, st>>>(h->G, h->F, h->W, h->O, T, ss,
-                                                             tin, tout, c3row, c3_load);
-      else
-        k_serial<false, double><<<kSerialBlocks, 64, 0, st>>>(h->G, h->F, h->W, h->O, T, ss,
-                                                              tin, tout, c3row, c3_load);
-      h->launches++;
+      launch_general<double>(h, last, T, ss, tin, tout, c3row, c3_load, nullptr);
     }
     cur ^= 1;
   }
@@ -1898,7 +1965,7 @@ int read_status(shoc_tr_gpu *h) {
 // sub-step minimum read back and the schedule built from it (tracers.c:
 // 591-720).  lateral: whether part A fills every tracer's lateral boundary.
 int probe_schedule(shoc_tr_gpu *h, bool lateral, Sched &s) {
-  int rc = launch_part_a(h, h->cur, lateral);
+  int rc = launch_part_a(h, h->cur, lateral, true);
   if (rc) return rc;
   rc = read_status(h);
   if (rc) return rc;
@@ -1950,7 +2017,7 @@ int step_async(shoc_tr_gpu *h) {
   }
   if (h->profile) {
     // profiling launches directly so each transport launch is timed
-    int rc = launch_part_a(h, h->cur);
+    int rc = launch_part_a(h, h->cur, true, false);
     if (rc) return rc;
     rc = launch_part_b(h, h->sched, h->cur, h->T);
     if (rc) return rc;
@@ -1969,7 +2036,7 @@ int step_async(shoc_tr_gpu *h) {
       cudaGraph_t graph;
       long long l0 = h->launches;
       CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-      int rc = launch_part_a(h, g);
+      int rc = launch_part_a(h, g, true, false);
       if (!rc) rc = launch_part_b(h, h->sched, g, h->T);
       cudaError_t e = cudaStreamEndCapture(h->stream, &graph);
       if (rc) return rc;
@@ -1995,7 +2062,7 @@ int step_async(shoc_tr_gpu *h) {
 // duplex) and every chunk's transport overlaps both.  Per tracer the kernels
 // and their order are those of a whole step: the tracers of a step are
 // independent apart from the general path's thin-surface cursor, which
-// k_serial carries from chunk to chunk (c3s); set_dz reads no tracer, so the
+// k_general carries from chunk to chunk (c3s); set_dz reads no tracer, so the
 // lateral boundaries of a chunk may follow it.
 
 // slots per chunk: about a twelfth of the tracers, so the first chunk is
@@ -2095,7 +2162,7 @@ int step_pipelined(shoc_tr_gpu *h, shoc_tr_state *st) {
     Tc.nslot = ns;
     Tc.ntb = std::max(0, std::min(h->T.ntb - s0, ns));
     CK(cudaStreamWaitEvent(h->stream, ev[1 + 2 * j], 0));
-    launch_lateral(h, cur, Tc);
+    launch_lateral(h, cur, Tc, false);
     rc = launch_part_b(h, s, cur, Tc, h->c3s, j > 0);
     if (rc) {
       pipe_drain(h);
@@ -2865,11 +2932,8 @@ int shoc_tr_gpu_substep_min(shoc_tr_gpu *h, double *dmin) {
   DeviceScope dev_(h->device);
   cudaStream_t st = h->stream;
   k_reset<<<1, 32, 0, st>>>(h->W, h->d_counts);
-  const int nb = (h->ncol + 127) / 128;
-  k_set_dz<<<nb, 128, 0, st>>>(h->G, h->F, h->W, h->O, h->tl, h->any_vdiff ? 1 : 0, h->d_counts,
-                               h->staged ? 1 : 0, h->esize == sizeof(float) ? 1 : 0, h->colown,
-                               1);
-  h->launches += 2;
+  h->launches++;
+  launch_set_dz(h, SD_PROBE | SD_SEARCH);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(h->h_dtm, h->W.dtm_bits, 8, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));

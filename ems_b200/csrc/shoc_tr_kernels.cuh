@@ -3,7 +3,8 @@
 // Device layout: tracers and per-cell fields stay in SHOC's sparse layout
 // (index = SHOC sparse coordinate), so 32 adjacent wet columns at one layer
 // are 32 consecutive cells and a warp's loads coalesce; host<->device copies
-// are plain memcpys.  One thread owns one (column, tracer) pair and walks its
+// are plain memcpys.  This file holds the general path (column_pass): one
+// thread owns one (column, tracer) pair and walks its
 // column bottom to top: horizontal and vertical face values, the ULTIMATE
 // limiter, the flux divergence, the interior update, surf_conc and tr_bounds,
 // and on the last sub-step the Thomas forward sweep; then it back-substitutes
@@ -113,7 +114,6 @@ struct Flow {
 
 struct Work {
   double *dz, *w5, *w9, *dbz, *dfz;     // per step
-  double *w6, *w7, *w8;                 // per sub-step
   double *vd_cm1, *vd_div, *vd_ud, *vd_dzdt;
   int *sur_t, *nsur_t;                  // [ncol] 0-based column
   ColInfo *col;                         // [ncol]
@@ -125,6 +125,29 @@ struct Work {
   float *dz32;
   float4 *lu32;
 };
+
+// Static per-cell / per-layer tables of the tile kernels (built once at
+// handle creation from the geometry maps).
+struct Tile {
+  const int *cellk;  // [nz][ncolp] cell of column col at layer k (0: none)
+  const int4 *nb1;   // [S] xm1, xp1, ym1, yp1
+  const int4 *nb2;   // [S] xm1(xm1), xp1(xp1), ym1(ym1), yp1(yp1)
+  const int2 *m2e;   // [S] m2d(xp1), m2d(yp1)
+  const uint8_t *fl; // [S] cflag(c) | xp1 wet, E1 | yp1 wet, E2 (FL_*)
+  const int *kof;    // [S] layer index of each cell (s2k)
+  const int4 *nbz;   // [S] zm1, zm1(zm1), zp1, zp1(zp1)
+  const int *colof;  // [S] 0-based column of each wet cell
+  const int *wet;    // [nwet] the wet cells (w3_t order)
+  const int *vdcol;  // [ncolp] columns in k_vd32 order: whole tiles of 32
+                     // adjacent columns, shallow tiles first (-1: padding)
+  int nclass;        // k_vd32 depth classes: tiles [ctile[i], ctile[i+1]) have
+  int ctile[5];      //   no cell below layer cbase[i]
+  int cbase[4];
+  const int4 *colrec;  // [ncolp] bottom cell, surface-layer cell, bottom layer
+  int ncolp;         // columns rounded up to whole tiles
+  int nwet;
+};
+constexpr int FL_XP_WET = 8, FL_XP_E1 = 16, FL_YP_WET = 32, FL_YP_E2 = 64;
 
 // FP32 copies of the flow fields (FP32-mixed path), made by set_flow.
 struct Flow32 {
@@ -301,14 +324,14 @@ __device__ __forceinline__ double hface_value(int trasc, bool eb, double cr, dou
 // Final e1 flux through the west face of wet cell c (advect + hor_diffuse):
 // tm2..tp1 = tr at xm1[xm1[c]], xm1[c], c, xp1[c].
 __device__ __forceinline__ double flux_x(const Geo &G, const Flow &F, const Work &W,
-                                         const Opt &O, uint8_t fl, bool adv, bool hdiff, int c,
+                                         const Opt &O, int fl, bool adv, bool hdiff, int c,
                                          int c2, double tm2, double tm1, double t0,
-                                         double tp1) {
+                                         double tp1, double dtu) {
   double v = 0.0;
   if (adv && O.trasc == SHOC_TR_ORDER1) {
     v = order1_flux(F.u1flux3d[c], tm1, t0);
   } else if (adv) {
-    double cr = W.w6[c];
+    double cr = F.u1[c] * dtu / G.h1au1[c2];  // w6 (:731)
     v = hface_value(O.trasc, (fl & CF_E1) != 0, cr, F.u1[c], G.fx[c2], tm2, tm1, t0, tp1);
     if (O.ultimate && (fl & CF_E1)) v = ultimate_face(cr, v, tm2, tm1, t0, tp1);
     v *= F.u1flux3d[c];
@@ -321,14 +344,14 @@ __device__ __forceinline__ double flux_x(const Geo &G, const Flow &F, const Work
 }
 
 __device__ __forceinline__ double flux_y(const Geo &G, const Flow &F, const Work &W,
-                                         const Opt &O, uint8_t fl, bool adv, bool hdiff, int c,
+                                         const Opt &O, int fl, bool adv, bool hdiff, int c,
                                          int c2, double tm2, double tm1, double t0,
-                                         double tp1) {
+                                         double tp1, double dtu) {
   double v = 0.0;
   if (adv && O.trasc == SHOC_TR_ORDER1) {
     v = order1_flux(F.u2flux3d[c], tm1, t0);
   } else if (adv) {
-    double cr = W.w7[c];
+    double cr = F.u2[c] * dtu / G.h2au2[c2];  // w7 (:733)
     v = hface_value(O.trasc, (fl & CF_E2) != 0, cr, F.u2[c], G.fy[c2], tm2, tm1, t0, tp1);
     if (O.ultimate && (fl & CF_E2)) v = ultimate_face(cr, v, tm2, tm1, t0, tp1);
     v *= F.u2flux3d[c];
@@ -348,7 +371,7 @@ __device__ __forceinline__ double flux_z(const Flow &F, const Work &W, const Opt
   const double wc = F.w[c];
   if (O.trasc == SHOC_TR_ORDER1)  // order1 (:1611-1616)
     return dtu * (0.5 * (wc + fabs(wc)) * tm1 + 0.5 * (wc - fabs(wc)) * t0);
-  double cz = W.w8[c];
+  double cz = wc * dtu / (w90 * 1.0);  // w8 (:735)
   double v;
   switch (O.trasc) {
     case SHOC_TR_QUICKEST:
@@ -369,16 +392,10 @@ __device__ __forceinline__ double flux_z(const Flow &F, const Work &W, const Opt
 
 namespace shoc {
 
-// Per-thread Thomas storage: the main kernel keeps sol(k) in shared memory
-// (layer-major, conflict free), the serial kernel in a local array.
-struct SmemSol {
-  double *base;
-  int stride;
-  __device__ __forceinline__ double &at(int k) { return base[(size_t)k * stride]; }
-};
-constexpr int kSerialMaxLayers = 128;
+// Thomas storage of one thread of the general path (local memory)
+constexpr int kMaxLayers = 128;
 struct LocalSol {
-  double v[kSerialMaxLayers];
+  double v[kMaxLayers];
   __device__ __forceinline__ double &at(int k) { return v[k]; }
 };
 
@@ -388,28 +405,24 @@ struct LocalSol {
 // (:3217-3324) and, when LAST, the implicit vertical diffusion
 // (implicit_vdiff_tr, :4067-4214) with the LU factors from k_set_dz.
 //
-// The loop over layers runs from kstart (the lowest bottom layer of the warp)
-// to the surface layer, so the lanes of a warp touch one layer at a time and
-// their loads coalesce; a lane acts once k reaches its own bottom layer.
+// The cells of the column and their neighbours come from the static tables, so
+// no load waits on a walk through the maps.
 // c3_moved carries tr_bounds' thin-surface cursor between tracers of one
-// column (tracers.c:3250-3270 does not reset it); the main kernel only runs
-// columns where the cursor cannot move.  TR is the tracer storage type
+// column (tracers.c:3250-3270 does not reset it).  TR is the tracer storage type
 // (double, or float for the FP32-mixed path); arithmetic is FP64 either way.
 template <bool LAST, class Sol, class TR>
 __device__ __forceinline__ void column_pass(const Geo &G, const Flow &F, const Work &W,
                                             const Opt &O, const TrSet &T, const SubStep &ss,
-                                            const TR *__restrict__ tri,
-                                            TR *__restrict__ tro, int col, int n, int kstart,
-                                            bool act, Sol &sol, bool &c3_moved,
-                                            unsigned long long &warn, int &stat) {
-  ColInfo ci = {0, 0, 0, 0, 0, 0};
-  int cbot = 0, ctop = 0, kb = G.nz;
-  if (act) {
-    ci = W.col[col];
-    cbot = G.col_bot[col];
-    ctop = G.col_top[col];
-    kb = G.col_kb[col];
-  }
+                                            const Tile &Tl, const TR *__restrict__ tri,
+                                            TR *__restrict__ tro, int col, int n, Sol &sol,
+                                            bool &c3_moved, unsigned long long &warn,
+                                            int &stat) {
+  const ColInfo ci = W.col[col];
+  const int cbot = G.col_bot[col], ctop = G.col_top[col], kb = G.col_kb[col];
+  // the cell of layer k (the top cell maps onto itself)
+  auto cell = [&](int k) {
+    return k < G.nz ? __ldg(&Tl.cellk[(size_t)k * Tl.ncolp + col]) : ctop;
+  };
   const uint8_t tf = T.trf[n];
   const bool tbdy = (tf & TR_TBDY) != 0;
   const bool wet = (ci.flags & COL_WET) != 0;
@@ -420,7 +433,7 @@ __device__ __forceinline__ void column_pass(const Geo &G, const Flow &F, const W
   const bool vd = vdf && !(ci.flags & (COL_SINGLE | COL_NOSOLVE));
   const double dtu = ss.dtu;
   const int c2 = ctop;
-  const double area = act ? G.cellarea[c2] : 1.0;
+  const double area = G.cellarea[c2];
   const double mn = T.mintr[n], mx = T.maxtr[n];
   const int s = ci.s, co = ci.co, cs = ci.cs, cbs = ci.cbs;
   // sub-step surface elevations (tracers.c:746-756, :1027-1031)
@@ -438,15 +451,14 @@ __device__ __forceinline__ void column_pass(const Geo &G, const Flow &F, const W
   double a_below = 0.0, solp = 0.0, ts_old = 0.0;
   int phase = 0, k_s = 0, k_cs = 0;
 
-  for (int k = kstart; k < G.nz; ++k) {
-    if (!act || k < kb) continue;
+  for (int k = kb; k < G.nz; ++k) {
     if (k == kb) {
       c = cbot;
       t0 = tri[c];
       tm1 = t0;  // sediment ghost holds the bottom value (tracers.c:827-830)
       tm2 = t0;
-      czp1 = G.zp1[c];
-      czp2 = G.zp1[czp1];
+      czp1 = cell(kb + 1);
+      czp2 = cell(kb + 2);
       tp1 = tri[czp1];
       tp2 = tri[czp2];
       w9m = 0.0;  // w9 of the sediment cell
@@ -458,7 +470,7 @@ __device__ __forceinline__ void column_pass(const Geo &G, const Flow &F, const W
     } else {
       c = czp1;
       czp1 = czp2;
-      czp2 = G.zp1[czp1];
+      czp2 = cell(k + 2);
       tm2 = tm1;
       tm1 = t0;
       t0 = tp1;
@@ -492,19 +504,23 @@ __device__ __forceinline__ void column_pass(const Geo &G, const Flow &F, const W
     // horizontal fluxes and their divergence (dtracer, tracers.c:888-892)
     double dtr = 0.0;
     if (adv || hd) {
-      const int xm1 = G.xm1[c], xp1 = G.xp1[c], ym1 = G.ym1[c], yp1 = G.yp1[c];
-      const uint8_t fc = G.cflag[c], fe = G.cflag[xp1], fn = G.cflag[yp1];
-      const double txm1 = tri[xm1], txp1 = tri[xp1], tym1 = tri[ym1], typ1 = tri[yp1];
-      const double txm2 = tri[G.xm1[xm1]], tym2 = tri[G.ym1[ym1]];
-      double Fxw = flux_x(G, F, W, O, fc, adv, hd, c, c2, txm2, txm1, t0, txp1);
-      double Fys = flux_y(G, F, W, O, fc, adv, hd, c, c2, tym2, tym1, t0, typ1);
+      const int4 n1 = __ldg(&Tl.nb1[c]), n2 = __ldg(&Tl.nb2[c]);
+      const int2 me = __ldg(&Tl.m2e[c]);
+      const int fc = __ldg(&Tl.fl[c]);
+      const int xp1 = n1.y, yp1 = n1.w;
+      const double txm1 = tri[n1.x], txp1 = tri[xp1], tym1 = tri[n1.z], typ1 = tri[yp1];
+      const double txm2 = tri[n2.x], tym2 = tri[n2.z];
+      double Fxw = flux_x(G, F, W, O, fc, adv, hd, c, c2, txm2, txm1, t0, txp1, dtu);
+      double Fys = flux_y(G, F, W, O, fc, adv, hd, c, c2, tym2, tym1, t0, typ1, dtu);
       double Fxe = 0.0, Fyn = 0.0;
-      if (fe & CF_WET)
-        Fxe = flux_x(G, F, W, O, fe, adv, hd, xp1, G.m2d[xp1], txm1, t0, txp1, tri[G.xp1[xp1]]);
+      if (fc & FL_XP_WET)
+        Fxe = flux_x(G, F, W, O, (fc & FL_XP_E1) ? CF_E1 : 0, adv, hd, xp1, me.x, txm1, t0,
+                     txp1, tri[n2.y], dtu);
       else if (adv && O.trasc == SHOC_TR_ORDER1)  // order1 fills the ghost cells' faces too
         Fxe = order1_flux(F.u1flux3d[xp1], t0, txp1);
-      if (fn & CF_WET)
-        Fyn = flux_y(G, F, W, O, fn, adv, hd, yp1, G.m2d[yp1], tym1, t0, typ1, tri[G.yp1[yp1]]);
+      if (fc & FL_YP_WET)
+        Fyn = flux_y(G, F, W, O, (fc & FL_YP_E2) ? CF_E2 : 0, adv, hd, yp1, me.y, tym1, t0,
+                     typ1, tri[n2.w], dtu);
       else if (adv && O.trasc == SHOC_TR_ORDER1)
         Fyn = order1_flux(F.u2flux3d[yp1], t0, typ1);
       dtr = (Fxe - Fxw + Fyn - Fys) * dtu;
@@ -564,14 +580,14 @@ __device__ __forceinline__ void column_pass(const Geo &G, const Flow &F, const W
       }
     }
   }
-  if (!act || !upd) {
-    if (act && vdf && (ci.flags & COL_SINGLE)) {
+  if (!upd) {
+    if (vdf && (ci.flags & COL_SINGLE)) {
       // one-layer column (tracers.c:4125-4132): max(dzcell, hmin)
       double h = W.dz[cs] > O.hmin ? W.dz[cs] : O.hmin;
       double v = tro[cs];
       tro[cs] = (TR)(v + F.dt * (0.0 - 0.0) / h);
       if (isnan(v)) stat |= ST_NAN;
-    } else if (act && vd) {
+    } else if (vd) {
       double x = sol.at(k_cs);
       double a = tro[cs];
       double fin = a + (x - a) * 1.0;

@@ -52,29 +52,6 @@
 
 namespace shoc {
 
-// Static per-cell / per-layer tables of the tile kernels (built once at
-// handle creation from the geometry maps).
-struct Tile {
-  const int *cellk;  // [nz][ncolp] cell of column col at layer k (0: none)
-  const int4 *nb1;   // [S] xm1, xp1, ym1, yp1
-  const int4 *nb2;   // [S] xm1(xm1), xp1(xp1), ym1(ym1), yp1(yp1)
-  const int2 *m2e;   // [S] m2d(xp1), m2d(yp1)
-  const uint8_t *fl; // [S] cflag(c) | xp1 wet, E1 | yp1 wet, E2 (FL_*)
-  const int *kof;    // [S] layer index of each cell (s2k)
-  const int4 *nbz;   // [S] zm1, zm1(zm1), zp1, zp1(zp1)
-  const int *colof;  // [S] 0-based column of each wet cell
-  const int *wet;    // [nwet] the wet cells (w3_t order)
-  const int *vdcol;  // [ncolp] columns in k_vd32 order: whole tiles of 32
-                     // adjacent columns, shallow tiles first (-1: padding)
-  int nclass;        // k_vd32 depth classes: tiles [ctile[i], ctile[i+1]) have
-  int ctile[5];      //   no cell below layer cbase[i]
-  int cbase[4];
-  const int4 *colrec;  // [ncolp] bottom cell, surface-layer cell, bottom layer
-  int ncolp;         // columns rounded up to whole tiles
-  int nwet;
-};
-constexpr int FL_XP_WET = 8, FL_XP_E1 = 16, FL_YP_WET = 32, FL_YP_E2 = 64;
-
 // asynchronous global -> shared copies; a thread waits for its own copies
 __device__ __forceinline__ void cp_async4(void *dst, const void *src) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(dst);
