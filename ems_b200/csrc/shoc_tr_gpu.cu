@@ -178,6 +178,15 @@ int dalloc(shoc_tr_gpu *h, T **p, size_t n) {
   return 0;
 }
 
+// Waits for the default stream: cudaMemset, and cudaMemcpy from pageable
+// memory, may still be under way when they return, and the handle's stream
+// is non-blocking.  Called after every use of them, before the handle's
+// stream may read what they write.
+int default_stream_done() {
+  CK(cudaStreamSynchronize(cudaStreamLegacy));
+  return 0;
+}
+
 template <class T>
 int dupload(shoc_tr_gpu *h, T **p, const T *src, size_t n) {
   int rc = dalloc(h, p, n);
@@ -1647,6 +1656,9 @@ int shoc_tr_gpu_create(const shoc_tr_geom *g, const shoc_tr_opts *o, int ntr, in
                            227 * 1024) != cudaSuccess ||
       tile32_set_smem_attr() != cudaSuccess)
     TRY(SHOC_TR_ECUDA);
+  // the uploads and fills above went to the default stream, which the
+  // handle's non-blocking stream does not wait for
+  if (default_stream_done() != 0) TRY(SHOC_TR_ECUDA);
 #undef TRY
   *out = h;
   return SHOC_TR_OK;
@@ -2328,6 +2340,7 @@ int shoc_tr_gpu_set_preamble(shoc_tr_gpu *h, int on) {
     if (!rc && !h->F.dzu1) rc = dupload<double>(h, (double **)&h->F.dzu1, nullptr, (size_t)h->S);
     if (!rc && !h->F.dzu2) rc = dupload<double>(h, (double **)&h->F.dzu2, nullptr, (size_t)h->S);
     if (!rc && !h->pre.detadt) rc = dupload<double>(h, &h->pre.detadt, nullptr, (size_t)h->S2);
+    if (!rc) rc = default_stream_done();
     if (rc) return rc;
   }
   if (h->pre.on != (on != 0)) {
@@ -2821,7 +2834,7 @@ int shoc_tr_gpu_halo_plan(shoc_tr_gpu *h, int nsend, const int *send_cells, int 
     CK(cudaMemcpy(h->halo_recv, recv_cells, (size_t)nrecv * sizeof(int), cudaMemcpyHostToDevice));
   h->nhalo_send = nsend;
   h->nhalo_recv = nrecv;
-  return SHOC_TR_OK;
+  return default_stream_done();
 }
 
 int shoc_tr_gpu_halo_pack(shoc_tr_gpu *h, void *buf) {
@@ -2922,6 +2935,7 @@ int shoc_tr_gpu_set_owned(shoc_tr_gpu *h, const int *owned2d) {
   for (int c = 0; c < h->ncol; c++) own[c] = owned2d[top[c]] ? 1 : 0;
   int *d = nullptr;
   int rc = dupload(h, &d, own.data(), (size_t)h->ncol);
+  if (!rc) rc = default_stream_done();
   if (rc) return rc;
   h->colown = d;
   return SHOC_TR_OK;
