@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
     const double tz = F.eta[c2] < F.oldeta[c2] ? F.eta[c2] : F.oldeta[c2];
     const double bz = SHOC_TR_DRY_FRAC * O.hmin + __ldg(&G.botz[c2]);
     wet = (tz > bz && js > 0);
-    pre_staged = O.tiled && wet && s == sur && s == nsur;
+    pre_staged = O.tiled && wet && (O.cross || (s == sur && s == nsur));
   }
   // thickness of layer j (:5824-5846): from the old surface down to the
   // bottom, the layers above the old surface copy the old surface cell's
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
   ci.cbs = cbs;
   ci.flags = flags;
   ci.ks = kb + js - 1;
-  const bool staged = on && O.tiled && staged_column(ci, bot);
+  const bool staged = on && O.tiled && staged_column(ci, bot, O.cross != 0);
   if (staged) ci.flags |= COL_STAGED;
   if (wy == 0) {
     if (solve) {
@@ -490,6 +490,7 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
         W.vd_div[cc] = div;
         W.vd_ud[cc] = ud;
         W.vd_dzdt[cc] = dzdt;
+        if (what & SD_LU64) W.vd_rdiv[cc] = div_range(div) == kDivLo ? 1.0 / div : 0.0;
       }
       if (what & SD_F32)
         W.lu32[cc] = make_float4((float)dzdt, (float)cm1, (float)(1.0 / div), (float)ud);
@@ -948,6 +949,7 @@ __global__ void k_halo_unpack(TR *tra, TR *trb, int S, int ntr, const int *cells
 }
 
 // shared memory of the column kernel of the handle's precision
+cudaError_t tile64_set_smem_attr();
 size_t vd_smem(const shoc_tr_gpu *h, int nd, int nw) {
   return h->esize == sizeof(float) ? vd32_smem(nd, nw, h->vd_pf, h->comp) : vd64_smem(nd, nw);
 }
@@ -1038,6 +1040,21 @@ int build_tile_tables(shoc_tr_gpu *h, const shoc_tr_geom *g, const std::vector<u
     h->vd_depth[i] = tdepth[t];
     for (int l = 0; l < 32; l++) vdcol[i * 32 + l] = (t * 32 + l < ncol) ? t * 32 + l : -1;
   }
+  // k_adv64's segments: columns in order, 32 to a warp; where the 32nd is the
+  // east neighbour of the 31st it is a halo lane and starts the next segment
+  std::vector<int> seg;
+  for (int col = 0; col < ncol;) {
+    const size_t b = seg.size();
+    seg.insert(seg.end(), 32, -1);
+    int l = 0;
+    for (; l < 32 && col < ncol; l++, col++) {
+      seg[b + l] = col;
+      if (l == 31 && g->xp1[g->w2_t[col]] == g->w2_t[col + 1]) {
+        seg[b + l] |= kSegHalo;
+        break;
+      }
+    }
+  }
   std::vector<int4> colrec(ncolp, make_int4(0, 0, nz, 0));
   for (int col = 0; col < ncol; col++)
     colrec[col] = make_int4(col_bot[col], g->w2_t[col + 1], col_kb[col], 0);
@@ -1070,6 +1087,9 @@ int build_tile_tables(shoc_tr_gpu *h, const shoc_tr_geom *g, const std::vector<u
   T.wet = ip;
   if ((rc = dupload(h, &ip, vdcol.data(), vdcol.size()))) return rc;
   T.vdcol = ip;
+  if ((rc = dupload(h, &ip, seg.data(), seg.size()))) return rc;
+  T.seg = ip;
+  T.nseg = (int)(seg.size() / 32);
   return 0;
 }
 
@@ -1453,7 +1473,8 @@ int shoc_tr_gpu_create(const shoc_tr_geom *g, const shoc_tr_opts *o, int ntr, in
   h->O.trasc = o->trasc;
   // order1 is monotonic and switches the limiter off (tracers.c:497-503)
   h->O.ultimate = o->trasc == SHOC_TR_ORDER1 ? 0 : o->ultimate;
-  h->O.tiled = (o->trasc == SHOC_TR_QUICKEST || o->trasc == SHOC_TR_VANLEER) ? 1 : 0;
+  h->O.cross = precision == SHOC_TR_FP64 ? 1 : 0;
+  h->O.tiled = (o->trasc == SHOC_TR_QUICKEST || o->trasc == SHOC_TR_VANLEER || h->O.cross) ? 1 : 0;
   h->O.substep =
       (o->stab & (SHOC_TR_SUB_STEP | SHOC_TR_SUB_STEP_NOSURF | SHOC_TR_SUB_STEP_TRACER)) ? 1 : 0;
   h->O.hmin = o->hmin;
@@ -1510,6 +1531,7 @@ int shoc_tr_gpu_create(const shoc_tr_geom *g, const shoc_tr_opts *o, int ntr, in
   TRY(dupload<double>(h, &W.vd_div, nullptr, S));
   TRY(dupload<double>(h, &W.vd_ud, nullptr, S));
   TRY(dupload<double>(h, &W.vd_dzdt, nullptr, S));
+  if (precision == SHOC_TR_FP64) TRY(dupload<double>(h, &W.vd_rdiv, nullptr, S));
   TRY(dupload<int>(h, &W.sur_t, nullptr, ncol));
   TRY(dupload<int>(h, &W.nsur_t, nullptr, ncol));
   TRY(dupload<ColInfo>(h, &W.col, nullptr, ncol));
@@ -1650,10 +1672,7 @@ int shoc_tr_gpu_create(const shoc_tr_geom *g, const shoc_tr_opts *o, int ntr, in
   h->h_counts = (int *)((char *)pin + 24);
   if (cudaFuncSetAttribute(k_set_dz, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)set_dz_smem(kMaxLayers)) != cudaSuccess ||
-      cudaFuncSetAttribute(k_vd64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           227 * 1024) != cudaSuccess ||
-      cudaFuncSetAttribute(k_vd64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           227 * 1024) != cudaSuccess ||
+      tile64_set_smem_attr() != cudaSuccess ||
       tile32_set_smem_attr() != cudaSuccess)
     TRY(SHOC_TR_ECUDA);
   // the uploads and fills above went to the default stream, which the
@@ -1810,21 +1829,59 @@ void launch_general(shoc_tr_gpu *h, bool last, const TrSet &T, const SubStep &ss
 
 // One FP64 transport sub-step over the staged columns: k_adv64, then one
 // k_vd64 launch per depth class.  Returns the kernels launched.
-template <bool Q, bool U, int M>
-void adv64(const shoc_tr_gpu *h, int grid, const SubStep &ss, const Tile &tl, const TrSet &T,
+//
+// Layers per warp of k_adv64: a longer climb computes fewer bottom faces twice
+// (one per chunk), a shorter one gives more warps.  The chip holds 148 x 16;
+// the chunks are the longest that still make about six rounds of them.
+template <int SCH, bool U>
+void adv64(const shoc_tr_gpu *h, const SubStep &ss, const Tile &tl, const TrSet &T,
            const double *tin, double *tout) {
-  k_adv64<Q, U, M><<<grid, kAdvBlock, 0, h->stream>>>(h->G, h->F, h->W, T, ss, tl, tin, tout,
-                                                      h->fzs64, h->any_hdiff ? 1 : 0);
-}
-template <bool Q, bool U>
-void adv64_mode(const shoc_tr_gpu *h, int grid, const SubStep &ss, const Tile &tl,
-                const TrSet &T, const double *tin, double *tout) {
+  const long long want = 148LL * 16 * 6;
+  const int ng = std::min(T.ntb, kAdv64Group), groups = (T.ntb + ng - 1) / ng;
+  const int lmax = (int)std::max<long long>(1, (long long)tl.nseg * h->nz * groups / want);
+  const int nch = (h->nz + std::min(lmax, h->nz) - 1) / std::min(lmax, h->nz);
+  const int L = (h->nz + nch - 1) / nch;
+  const dim3 grid((tl.nseg + kAdv64Warps - 1) / kAdv64Warps * nch, groups);
+  const size_t smem = adv64_smem(ng);
   if (h->adv_flags == 1)
-    adv64<Q, U, 1>(h, grid, ss, tl, T, tin, tout);
-  else if (h->adv_flags == 2)
-    adv64<Q, U, 2>(h, grid, ss, tl, T, tin, tout);
+    k_adv64<SCH, U, true><<<grid, kAdv64Warps * 32, smem, h->stream>>>(
+        h->G, h->F, h->W, h->O, T, ss, tl, tin, tout, h->fzs64, nch, L, ng);
   else
-    adv64<Q, U, 0>(h, grid, ss, tl, T, tin, tout);
+    k_adv64<SCH, U, false><<<grid, kAdv64Warps * 32, smem, h->stream>>>(
+        h->G, h->F, h->W, h->O, T, ss, tl, tin, tout, h->fzs64, nch, L, ng);
+}
+template <int SCH>
+void adv64_ult(const shoc_tr_gpu *h, const SubStep &ss, const Tile &tl, const TrSet &T,
+               const double *tin, double *tout) {
+  if (h->O.ultimate)
+    adv64<SCH, true>(h, ss, tl, T, tin, tout);
+  else
+    adv64<SCH, false>(h, ss, tl, T, tin, tout);
+}
+template <int SCH>
+cudaError_t adv64_attr() {
+  cudaError_t e = cudaSuccess;
+  const int bytes = (int)adv64_smem(kAdv64Group);
+  for (auto k : {k_adv64<SCH, false, false>, k_adv64<SCH, false, true>, k_adv64<SCH, true, false>,
+                 k_adv64<SCH, true, true>}) {
+    const cudaError_t r =
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (r != cudaSuccess) e = r;
+  }
+  return e;
+}
+cudaError_t tile64_set_smem_attr() {
+  const cudaError_t r[] = {
+      adv64_attr<SHOC_TR_QUICKEST>(),    adv64_attr<SHOC_TR_VANLEER>(),
+      adv64_attr<SHOC_TR_ORDER1>(),      adv64_attr<SHOC_TR_ORDER2>(),
+      adv64_attr<SHOC_TR_ORDER4>(),      adv64_attr<SHOC_TR_QUICKEST_CO>(),
+      adv64_attr<SHOC_TR_ORDER2_UW>(),
+      cudaFuncSetAttribute(k_vd64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024),
+      cudaFuncSetAttribute(k_vd64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           227 * 1024)};
+  for (auto x : r)
+    if (x != cudaSuccess) return x;
+  return cudaSuccess;
 }
 int tile64_substep(const shoc_tr_gpu *h, bool last, const SubStep &ss, const Tile &tl,
                    const TrSet &T, const double *tin, double *tout, int nw, cudaEvent_t *ev) {
@@ -1832,16 +1889,15 @@ int tile64_substep(const shoc_tr_gpu *h, bool last, const SubStep &ss, const Til
   int nl = 0;
   if (ev) cudaEventRecord(ev[0], st);
   if (T.ntb > 0 && tl.nwet > 0) {
-    const int grid = (tl.nwet + kAdvBlock - 1) / kAdvBlock;
-    const bool q = h->O.trasc == SHOC_TR_QUICKEST, u = h->O.ultimate != 0;
-    if (q && u)
-      adv64_mode<true, true>(h, grid, ss, tl, T, tin, tout);
-    else if (q)
-      adv64_mode<true, false>(h, grid, ss, tl, T, tin, tout);
-    else if (u)
-      adv64_mode<false, true>(h, grid, ss, tl, T, tin, tout);
-    else
-      adv64_mode<false, false>(h, grid, ss, tl, T, tin, tout);
+    switch (h->O.trasc) {
+      case SHOC_TR_QUICKEST: adv64_ult<SHOC_TR_QUICKEST>(h, ss, tl, T, tin, tout); break;
+      case SHOC_TR_VANLEER: adv64_ult<SHOC_TR_VANLEER>(h, ss, tl, T, tin, tout); break;
+      case SHOC_TR_ORDER1: adv64_ult<SHOC_TR_ORDER1>(h, ss, tl, T, tin, tout); break;
+      case SHOC_TR_ORDER2: adv64_ult<SHOC_TR_ORDER2>(h, ss, tl, T, tin, tout); break;
+      case SHOC_TR_ORDER4: adv64_ult<SHOC_TR_ORDER4>(h, ss, tl, T, tin, tout); break;
+      case SHOC_TR_QUICKEST_CO: adv64_ult<SHOC_TR_QUICKEST_CO>(h, ss, tl, T, tin, tout); break;
+      case SHOC_TR_ORDER2_UW: adv64_ult<SHOC_TR_ORDER2_UW>(h, ss, tl, T, tin, tout); break;
+    }
     nl++;
   }
   if (ev) cudaEventRecord(ev[1], st);
@@ -1854,11 +1910,11 @@ int tile64_substep(const shoc_tr_gpu *h, bool last, const SubStep &ss, const Til
     if (last)
       k_vd64<true><<<nt * nchunk, blk, smem, st>>>(
           h->G, h->F, h->W, h->O, T, ss, tl, tin, tout, h->fzs64, h->W.vd_dzdt, h->W.vd_cm1,
-          h->W.vd_div, h->W.vd_ud, nw, nchunk, t0, kbase);
+          h->W.vd_div, h->W.vd_rdiv, h->W.vd_ud, nw, nchunk, t0, kbase);
     else
       k_vd64<false><<<nt * nchunk, blk, smem, st>>>(
           h->G, h->F, h->W, h->O, T, ss, tl, tin, tout, h->fzs64, h->W.vd_dzdt, h->W.vd_cm1,
-          h->W.vd_div, h->W.vd_ud, nw, nchunk, t0, kbase);
+          h->W.vd_div, h->W.vd_rdiv, h->W.vd_ud, nw, nchunk, t0, kbase);
     nl++;
   }
   if (ev) cudaEventRecord(ev[2], st);

@@ -115,6 +115,7 @@ struct Flow {
 struct Work {
   double *dz, *w5, *w9, *dbz, *dfz;     // per step
   double *vd_cm1, *vd_div, *vd_ud, *vd_dzdt;
+  double *vd_rdiv;                      // FP64: 1 / vd_div (0: not for div_known)
   int *sur_t, *nsur_t;                  // [ncol] 0-based column
   ColInfo *col;                         // [ncol]
   int *status;
@@ -144,9 +145,15 @@ struct Tile {
   int ctile[5];      //   no cell below layer cbase[i]
   int cbase[4];
   const int4 *colrec;  // [ncolp] bottom cell, surface-layer cell, bottom layer
+  // k_adv64's segments of the column order, [nseg][32]: columns, -1: none,
+  // with kSegHalo: the column only lends its west flux (it is the next
+  // segment's first own one)
+  const int *seg;
+  int nseg;
   int ncolp;         // columns rounded up to whole tiles
   int nwet;
 };
+constexpr int kSegHalo = 0x40000000;
 constexpr int FL_XP_WET = 8, FL_XP_E1 = 16, FL_YP_WET = 32, FL_YP_E2 = 64;
 
 // FP32 copies of the flow fields (FP32-mixed path), made by set_flow.
@@ -160,8 +167,9 @@ struct Flow32 {
 struct Opt {
   int trasc, ultimate, substep;
   double hmin;
-  int tiled;  // the scheme has tile kernels (QUICKEST, Van Leer); else every
-              // column takes the general path
+  int tiled;  // the scheme has tile kernels (FP64: every scheme; FP32-mixed:
+              // QUICKEST, Van Leer); else every column takes the general path
+  int cross;  // they step columns whose surface crosses a layer face (FP64)
 };
 
 // Per-tracer attributes (device arrays indexed by tracer number).

@@ -1,20 +1,21 @@
 // shoc_tr_stage.cuh -- FP32 face arithmetic of the FP32-mixed path and the
 // test that picks the columns the column-tile kernel handles.
 //
-// Columns whose free surface crosses a layer face during the step, whose
-// tr_bounds thin-surface cursor couples tracers, or whose implicit solve is
+// Columns whose free surface crosses a layer face during the step (FP32-mixed),
+// whose tr_bounds thin-surface cursor couples tracers, or whose implicit solve is
 // degenerate go through the general column path (column_pass) instead.
 #pragma once
 #include "shoc_tr_kernels.cuh"
 
 namespace shoc {
 
-// Columns the column-tile kernel handles: wet, surface cell unchanged this step
-// (s == co == cs), implicit solve spanning the whole column (or one layer).
-__device__ __forceinline__ bool staged_column(const ColInfo &ci, int cbot) {
+// Columns the column-tile kernels handle: wet, implicit solve spanning the
+// whole column (or one layer) and, unless they take crossings (cross),
+// surface cell unchanged this step (s == co == cs).
+__device__ __forceinline__ bool staged_column(const ColInfo &ci, int cbot, bool cross) {
   if (!(ci.flags & COL_WET)) return false;
   if (ci.flags & (COL_SERIAL | COL_NOSOLVE)) return false;
-  if (ci.s != ci.co || ci.s != ci.cs) return false;
+  if (!cross && (ci.s != ci.co || ci.s != ci.cs)) return false;
   if (!(ci.flags & COL_SINGLE) && ci.cbs != cbot) return false;
   return true;
 }

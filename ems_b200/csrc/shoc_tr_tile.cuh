@@ -142,7 +142,6 @@ __device__ __forceinline__ void zface(Face &f, bool quick, bool ult, float dzm2,
 // ---------------------------------------------------------------------------
 // k_adv32
 
-constexpr int kAdvBlock = 256;     // k_adv64
 // k_adv32: 128 threads, 5 blocks per SM (at most 102 registers a thread: 20
 // warps per SM where 256-thread blocks fit 16; measured 13.0 ms against 14.3
 // on stiff2048)

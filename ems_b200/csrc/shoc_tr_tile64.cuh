@@ -1,12 +1,12 @@
-// shoc_tr_tile64.cuh -- the plain FP64 transport kernels of the staged columns
-// (surface cell stays in its layer during the step), bitwise equal to the
-// reference: the same two-kernel structure as the FP32-mixed path
-// (shoc_tr_tile.cuh), with model/hd/tracers/tracers.c's arithmetic operation
-// by operation (compiled without FMA contraction, IEEE division).
+// shoc_tr_tile64.cuh -- the plain FP64 transport kernels, bitwise equal to the
+// reference: model/hd/tracers/tracers.c's arithmetic operation by operation
+// (compiled without FMA contraction; quotients correctly rounded).  They step
+// every scheme and every wet column but those whose thin-surface cursor
+// couples tracers or whose implicit solve is degenerate (k_general).
 //
-//  k_adv64  one thread per wet cell: the QUICKEST / Van Leer face values with
-//           ULTIMATE and horizontal diffusion of the cell's west, south,
-//           north, (east) and bottom and top faces (quickest :1819-1931,
+//  k_adv64  a warp per segment of columns and chunk of layers: the face
+//           values of the scheme with ULTIMATE and horizontal diffusion of the
+//           cell's west, south, north and top faces (quickest :1819-1931,
 //           ulimate_filter :3501-3557, van_leer_do :2087-2119, hor_diffuse
 //           :3595-3668), the flux divergence and the interior update
 //           (advect_diffuse :888-925).  The Courant numbers are formed in the
@@ -16,210 +16,548 @@
 //           implicit vertical diffusion (implicit_vdiff_tr :4067-4214) with
 //           the LU factors k_set_dz builds.
 //
-// Every face value is computed from the same operands in the same order as
-// column_pass computes it (a cell's top face is the next cell's bottom face:
-// the same call with the same arguments), so the results are identical.
+// A face two cells share is computed from the same operands in the same order
+// wherever it is computed, so the results are those of column_pass.
 #pragma once
+#include <type_traits>
+
 #include "shoc_tr_tile.cuh"
 
 namespace shoc {
 
 // shared memory of k_vd64 (bytes) for columns of at most nd layers:
-// colC int[nd][32], A, S double[nd][nw][32]
+// S double[nd][nw][32], colC int[nd][32]
 inline size_t vd64_smem(int nd, int nw) {
-  return (size_t)nd * 32 * 4 + (size_t)2 * nd * nw * 32 * 8;
-}
-
-// One horizontal face (advect + hor_diffuse) at a cell with Courant number cr,
-// velocity vel (Van Leer's sign), metric factors m, volume flux U; the
-// diffusion term is (P (t0 - tm1)) / H with P = dzu h2au1 1.0 u1kh and
-// H = h1au1 (x; the e2 analogue for y), as flux_x / flux_y form it.
-template <bool QUICK, bool ULT>
-__device__ __forceinline__ double hface64(bool eb, bool adv, bool hd, double cr, double vel,
-                                          const Face2D &m, double U, double P, double H,
-                                          double tm2, double tm1, double t0, double tp1) {
-  double v = 0.0;
-  if (adv) {
-    if (QUICK)
-      v = quickest_face(cr, m, tm2, tm1, t0, tp1);
-    else if (eb)
-      v = vanleer_face(vel, cr, tm2, tm1, t0, tp1);
-    if (ULT && eb) v = ultimate_face(cr, v, tm2, tm1, t0, tp1);
-    v *= U;
-  }
-  if (hd) v -= (P * (t0 - tm1) / H);
-  return v;
-}
-
-// The vertical face of flux_z at cell c (below it zm, above it zp) with its
-// Courant number cz = w dtu / w9 and w dtu precomputed; the work-array
-// values are read here (cached loads) to keep them out of registers.
-template <bool QUICK, bool ULT>
-__device__ __forceinline__ double zface64(const Flow &F, const Work &W, int c, int zm, int zp,
-                                          double cz, double wdtu, double tm2, double tm1,
-                                          double t0, double tp1) {
-  double v;
-  if (QUICK)
-    v = quickest_zface(cz, W.w5[c], W.dbz[c], W.dfz[c], W.w9[zm], W.w9[c], W.w9[zp], tm2, tm1,
-                       t0, tp1);
-  else
-    v = vanleer_face(F.w[c], cz, tm2, tm1, t0, tp1);
-  if (ULT) v = ultimate_face(cz, v, tm2, tm1, t0, tp1);
-  return v * wdtu;
+  return (size_t)nd * 32 * 4 + (size_t)nd * nw * 32 * 8;
 }
 
 // ---------------------------------------------------------------------------
 // k_adv64
+//
+// A warp owns a segment of the column order (Tile::seg: up to 32 neighbouring
+// columns; where the 32nd is the east neighbour of the 31st it only lends its
+// west flux, the halo lane) and a chunk of layers, and climbs the chunk: the
+// east flux is the next lane's west flux (a shuffle) and the bottom flux the
+// top flux of the layer below (kept per tracer in shared memory), so a cell
+// costs four face values where one thread per cell and no climbing cost six
+// executed ones (the east one for a warp's last lane alone).  The warps are
+// independent of one another.
+//
+// What bounds it: FP64 instructions and the latency of their chains.  The
+// reference divides by 6, by the cell area and thickness and up to four times
+// in ULTIMATE for every face; nothing but its own operation order gives its
+// bits.  So
+//  - quotients by divisors no tracer changes (6, area, dz, |cr|) come from the
+//    correctly rounded reciprocal and two residual corrections (quot), and
+//    ULTIMATE's by td - tu from one reciprocal that Van Leer's slope shares;
+//  - all of it is computed for every face and selected, so a cell's faces are
+//    one straight line of code the compiler interleaves; one check of the
+//    exponents of the cell's stencil values decides whether quotients may be
+//    formed this way, and a cell that fails it (values below 2^-400 or above
+//    2^490, NaN) computes its faces by the reference's divisions;
+//  - the faces' factors live in shared memory, written when a layer is set up
+//    (in registers they left 12 warps on an SM), and a tracer's stencil values
+//    are loaded while the one before it is computed, of the two values beyond a
+//    face only the upwind one.
+// 384 x 320 x 40, 10 tracers (B200), a sub-step: 1.75 ms with one thread per
+// cell and the reference's divisions; climbing, 2.35 ms with the limiter's
+// cases as branches, 1.15 ms as selections, 1.08 ms with upwind loads alone,
+// 1.00 ms with loads a tracer ahead and one-warp blocks (four-warp blocks wait
+// for their deepest column: 1.04).  A warp per face with the fluxes meeting in
+// shared memory took 1.25 ms: more warps, but a quarter more instructions.
 
-template <bool QUICK, bool ULT, int MODE>
-__global__ void __launch_bounds__(kAdvBlock, 2) k_adv64(Geo G, Flow F, Work W, TrSet T,
-                                                     SubStep ss, Tile Tl,
-                                                     const double *__restrict__ tri,
-                                                     double *__restrict__ tro,
-                                                     double *__restrict__ fzs, int any_hd) {
+// Correctly rounded a / b from y = RN(1 / b) (P. Markstein, IBM J. Res. Dev.
+// 34, 1990: with y the correctly rounded reciprocal, q within an ulp of a / b
+// and r = a - b q exact, RN(q + r y) is RN(a / b); the first correction brings
+// RN(a y) within an ulp) where neither a, b nor a / b are near the ends of the
+// range, or a is 0
+__device__ __forceinline__ double quot(double a, double b, double y) {
+  double q = __dmul_rn(a, y);
+  q = __fma_rn(__fma_rn(-b, q, a), y, q);
+  return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+// |x| outside 2^-lim .. 2^lim (a zero too)
+template <unsigned LIM>
+__device__ __forceinline__ bool far_out(double x) {
+  return ((unsigned)__double2hiint(x) & 0x7fffffffu) - ((1023u - LIM) << 20) >= ((2 * LIM) << 20);
+}
+// a / b for any a and a b the caller keeps y = 1 / b of.  lo: kDivLo where b
+// lies in 2^-200 .. 2^200, so that nothing under- or overflows for |a| in
+// 2^-700 .. 2^700; kDivNever where it does not.  Else the division.
+constexpr unsigned kDivLo = (1023u - 700u) << 20, kDivSpan = 1400u << 20;
+constexpr unsigned kDivNever = 0x80000000u;
+__device__ __noinline__ double div_slow(double a, double b) { return a / b; }
+__device__ __forceinline__ unsigned div_range(double b) {
+  return far_out<200>(b) ? kDivNever : kDivLo;
+}
+__device__ __forceinline__ double div_known(double a, double b, double y, unsigned lo) {
+  double q = quot(a, b, y);
+  const unsigned e = ((unsigned)__double2hiint(a) & 0x7fffffffu) - lo;
+  if (e >= kDivSpan) q = (a == 0.0 && lo != kDivNever) ? __dmul_rn(a, y) : div_slow(a, b);
+  return q;
+}
+// RN(1 / d) for |d| in 2^-500 .. 2^500: Newton steps from the hardware's
+// approximation (20 bits); the last one starts within an ulp, so it rounds
+// correctly (Markstein)
+__device__ __forceinline__ double recip(double d) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  y = __fma_rn(__fma_rn(-d, y, 1.0), y, y);
+  y = __fma_rn(__fma_rn(-d, y, 1.0), y, y);
+  return __fma_rn(__fma_rn(-d, y, 1.0), y, y);
+}
+
+// One face, set up once per cell for every tracer, in the warp's shared memory
+// (a row of 32 doubles each): the Courant number, the scheme's factors for its
+// sign (the curvature is D (P td + Q tu) - 2 tc; e: 1 - cr^2, Van Leer
+// (1 -+ cr) / 2), 1 / |cr| for the limiter and the volume flux
+enum { FC_CR, FC_U, FC_E, FC_Y, FC_D, FC_DB, FC_P, FC_Q, FC_N };
+constexpr int F64_POS = 1, F64_MOVE = 2, F64_VNZ = 4, F64_LIM = 8, F64_VAL = 16, F64_REF = 32;
+
+// hm, h0, hp: the metric at the cell behind, at and ahead of the face; val:
+// the scheme fills this face; lim: the limiter acts on it.  Returns its flags.
+template <int SCH>
+__device__ __forceinline__ int set_face_64(double *f, double cr, double vel, double d, double db,
+                                           double df, double hm, double h0, double hp, double U,
+                                           bool val, bool lim) {
+  constexpr bool byvel = SCH == SHOC_TR_VANLEER || SCH == SHOC_TR_ORDER2_UW;
+  const bool pos = byvel ? vel > 0.0 : cr > 0.0;
+  if (byvel) val = val && vel != 0.0;
+  int bits = (pos ? F64_POS : 0) | (cr != 0.0 ? F64_MOVE : 0) | (val ? F64_VAL : 0);
+  bool ref = false;
+  f[FC_U * 32] = U;
+  f[FC_CR * 32] = cr;
+  if (SCH == SHOC_TR_QUICKEST || SCH == SHOC_TR_QUICKEST_CO) f[FC_E * 32] = 1.0 - cr * cr;
+  if (SCH == SHOC_TR_VANLEER) f[FC_E * 32] = pos ? 0.5 * (1.0 - cr) : 0.5 * (1.0 + cr);
+  if (SCH == SHOC_TR_QUICKEST) {
+    const double D = pos ? db : df, P = pos ? hm : hp;
+    f[FC_D * 32] = d;
+    f[FC_DB * 32] = D;
+    f[FC_P * 32] = P;
+    f[FC_Q * 32] = h0;
+    ref = far_out<60>(D) || far_out<60>(P) || far_out<60>(h0);
+  }
+  if (SCH == SHOC_TR_ORDER2) f[FC_D * 32] = d;
+  if (lim && cr != 0.0) {
+    const double acr = fabs(cr);
+    f[FC_Y * 32] = 1.0 / acr;
+    bits |= F64_LIM;
+    // by velocity's sign the limiter's upwind side is the scheme's
+    ref = ref || far_out<200>(acr) || acr > 0x1p20 || (byvel && pos != (cr > 0.0));
+  } else {
+    f[FC_Y * 32] = 1.0;
+  }
+  return bits | (ref ? F64_REF : 0);
+}
+
+// The flux by the reference's operations and divisions; of tm2 and tp1 (the
+// values at i-2 and i+1) only the upwind one, tu, is needed but by ORDER4
+template <int SCH, bool ULT>
+__device__ __noinline__ double face_ref64(const double *f, int bits, double tu, double tm1,
+                                          double t0, double tm2, double tp1) {
+  const double cr = f[FC_CR * 32];
+  const bool pos = (bits & F64_POS) != 0;
+  const double vel = (bits & F64_VAL) ? (pos ? 1.0 : -1.0) : 0.0;
+  double v = 0.0;
+  if (SCH == SHOC_TR_QUICKEST) {
+    const double grad = t0 - tm1, tc = pos ? tm1 : t0, td = pos ? t0 : tm1;
+    v = f[FC_D * 32] * grad + tm1;
+    double curv = 0.0;
+    if (bits & F64_MOVE)
+      curv = f[FC_DB * 32] * (f[FC_P * 32] * td + f[FC_Q * 32] * tu) - 2.0 * tc;
+    v = v - 0.5 * cr * grad - f[FC_E * 32] * curv / 6.0;
+  } else if (SCH == SHOC_TR_QUICKEST_CO) {
+    v = quickest_co_face(cr, tu, tm1, t0, tu);
+  } else if (SCH == SHOC_TR_VANLEER) {
+    v = vanleer_face(vel, cr, tu, tm1, t0, tu);
+  } else if (SCH == SHOC_TR_ORDER2 && (bits & F64_VAL)) {
+    v = order2_face(f[FC_D * 32], tm1, t0);
+  } else if (SCH == SHOC_TR_ORDER4 && (bits & F64_VAL)) {
+    v = order4_face(tm2, tm1, t0, tp1);
+  } else if (SCH == SHOC_TR_ORDER2_UW) {
+    v = order2_uw_face(vel, cr, tu, tm1, t0, tu);
+  }
+  if (ULT && (bits & F64_LIM))  // (its unused side's value is not read)
+    v = cr > 0.0 ? ultimate_face(cr, v, SCH == SHOC_TR_ORDER4 ? tm2 : tu, tm1, t0, t0)
+                 : ultimate_face(cr, v, t0, tm1, t0, SCH == SHOC_TR_ORDER4 ? tp1 : tu);
+  return v * f[FC_U * 32];
+}
+
+// The face's flux from the values tm1, t0 beside it and the upwind one beyond
+// them, tu (i-2 for a positive Courant number, i+1 for a negative one; tm2 and
+// tp1, both of them, for ORDER4) (advect: quickest :1870-1884, van_leer_do
+// :2102-2117, the other schemes, then ulimate_filter), without horizontal
+// diffusion, for values in the checked range
+template <int SCH, bool ULT>
+__device__ __forceinline__ double face_flux64(const double *f, int bits, double tu, double tm1,
+                                              double t0, double tm2, double tp1) {
+  if (SCH == SHOC_TR_ORDER1) return order1_flux(f[FC_U * 32], tm1, t0);
+  const bool pos = (bits & F64_POS) != 0, val = (bits & F64_VAL) != 0;
+  const double tc = pos ? tm1 : t0, td = pos ? t0 : tm1;
+  const double diff = td - tu, c = tc - tu, cr = f[FC_CR * 32];
+  double y = 0.0;
+  if (ULT || SCH == SHOC_TR_VANLEER) y = recip(diff);
+  double v;
+  if (SCH == SHOC_TR_QUICKEST) {
+    const double grad = t0 - tm1;
+    v = f[FC_D * 32] * grad + tm1;
+    // (2 tc is exact, so its fused subtraction rounds as the separate one)
+    const double curv =
+        __fma_rn(-2.0, tc, f[FC_DB * 32] * (f[FC_P * 32] * td + f[FC_Q * 32] * tu));
+    const double q = v - 0.5 * cr * grad - quot(f[FC_E * 32] * curv, 6.0, 1.0 / 6.0);
+    v = (bits & F64_MOVE) ? q : v;
+  } else if (SCH == SHOC_TR_QUICKEST_CO) {
+    const double curv = pos ? t0 - 2.0 * tm1 + tu : tu - 2.0 * t0 + tm1;
+    const double w = (bits & F64_MOVE) ? f[FC_E * 32] * curv : 0.0;
+    v = 0.5 * (t0 + tm1) - 0.5 * cr * (t0 - tm1) - quot(w, 6.0, 1.0 / 6.0);
+  } else if (SCH == SHOC_TR_VANLEER) {
+    // with the flow negative the reference's differences, and their quotient,
+    // have the opposite signs, and the value is t0 minus the term
+    const double p = c * (td - tc);
+    const double s = p > 0.0 ? quot(2.0 * p, diff, y) : 0.0;
+    v = val ? tc + f[FC_E * 32] * s : 0.0;
+  } else if (SCH == SHOC_TR_ORDER2) {
+    v = val ? order2_face(f[FC_D * 32], tm1, t0) : 0.0;
+  } else if (SCH == SHOC_TR_ORDER4) {
+    v = val ? quot(7.0 * (tm1 + t0) - (tp1 + tm2), 12.0, 1.0 / 12.0) : 0.0;
+  } else {  // ORDER2_UW
+    v = val ? 0.5 * (3.0 - cr) * tc - 0.5 * (1.0 - cr) * tu : 0.0;
+  }
+  if (ULT) {
+    const double nc = quot(c, diff, y), nu = quot(v - tu, diff, y), acr = fabs(cr);
+    const double ya = f[FC_Y * 32], p = nc * diff;
+    const bool in = nc >= 0.0 && nc <= 1.0;
+    const bool cap = nu > quot(nc, acr, ya);
+    const double up = tu + p, upc = tu + quot(p, acr, ya);
+    double l = cap ? upc : v;
+    l = nu < nc ? up : l;
+    l = nu > 1.0 ? td : l;
+    l = in ? l : up;
+    v = (diff != 0.0 && (bits & F64_LIM)) ? l : v;
+  }
+  return v * f[FC_U * 32];
+}
+
+// A face outside the climb, by the reference's own operations: the east face of
+// a cell whose east neighbour is not the next lane's (maps that join columns
+// out of order), or the bottom face of a column whose floor lies inside a
+// chunk and lets water through
+__device__ __noinline__ double east_flux(const Geo &G, const Flow &F, const Work &W, const Opt &O,
+                                         const Tile &Tl, int c, bool adv, bool hd,
+                                         const double *tr, double dtu) {
+  const int4 n1 = Tl.nb1[c], n2 = Tl.nb2[c];
+  return flux_x(G, F, W, O, (Tl.fl[c] & FL_XP_E1) ? CF_E1 : 0, adv, hd, n1.y, Tl.m2e[c].x,
+                tr[n1.x], tr[c], tr[n1.y], tr[n2.y], dtu);
+}
+__device__ __noinline__ double floor_flux(const Flow &F, const Work &W, const Opt &O, int c,
+                                          int sed, int zp, double t0, double tp1, double dtu) {
+  return flux_z(F, W, O, c, W.w9[sed], W.w9[c], W.w9[zp], t0, t0, t0, tp1, dtu);
+}
+
+// Whether every value of a list lies in 2^-400 .. 2^490 or is 0: differences
+// of such values are 0 or above 2^-453, and the faces' quotients stay inside
+// the range quot takes.  (h - 1 orders a zero high word last; a subnormal
+// below 2^-1042 counts as 0 only where its low word is 0 too.)
+struct ExpCheck {
+  unsigned hi = 0, lo = 0xffffffffu;
+  __device__ __forceinline__ void add(double x) {
+    const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    hi = max(hi, h);
+    lo = min(lo, (h | min((unsigned)__double2loint(x), 1u)) - 1u);
+  }
+  __device__ __forceinline__ bool bad() const {
+    return hi >= ((1023u + 490u) << 20) || lo < ((1023u - 400u) << 20) - 1u;
+  }
+};
+
+constexpr int kAdv64Warps = 1;   // warps of a block (they share nothing)
+constexpr int kAdv64Group = 32;  // tracers whose bottom fluxes a launch row keeps
+constexpr int kAdv64Faces = 4;   // west, south, north, top
+inline size_t adv64_smem(int ng) {
+  return (size_t)kAdv64Warps * (kAdv64Faces * FC_N + ng) * 32 * sizeof(double);
+}
+
+// PLAIN: every advected tracer is advected without horizontal diffusion.
+// Block b: segments kAdv64Warps (b / nch) .., layers [ch L, ch L + L) of chunk
+// ch = b % nch; blockIdx.y: groups of ng tracers.
+template <int SCH, bool ULT, bool PLAIN>
+__global__ void __launch_bounds__(kAdv64Warps * 32, 16)
+    k_adv64(Geo G, Flow F, Work W, Opt O, TrSet T, SubStep ss, Tile Tl,
+            const double *__restrict__ tri, double *__restrict__ tro, double *__restrict__ fzs,
+            int nch, int L, int ng) {
+  extern __shared__ double sAdv[];  // per warp: [kAdv64Faces][FC_N][32], [ng][32]
   constexpr unsigned FULL = 0xffffffffu;
-  __shared__ int sTr[kMaxTracers], sTf[kMaxTracers];
-  const int i = blockIdx.x * kAdvBlock + threadIdx.x;
-  const int lane = threadIdx.x & 31;
-  const int nz = G.nz;
-  for (int s = threadIdx.x; s < T.ntb; s += kAdvBlock) {
-    const int n = T.slot_tr[s];
-    sTr[s] = n;
-    sTf[s] = T.trf[n];
-  }
-  __syncthreads();
+  const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
+  const int seg = (blockIdx.x / nch) * kAdv64Warps + wy;
+  if (seg >= Tl.nseg) return;
+  const int k0 = (blockIdx.x % nch) * L, k1 = min(G.nz, k0 + L);
+  const int sl0 = blockIdx.y * ng, sl1 = min(T.ntb, sl0 + ng);
+  double *const fw = sAdv + (size_t)wy * (kAdv64Faces * FC_N + ng) * 32 + lane;
+  double *const fs = fw + FC_N * 32, *const fn = fs + FC_N * 32, *const ft = fn + FC_N * 32;
+  double *const sF = ft + FC_N * 32;  // the flux through the layer's bottom, per tracer
 
-  int c = 0, col = 0, kb = nz, ks = 0, k = 0, c2 = 0, ntc = 0;
-  if (i < Tl.nwet) {
-    c = Tl.wet[i];
-    col = Tl.colof[c];
-    k = Tl.kof[c];
-    const TileCol tc = tile_column(G, W, Tl, col);
-    if (tc.act) {
-      kb = tc.kb;
-      ks = tc.ks;
-      c2 = tc.c2;
-      ntc = G.colntr[col];
-    } else {
-      c = 0;
-    }
+  const int sc = Tl.seg[seg * 32 + lane];
+  const bool own = sc >= 0 && !(sc & kSegHalo);
+  const int col = sc >= 0 ? (sc & ~kSegHalo) : -1;
+  int kb = G.nz, ks = -1, c2 = 0, ntc = 0;
+  bool staged = false;
+  if (col >= 0) {
+    const int4 r = __ldg(&Tl.colrec[col]);
+    kb = r.z;
+    c2 = r.y;
+    const ColInfo ci = W.col[col];
+    staged = own && (ci.flags & COL_STAGED);
+    ks = ci.ks;
+    ntc = __ldg(&G.colntr[col]);
   }
-  const bool on = c != 0;
-  int4 n1 = make_int4(0, 0, 0, 0), n2 = n1, nzv = n1;
-  int2 me = make_int2(0, 0);
-  int fl = 0;
-  if (on) {
-    n1 = Tl.nb1[c];
-    n2 = Tl.nb2[c];
-    nzv = Tl.nbz[c];
-    me = Tl.m2e[c];
-    fl = Tl.fl[c];
-  }
-  const int cd1 = __shfl_down_sync(FULL, c, 1);
-  const bool sxp1 = on && lane <= 30 && cd1 && n1.y == cd1;
-
-  // tracer-independent face data: Courant numbers and volume fluxes (the
-  // metric factors and work arrays are read per face from cache)
+  if (!__any_sync(FULL, staged)) return;
   const double dtu = ss.dtu;
-  const bool hdf = any_hd != 0;
-  const int xp = n1.y, yp = n1.w, zp = nzv.z, zm = nzv.x;
-  const bool e1 = fl & CF_E1, e2 = fl & CF_E2;
-  const bool ewet = !sxp1 && (fl & FL_XP_WET), nwet = fl & FL_YP_WET;
-  const bool e1e = fl & FL_XP_E1, e2n = fl & FL_YP_E2;
-  double crw = 0.0, crs = 0.0, crn = 0.0, cre = 0.0, czb = 0.0, czt = 0.0;
-  double Uw = 0.0, Us = 0.0, Un = 0.0, Ue = 0.0, wdb = 0.0, wdt = 0.0;
-  const bool zf = on && k <= ks, ztop = on && k < ks;
-  if (on) {
-    // Courant numbers as tracers.c:730-736 (w6, w7, w8)
-    crw = F.u1[c] * dtu / G.h1au1[c2];
-    crs = F.u2[c] * dtu / G.h2au2[c2];
-    Uw = F.u1flux3d[c];
-    Us = F.u2flux3d[c];
-    if (nwet) {
-      crn = F.u2[yp] * dtu / G.h2au2[me.y];
-      Un = F.u2flux3d[yp];
+  const double area = col >= 0 ? __ldg(&G.cellarea[c2]) : 1.0;
+  const double yarea = 1.0 / area;
+  // the bottom face of cell cc (below it zm, above it zp)
+  auto zset = [&](double *f, int cc, int zm, int zp) {
+    const double w9c = W.w9[cc], w = __ldg(&F.w[cc]);
+    return set_face_64<SCH>(f, w * dtu / (w9c * 1.0), w,
+                            (SCH == SHOC_TR_QUICKEST || SCH == SHOC_TR_ORDER2) ? W.w5[cc] : 0.0,
+                            W.dbz[cc], W.dfz[cc], W.w9[zm], w9c, W.w9[zp],
+                            SCH == SHOC_TR_ORDER1 ? w : w * dtu, true, ULT);
+  };
+  // the tracers of this row (at most 32), a lane each
+  const int my_tr = sl0 + lane < sl1 ? __ldg(&T.slot_tr[sl0 + lane]) : 0;
+  // order1's vertical flux (:1611-1616)
+  auto order1_z = [&](double w, double tm1, double t0) {
+    return dtu * (0.5 * (w + fabs(w)) * tm1 + 0.5 * (w - fabs(w)) * t0);
+  };
+
+  // the flux through the bottom of the chunk's first layer, for every tracer
+  {
+    const int c = (staged && k0 >= kb && k0 <= ks) ? __ldg(&Tl.cellk[(size_t)k0 * Tl.ncolp + col])
+                                                   : 0;
+    int4 nzv = make_int4(0, 0, 0, 0);
+    int bits = 0;
+    bool flow = false;  // through a closed floor v * 0
+    if (c) {
+      nzv = __ldg(&Tl.nbz[c]);
+      flow = __ldg(&F.w[c]) * dtu != 0.0;
+      if (flow) bits = zset(ft, c, nzv.x, nzv.z);
     }
-    if (ewet) {
-      cre = F.u1[xp] * dtu / G.h1au1[me.x];
-      Ue = F.u1flux3d[xp];
-    }
-    if (zf) {
-      czb = F.w[c] * dtu / (W.w9[c] * 1.0);
-      wdb = F.w[c] * dtu;
-    }
-    if (ztop) {
-      czt = F.w[zp] * dtu / (W.w9[zp] * 1.0);
-      wdt = F.w[zp] * dtu;
+    const int vm1 = (k0 - 1 >= kb) ? nzv.x : c, vm2 = (k0 - 2 >= kb) ? nzv.y : vm1;
+    for (int s = sl0; s < sl1; ++s) {
+      double Fz = 0.0;
+      const int n = __ldg(&T.slot_tr[s]);
+      if (flow && n < ntc && (PLAIN || (__ldg(&T.trf[n]) & TR_ADV))) {
+        const double *__restrict__ tr = tri + (size_t)n * G.S;
+        const double tm2 = tr[vm2], tm1 = tr[vm1], t0 = tr[c], tp1 = tr[nzv.z];
+        const double tu = (bits & F64_POS) ? tm2 : tp1;
+        ExpCheck ec;
+        ec.add(tu);
+        ec.add(tm1);
+        ec.add(t0);
+        if (SCH == SHOC_TR_ORDER1)
+          Fz = order1_z(ft[FC_U * 32], tm1, t0);
+        else if (ec.bad() || (bits & F64_REF))
+          Fz = face_ref64<SCH, ULT>(ft, bits, tu, tm1, t0, tm2, tp1);
+        else
+          Fz = face_flux64<SCH, ULT>(ft, bits, tu, tm1, t0, tm2, tp1);
+      }
+      sF[(s - sl0) * 32] = Fz;
     }
   }
-  // hor_diffuse (tracers.c:3654-3667): csx = dzu1 h2au1 mdx, then
-  // csx u1kh (t0 - tm1) / h1au1 (the e2 analogue for y)
-  auto Px = [&](int cc, int cc2) { return F.dzu1[cc] * G.h2au1[cc2] * 1.0 * F.u1kh[cc]; };
-  auto Py = [&](int cc, int cc2) { return F.dzu2[cc] * G.h1au2[cc2] * 1.0 * F.u2kh[cc]; };
-  // vertical neighbours (bottom: the sediment ghost holds the bottom value)
-  const int vm1 = (k - 1 >= kb) ? nzv.x : c;
-  const int vm2 = (k - 2 >= kb) ? nzv.y : vm1;
-  const int idx[13] = {c,   n1.z, n2.z, n1.w, n2.w, vm1, vm2,
-                       zp,  nzv.w, n1.x, n2.x, n1.y, n2.y};
-  const int ntb = T.ntb;
 
-  for (int s = 0; s < ntb; ++s) {
-    const int n = sTr[s];
-    const int tf = sTf[s];
-    if (!__any_sync(FULL, on && n < ntc)) continue;  // no lane carries it
-    const bool adv = MODE != 0 || (tf & TR_ADV);
-    const bool hd = MODE == 2 || (MODE == 0 && (tf & TR_HDIFF));
-    const double *__restrict__ tr = tri + (size_t)n * G.S;
-    double v[13];
+  for (int k = k0; k < k1; ++k) {
+    const int c = (col >= 0 && k >= kb) ? __ldg(&Tl.cellk[(size_t)k * Tl.ncolp + col]) : 0;
+    const bool on = c != 0, st = on && staged;
+    if (!__any_sync(FULL, st)) continue;
+    int4 n1 = make_int4(0, 0, 0, 0), n2 = n1, nzv = n1;
+    int2 me = make_int2(0, 0);
+    int fl = 0;
+    if (on) {
+      n1 = __ldg(&Tl.nb1[c]);
+      n2 = __ldg(&Tl.nb2[c]);
+      nzv = __ldg(&Tl.nbz[c]);
+      me = __ldg(&Tl.m2e[c]);
+      fl = __ldg(&Tl.fl[c]);
+    }
+    const int cd1 = __shfl_down_sync(FULL, c, 1);
+    const bool sxp = on && lane < 31 && cd1 && n1.y == cd1;
+    const bool nwet = (fl & FL_YP_WET) != 0;
+    const bool eslow = st && !sxp && (SCH == SHOC_TR_ORDER1 || (fl & FL_XP_WET));
+    const bool below = k < ks;  // interior cell: its top face is in the water
+
+    int bw = 0, bs = 0, bn = 0, bt = 0;
+    double ydz = 0.0, dzc = 1.0;
+    unsigned rng = kDivNever;
+    if (on) {
+      const Face2D mx = G.fx[c2];
+      const double h = __ldg(&G.h1au1[c2]), u = __ldg(&F.u1[c]);
+      const bool e1 = fl & CF_E1;
+      bw = set_face_64<SCH>(fw, u * dtu / h, u, mx.d, mx.db, mx.df, mx.hm, mx.h0, mx.hp,
+                            __ldg(&F.u1flux3d[c]), e1, ULT && e1);
+    }
+    if (st) {
+      const Face2D my = G.fy[c2];
+      const double h = __ldg(&G.h2au2[c2]), u = __ldg(&F.u2[c]);
+      const bool e2 = fl & CF_E2;
+      bs = set_face_64<SCH>(fs, u * dtu / h, u, my.d, my.db, my.df, my.hm, my.h0, my.hp,
+                            __ldg(&F.u2flux3d[c]), e2, ULT && e2);
+      if (nwet || SCH == SHOC_TR_ORDER1) {  // order1 fills the ghost cells' faces too
+        const int yp = n1.w;
+        const Face2D mn = G.fy[me.y];
+        const double hn = nwet ? __ldg(&G.h2au2[me.y]) : 1.0, un = __ldg(&F.u2[yp]);
+        const bool e2n = fl & FL_YP_E2;
+        bn = set_face_64<SCH>(fn, un * dtu / hn, un, mn.d, mn.db, mn.df, mn.hm, mn.h0, mn.hp,
+                              __ldg(&F.u2flux3d[yp]), e2n, ULT && e2n);
+      } else {
+        fn[FC_U * 32] = 0.0;
+      }
+      if (below)
+        bt = zset(ft, nzv.z, c, nzv.w);  // the bottom face of the cell above
+      else
+        ft[FC_U * 32] = 0.0;
+      dzc = W.dz[c];
+      ydz = 1.0 / dzc;
+      rng = div_range(dzc) == kDivLo && div_range(area) == kDivLo ? kDivLo : kDivNever;
+    }
+    const int refs = (bw | bs | bn | bt) & F64_REF;
+    // vertical neighbour (bottom: the sediment ghost holds the bottom value,
+    // tracers.c:827-830)
+    const int vm1 = (k - 1 >= kb) ? nzv.x : c;
+    // the upwind value beyond each face: one load instead of two and a choice
+    const int uw = (bw & F64_POS) ? n2.x : n1.y, us = (bs & F64_POS) ? n2.z : n1.w;
+    const int un = (bn & F64_POS) ? n1.z : n2.w, ut = (bt & F64_POS) ? vm1 : nzv.w;
+    // the floor inside the chunk: where it lets water through
+    const bool fbot = k == kb && k > k0;
+    const bool fslow = st && fbot && k <= ks && __ldg(&F.w[c]) * dtu != 0.0;
+
+    // the next tracer's stencil values are loaded while this one is computed
+    constexpr int NV = 9;
+    const int idx[NV] = {c, n1.x, n1.z, n1.w, nzv.z, uw, us, un, ut};
+    double nv[NV];
+    int nn = __shfl_sync(FULL, my_tr, 0), nn2 = __shfl_sync(FULL, my_tr, 1);
+    auto fetch = [&](int n) {
+      const double *__restrict__ p = tri + (size_t)n * G.S;
 #pragma unroll
-    for (int q = 0; q < 13; ++q) v[q] = tr[idx[q]];
-    const double t0 = v[0];
-    const double tym1 = v[1], tym2 = v[2], typ1 = v[3], typ2 = v[4];
-    const double tm1 = v[5], tm2 = v[6], tp1 = v[7], tp2 = v[8];
-    const double txm1 = v[9], txm2 = v[10], txp1 = v[11], txp2 = v[12];
-    const bool hor = adv || hd;
-    double Fxw = 0.0, Fys = 0.0, Fyn = 0.0, Fxe = 0.0;
-    if (on && hor) {
-      const bool h = hdf && hd;
-      Fxw = hface64<QUICK, ULT>(e1, adv, hd, crw, F.u1[c], G.fx[c2], Uw, h ? Px(c, c2) : 0.0,
-                                G.h1au1[c2], txm2, txm1, t0, txp1);
-      Fys = hface64<QUICK, ULT>(e2, adv, hd, crs, F.u2[c], G.fy[c2], Us, h ? Py(c, c2) : 0.0,
-                                G.h2au2[c2], tym2, tym1, t0, typ1);
-      if (nwet)
-        Fyn = hface64<QUICK, ULT>(e2n, adv, hd, crn, F.u2[yp], G.fy[me.y], Un,
-                                  h ? Py(yp, me.y) : 0.0, G.h2au2[me.y], tym1, t0, typ1, typ2);
-      if (ewet)
-        Fxe = hface64<QUICK, ULT>(e1e, adv, hd, cre, F.u1[xp], G.fx[me.x], Ue,
-                                  h ? Px(xp, me.x) : 0.0, G.h1au1[me.x], txm1, t0, txp1, txp2);
+      for (int q = 0; q < NV; ++q) nv[q] = p[idx[q]];
+    };
+    fetch(nn);
+    for (int s = sl0; s < sl1; ++s) {
+      const int n = nn;
+      const double t0 = nv[0], txm1 = nv[1], tym1 = nv[2], typ1 = nv[3], tp1 = nv[4];
+      const double tuw = nv[5], tus = nv[6], tun = nv[7], tut = nv[8];
+      if (s + 1 < sl1) {
+        nn = nn2;
+        nn2 = __shfl_sync(FULL, my_tr, (s + 2 - sl0) & 31);
+        fetch(nn);
+      }
+      if (!__any_sync(FULL, st && n < ntc)) continue;  // no lane carries it
+      const int tf = PLAIN ? TR_ADV : __ldg(&T.trf[n]);
+      const bool adv = PLAIN || (tf & TR_ADV), hd = !PLAIN && (tf & TR_HDIFF);
+      const double *__restrict__ tr = tri + (size_t)n * G.S;
+      double txm2 = 0.0, txp1 = 0.0, tym2 = 0.0, typ2 = 0.0, tm1 = 0.0, tp2 = 0.0;
+      if (SCH == SHOC_TR_ORDER4) {  // both values beyond each face
+        txm2 = tr[n2.x];
+        txp1 = tr[n1.y];
+        tym2 = tr[n2.z];
+        typ2 = tr[n2.w];
+        tm1 = tr[vm1];
+        tp2 = tr[nzv.w];
+      }
+      double Fxw = 0.0, Fys = 0.0, Fyn = 0.0, Fzt = 0.0;
+      if (adv) {
+        // (faces a lane does not have hold whatever their factors give: they
+        // are not used)
+        Fxw = face_flux64<SCH, ULT>(fw, bw, tuw, txm1, t0, txm2, txp1);
+        Fys = face_flux64<SCH, ULT>(fs, bs, tus, tym1, t0, tym2, typ1);
+        Fyn = face_flux64<SCH, ULT>(fn, bn, tun, t0, typ1, tym1, typ2);
+        Fzt = SCH == SHOC_TR_ORDER1 ? order1_z(ft[FC_U * 32], t0, tp1)
+                                    : face_flux64<SCH, ULT>(ft, bt, tut, t0, tp1, tm1, tp2);
+        if (SCH != SHOC_TR_ORDER1) {
+          ExpCheck ec;
+          ec.add(t0);
+          ec.add(txm1);
+          ec.add(tym1);
+          ec.add(typ1);
+          ec.add(tp1);
+          ec.add(tuw);
+          ec.add(tus);
+          ec.add(tun);
+          ec.add(tut);
+          if (SCH == SHOC_TR_ORDER4) {
+            ec.add(txm2);
+            ec.add(txp1);
+            ec.add(tym2);
+            ec.add(typ2);
+            ec.add(tm1);
+            ec.add(tp2);
+          }
+          if (ec.bad() || refs) {
+            if (on) Fxw = face_ref64<SCH, ULT>(fw, bw, tuw, txm1, t0, txm2, txp1);
+            if (st) {
+              Fys = face_ref64<SCH, ULT>(fs, bs, tus, tym1, t0, tym2, typ1);
+              if (nwet) Fyn = face_ref64<SCH, ULT>(fn, bn, tun, t0, typ1, tym1, typ2);
+              if (below) Fzt = face_ref64<SCH, ULT>(ft, bt, tut, t0, tp1, tm1, tp2);
+            }
+          }
+        }
+      }
+      if (hd && on) {
+        // hor_diffuse (tracers.c:3654-3667): csx = dzu1 h2au1 mdx, then
+        // csx u1kh (t0 - tm1) / h1au1 (the e2 analogue for y)
+        Fxw -= F.dzu1[c] * G.h2au1[c2] * 1.0 * F.u1kh[c] * (t0 - txm1) / G.h1au1[c2];
+        if (st) {
+          Fys -= F.dzu2[c] * G.h1au2[c2] * 1.0 * F.u2kh[c] * (t0 - tym1) / G.h2au2[c2];
+          if (nwet) {
+            const int yp = n1.w;
+            Fyn -= F.dzu2[yp] * G.h1au2[me.y] * 1.0 * F.u2kh[yp] * (typ1 - t0) / G.h2au2[me.y];
+          }
+        }
+      }
+      double Fxe = __shfl_down_sync(FULL, Fxw, 1);
+      if (!st || n >= ntc) continue;
+      if (!sxp) Fxe = 0.0;
+      if (SCH != SHOC_TR_ORDER1 && !nwet) Fyn = 0.0;
+      if (eslow) {
+        if (fl & FL_XP_WET)
+          Fxe = east_flux(G, F, W, O, Tl, c, adv, hd, tr, dtu);
+        else if (adv)
+          Fxe = order1_flux(F.u1flux3d[n1.y], t0, tr[n1.y]);
+      }
+      // dtracer (tracers.c:888-892)
+      const double dtr = (Fxe - Fxw + Fyn - Fys) * dtu;
+      double val = dtr;
+      if (k <= ks) {
+        double Fzb = 0.0;
+        if (!fbot)
+          Fzb = sF[(s - sl0) * 32];
+        else if (fslow && adv)
+          Fzb = floor_flux(F, W, O, c, nzv.x, nzv.z, t0, tp1, dtu);
+        if (below) {
+          sF[(s - sl0) * 32] = Fzt;
+          // interior cell (tracers.c:912-925); Ds = Hn1 = 1 in z coordinates
+          val = t0 - div_known(div_known(dtr, area, yarea, rng) + (Fzt - Fzb), dzc, ydz, rng);
+        } else {
+          fzs[(size_t)n * G.ncol + col] = Fzb;
+        }
+      }
+      tro[(size_t)n * G.S + c] = val;
     }
-    const double Fnext = __shfl_down_sync(FULL, Fxw, 1);
-    if (!on || n >= ntc) continue;
-    if (sxp1) Fxe = Fnext;
-    // dtracer (tracers.c:888-892)
-    const double dtr = (Fxe - Fxw + Fyn - Fys) * dtu;
-    double val;
-    if (ztop) {
-      // interior cell (tracers.c:912-925); Ds = Hn1 = 1 in z coordinates
-      const double Fzb =
-          adv ? zface64<QUICK, ULT>(F, W, c, zm, zp, czb, wdb, tm2, tm1, t0, tp1) : 0.0;
-      const double Fzt =
-          adv ? zface64<QUICK, ULT>(F, W, zp, c, nzv.w, czt, wdt, tm1, t0, tp1, tp2) : 0.0;
-      double a = t0 * 1.0;
-      a -= ((dtr / G.cellarea[c2] + (Fzt - Fzb)) / W.dz[c]);
-      a /= 1.0;
-      val = a;
-    } else {
-      val = dtr;
-      if (k == ks)
-        fzs[(size_t)n * G.ncol + col] =
-            adv ? zface64<QUICK, ULT>(F, W, c, zm, zp, czb, wdb, tm2, tm1, t0, tp1) : 0.0;
-    }
-    tro[(size_t)n * G.S + c] = val;
   }
 }
 
 // ---------------------------------------------------------------------------
 // k_vd64
+//
+// One thread per (column, tracer), a warp per 32 columns of one tracer.  What
+// bounds it: the serial chain of the Thomas sweeps (memory is 16 bytes a
+// value).  The forward sweep's IEEE division was most of the chain: the
+// divisor does not depend on the tracer, so k_set_dz stores its reciprocal and
+// div_known takes five dependent operations.  The advected values are copied
+// to shared memory in one batch of asynchronous copies and replaced by the
+// forward sweep's row by row; the back substitution reads them again (from
+// L2), so a warp keeps one array instead of two and twice the warps fit.
+// Columns whose surface crosses layer faces during the step run here too: the
+// cells from the lower of the old and new surface cells up to the old one add
+// to the surface balance, and the solve runs up to the new one.
 
 template <bool LAST>
 __global__ void __launch_bounds__(256) k_vd64(Geo G, Flow F, Work W, Opt O, TrSet T,
@@ -230,12 +568,12 @@ __global__ void __launch_bounds__(256) k_vd64(Geo G, Flow F, Work W, Opt O, TrSe
                                               const double *__restrict__ vdzdt,
                                               const double *__restrict__ vcm1,
                                               const double *__restrict__ vdiv,
+                                              const double *__restrict__ vrdiv,
                                               const double *__restrict__ vud, int nw,
                                               int nchunk, int tile0, int kbase) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int nz = G.nz, nd = nz - kbase;
-  double *A = reinterpret_cast<double *>(smem);          // [nd][nw][32]
-  double *Sv = A + nd * nw * 32;                         // [nd][nw][32]
+  double *Sv = reinterpret_cast<double *>(smem);           // [nd][nw][32]
   int *colC = reinterpret_cast<int *>(Sv + nd * nw * 32);  // [nd][32]
 
   const int lane = threadIdx.x, wy = threadIdx.y;
@@ -268,106 +606,107 @@ __global__ void __launch_bounds__(256) k_vd64(Geo G, Flow F, Work W, Opt O, TrSe
   const bool solve = vdf && !single;
   const double *tr = tri + (size_t)n * G.S;
   double *to = tro + (size_t)n * G.S;
-  double *const A0 = A + (kb - kbase) * sa + wy * 32 + lane;
+  // the column: advection results (advected tracers) or the old values
+  const double *src = tbdy ? to : tr;
   double *const S0 = Sv + (kb - kbase) * sa + wy * 32 + lane;
   const int *const C0 = colC + (kb - kbase) * 32 + lane;
   const int nk = ks - kb, nl = nz - kb;
-  {  // the column: advection results (advected tracers) or the old values
-    const double *src = tbdy ? to : tr;
-    for (int j = 0; j < nl; ++j) cp_async8(&A0[j * sa], src + C0[j * 32]);
-    cp_async_commit();
-  }
+  for (int j = 0; j < nl; ++j) cp_async8(&S0[j * sa], src + C0[j * 32]);
+  cp_async_commit();
   const double mn = T.mintr[n], mx = T.maxtr[n];
   {  // sediment ghost (tracers.c:827-830)
     const int sed = G.zm1[cbot];
     to[sed] = tbdy ? tr[cbot] : tr[sed];
   }
-  const int cs = ci.s;  // the surface cell (= old and new surface)
-  const double ts_old = tr[cs];
+  // s: the lower of the old (co) and new (cs) surface cells
+  const int cell_s = ci.s, cs = ci.cs;
+  const int nc = (cs == cell_s) ? nk : G.kof[cs] - kb;        // rows up to the new surface
+  const int no = (ci.co == cell_s) ? nk : G.kof[ci.co] - kb;  // up to the old one
+  const double ts_old = tr[cell_s];
   const double area = G.cellarea[c2];
   cp_async_wait<0>();
 
   unsigned long long nwarn = 0;
   int stat = 0;
   double solp = 0.0;
+  const bool clip = mn <= kClipEps;
+  // row j of the forward sweep (:4185-4196) for the value a
+  auto forward = [&](int j, double a) {
+    const int cc = C0[j * 32];
+    const double div = __ldg(&vdiv[cc]), y = __ldg(&vrdiv[cc]);
+    double rhs = __ldg(&vdzdt[cc]) * a;
+    if (j == 0) {
+      rhs = rhs + 0.0;
+    } else {
+      if (j == nc) rhs = rhs - 0.0;
+      rhs = rhs - __ldg(&vcm1[cc]) * solp;
+    }
+    solp = div_known(rhs, div, y, __double2hiint(y) ? kDivLo : kDivNever);
+    S0[j * sa] = solp;
+  };
+  double vs = ts_old;
   if (!tbdy) {
     // tracers without advection / diffusion keep their values, then diffuse
     for (int j = 0; j < nl; ++j) {
-      to[C0[j * 32]] = A0[j * sa];
-      if (isnan(A0[j * sa])) stat |= ST_NAN;
+      const double a = S0[j * sa];
+      to[C0[j * 32]] = a;
+      if (isnan(a)) stat |= ST_NAN;
     }
     if (vdf && single) {
       const double h = W.dz[cs] > O.hmin ? W.dz[cs] : O.hmin;
-      const double v = A0[nk * sa];
+      const double v = S0[nc * sa];
       to[cs] = v + F.dt * (0.0 - 0.0) / h;
     } else if (solve) {
 #pragma unroll 4
-      for (int j = 0; j <= nk; ++j) {
-        const int cc = C0[j * 32];
-        double rhs = __ldg(&vdzdt[cc]) * A0[j * sa];
-        double sl;
-        if (j == 0) {
-          rhs = rhs + 0.0;
-          sl = rhs / __ldg(&vdiv[cc]);
-        } else {
-          if (j == nk) rhs = rhs - 0.0;
-          sl = (rhs - __ldg(&vcm1[cc]) * solp) / __ldg(&vdiv[cc]);
-        }
-        S0[j * sa] = sl;
-        solp = sl;
-      }
+      for (int j = 0; j <= nc; ++j) forward(j, S0[j * sa]);
     }
   } else {
-    double a_below = 0.0;
-#pragma unroll 4
-    for (int j = 0; j < nk; ++j) {
-      const int cc = C0[j * 32];
-      double a = A0[j * sa];
-      if (j == nk - 1) a_below = a;
-      // tr_bounds clip and range check (:3278-3293)
-      if (mn <= kClipEps && a < mn) a = mn;
-      if (a < mn || a > mx) nwarn++;
-      if (isnan(a)) stat |= ST_NAN;
-      if (solve) {
-        A0[j * sa] = a;
-        double rhs = __ldg(&vdzdt[cc]) * a;
-        double sl;
-        if (j == 0) {
-          rhs = rhs + 0.0;
-          sl = rhs / __ldg(&vdiv[cc]);
-        } else {
-          sl = (rhs - __ldg(&vcm1[cc]) * solp) / __ldg(&vdiv[cc]);
-        }
-        S0[j * sa] = sl;
-        solp = sl;
-      } else {
-        to[cc] = a;
-      }
-    }
-    // surf_conc with s == co (tracers.c:3097-3206)
-    double vs = ts_old;
+    // surf_conc's balance (tracers.c:3097-3206), before the sweep replaces
+    // the divergences at and above s
+    double sv = 0.0;
     if (adv) {
       const double Fzb = fzs[(size_t)n * G.ncol + col];
       const double fcbot = -Fzb * area;
       double surftr = -fcbot;
-      const double wbot = (cs == cbot) ? G.botz[c2] : G.gridz[cs];
+      double wbot = (cell_s == cbot) ? G.botz[c2] : G.gridz[cell_s];
       const double eta = F.eta[c2], oe = F.oldeta[c2];
       const double sub = oe + ss.subeta_f * (eta - oe);
       const double osub = ss.first ? oe : oe + ss.osub_f * (eta - oe);
       const double dzs = sub - wbot;
       const double svol = dzs * area;
-      surftr += (ts_old * area * (osub - wbot) - A0[nk * sa]);
-      for (int j = nk + 1; j < nl; ++j) surftr -= (A0[j * sa]);
-      double sv;
+      double t0 = ts_old;
+      int j = nk;
+      for (; j < no; ++j) {  // cells the old surface was above
+        const double wtop = G.gridz[C0[(j + 1) * 32]];
+        surftr += (t0 * area * (wtop - wbot) - S0[j * sa]);
+        wbot = wtop;
+        t0 = tr[C0[(j + 1) * 32]];
+      }
+      const double wb = (ci.co == cbot) ? G.botz[c2] : G.gridz[ci.co];
+      surftr += (t0 * area * (osub - wb) - S0[j * sa]);
+      for (++j; j < nl; ++j) surftr -= (S0[j * sa]);
       if (svol == 0.0 || (surftr < 0.0 && dzs <= O.hmin))
         sv = 0.0;
       else
         sv = surftr / svol;
-      vs = (G.botz[c2] > 0.0 && W.dz[cs] < O.hmin) ? ts_old : sv;
+      vs = (G.botz[c2] > 0.0 && W.dz[cell_s] < O.hmin) ? ts_old : sv;
+    }
+    double a_below = nk > 0 ? S0[(nk - 1) * sa] : 0.0;
+#pragma unroll 4
+    for (int j = 0; j < nk; ++j) {
+      double a = S0[j * sa];
+      // tr_bounds clip and range check (:3278-3293)
+      if (clip && a < mn) a = mn;
+      if (a < mn || a > mx) nwarn++;
+      if (isnan(a)) stat |= ST_NAN;
+      if (solve)
+        forward(j, a);
+      else
+        to[C0[j * 32]] = a;
     }
     // tr_bounds thin-surface fix (:3250-3272); the cursor cannot move here
     if ((ci.flags & COL_THIN) && (vs < mn || vs > mx)) vs = a_below;
-    if (mn <= kClipEps && vs < mn) vs = mn;
+    if (clip && vs < mn) vs = mn;
     if (vs < mn || vs > mx) nwarn++;
     if (isnan(vs)) stat |= ST_NAN;
     for (int j = nk; j < nl; ++j) to[C0[j * 32]] = vs;
@@ -375,36 +714,44 @@ __global__ void __launch_bounds__(256) k_vd64(Geo G, Flow F, Work W, Opt O, TrSe
       const double h = W.dz[cs] > O.hmin ? W.dz[cs] : O.hmin;
       to[cs] = vs + F.dt * (0.0 - 0.0) / h;
     } else if (solve) {
-      A0[nk * sa] = vs;
-      double rhs = __ldg(&vdzdt[cs]) * vs;
-      double sl;
-      if (nk == 0) {
-        rhs = rhs + 0.0;
-        sl = rhs / __ldg(&vdiv[cs]);
-      } else {
-        rhs = rhs - 0.0;
-        sl = (rhs - __ldg(&vcm1[cs]) * solp) / __ldg(&vdiv[cs]);
-      }
-      S0[nk * sa] = sl;
+      for (int j = nk; j <= nc; ++j) forward(j, vs);
     }
   }
   if (solve) {
-    // back substitution and update (:4197-4205)
-    double x = S0[nk * sa];
-    double a = A0[nk * sa];
+    // back substitution and update (:4197-4205); a: the value before the solve
+    auto before = [&](int j) {
+      if (tbdy && j >= nk) return vs;
+      double a = src[C0[j * 32]];
+      if (tbdy && clip && a < mn) a = mn;
+      return a;
+    };
+    double x = S0[nc * sa];
+    double a = before(nc);
     double fin = a + (x - a) * 1.0;
-    to[cs] = fin;
     if (isnan(fin)) stat |= ST_NAN;
     double udp = __ldg(&vud[cs]);
-#pragma unroll 4
-    for (int j = nk - 1; j >= 0; --j) {
-      const int cc = C0[j * 32];
-      x = S0[j * sa] - udp * x;
-      a = A0[j * sa];
-      fin = a + (x - a) * 1.0;
-      to[cc] = fin;
-      if (isnan(fin)) stat |= ST_NAN;
-      udp = __ldg(&vud[cc]);
+    // the values of kBack rows are read ahead of the rows they replace
+    constexpr int kBack = 4;
+    to[cs] = fin;
+    for (int j0 = nc - 1; j0 >= 0; j0 -= kBack) {
+      double av[kBack], uv[kBack];
+      int cv[kBack];
+#pragma unroll
+      for (int q = 0; q < kBack; ++q) {
+        const int j = max(j0 - q, 0);
+        cv[q] = C0[j * 32];
+        av[q] = before(j);
+        uv[q] = __ldg(&vud[cv[q]]);
+      }
+#pragma unroll
+      for (int q = 0; q < kBack; ++q) {
+        if (j0 - q < 0) break;
+        x = S0[(j0 - q) * sa] - udp * x;
+        const double f = av[q] + (x - av[q]) * 1.0;
+        to[cv[q]] = f;
+        if (isnan(f)) stat |= ST_NAN;
+        udp = uv[q];
+      }
     }
   }
   if (nwarn) atomicAdd(W.nwarn, nwarn);

@@ -1,0 +1,69 @@
+"""The FP64 kernels at the edges of their tiles, bitwise against the oracle.
+
+A warp of the advection kernel holds up to 32 neighbouring columns (the last
+one only lending its west flux) and a chunk of layers; the column kernel 32
+columns of one tracer.  Windows just below, at and above those sizes, one
+tracer to more than a launch row of them, one layer to many, and tracers whose
+values leave the range in which quotients are formed from reciprocals and the
+limiter's cases from products.  Tolerance: none, the results are the
+reference's bits.
+"""
+import numpy as np
+import pytest
+
+import oracle
+from ems_b200 import _abi, gpu, synth
+
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("need_gpu")]
+
+
+def window(nx, ny, nz, ntr, **kw):
+    d = dict(seed=91, ntr=ntr, depth=(3.0, 5.0 * nz - 1.0), land_frac=0.15, cell=(400.0, 900.0),
+             curvilinear=True, umax=0.8, kz=("logu", 1e-5, 1e-1), tracers=("logn", 1e-2, 10.0))
+    d.update(kw)
+    layers = d.pop("layers", synth.uniform_layers(nz, 5.0 * nz))
+    return synth.build_case("edge", nx, ny, layers, **d)
+
+
+def check(case, nsteps=3):
+    t = gpu.TracerStep(case)
+    t.start()
+    t.run(nsteps)
+    t.sync()
+    tr = t.download()
+    sur, nsur = t.surface()
+    t.close()
+    rc, ref, rsur, rnsur, _ = oracle.run_oracle(case, nsteps)
+    assert rc == 0
+    np.testing.assert_array_equal(tr[:, 1:], ref[:, 1:])
+    np.testing.assert_array_equal(sur, rsur)
+    np.testing.assert_array_equal(nsur, rnsur)
+
+
+@pytest.mark.parametrize("nx,ny,nz,ntr", [
+    (30, 9, 7, 2), (31, 9, 7, 2), (32, 9, 7, 2), (33, 9, 7, 2), (63, 5, 2, 3), (64, 5, 9, 1),
+    (9, 40, 40, 5), (97, 6, 128, 1), (40, 12, 5, 70)])
+def test_sizes(nx, ny, nz, ntr):
+    check(window(nx, ny, nz, ntr))
+
+
+@pytest.mark.parametrize("scheme,ultimate", [(_abi.QUICKEST, 1), (_abi.QUICKEST, 0),
+                                             (_abi.VANLEER, 1), (_abi.VANLEER, 0)])
+@pytest.mark.parametrize("hdiff", [None, (40.0, [1, 0, 1])])
+def test_crossing_surface(scheme, ultimate, hdiff):
+    """The surface moves through layer faces at -1.0 and 0.6 m."""
+    layers = np.array([-30.0, -22.0, -14.0, -8.0, -3.0, -1.0, 0.6, 2.5])
+    check(window(45, 20, 7, 3, layers=layers, depth=(4.0, 29.0), eta_offset=(1.9, -1.7),
+                 trasc=scheme, ultimate=ultimate, hdiff=hdiff), nsteps=4)
+
+
+@pytest.mark.parametrize("scale", [1e-308, 1e-290, 1e-160, 1e-120, 1e120, 1e160, 1e290])
+def test_extreme_values(scale):
+    """Every other tracer holds zeros, equal neighbours and sign changes too."""
+    case = window(40, 12, 6, 4)
+    c = case.win.wet_cells()
+    case.tr *= scale
+    case.tr[1, c[::3]] = 0.0
+    case.tr[2, c] = np.where(c % 5 < 2, -case.tr[2, c], case.tr[2, c])
+    case.tr[3, c] = scale * (c % 2)
+    check(case)
