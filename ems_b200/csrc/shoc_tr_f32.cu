@@ -12,18 +12,17 @@ cudaError_t attr(K k, int bytes = 227 * 1024) {
   return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
-template <bool Q, bool U, int M>
+template <bool Q, bool U, bool P>
 void adv(int grid, cudaStream_t st, const Geo &G, const Flow32 &F3, const Work &W, const TrSet &T,
          const SubStep &ss, const Tile &Tl, const f32::Face2 *fx2, const f32::Face2 *fy2,
          const float *tin, float *tout, float *rnd, double *fzs, int hd,
          const int16_t *loi) {
-  const size_t sm = M != 0 ? kAdvSmem : 0;
   if (loi)
-    k_adv32<Q, U, M, true><<<grid, kAdv32Block, sm, st>>>(G, F3, W, T, ss, Tl, fx2, fy2, tin,
-                                                          tout, rnd, fzs, hd, loi);
+    k_adv32<Q, U, P, true><<<grid, kAdv32Block, kAdvSmem, st>>>(G, F3, W, T, ss, Tl, fx2, fy2,
+                                                                tin, tout, rnd, fzs, hd, loi);
   else
-    k_adv32<Q, U, M, false><<<grid, kAdv32Block, sm, st>>>(G, F3, W, T, ss, Tl, fx2, fy2, tin,
-                                                           tout, rnd, fzs, hd, nullptr);
+    k_adv32<Q, U, P, false><<<grid, kAdv32Block, kAdvSmem, st>>>(
+        G, F3, W, T, ss, Tl, fx2, fy2, tin, tout, rnd, fzs, hd, nullptr);
 }
 template <bool Q, bool U>
 void adv_mode(int mode, int grid, cudaStream_t st, const Geo &G, const Flow32 &F3,
@@ -31,30 +30,19 @@ void adv_mode(int mode, int grid, cudaStream_t st, const Geo &G, const Flow32 &F
               const f32::Face2 *fx2, const f32::Face2 *fy2, const float *tin, float *tout,
               float *rnd, double *fzs, int hd, const int16_t *loi) {
   if (mode == 1)
-    adv<Q, U, 1>(grid, st, G, F3, W, T, ss, Tl, fx2, fy2, tin, tout, rnd, fzs, hd, loi);
-  else if (mode == 2)
-    adv<Q, U, 2>(grid, st, G, F3, W, T, ss, Tl, fx2, fy2, tin, tout, rnd, fzs, hd, loi);
+    adv<Q, U, true>(grid, st, G, F3, W, T, ss, Tl, fx2, fy2, tin, tout, rnd, fzs, hd, loi);
   else
-    adv<Q, U, 0>(grid, st, G, F3, W, T, ss, Tl, fx2, fy2, tin, tout, rnd, fzs, hd, loi);
+    adv<Q, U, false>(grid, st, G, F3, W, T, ss, Tl, fx2, fy2, tin, tout, rnd, fzs, hd, loi);
 }
 }  // namespace
 
 cudaError_t tile32_set_smem_attr() {
   cudaError_t e = cudaSuccess;
-  const int a = (int)kAdvSmem;
-  const cudaError_t r[24] = {
-      attr(k_vd32<true, false, false>),  attr(k_vd32<false, false, false>),
-      attr(k_vd32<true, true, false>),   attr(k_vd32<false, true, false>),
-      attr(k_vd32<true, false, true>),   attr(k_vd32<false, false, true>),
-      attr(k_vd32<true, true, true>),    attr(k_vd32<false, true, true>),
-      attr(k_adv32<true, true, 1, false>, a), attr(k_adv32<true, true, 2, false>, a),
-      attr(k_adv32<true, false, 1, false>, a), attr(k_adv32<true, false, 2, false>, a),
-      attr(k_adv32<false, true, 1, false>, a), attr(k_adv32<false, true, 2, false>, a),
-      attr(k_adv32<false, false, 1, false>, a), attr(k_adv32<false, false, 2, false>, a),
-      attr(k_adv32<true, true, 1, true>, a), attr(k_adv32<true, true, 2, true>, a),
-      attr(k_adv32<true, false, 1, true>, a), attr(k_adv32<true, false, 2, true>, a),
-      attr(k_adv32<false, true, 1, true>, a), attr(k_adv32<false, true, 2, true>, a),
-      attr(k_adv32<false, false, 1, true>, a), attr(k_adv32<false, false, 2, true>, a)};
+  const cudaError_t r[8] = {
+      attr(k_vd32<true, false, false>), attr(k_vd32<false, false, false>),
+      attr(k_vd32<true, true, false>),  attr(k_vd32<false, true, false>),
+      attr(k_vd32<true, false, true>),  attr(k_vd32<false, false, true>),
+      attr(k_vd32<true, true, true>),   attr(k_vd32<false, true, true>)};
   for (auto x : r)
     if (x != cudaSuccess) e = x;
   return e;

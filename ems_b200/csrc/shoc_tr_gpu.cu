@@ -424,7 +424,10 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
   ci.cbs = cbs;
   ci.flags = flags;
   ci.ks = kb + js - 1;
-  const bool staged = on && O.tiled && staged_column(ci, bot, O.cross != 0);
+  // (k_adv64 takes floors as closed: a column whose floor lets water through
+  // goes the general path)
+  const bool staged = on && O.tiled && staged_column(ci, bot, O.cross != 0) &&
+                      !(O.cross && F.w[bot] != 0.0);
   if (staged) ci.flags |= COL_STAGED;
   if (wy == 0) {
     if (solve) {
@@ -1002,24 +1005,37 @@ int build_tile_tables(shoc_tr_gpu *h, const shoc_tr_geom *g, const std::vector<u
       const int c = cellk[(size_t)k * ncolp + col];
       if (c) colof[c] = col;
     }
-  // k_adv32 cell order: tile by tile (32 adjacent columns), layer by layer
-  // within a tile, so the vertical and y-neighbours a block reads were read
+  // k_adv32 cell order: segment by segment (up to 31 adjacent columns), layer by
+  // layer within one, so the vertical and y-neighbours a block reads were read
   // by blocks shortly before it (cache reuse) and a warp's cells are mostly
-  // adjacent cells of one layer
+  // adjacent cells of one layer.  A cell's east neighbour, where it is wet, is
+  // the next lane's: a run that goes on beyond the segment, or beyond a warp's
+  // last lane, is given a halo lane there.
   std::vector<uint8_t> is_wet(S, 0);
   for (int i = 1; i <= g->a3_t; i++) {
     const int c = g->w3_t[i];
     if (c > 0 && c < S) is_wet[c] = 1;
   }
   std::vector<int> wet;
-  wet.reserve(g->a3_t);
-  for (int t = 0; t < ncolp / 32; t++)
+  wet.reserve((size_t)g->a3_t + g->a3_t / 16);
+  for (int col0 = 0; col0 < ncol; col0 += 31)
     for (int k = nz - 1; k >= 0; k--)
-      for (int l = 0; l < 32; l++) {
-        const int col = t * 32 + l;
-        if (col >= ncol) break;
+      for (int col = col0; col < std::min(ncol, col0 + 31); col++) {
         const int c = cellk[(size_t)k * ncolp + col];
-        if (c && is_wet[c]) wet.push_back(c);
+        if (!c || !is_wet[c]) continue;
+        const int e = in(g->xp1[c]);
+        if ((wet.size() & 31) == 31) {  // a warp's last lane: the cell itself only
+          if (is_wet[e] && !wet.empty() && (wet.back() & ~kSegHalo) != 0 &&
+              in(g->xp1[wet.back() & ~kSegHalo]) == c) {
+            wet.push_back(c | kSegHalo);  // lends its west flux to the lane before it
+          } else if (is_wet[e]) {
+            wet.push_back(-1);
+          }
+        }
+        wet.push_back(c);
+        // the run's end in this segment with a wet east neighbour beyond it
+        const int nx = col + 1 < std::min(ncol, col0 + 31) ? cellk[(size_t)k * ncolp + col + 1] : 0;
+        if (is_wet[e] && nx != e) wet.push_back(e | kSegHalo);
       }
   // k_vd32 column order: tiles of 32 adjacent columns (a warp's lanes at one
   // layer are adjacent cells: coalesced loads and stores), the tiles sorted
@@ -1040,21 +1056,34 @@ int build_tile_tables(shoc_tr_gpu *h, const shoc_tr_geom *g, const std::vector<u
     h->vd_depth[i] = tdepth[t];
     for (int l = 0; l < 32; l++) vdcol[i * 32 + l] = (t * 32 + l < ncol) ? t * 32 + l : -1;
   }
-  // k_adv64's segments: columns in order, 32 to a warp; where the 32nd is the
-  // east neighbour of the 31st it is a halo lane and starts the next segment
+  // k_adv64's segments: columns in order, 32 to a warp.  A column's wet east
+  // neighbours are the next lane's cells: where the next column is not its east
+  // neighbour, or the warp is full, that one is added as a halo lane.
+  std::vector<int> col_of_top(h->S2, -1);
+  for (int col = 0; col < ncol; col++) col_of_top[g->w2_t[col + 1]] = col;
+  auto east = [&](int col) {
+    const int e = in(g->xp1[g->w2_t[col + 1]]);
+    return e < h->S2 ? col_of_top[e] : -1;
+  };
   std::vector<int> seg;
-  for (int col = 0; col < ncol;) {
-    const size_t b = seg.size();
-    seg.insert(seg.end(), 32, -1);
-    int l = 0;
-    for (; l < 32 && col < ncol; l++, col++) {
-      seg[b + l] = col;
-      if (l == 31 && g->xp1[g->w2_t[col]] == g->w2_t[col + 1]) {
-        seg[b + l] |= kSegHalo;
-        break;
-      }
+  for (int col = 0; col < ncol; col++) {
+    const int e = east(col);
+    if ((seg.size() & 31) == 31 && e >= 0) {  // the last lane: a halo lane, or none
+      const int b = seg.back();
+      seg.push_back(b >= 0 && !(b & kSegHalo) && east(b) == col ? col | kSegHalo : -1);
     }
+    seg.push_back(col);
+    if (e >= 0 && e != col + 1) seg.push_back(e | kSegHalo);
   }
+  while (seg.size() & 31) seg.push_back(-1);
+  // maps that do not stack (a cell's east neighbour outside its column's east
+  // column): every column goes the general path
+  if (h->O.cross)
+    for (int c = 1; c < S; c++) {
+      const int e = in(g->xp1[c]);
+      if (is_wet[c] && is_wet[e] && (east(colof[c]) != colof[e] || g->s2k[c] != g->s2k[e]))
+        h->O.tiled = 0;
+    }
   std::vector<int4> colrec(ncolp, make_int4(0, 0, nz, 0));
   for (int col = 0; col < ncol; col++)
     colrec[col] = make_int4(col_bot[col], g->w2_t[col + 1], col_kb[col], 0);
@@ -1845,10 +1874,10 @@ void adv64(const shoc_tr_gpu *h, const SubStep &ss, const Tile &tl, const TrSet 
   const size_t smem = adv64_smem(ng);
   if (h->adv_flags == 1)
     k_adv64<SCH, U, true><<<grid, kAdv64Warps * 32, smem, h->stream>>>(
-        h->G, h->F, h->W, h->O, T, ss, tl, tin, tout, h->fzs64, nch, L, ng);
+        h->G, h->F, h->W, T, ss, tl, tin, tout, h->fzs64, nch, L, ng);
   else
     k_adv64<SCH, U, false><<<grid, kAdv64Warps * 32, smem, h->stream>>>(
-        h->G, h->F, h->W, h->O, T, ss, tl, tin, tout, h->fzs64, nch, L, ng);
+        h->G, h->F, h->W, T, ss, tl, tin, tout, h->fzs64, nch, L, ng);
 }
 template <int SCH>
 void adv64_ult(const shoc_tr_gpu *h, const SubStep &ss, const Tile &tl, const TrSet &T,
@@ -1858,24 +1887,10 @@ void adv64_ult(const shoc_tr_gpu *h, const SubStep &ss, const Tile &tl, const Tr
   else
     adv64<SCH, false>(h, ss, tl, T, tin, tout);
 }
-template <int SCH>
-cudaError_t adv64_attr() {
-  cudaError_t e = cudaSuccess;
-  const int bytes = (int)adv64_smem(kAdv64Group);
-  for (auto k : {k_adv64<SCH, false, false>, k_adv64<SCH, false, true>, k_adv64<SCH, true, false>,
-                 k_adv64<SCH, true, true>}) {
-    const cudaError_t r =
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (r != cudaSuccess) e = r;
-  }
-  return e;
-}
+static_assert(kAdv64Warps * (kAdv64Faces * FC_N + kAdv64Group) * 32 * 8 <= 48 * 1024,
+              "k_adv64 stays below the opt-in shared memory size");
 cudaError_t tile64_set_smem_attr() {
   const cudaError_t r[] = {
-      adv64_attr<SHOC_TR_QUICKEST>(),    adv64_attr<SHOC_TR_VANLEER>(),
-      adv64_attr<SHOC_TR_ORDER1>(),      adv64_attr<SHOC_TR_ORDER2>(),
-      adv64_attr<SHOC_TR_ORDER4>(),      adv64_attr<SHOC_TR_QUICKEST_CO>(),
-      adv64_attr<SHOC_TR_ORDER2_UW>(),
       cudaFuncSetAttribute(k_vd64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024),
       cudaFuncSetAttribute(k_vd64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            227 * 1024)};

@@ -138,7 +138,8 @@ struct Tile {
   const int *kof;    // [S] layer index of each cell (s2k)
   const int4 *nbz;   // [S] zm1, zm1(zm1), zp1, zp1(zp1)
   const int *colof;  // [S] 0-based column of each wet cell
-  const int *wet;    // [nwet] the wet cells (w3_t order)
+  const int *wet;    // [nwet] k_adv32's cells, a lane each: cell, cell | kSegHalo (lends
+                     // its west flux only), -1: none
   const int *vdcol;  // [ncolp] columns in k_vd32 order: whole tiles of 32
                      // adjacent columns, shallow tiles first (-1: padding)
   int nclass;        // k_vd32 depth classes: tiles [ctile[i], ctile[i+1]) have
@@ -146,8 +147,7 @@ struct Tile {
   int cbase[4];
   const int4 *colrec;  // [ncolp] bottom cell, surface-layer cell, bottom layer
   // k_adv64's segments of the column order, [nseg][32]: columns, -1: none,
-  // with kSegHalo: the column only lends its west flux (it is the next
-  // segment's first own one)
+  // with kSegHalo: the column only lends its west flux
   const int *seg;
   int nseg;
   int ncolp;         // columns rounded up to whole tiles

@@ -102,7 +102,7 @@ __device__ __forceinline__ void set_face(Face &f, bool quick, float cr, float d,
 // weight formed in FP64 and rounded once, and V = U / |cr| in FP64: the
 // volume flux per unit of tc - tu of a face ULTIMATE caps at its Courant
 // bound (tu + (tc - tu) / |cr|).  That cap does not shrink with the Courant
-// number, so it is applied in FP64 to compensated values (face_c).
+// number, so it is applied in FP64 to compensated values (face_cu).
 __device__ __forceinline__ void set_face64(Face &f, bool quick, double cr, double d, double Ap,
                                            double Bp, double Am, double Bm, double U, bool ult,
                                            float K) {
@@ -131,24 +131,26 @@ __device__ __forceinline__ void set_face64(Face &f, bool quick, double cr, doubl
 }
 
 // One face flux, every rounding explicit: the QUICKEST or Van Leer face value
-// from the values tm2..tp1 at i-2..i+1 of the face's cell (FP32), then
-// ULTIMATE, times the FP64 volume flux, minus the horizontal-diffusion term.
+// from the values tm1, t0 beside the face (FP32) and the upwind one beyond them,
+// tu (at i-2 for FB_POS, else at i+1), then ULTIMATE, times the FP64 volume
+// flux, minus the horizontal-diffusion term.
 template <bool QUICK, bool ULT>
-__device__ __forceinline__ double face(const Face &f, bool adv, bool hd, float tm2, float tm1,
-                                       float t0, float tp1) {
+__device__ __forceinline__ double face_u(const Face &f, bool adv, bool hd, float tu, float tm1,
+                                         float t0) {
   double flux = 0.0;
   if (adv) {
     const bool pos = (f.bits & FB_POS) != 0;
-    const float tu = pos ? tm2 : tp1;
+    const float tc = pos ? tm1 : t0, td = pos ? t0 : tm1;
     float F;
     if (QUICK) {
-      const float tc = pos ? tm1 : t0;
       F = __fmaf_rn(f.wa, __fsub_rn(tu, tc), __fmaf_rn(f.wg, __fsub_rn(t0, tm1), tm1));
     } else {
       const bool neg = (f.bits & FB_NEG) != 0;
-      const float p = pos ? __fsub_rn(tm1, tm2) : __fsub_rn(t0, tm1);
-      const float q = pos ? __fsub_rn(t0, tm1) : __fsub_rn(tp1, t0);
-      const float den = pos ? __fsub_rn(t0, tm2) : __fsub_rn(tp1, tm1);
+      // (differences are exact negatives of each other taken the other way)
+      const float g01 = __fsub_rn(t0, tm1), cu = __fsub_rn(tc, tu), du = __fsub_rn(td, tu);
+      const float p = pos ? cu : g01;
+      const float q = pos ? g01 : -cu;
+      const float den = pos ? du : -du;
       const float pq = __fmul_rn(p, q);
       const float df = pq > 0.f ? __fmul_rn(2.f, __fdiv_rn(pq, den)) : 0.f;
       F = pos ? __fmaf_rn(f.wa, df, tm1) : (neg ? __fmaf_rn(-f.wa, df, t0) : 0.f);
@@ -162,7 +164,6 @@ __device__ __forceinline__ double face(const Face &f, bool adv, bool hd, float t
       // tc equals them too: in FP64 they almost always differ by a few ulps
       // and the limiter falls back to upwind, so FP32 rounding of the stored
       // tracer does not flip the limiter's decision.
-      const float tc = pos ? tm1 : t0, td = pos ? t0 : tm1;
       const float diff = __fsub_rn(td, tu);
       const float sg = diff < 0.f ? -1.f : 1.f;
       const float d = fabsf(diff);
@@ -183,8 +184,15 @@ __device__ __forceinline__ double face(const Face &f, bool adv, bool hd, float t
   return flux;
 }
 
-// FP32_COMP face flux: face() on compensated values, each value the stored
-// FP32 one (tm2..tp1) plus its compensation (lm2..lp1).  Differences are
+// the same from all four values at i-2..i+1
+template <bool QUICK, bool ULT>
+__device__ __forceinline__ double face(const Face &f, bool adv, bool hd, float tm2, float tm1,
+                                       float t0, float tp1) {
+  return face_u<QUICK, ULT>(f, adv, hd, (f.bits & FB_POS) ? tm2 : tp1, tm1, t0);
+}
+
+// FP32_COMP face flux: face_u() on compensated values, each value the stored
+// FP32 one (tu, tm1, t0) plus its compensation (lu, lm1, l0).  Differences are
 // the stored difference plus the compensations' difference (FP32, accurate
 // to their own size), so the limiter decides as on the FP64 values.  The face
 // value is a base value (a stored value) plus a correction (its compensation
@@ -192,12 +200,10 @@ __device__ __forceinline__ double face(const Face &f, bool adv, bool hd, float t
 // capped at ULTIMATE's Courant bound carries U (tu + lu) + V (tc - tu), the
 // second term with the FP64 V.
 template <bool QUICK, bool ULT>
-__device__ __forceinline__ double face_c(const Face &f, bool adv, bool hd, float tm2, float tm1,
-                                         float t0, float tp1, float lm2, float lm1, float l0,
-                                         float lp1) {
+__device__ __forceinline__ double face_cu(const Face &f, bool adv, bool hd, float tu, float tm1,
+                                          float t0, float lu, float lm1, float l0) {
   const bool pos = (f.bits & FB_POS) != 0;
-  const float tu = pos ? tm2 : tp1, tc = pos ? tm1 : t0;
-  const float lu = pos ? lm2 : lp1, lc = pos ? lm1 : l0;
+  const float tc = pos ? tm1 : t0, lc = pos ? lm1 : l0;
   const float g01 = __fadd_rn(__fsub_rn(t0, tm1), __fsub_rn(l0, lm1));  // t0 - tm1
   const float dc = __fadd_rn(__fsub_rn(tc, tu), __fsub_rn(lc, lu));   // tc - tu
   float base, lbase, inc;
@@ -207,10 +213,9 @@ __device__ __forceinline__ double face_c(const Face &f, bool adv, bool hd, float
     lbase = lm1;
   } else {
     const bool neg = (f.bits & FB_NEG) != 0;
-    const float p = pos ? __fadd_rn(__fsub_rn(tm1, tm2), __fsub_rn(lm1, lm2)) : g01;
-    const float q = pos ? g01 : __fadd_rn(__fsub_rn(tp1, t0), __fsub_rn(lp1, l0));
-    const float den = pos ? __fadd_rn(__fsub_rn(t0, tm2), __fsub_rn(l0, lm2))
-                          : __fadd_rn(__fsub_rn(tp1, tm1), __fsub_rn(lp1, lm1));
+    const float td = pos ? t0 : tm1, ld = pos ? l0 : lm1;
+    const float du = __fadd_rn(__fsub_rn(td, tu), __fsub_rn(ld, lu));
+    const float p = pos ? dc : g01, q = pos ? g01 : -dc, den = pos ? du : -du;
     const float pq = __fmul_rn(p, q);
     const float df = pq > 0.f ? __fmul_rn(2.f, __fdiv_rn(pq, den)) : 0.f;
     inc = pos ? __fmul_rn(f.wa, df) : (neg ? -__fmul_rn(f.wa, df) : 0.f);

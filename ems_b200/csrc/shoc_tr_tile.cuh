@@ -4,8 +4,8 @@
 // One sub-step is two launches:
 //
 //  k_adv32  advection and horizontal diffusion (advect_diffuse, tracers.c:
-//           849-925): one thread per wet cell, in SHOC's cell order (layer by
-//           layer, i fastest), so a warp's cells are adjacent cells of one
+//           849-925): one thread per wet cell, tile by tile (columns side by
+//           side), layer by layer, so a warp's cells are adjacent cells of one
 //           layer and its loads coalesce.  The thread folds its cell's
 //           tracer-independent face coefficients once (QUICKEST weights,
 //           ULTIMATE 1/|cr|, volume flux, horizontal-diffusion factor) and
@@ -141,37 +141,98 @@ __device__ __forceinline__ void zface(Face &f, bool quick, bool ult, float dzm2,
 
 // ---------------------------------------------------------------------------
 // k_adv32
+//
+// What bounds it: instructions issued, compares and selections above all (ALU
+// pipe), DRAM runs far below its peak.  So a cell evaluates five faces, its
+// east flux always being the next lane's west flux: the cell list (Tile::wet)
+// gives a run of cells that goes on beyond a warp's last lane or its tile a
+// halo lane, whose west flux is used and which the next warp updates.  Of the
+// two values beyond a face only the upwind one is fetched.  The vertical
+// neighbours are read from warps of the same block (four layers of a tile):
+// climbing a chunk of layers with the bottom flux kept, as k_adv64 does,
+// needs four faces and nine values but lost that reuse (4.6 ms on the case
+// below at first, 3.4 at best).  A third stage of the values' ring, and four or six
+// blocks an SM, were no faster.  No function is called from the loop: one that
+// took the kernel's parameters by reference put them in local memory (4.3 ms).
+// 1024 x 512 x 50, 24 tracers (B200), a sub-step: 3.45 ms with six faces and
+// thirteen values, 3.02 ms so; with compensations (448 x 300 x 50, 16 tracers)
+// 1.17 and 1.04 ms.
 
-// k_adv32: 128 threads, 5 blocks per SM (at most 102 registers a thread: 20
-// warps per SM where 256-thread blocks fit 16; measured 13.0 ms against 14.3
-// on stiff2048)
+// 128 threads, 5 blocks per SM (at most 102 registers a thread: 20 warps per SM
+// where 256-thread blocks fit 16; measured 13.0 ms against 14.3 on stiff2048)
 constexpr int kAdv32Block = 128, kAdv32MinBlocks = 5;
-constexpr int kAdvGroup = 1;       // tracers whose loads a thread issues together
-// dynamic shared memory of k_adv32 with uniform flags: the double-buffered
-// stencil values of a group of tracers per thread
-constexpr size_t kAdvSmem = (size_t)2 * kAdvGroup * 13 * kAdv32Block * sizeof(float);
+constexpr int kAdvValues = 11;     // stencil values of a cell and tracer
+// dynamic shared memory of k_adv32: the double-buffered stencil values
+constexpr size_t kAdvSmem = (size_t)2 * kAdvValues * kAdv32Block * sizeof(float);
 constexpr int kMaxTracers = 256;   // tracers a handle of the FP32-mixed path may carry
 
-// MODE: 0 tracers with their own advect / diffuse flags, 1 every advected
-// tracer advected without horizontal diffusion, 2 advected with it.
-// COMP (FP32_COMP): faces set up in FP64 (set_face64) and every stencil
-// value read with its compensation from loi (face_c); 4 blocks per SM.
-template <bool QUICK, bool ULT, int MODE, bool COMP>
-__global__ void __launch_bounds__(kAdv32Block, COMP ? 4 : kAdv32MinBlocks) k_adv32(Geo G, Flow32 F3, Work W, TrSet T,
-                                                     SubStep ss, Tile Tl,
-                                                     const f32::Face2 *__restrict__ fx2,
-                                                     const f32::Face2 *__restrict__ fy2,
-                                                     const float *__restrict__ tri,
-                                                     float *__restrict__ tro,
-                                                     float *__restrict__ rso,
-                                                     double *__restrict__ fzs, int any_hd,
-                                                     const int16_t *__restrict__ loi) {
+namespace f32 {
+
+// The faces of k_adv32's cells.  COMP (FP32_COMP): set up in FP64 (set_face64)
+template <bool QUICK, bool ULT, bool COMP>
+struct Faces {
+  const Geo &G;
+  const Flow32 &F3;
+  const Work &W;
+  const Face2 *__restrict__ fx2, *__restrict__ fy2;
+  double dtu;
+  float fdtu;
+  bool hdf;  // horizontal diffusion factors exist
+
+  // the backward face of cell c with 2D cell c2 along x (or y): wet: c is wet
+  // (else the face carries nothing), eb: an interior face
+  __device__ __forceinline__ void h(Face &f, bool x, int c, int c2, bool wet, bool eb) const {
+    const float K = hdf ? (x ? F3.khx[c] : F3.khy[c]) : 0.f;
+    const double U = x ? F3.u1flux3d[c] : F3.u2flux3d[c];
+    if constexpr (COMP) {
+      // FP64 Courant number (tracers.c:730-736) and metric factors
+      if (!wet) {
+        face_zero(f);
+      } else if (!QUICK && !eb) {  // Van Leer advects interior faces only
+        face_zero(f);
+        f.K = K;
+      } else {
+        const Face2D m = x ? G.fx[c2] : G.fy[c2];
+        const double u = x ? F3.u1_64[c] : F3.u2_64[c], hh = x ? G.h1au1[c2] : G.h2au2[c2];
+        set_face64(f, QUICK, u * dtu / hh, m.d, m.db * m.hm, m.db * m.h0, m.df * m.h0,
+                   m.df * m.hp, U, ULT && eb, K);
+      }
+    } else {
+      const Face2 m = x ? fx2[c2] : fy2[c2];
+      const float u = x ? F3.u1[c] : F3.u2[c];
+      hface(f, wet, eb, QUICK, ULT, __fmul_rn(__fmul_rn(u, fdtu), m.ih), U, K, m);
+    }
+  }
+  // the bottom face of cell c: below it zm and zmm, above it zp
+  __device__ __forceinline__ void z(Face &f, int c, int zm, int zmm, int zp) const {
+    const double U = __dmul_rn(F3.w64[c], dtu);
+    if constexpr (COMP) {
+      const double w90 = W.w9[c];
+      set_face64(f, QUICK, F3.w64[c] * dtu / (w90 * 1.0), W.w5[c], W.dbz[c] * W.w9[zm],
+                 W.dbz[c] * w90, W.dfz[c] * w90, W.dfz[c] * W.w9[zp], U, ULT, 0.f);
+    } else {
+      // (the sediment has no thickness, the surface-layer cell maps onto itself)
+      zface(f, QUICK, ULT, W.dz32[zmm], W.dz32[zm], W.dz32[c], W.dz32[zp], zp == c,
+            __fmul_rn(F3.w[c], fdtu), U);
+    }
+  }
+};
+
+}  // namespace f32
+
+// PLAIN: every advected tracer is advected without horizontal diffusion.
+// COMP (FP32_COMP): every stencil value is read with its compensation from loi
+// (face_cu); 4 blocks per SM.
+template <bool QUICK, bool ULT, bool PLAIN, bool COMP>
+__global__ void __launch_bounds__(kAdv32Block, COMP ? 4 : kAdv32MinBlocks)
+    k_adv32(Geo G, Flow32 F3, Work W, TrSet T, SubStep ss, Tile Tl,
+            const f32::Face2 *__restrict__ fx2, const f32::Face2 *__restrict__ fy2,
+            const float *__restrict__ tri, float *__restrict__ tro, float *__restrict__ rso,
+            double *__restrict__ fzs, int any_hd, const int16_t *__restrict__ loi) {
   using namespace f32;
   constexpr unsigned FULL = 0xffffffffu;
   __shared__ int sTr[kMaxTracers], sTf[kMaxTracers];
   const int i = blockIdx.x * kAdv32Block + threadIdx.x;
-  const int lane = threadIdx.x & 31;
-  const int nz = G.nz;
   for (int s = threadIdx.x; s < T.ntb; s += kAdv32Block) {
     const int n = T.slot_tr[s];
     sTr[s] = n;
@@ -179,129 +240,55 @@ __global__ void __launch_bounds__(kAdv32Block, COMP ? 4 : kAdv32MinBlocks) k_adv
   }
   __syncthreads();
 
-  // this thread's cell and its column (ntc: tracers carried by the column)
-  int c = 0, col = 0, kb = nz, ks = 0, k = 0, c2 = 0, ntc = 0;
+  // this thread's cell and its column (ntc: tracers carried by the column); st:
+  // its to update (not a halo lane, not a column of the general path)
+  int c = 0, col = 0, kb = G.nz, ks = 0, k = 0, c2 = 0, ntc = 0;
+  bool st = false;
   if (i < Tl.nwet) {
-    c = Tl.wet[i];
-    col = Tl.colof[c];
-    k = Tl.kof[c];
-    const TileCol tc = tile_column(G, W, Tl, col);
-    if (tc.act) {
-      kb = tc.kb;
-      ks = tc.ks;
-      c2 = tc.c2;
+    const int e = Tl.wet[i];
+    if (e >= 0) {
+      c = e & ~kSegHalo;
+      col = Tl.colof[c];
+      k = Tl.kof[c];
+      const int4 r = Tl.colrec[col];
+      const ColInfo ci = W.col[col];
+      kb = r.z;
+      c2 = r.y;
+      ks = ci.ks;
+      st = !(e & kSegHalo) && (ci.flags & COL_STAGED);
       ntc = G.colntr[col];
-    } else {
-      c = 0;
     }
   }
   const bool on = c != 0;
+  if (!__any_sync(FULL, st)) return;
   int4 n1 = make_int4(0, 0, 0, 0), n2 = n1, nzv = n1;
-  int2 me = make_int2(0, 0);
   int fl = 0;
   if (on) {
     n1 = Tl.nb1[c];
     n2 = Tl.nb2[c];
     nzv = Tl.nbz[c];
-    me = Tl.m2e[c];
     fl = Tl.fl[c];
   }
-  // x-neighbours that are the cells of neighbouring lanes
-  const int cu1 = __shfl_up_sync(FULL, c, 1), cu2 = __shfl_up_sync(FULL, c, 2);
-  const int cd1 = __shfl_down_sync(FULL, c, 1), cd2 = __shfl_down_sync(FULL, c, 2);
-  const bool sxm1 = on && lane >= 1 && cu1 && n1.x == cu1;
-  const bool sxm2 = on && lane >= 2 && cu2 && n2.x == cu2;
-  const bool sxp1 = on && lane <= 30 && cd1 && n1.y == cd1;
-  const bool sxp2 = on && lane <= 29 && cd2 && n2.y == cd2;
+  // a wet east neighbour is the next lane's cell (the cell list sees to it)
+  const bool ewet = (fl & FL_XP_WET) != 0;
+  const bool zf = k <= ks, zt = k < ks;
 
   // tracer-independent face coefficients
   const double dtu = ss.dtu;
-  const float fdtu = (float)dtu;
-  const bool hdf = any_hd != 0;
-  Face fw, fs, fn, fe, fzb, fzt;
+  const Faces<QUICK, ULT, COMP> set{G, F3, W, fx2, fy2, dtu, (float)dtu, any_hd != 0};
+  Face fw, fs, fn, fzb, fzt;
   face_zero(fw);
   face_zero(fs);
   face_zero(fn);
-  face_zero(fe);
   face_zero(fzb);
   face_zero(fzt);
   double idz = 0.0, ia = 0.0;
-  if (on && COMP) {
-    // FP64 Courant numbers (tracers.c:730-736) and metric factors
-    auto hset = [&](Face &f, bool wet, bool eb, double u, double h, const Face2D &m, double U,
-                    float K) {
-      if (!wet) {
-        face_zero(f);
-      } else if (!QUICK && !eb) {  // Van Leer advects interior faces only
-        face_zero(f);
-        f.K = K;
-      } else {
-        set_face64(f, QUICK, u * dtu / h, m.d, m.db * m.hm, m.db * m.h0, m.df * m.h0,
-                   m.df * m.hp, U, ULT && eb, K);
-      }
-    };
-    // the face at the bottom of cell cc (below it zm, above it zp), from the
-    // work arrays as quickest_zface takes them
-    auto zset = [&](Face &f, int cc, int zm, int zp) {
-      const double w90 = W.w9[cc];
-      set_face64(f, QUICK, F3.w64[cc] * dtu / (w90 * 1.0), W.w5[cc], W.dbz[cc] * W.w9[zm],
-                 W.dbz[cc] * w90, W.dfz[cc] * w90, W.dfz[cc] * W.w9[zp],
-                 __dmul_rn(F3.w64[cc], dtu), ULT, 0.f);
-    };
-    hset(fw, fl & CF_WET, fl & CF_E1, F3.u1_64[c], G.h1au1[c2], G.fx[c2], F3.u1flux3d[c],
-         hdf ? F3.khx[c] : 0.f);
-    hset(fs, fl & CF_WET, fl & CF_E2, F3.u2_64[c], G.h2au2[c2], G.fy[c2], F3.u2flux3d[c],
-         hdf ? F3.khy[c] : 0.f);
-    if (fl & FL_YP_WET) {
-      const int yp = n1.w;
-      hset(fn, true, fl & FL_YP_E2, F3.u2_64[yp], G.h2au2[me.y], G.fy[me.y], F3.u2flux3d[yp],
-           hdf ? F3.khy[yp] : 0.f);
-    }
-    if (!sxp1 && (fl & FL_XP_WET)) {
-      const int xp = n1.y;
-      hset(fe, true, fl & FL_XP_E1, F3.u1_64[xp], G.h1au1[me.x], G.fx[me.x], F3.u1flux3d[xp],
-           hdf ? F3.khx[xp] : 0.f);
-    }
-    if (k <= ks) {
-      zset(fzb, c, nzv.x, nzv.z);
-      if (k < ks) zset(fzt, nzv.z, c, nzv.w);  // the bottom face of the cell above
-    }
-    idz = 1.0 / W.dz[c];
-    ia = 1.0 / G.cellarea[c2];
-  } else if (on) {
-    const Face2 mx = fx2[c2], my = fy2[c2];
-    hface(fw, fl & CF_WET, fl & CF_E1, QUICK, ULT, __fmul_rn(__fmul_rn(F3.u1[c], fdtu), mx.ih),
-          F3.u1flux3d[c], hdf ? F3.khx[c] : 0.f, mx);
-    hface(fs, fl & CF_WET, fl & CF_E2, QUICK, ULT, __fmul_rn(__fmul_rn(F3.u2[c], fdtu), my.ih),
-          F3.u2flux3d[c], hdf ? F3.khy[c] : 0.f, my);
-    if (fl & FL_YP_WET) {
-      const int yp = n1.w;
-      const Face2 mn = fy2[me.y];
-      hface(fn, true, fl & FL_YP_E2, QUICK, ULT, __fmul_rn(__fmul_rn(F3.u2[yp], fdtu), mn.ih),
-            F3.u2flux3d[yp], hdf ? F3.khy[yp] : 0.f, mn);
-    }
-    if (!sxp1 && (fl & FL_XP_WET)) {
-      const int xp = n1.y;
-      const Face2 mxe = fx2[me.x];
-      hface(fe, true, fl & FL_XP_E1, QUICK, ULT, __fmul_rn(__fmul_rn(F3.u1[xp], fdtu), mxe.ih),
-            F3.u1flux3d[xp], hdf ? F3.khx[xp] : 0.f, mxe);
-    }
-    const float dz0 = W.dz32[c];
-    if (k <= ks) {
-      // thicknesses below, at and above the cell (the sediment has none, the
-      // surface-layer cell maps onto itself)
-      const float dzm1 = W.dz32[nzv.x], dzm2 = W.dz32[nzv.y];
-      const bool top = (nzv.z == c);
-      const float dzp1 = W.dz32[nzv.z];
-      zface(fzb, QUICK, ULT, dzm2, dzm1, dz0, dzp1, top, __fmul_rn(F3.w[c], fdtu),
-            __dmul_rn(F3.w64[c], dtu));
-      if (k < ks) {  // the bottom face of the cell above
-        const bool top1 = (nzv.w == nzv.z);
-        const float dzp2 = W.dz32[nzv.w];
-        zface(fzt, QUICK, ULT, dzm1, dz0, dzp1, dzp2, top1, __fmul_rn(F3.w[nzv.z], fdtu),
-              __dmul_rn(F3.w64[nzv.z], dtu));
-      }
-    }
+  if (on) set.h(fw, true, c, c2, fl & CF_WET, fl & CF_E1);
+  if (st) {
+    set.h(fs, false, c, c2, fl & CF_WET, fl & CF_E2);
+    if (fl & FL_YP_WET) set.h(fn, false, n1.w, Tl.m2e[c].y, true, fl & FL_YP_E2);
+    if (zf) set.z(fzb, c, nzv.x, nzv.y, nzv.z);
+    if (zt) set.z(fzt, nzv.z, c, nzv.x, nzv.w);  // the bottom face of the cell above
     idz = 1.0 / W.dz[c];  // the FP64 thickness: the update conserves mass to FP64 round-off
     ia = 1.0 / G.cellarea[c2];
   }
@@ -309,223 +296,94 @@ __global__ void __launch_bounds__(kAdv32Block, COMP ? 4 : kAdv32MinBlocks) k_adv
   // tracers.c:827-830)
   const int vm1 = (k - 1 >= kb) ? nzv.x : c;
   const int vm2 = (k - 2 >= kb) ? nzv.y : vm1;
-  const int vp1 = nzv.z, vp2 = nzv.w;
-  const bool zf = k <= ks, zt = k < ks;
   const int ntb = T.ntb;
 
-  // The advected tracers in groups of U: every stencil value of the group is
-  // loaded before any of it is used, so a thread has U tracers' loads in
-  // flight at once.
-  constexpr int U = kAdvGroup;
-  if constexpr (MODE != 0) {
-    // uniform flags: every stencil value is loaded (threads without a cell,
-    // and neighbours a cell does not use, read valid cells) and the face
-    // code has no per-tracer branches
-    constexpr bool HD = MODE == 2;
-    constexpr int NQ = 13;
-    const int idx[NQ] = {c,    n1.z, n2.z, n1.w, n2.w, vm1, vm2,
-                         vp1,  vp2,  n1.x, n2.x, n1.y, n2.y};
-    // the stencil values of the next group of tracers are copied into this
-    // thread's slots of a double buffer while the current group is computed
-    extern __shared__ float pf[];  // [2][U][NQ][kAdv32Block]
-    auto issue = [&](int s0, int buf) {
+  // The stencil values of the next tracer are copied into this thread's slots of
+  // a double buffer while the current one is computed: the cell, its west,
+  // south, north, bottom and top neighbours, and the upwind value beyond each
+  // face (threads without a cell, and neighbours a cell does not use, read
+  // valid cells).
+  constexpr int NQ = kAdvValues, B = kAdv32Block;
+  const int idx[NQ] = {c,
+                       n1.x,
+                       n1.z,
+                       n1.w,
+                       vm1,
+                       nzv.z,
+                       (fw.bits & FB_POS) ? n2.x : n1.y,
+                       (fs.bits & FB_POS) ? n2.z : n1.w,
+                       (fn.bits & FB_POS) ? n1.z : n2.w,
+                       (fzb.bits & FB_POS) ? vm2 : nzv.z,
+                       (fzt.bits & FB_POS) ? vm1 : nzv.w};
+  extern __shared__ float pf[];  // [2][NQ][kAdv32Block]
+  auto issue = [&](int s, int buf) {
+    const float *tr = tri + (size_t)sTr[s] * G.S;
+    float *d = pf + buf * NQ * B + threadIdx.x;
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int s = s0 + u < ntb ? s0 + u : s0;
-        const float *tr = tri + (size_t)sTr[s] * G.S;
-        float *d = pf + (buf * U + u) * NQ * kAdv32Block + threadIdx.x;
+    for (int q = 0; q < NQ; ++q) cp_async4(d + q * B, tr + idx[q]);
+    cp_async_commit();
+  };
+  issue(0, 0);
+  for (int s = 0; s < ntb; ++s) {
+    const int n = sTr[s];
+    // COMP: the stencil's compensations, in flight while the stencil values'
+    // copies complete
+    int16_t lq[NQ];
+    if constexpr (COMP) {
+      const int16_t *Lp = loi + (size_t)n * G.S;
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) cp_async4(d + q * kAdv32Block, tr + idx[q]);
-      }
-      cp_async_commit();
-    };
-    issue(0, 0);
-    static_assert(U == 1, "the compensations are loaded for one tracer at a time");
-    for (int s0 = 0, g = 0; s0 < ntb; s0 += U, ++g) {
-      // COMP: the stencil's compensations, in flight while the stencil
-      // values' copies complete
-      int16_t lq[NQ];
-      if constexpr (COMP) {
-        const int16_t *Lp = loi + (size_t)sTr[s0] * G.S;
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) lq[q] = Lp[idx[q]];
-      }
-      if (s0 + U < ntb) {
-        issue(s0 + U, (g + 1) & 1);
-        cp_async_wait<1>();
-      } else {
-        cp_async_wait<0>();
-      }
-      // tracers are ascending when columns carry different numbers of them
-      if (!__any_sync(FULL, on && sTr[s0] < ntc)) continue;
-      const float *P = pf + (g & 1) * U * NQ * kAdv32Block + threadIdx.x;
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int s = s0 + u;
-        if (s >= ntb) break;
-        const float *v = P + u * NQ * kAdv32Block;
-        const float t0 = v[0];
-        const float tym1 = v[1 * kAdv32Block], tym2 = v[2 * kAdv32Block];
-        const float typ1 = v[3 * kAdv32Block], typ2 = v[4 * kAdv32Block];
-        const float tm1 = v[5 * kAdv32Block], tm2 = v[6 * kAdv32Block];
-        const float tp1 = v[7 * kAdv32Block], tp2 = v[8 * kAdv32Block];
-        const float txm1 = v[9 * kAdv32Block], txm2 = v[10 * kAdv32Block];
-        const float txp1 = v[11 * kAdv32Block], txp2 = v[12 * kAdv32Block];
-        double Fxw, Fys, Fyn, Fxe, Fzb;
-        float l0 = 0.f, lm1 = 0.f, lm2 = 0.f, lp1 = 0.f, lp2 = 0.f;
-        if constexpr (COMP) {
-          l0 = lo_val(lq[0]);
-          const float lym1 = lo_val(lq[1]), lym2 = lo_val(lq[2]);
-          const float lyp1 = lo_val(lq[3]), lyp2 = lo_val(lq[4]);
-          lm1 = lo_val(lq[5]);
-          lm2 = lo_val(lq[6]);
-          lp1 = lo_val(lq[7]);
-          lp2 = lo_val(lq[8]);
-          const float lxm1 = lo_val(lq[9]), lxm2 = lo_val(lq[10]);
-          const float lxp1 = lo_val(lq[11]), lxp2 = lo_val(lq[12]);
-          Fxw = face_c<QUICK, ULT>(fw, true, HD, txm2, txm1, t0, txp1, lxm2, lxm1, l0, lxp1);
-          Fys = face_c<QUICK, ULT>(fs, true, HD, tym2, tym1, t0, typ1, lym2, lym1, l0, lyp1);
-          Fyn = face_c<QUICK, ULT>(fn, true, HD, tym1, t0, typ1, typ2, lym1, l0, lyp1, lyp2);
-          const double Fnext = __shfl_down_sync(FULL, Fxw, 1);
-          Fxe = sxp1 ? Fnext
-                     : face_c<QUICK, ULT>(fe, true, HD, txm1, t0, txp1, txp2, lxm1, l0, lxp1,
-                                          lxp2);
-          Fzb = zf ? face_c<QUICK, ULT>(fzb, true, false, tm2, tm1, t0, tp1, lm2, lm1, l0, lp1)
-                   : 0.0;
-        } else {
-          Fxw = face<QUICK, ULT>(fw, true, HD, txm2, txm1, t0, txp1);
-          Fys = face<QUICK, ULT>(fs, true, HD, tym2, tym1, t0, typ1);
-          Fyn = face<QUICK, ULT>(fn, true, HD, tym1, t0, typ1, typ2);
-          const double Fnext = __shfl_down_sync(FULL, Fxw, 1);
-          Fxe = sxp1 ? Fnext : face<QUICK, ULT>(fe, true, HD, txm1, t0, txp1, txp2);
-          Fzb = zf ? face<QUICK, ULT>(fzb, true, false, tm2, tm1, t0, tp1) : 0.0;
-        }
-        const int n = sTr[s];
-        if (!on || n >= ntc) continue;
-        // FP64 flux divergence (tracers.c:888-892)
-        const double dtr = ((Fxe - Fxw) + (Fyn - Fys)) * dtu;
-        double a = dtr;
-        if (zt) {
-          const double Fzt =
-              COMP ? face_c<QUICK, ULT>(fzt, true, false, tm1, t0, tp1, tp2, lm1, l0, lp1, lp2)
-                   : face<QUICK, ULT>(fzt, true, false, tm1, t0, tp1, tp2);
-          const double t0d = COMP ? (double)t0 + (double)l0 : (double)t0;
-          a = t0d - (dtr * ia + (Fzt - Fzb)) * idz;
-        } else if (zf) {
-          fzs[(size_t)n * G.ncol + col] = Fzb;
-        }
-        const float val = (float)a;
-        tro[(size_t)n * G.S + c] = val;
-        rso[(size_t)n * G.S + c] = (float)(a - (double)val);
-      }
+      for (int q = 0; q < NQ; ++q) lq[q] = Lp[idx[q]];
     }
-  } else {
-  for (int s0 = 0; s0 < ntb; s0 += U) {
-    float v[U][13];  // t0, y-2..y+2, z-2..z+2, x-2..x+2 (off-tile x only)
-    float lv[U][13];  // COMP: their compensations (x-neighbours read for every cell)
-    int nn[U], tf[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int s = s0 + u;
-      nn[u] = s < ntb ? sTr[s] : 0;
-      tf[u] = s < ntb ? sTf[s] : 0;
-      const float *__restrict__ tr = tri + (size_t)nn[u] * G.S;
-      const bool hor = on && (tf[u] & (TR_ADV | TR_HDIFF));
-      const bool vz = on && (tf[u] & TR_ADV) && zf;
-      v[u][0] = on && s < ntb ? tr[c] : 0.f;
-      v[u][1] = hor ? tr[n1.z] : 0.f;
-      v[u][2] = hor ? tr[n2.z] : 0.f;
-      v[u][3] = hor ? tr[n1.w] : 0.f;
-      v[u][4] = hor ? tr[n2.w] : 0.f;
-      v[u][5] = vz ? tr[vm1] : 0.f;
-      v[u][6] = vz ? tr[vm2] : 0.f;
-      v[u][7] = vz ? tr[vp1] : 0.f;
-      v[u][8] = (vz && zt) ? tr[vp2] : 0.f;
-      v[u][9] = (hor && !sxm1) ? tr[n1.x] : 0.f;
-      v[u][10] = (hor && !sxm2) ? tr[n2.x] : 0.f;
-      v[u][11] = (hor && !sxp1) ? tr[n1.y] : 0.f;
-      v[u][12] = (hor && !sxp1 && !sxp2) ? tr[n2.y] : 0.f;
-      if constexpr (COMP) {
-        const int16_t *L = loi + (size_t)nn[u] * G.S;
-        lv[u][0] = on && s < ntb ? lo_val(L[c]) : 0.f;
-        lv[u][1] = hor ? lo_val(L[n1.z]) : 0.f;
-        lv[u][2] = hor ? lo_val(L[n2.z]) : 0.f;
-        lv[u][3] = hor ? lo_val(L[n1.w]) : 0.f;
-        lv[u][4] = hor ? lo_val(L[n2.w]) : 0.f;
-        lv[u][5] = vz ? lo_val(L[vm1]) : 0.f;
-        lv[u][6] = vz ? lo_val(L[vm2]) : 0.f;
-        lv[u][7] = vz ? lo_val(L[vp1]) : 0.f;
-        lv[u][8] = (vz && zt) ? lo_val(L[vp2]) : 0.f;
-        lv[u][9] = hor ? lo_val(L[n1.x]) : 0.f;
-        lv[u][10] = hor ? lo_val(L[n2.x]) : 0.f;
-        lv[u][11] = hor ? lo_val(L[n1.y]) : 0.f;
-        lv[u][12] = hor ? lo_val(L[n2.y]) : 0.f;
-      }
+    if (s + 1 < ntb) {
+      issue(s + 1, (s + 1) & 1);
+      cp_async_wait<1>();
+    } else {
+      cp_async_wait<0>();
     }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int s = s0 + u;
-      if (s >= ntb) break;
-      const bool adv = (tf[u] & TR_ADV) != 0, hd = (tf[u] & TR_HDIFF) != 0;
-      const float t0 = v[u][0];
-      const float u1v = __shfl_up_sync(FULL, t0, 1), u2v = __shfl_up_sync(FULL, t0, 2);
-      const float d1v = __shfl_down_sync(FULL, t0, 1), d2v = __shfl_down_sync(FULL, t0, 2);
-      double Fxw = 0.0, Fxe = 0.0, Fys = 0.0, Fyn = 0.0, Fzb = 0.0, Fzt = 0.0;
-      if (on && (adv || hd)) {
-        const float txm1 = sxm1 ? u1v : v[u][9];
-        const float txm2 = sxm2 ? u2v : v[u][10];
-        const float txp1 = sxp1 ? d1v : v[u][11];
-        const float tym1 = v[u][1], tym2 = v[u][2], typ1 = v[u][3], typ2 = v[u][4];
-        if constexpr (COMP) {
-          const float *l = lv[u];
-          Fxw = face_c<QUICK, ULT>(fw, adv, hd, txm2, txm1, t0, txp1, l[10], l[9], l[0], l[11]);
-          Fys = face_c<QUICK, ULT>(fs, adv, hd, tym2, tym1, t0, typ1, l[2], l[1], l[0], l[3]);
-          Fyn = face_c<QUICK, ULT>(fn, adv, hd, tym1, t0, typ1, typ2, l[1], l[0], l[3], l[4]);
-          if (!sxp1) {
-            const float txp2 = sxp2 ? d2v : v[u][12];
-            Fxe = face_c<QUICK, ULT>(fe, adv, hd, txm1, t0, txp1, txp2, l[9], l[0], l[11],
-                                     l[12]);
-          }
-          if (adv && zf) {
-            const float tm1 = v[u][5], tm2 = v[u][6], tp1 = v[u][7];
-            Fzb = face_c<QUICK, ULT>(fzb, true, false, tm2, tm1, t0, tp1, l[6], l[5], l[0],
-                                     l[7]);
-            if (zt)
-              Fzt = face_c<QUICK, ULT>(fzt, true, false, tm1, t0, tp1, v[u][8], l[5], l[0],
-                                       l[7], l[8]);
-          }
-        } else {
-          Fxw = face<QUICK, ULT>(fw, adv, hd, txm2, txm1, t0, txp1);
-          Fys = face<QUICK, ULT>(fs, adv, hd, tym2, tym1, t0, typ1);
-          Fyn = face<QUICK, ULT>(fn, adv, hd, tym1, t0, typ1, typ2);
-          if (!sxp1) {
-            const float txp2 = sxp2 ? d2v : v[u][12];
-            Fxe = face<QUICK, ULT>(fe, adv, hd, txm1, t0, txp1, txp2);
-          }
-          if (adv && zf) {
-            const float tm1 = v[u][5], tm2 = v[u][6], tp1 = v[u][7];
-            Fzb = face<QUICK, ULT>(fzb, true, false, tm2, tm1, t0, tp1);
-            if (zt) Fzt = face<QUICK, ULT>(fzt, true, false, tm1, t0, tp1, v[u][8]);
-          }
-        }
-      }
-      const double Fnext = __shfl_down_sync(FULL, Fxw, 1);
-      if (!on || nn[u] >= ntc) continue;
-      if (sxp1) Fxe = Fnext;
-      // FP64 flux divergence (tracers.c:888-892)
-      const double dtr = ((Fxe - Fxw) + (Fyn - Fys)) * dtu;
-      double a = dtr;
-      if (zt) {
-        const double t0d = COMP ? (double)t0 + (double)lv[u][0] : (double)t0;
-        a = t0d - (dtr * ia + (Fzt - Fzb)) * idz;
-      }
-      else if (k == ks)
-        fzs[(size_t)nn[u] * G.ncol + col] = Fzb;
-      const float val = (float)a;
-      tro[(size_t)nn[u] * G.S + c] = val;
-      rso[(size_t)nn[u] * G.S + c] = (float)(a - (double)val);
+    // tracers are ascending when columns carry different numbers of them
+    if (!__any_sync(FULL, st && n < ntc)) continue;
+    const int tf = PLAIN ? TR_ADV : sTf[s];
+    const bool adv = PLAIN || (tf & TR_ADV), hd = !PLAIN && (tf & TR_HDIFF);
+    const float *v = pf + (s & 1) * NQ * B + threadIdx.x;
+    const float t0 = v[0], txm1 = v[B], tym1 = v[2 * B], typ1 = v[3 * B], tm1 = v[4 * B];
+    const float tp1 = v[5 * B], tuw = v[6 * B], tus = v[7 * B], tun = v[8 * B];
+    const float tub = v[9 * B], tut = v[10 * B];
+    double Fxw, Fys, Fyn, Fzb = 0.0, Fzt = 0.0;
+    float l0 = 0.f;
+    if constexpr (COMP) {
+      l0 = lo_val(lq[0]);
+      const float lxm1 = lo_val(lq[1]), lym1 = lo_val(lq[2]), lyp1 = lo_val(lq[3]);
+      const float lm1 = lo_val(lq[4]), lp1 = lo_val(lq[5]), luw = lo_val(lq[6]);
+      const float lus = lo_val(lq[7]), lun = lo_val(lq[8]), lub = lo_val(lq[9]);
+      const float lut = lo_val(lq[10]);
+      Fxw = face_cu<QUICK, ULT>(fw, adv, hd, tuw, txm1, t0, luw, lxm1, l0);
+      Fys = face_cu<QUICK, ULT>(fs, adv, hd, tus, tym1, t0, lus, lym1, l0);
+      Fyn = face_cu<QUICK, ULT>(fn, adv, hd, tun, t0, typ1, lun, l0, lyp1);
+      if (zf) Fzb = face_cu<QUICK, ULT>(fzb, adv, false, tub, tm1, t0, lub, lm1, l0);
+      if (zt) Fzt = face_cu<QUICK, ULT>(fzt, adv, false, tut, t0, tp1, lut, l0, lp1);
+    } else {
+      Fxw = face_u<QUICK, ULT>(fw, adv, hd, tuw, txm1, t0);
+      Fys = face_u<QUICK, ULT>(fs, adv, hd, tus, tym1, t0);
+      Fyn = face_u<QUICK, ULT>(fn, adv, hd, tun, t0, typ1);
+      if (zf) Fzb = face_u<QUICK, ULT>(fzb, adv, false, tub, tm1, t0);
+      if (zt) Fzt = face_u<QUICK, ULT>(fzt, adv, false, tut, t0, tp1);
     }
-  }
+    double Fxe = __shfl_down_sync(FULL, Fxw, 1);
+    if (!st || n >= ntc) continue;
+    if (!ewet) Fxe = 0.0;
+    // FP64 flux divergence (tracers.c:888-892)
+    const double dtr = ((Fxe - Fxw) + (Fyn - Fys)) * dtu;
+    double a = dtr;
+    if (zt) {
+      const double t0d = COMP ? (double)t0 + (double)l0 : (double)t0;
+      a = t0d - (dtr * ia + (Fzt - Fzb)) * idz;
+    } else if (zf) {
+      fzs[(size_t)n * G.ncol + col] = Fzb;
+    }
+    const float val = (float)a;
+    const size_t o = (size_t)n * G.S + c;
+    tro[o] = val;
+    rso[o] = (float)(a - (double)val);
   }
 }
 

@@ -83,17 +83,19 @@ __device__ __forceinline__ bool far_out(double x) {
 }
 // a / b for any a and a b the caller keeps y = 1 / b of.  lo: kDivLo where b
 // lies in 2^-200 .. 2^200, so that nothing under- or overflows for |a| in
-// 2^-700 .. 2^700; kDivNever where it does not.  Else the division.
+// 2^-700 .. 2^700 (div_fast); kDivNever where it does not.  Else the division.
 constexpr unsigned kDivLo = (1023u - 700u) << 20, kDivSpan = 1400u << 20;
 constexpr unsigned kDivNever = 0x80000000u;
 __device__ __noinline__ double div_slow(double a, double b) { return a / b; }
 __device__ __forceinline__ unsigned div_range(double b) {
   return far_out<200>(b) ? kDivNever : kDivLo;
 }
+__device__ __forceinline__ bool div_fast(double a, unsigned lo) {
+  return ((unsigned)__double2hiint(a) & 0x7fffffffu) - lo < kDivSpan;
+}
 __device__ __forceinline__ double div_known(double a, double b, double y, unsigned lo) {
   double q = quot(a, b, y);
-  const unsigned e = ((unsigned)__double2hiint(a) & 0x7fffffffu) - lo;
-  if (e >= kDivSpan) q = (a == 0.0 && lo != kDivNever) ? __dmul_rn(a, y) : div_slow(a, b);
+  if (!div_fast(a, lo)) q = (a == 0.0 && lo != kDivNever) ? __dmul_rn(a, y) : div_slow(a, b);
   return q;
 }
 // RN(1 / d) for |d| in 2^-500 .. 2^500: Newton steps from the hardware's
@@ -238,22 +240,6 @@ __device__ __forceinline__ double face_flux64(const double *f, int bits, double 
   return v * f[FC_U * 32];
 }
 
-// A face outside the climb, by the reference's own operations: the east face of
-// a cell whose east neighbour is not the next lane's (maps that join columns
-// out of order), or the bottom face of a column whose floor lies inside a
-// chunk and lets water through
-__device__ __noinline__ double east_flux(const Geo &G, const Flow &F, const Work &W, const Opt &O,
-                                         const Tile &Tl, int c, bool adv, bool hd,
-                                         const double *tr, double dtu) {
-  const int4 n1 = Tl.nb1[c], n2 = Tl.nb2[c];
-  return flux_x(G, F, W, O, (Tl.fl[c] & FL_XP_E1) ? CF_E1 : 0, adv, hd, n1.y, Tl.m2e[c].x,
-                tr[n1.x], tr[c], tr[n1.y], tr[n2.y], dtu);
-}
-__device__ __noinline__ double floor_flux(const Flow &F, const Work &W, const Opt &O, int c,
-                                          int sed, int zp, double t0, double tp1, double dtu) {
-  return flux_z(F, W, O, c, W.w9[sed], W.w9[c], W.w9[zp], t0, t0, t0, tp1, dtu);
-}
-
 // Whether every value of a list lies in 2^-400 .. 2^490 or is 0: differences
 // of such values are 0 or above 2^-453, and the faces' quotients stay inside
 // the range quot takes.  (h - 1 orders a zero high word last; a subnormal
@@ -282,7 +268,7 @@ inline size_t adv64_smem(int ng) {
 // ch = b % nch; blockIdx.y: groups of ng tracers.
 template <int SCH, bool ULT, bool PLAIN>
 __global__ void __launch_bounds__(kAdv64Warps * 32, 16)
-    k_adv64(Geo G, Flow F, Work W, Opt O, TrSet T, SubStep ss, Tile Tl,
+    k_adv64(Geo G, Flow F, Work W, TrSet T, SubStep ss, Tile Tl,
             const double *__restrict__ tri, double *__restrict__ tro, double *__restrict__ fzs,
             int nch, int L, int ng) {
   extern __shared__ double sAdv[];  // per warp: [kAdv64Faces][FC_N][32], [ng][32]
@@ -335,13 +321,12 @@ __global__ void __launch_bounds__(kAdv64Warps * 32, 16)
                                                    : 0;
     int4 nzv = make_int4(0, 0, 0, 0);
     int bits = 0;
-    bool flow = false;  // through a closed floor v * 0
-    if (c) {
+    const bool flow = c && k0 > kb;  // (a column's floor is closed)
+    if (flow) {
       nzv = __ldg(&Tl.nbz[c]);
-      flow = __ldg(&F.w[c]) * dtu != 0.0;
-      if (flow) bits = zset(ft, c, nzv.x, nzv.z);
+      bits = zset(ft, c, nzv.x, nzv.z);
     }
-    const int vm1 = (k0 - 1 >= kb) ? nzv.x : c, vm2 = (k0 - 2 >= kb) ? nzv.y : vm1;
+    const int vm1 = nzv.x, vm2 = (k0 - 2 >= kb) ? nzv.y : vm1;
     for (int s = sl0; s < sl1; ++s) {
       double Fz = 0.0;
       const int n = __ldg(&T.slot_tr[s]);
@@ -378,10 +363,9 @@ __global__ void __launch_bounds__(kAdv64Warps * 32, 16)
       me = __ldg(&Tl.m2e[c]);
       fl = __ldg(&Tl.fl[c]);
     }
-    const int cd1 = __shfl_down_sync(FULL, c, 1);
-    const bool sxp = on && lane < 31 && cd1 && n1.y == cd1;
+    // a wet east neighbour is the next lane's cell (the segments see to it)
+    const bool ewet = (fl & FL_XP_WET) != 0;
     const bool nwet = (fl & FL_YP_WET) != 0;
-    const bool eslow = st && !sxp && (SCH == SHOC_TR_ORDER1 || (fl & FL_XP_WET));
     const bool below = k < ks;  // interior cell: its top face is in the water
 
     int bw = 0, bs = 0, bn = 0, bt = 0;
@@ -425,10 +409,6 @@ __global__ void __launch_bounds__(kAdv64Warps * 32, 16)
     // the upwind value beyond each face: one load instead of two and a choice
     const int uw = (bw & F64_POS) ? n2.x : n1.y, us = (bs & F64_POS) ? n2.z : n1.w;
     const int un = (bn & F64_POS) ? n1.z : n2.w, ut = (bt & F64_POS) ? vm1 : nzv.w;
-    // the floor inside the chunk: where it lets water through
-    const bool fbot = k == kb && k > k0;
-    const bool fslow = st && fbot && k <= ks && __ldg(&F.w[c]) * dtu != 0.0;
-
     // the next tracer's stencil values are loaded while this one is computed
     constexpr int NV = 9;
     const int idx[NV] = {c, n1.x, n1.z, n1.w, nzv.z, uw, us, un, ut};
@@ -491,11 +471,18 @@ __global__ void __launch_bounds__(kAdv64Warps * 32, 16)
             ec.add(tp2);
           }
           if (ec.bad() || refs) {
-            if (on) Fxw = face_ref64<SCH, ULT>(fw, bw, tuw, txm1, t0, txm2, txp1);
-            if (st) {
-              Fys = face_ref64<SCH, ULT>(fs, bs, tus, tym1, t0, tym2, typ1);
-              if (nwet) Fyn = face_ref64<SCH, ULT>(fn, bn, tun, t0, typ1, tym1, typ2);
-              if (below) Fzt = face_ref64<SCH, ULT>(ft, bt, tut, t0, tp1, tm1, tp2);
+#pragma unroll 1
+            for (int q = 0; q < 4; ++q) {  // (one call: four would cost registers)
+              const bool w = q == 0, y = q == 1, z = q == 3;
+              const double v = face_ref64<SCH, ULT>(
+                  fw + q * FC_N * 32, w ? bw : y ? bs : z ? bt : bn,
+                  w ? tuw : y ? tus : z ? tut : tun, w ? txm1 : y ? tym1 : t0,
+                  (w || y) ? t0 : z ? tp1 : typ1, w ? txm2 : y ? tym2 : z ? tm1 : tym1,
+                  w ? txp1 : y ? typ1 : z ? tp2 : typ2);
+              if (w) Fxw = v;
+              else if (y) Fys = v;
+              else if (z) Fzt = v;
+              else Fyn = v;
             }
           }
         }
@@ -514,27 +501,21 @@ __global__ void __launch_bounds__(kAdv64Warps * 32, 16)
       }
       double Fxe = __shfl_down_sync(FULL, Fxw, 1);
       if (!st || n >= ntc) continue;
-      if (!sxp) Fxe = 0.0;
+      if (!ewet)  // order1 fills the ghost cells' faces too
+        Fxe = (SCH == SHOC_TR_ORDER1 && adv) ? order1_flux(F.u1flux3d[n1.y], t0, tr[n1.y]) : 0.0;
       if (SCH != SHOC_TR_ORDER1 && !nwet) Fyn = 0.0;
-      if (eslow) {
-        if (fl & FL_XP_WET)
-          Fxe = east_flux(G, F, W, O, Tl, c, adv, hd, tr, dtu);
-        else if (adv)
-          Fxe = order1_flux(F.u1flux3d[n1.y], t0, tr[n1.y]);
-      }
       // dtracer (tracers.c:888-892)
       const double dtr = (Fxe - Fxw + Fyn - Fys) * dtu;
       double val = dtr;
       if (k <= ks) {
-        double Fzb = 0.0;
-        if (!fbot)
-          Fzb = sF[(s - sl0) * 32];
-        else if (fslow && adv)
-          Fzb = floor_flux(F, W, O, c, nzv.x, nzv.z, t0, tp1, dtu);
+        const double Fzb = sF[(s - sl0) * 32];
         if (below) {
           sF[(s - sl0) * 32] = Fzt;
           // interior cell (tracers.c:912-925); Ds = Hn1 = 1 in z coordinates
-          val = t0 - div_known(div_known(dtr, area, yarea, rng) + (Fzt - Fzb), dzc, ydz, rng);
+          const double net = quot(dtr, area, yarea) + (Fzt - Fzb);
+          val = t0 - quot(net, dzc, ydz);
+          if (!((div_fast(dtr, rng) || dtr == 0.0) && (div_fast(net, rng) || net == 0.0)))
+            val = t0 - (dtr / area + (Fzt - Fzb)) / dzc;
         } else {
           fzs[(size_t)n * G.ncol + col] = Fzb;
         }
