@@ -2,6 +2,8 @@
 // launcher.  Compiled with FMA contraction on (the FP64 reference path in
 // shoc_tr_gpu.cu is compiled without it); the FP64 sums of the kernels use
 // explicitly rounded operations where contraction would change them.
+#include <algorithm>
+
 #include "shoc_tr_launch.h"
 
 namespace shoc {
@@ -71,19 +73,19 @@ void tile32_substep(bool last, bool quick, bool ult, cudaStream_t st, const Geo 
                              fzs, any_hd, lo_in);
   }
   if (ev) cudaEventRecord(ev[1], st);
-  const dim3 blk(32, vd_nw);
-  for (int i = 0; i < Tl.nclass; i++) {
-    const int t0 = Tl.ctile[i], nt = Tl.ctile[i + 1] - t0, kbase = Tl.cbase[i];
-    if (nt <= 0) continue;
-    const bool comp = lo_out != nullptr;
-    const size_t smem = vd32_smem(G.nz - kbase, vd_nw, vd_pf != 0, comp);
-    auto kern = comp ? (last ? (vd_pf ? k_vd32<true, true, true> : k_vd32<true, false, true>)
-                             : (vd_pf ? k_vd32<false, true, true> : k_vd32<false, false, true>))
-                     : (last ? (vd_pf ? k_vd32<true, true, false> : k_vd32<true, false, false>)
-                             : (vd_pf ? k_vd32<false, true, false> : k_vd32<false, false, false>));
-    kern<<<nt, blk, smem, st>>>(G, F, W, O, T, ss, Tl, W.lu32, tin, tout, rnd, carry, fzs, lo_in,
-                                lo_out, vd_nw, t0, kbase);
-  }
+  // one launch for every depth: blocks of the shared memory vd_nw warps need at
+  // full depth, and as many warps, for the shallow tiles to use it up, as the
+  // registers allow those blocks (16 warps an SM)
+  const bool comp = lo_out != nullptr;
+  const int bytes = (int)vd32_smem(G.nz, vd_nw, vd_pf != 0, comp);
+  const int blocks = std::max(1, 233472 / (bytes + 1024));
+  const dim3 blk(32, std::min(T.nslot, std::max(vd_nw, kVd32MaxWarps / blocks)));
+  auto kern = comp ? (last ? (vd_pf ? k_vd32<true, true, true> : k_vd32<true, false, true>)
+                           : (vd_pf ? k_vd32<false, true, true> : k_vd32<false, false, true>))
+                   : (last ? (vd_pf ? k_vd32<true, true, false> : k_vd32<true, false, false>)
+                           : (vd_pf ? k_vd32<false, true, false> : k_vd32<false, false, false>));
+  kern<<<Tl.ncolp / 32, blk, bytes, st>>>(G, F, W, O, T, ss, Tl, W.lu32, tin, tout, rnd, carry,
+                                          fzs, lo_in, lo_out, bytes);
   if (ev) cudaEventRecord(ev[2], st);
 }
 

@@ -57,6 +57,15 @@ struct Fused {
   int ngrp;           // advected tracers per phase-A reduction pass
 };
 
+// row j of a column's tridiagonal factors in k_step32's shared memory
+struct FacVec {
+  const float4 *l;
+  __device__ __forceinline__ float dzdt(int j) const { return l[j * 32].x; }
+  __device__ __forceinline__ float cm1(int j) const { return l[j * 32].y; }
+  __device__ __forceinline__ float rdiv(int j) const { return l[j * 32].z; }
+  __device__ __forceinline__ float re(int j) const { return l[j * 32].w; }
+};
+
 // shared memory of k_step32 (bytes) for columns of at most nd layers, nwb
 // phase-B warps, ntb advected tracers and reduction groups of ngrp tracers:
 // LU float4 [nd][32], thicknesses double [nd][32], cells int [nd][32], a
@@ -301,8 +310,10 @@ __global__ void __launch_bounds__(kFusedThreads, 2)
     const double *const D0 = DZ + (kb - kbase) * 32 + lane;
     const bool steady = F.eta[c2] == F.oldeta[c2];
     const int *const C0 = colC + (kb - kbase) * 32 + lane;
-    const float4 *const L0 = LU + (kb - kbase) * 32 + lane;
+    const FacVec fac{LU + (kb - kbase) * 32 + lane};
     const int nk = ks - kb;  // cells below the surface cell
+    double H = D0[nk * 32];  // the water depth
+    for (int j = 0; j < nk; ++j) H += D0[j * 32];
     const double idt = 1.0 / F.dt;  // the residual's diagonal is dz / dt in FP64
     long long nwarn = 0;
     for (int slot = w; slot < T.nslot; slot += nwb) {
@@ -331,9 +342,9 @@ __global__ void __launch_bounds__(kFusedThreads, 2)
                        adv ? accF[slot * 32 + lane] : 0.0};
       bool bad = false;
       cp_async_wait<0>();
-      column_finish<LAST, false>(G, F, W, O, T, ss, tc, col, n, tbdy, adv, vdf, A0, S0, 32, L0,
-                                 C0, D0, tr, to, area, ia, idt, cs, Fu.carry, steady,
-                                 nwarn, bad);
+      column_finish<LAST, false>(G, F, W, O, T, ss, tc, col, n, tbdy, adv, vdf, A0, S0, 32, fac,
+                                 C0, D0, H, tr, to, area, ia, idt, cs, Fu.carry,
+                                 steady, nwarn, bad);
       if (bad) nstat |= ST_NAN;
     }
     if (nwarn) atomicAdd(W.nwarn, (unsigned long long)nwarn);

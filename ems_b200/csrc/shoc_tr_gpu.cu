@@ -272,9 +272,9 @@ constexpr int SD_WORK = 8;    // w5, w9, dbz, dfz of the tile kernels' columns
 constexpr int SD_LU64 = 16;   // FP64 LU factors of the tile kernels' columns
                               // (the general path's columns get all of them)
 constexpr int kSetDzWarps = 8;
-// bytes: FP64 faces (then ud), rows cm1 and dz/dt (then div) and the cells of
-// nz layers of 32 columns
-inline size_t set_dz_smem(int nz) { return (size_t)nz * 32 * (3 * 8 + 4); }
+// bytes: FP64 faces (then ud), rows cm1 and dz/dt (then div; for SD_F32 once
+// more, then the UL diagonal) and the cells of nz layers of 32 columns
+inline size_t set_dz_smem(int nz, bool f32) { return (size_t)nz * 32 * ((f32 ? 4 : 3) * 8 + 4); }
 
 __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
     k_set_dz(Geo G, Flow F, Work W, Opt O, Tile Tl, int any_vdiff, int *counts, int list_all,
@@ -285,7 +285,10 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
   double *const sZ = reinterpret_cast<double *>(smem) + lane;  // bottom face z, then ud
   double *const sCm = sZ + nz * 32;                            // cm1
   double *const sDv = sCm + nz * 32;                           // dz / dt, then div
-  int *const sC = reinterpret_cast<int *>(reinterpret_cast<double *>(smem) + 3 * nz * 32) + lane;
+  double *const sE = sDv + nz * 32;                            // dz / dt, then e (SD_F32)
+  int *const sC = reinterpret_cast<int *>(reinterpret_cast<double *>(smem) +
+                                          ((what & SD_F32) ? 4 : 3) * nz * 32) +
+                  lane;
   __shared__ int sJa[32];        // highest layer <= jn of zero thickness
   __shared__ double sMin[kSetDzWarps];
   const int col = blockIdx.x * 32 + lane;
@@ -365,6 +368,7 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
     if (j <= jn && !dzc) atomicMax(&sJa[lane], j);
     if (any_vdiff) {  // rows of the implicit solve (:3841-3889)
       sDv[k * 32] = dzc / dt;
+      if (what & SD_F32) sE[k * 32] = dzc / dt;
       sCm[k * 32] = -__ldg(&F.Kz[cc]) / (0.5 * (dzm + dzc));
     }
     if (search && j <= js) {
@@ -454,6 +458,21 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
       }
     }
     if (stat) atomicOr(W.status, stat);
+  }
+  if (wy == 1 && solve && (what & SD_F32)) {
+    // the same matrix eliminated from the top (the FP32-mixed correction
+    // solve): e(j) = C(j) - cm1(j+1) cm1(j+1) / e(j+1)
+    const int kt = kb + jn - 1, kl = kb + jb - 1;
+    double up = sCm[kt * 32], e = sE[kt * 32] - up;
+    sE[kt * 32] = e;
+    for (int k = kt - 1; k >= kl; --k) {
+      const double cm1 = k > kl ? sCm[k * 32] : 0.0;
+      e = (sE[k * 32] - cm1 - up) - up * (up / e);
+      sE[k * 32] = e;
+      up = cm1;
+    }
+  }
+  if (wy == 0) {
     if (on) {
       if (!(what & SD_PROBE)) {
         W.sur_t[col] = sur;
@@ -496,7 +515,8 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
         if (what & SD_LU64) W.vd_rdiv[cc] = div_range(div) == kDivLo ? 1.0 / div : 0.0;
       }
       if (what & SD_F32)
-        W.lu32[cc] = make_float4((float)dzdt, (float)cm1, (float)(1.0 / div), (float)ud);
+        W.lu32[cc] =
+            make_float4((float)dzdt, (float)cm1, (float)(1.0 / div), (float)(1.0 / sE[k * 32]));
     }
     if (late) {
       const double dzm = j > 1 ? W.dz[sC[(k - 1) * 32]] : dzsed;
@@ -1011,32 +1031,29 @@ int build_tile_tables(shoc_tr_gpu *h, const shoc_tr_geom *g, const std::vector<u
   // adjacent cells of one layer.  A cell's east neighbour, where it is wet, is
   // the next lane's: a run that goes on beyond the segment, or beyond a warp's
   // last lane, is given a halo lane there.
-  std::vector<uint8_t> is_wet(S, 0);
-  for (int i = 1; i <= g->a3_t; i++) {
-    const int c = g->w3_t[i];
-    if (c > 0 && c < S) is_wet[c] = 1;
-  }
   std::vector<int> wet;
   wet.reserve((size_t)g->a3_t + g->a3_t / 16);
-  for (int col0 = 0; col0 < ncol; col0 += 31)
-    for (int k = nz - 1; k >= 0; k--)
-      for (int col = col0; col < std::min(ncol, col0 + 31); col++) {
-        const int c = cellk[(size_t)k * ncolp + col];
-        if (!c || !is_wet[c]) continue;
-        const int e = in(g->xp1[c]);
-        if ((wet.size() & 31) == 31) {  // a warp's last lane: the cell itself only
-          if (is_wet[e] && !wet.empty() && (wet.back() & ~kSegHalo) != 0 &&
-              in(g->xp1[wet.back() & ~kSegHalo]) == c) {
-            wet.push_back(c | kSegHalo);  // lends its west flux to the lane before it
-          } else if (is_wet[e]) {
-            wet.push_back(-1);
-          }
+  for (int col0 = 0; col0 < ncol; col0 += 31) {
+    const int col1 = std::min(ncol, col0 + 31);
+    for (int k = nz - 1; k >= 0; k--) {
+      const int *row = &cellk[(size_t)k * ncolp];
+      for (int col = col0; col < col1; col++) {
+        const int c = row[col];
+        if (!c || !(fl[c] & CF_WET)) continue;
+        const int e = (fl[c] & FL_XP_WET) ? nb1[c].y : 0;  // its wet east neighbour
+        if ((wet.size() & 31) == 31 && e) {
+          // a warp's last lane: the cell lends its west flux to the lane before
+          // it, or the lane stays empty
+          const int w = wet.back() & ~kSegHalo;
+          wet.push_back((wet.back() >= 0 && (fl[w] & FL_XP_WET) && nb1[w].y == c)
+                            ? c | kSegHalo : -1);
         }
         wet.push_back(c);
         // the run's end in this segment with a wet east neighbour beyond it
-        const int nx = col + 1 < std::min(ncol, col0 + 31) ? cellk[(size_t)k * ncolp + col + 1] : 0;
-        if (is_wet[e] && nx != e) wet.push_back(e | kSegHalo);
+        if (e && (col + 1 >= col1 || row[col + 1] != e)) wet.push_back(e | kSegHalo);
       }
+    }
+  }
   // k_vd32 column order: tiles of 32 adjacent columns (a warp's lanes at one
   // layer are adjacent cells: coalesced loads and stores), the tiles sorted
   // by depth so launches per depth class size shared memory to their tiles
@@ -1061,16 +1078,17 @@ int build_tile_tables(shoc_tr_gpu *h, const shoc_tr_geom *g, const std::vector<u
   // neighbour, or the warp is full, that one is added as a halo lane.
   std::vector<int> col_of_top(h->S2, -1);
   for (int col = 0; col < ncol; col++) col_of_top[g->w2_t[col + 1]] = col;
-  auto east = [&](int col) {
+  std::vector<int> east_of(ncol, -1);
+  for (int col = 0; col < ncol; col++) {
     const int e = in(g->xp1[g->w2_t[col + 1]]);
-    return e < h->S2 ? col_of_top[e] : -1;
-  };
+    if (e < h->S2) east_of[col] = col_of_top[e];
+  }
   std::vector<int> seg;
   for (int col = 0; col < ncol; col++) {
-    const int e = east(col);
+    const int e = east_of[col];
     if ((seg.size() & 31) == 31 && e >= 0) {  // the last lane: a halo lane, or none
       const int b = seg.back();
-      seg.push_back(b >= 0 && !(b & kSegHalo) && east(b) == col ? col | kSegHalo : -1);
+      seg.push_back(b >= 0 && !(b & kSegHalo) && east_of[b] == col ? col | kSegHalo : -1);
     }
     seg.push_back(col);
     if (e >= 0 && e != col + 1) seg.push_back(e | kSegHalo);
@@ -1080,9 +1098,9 @@ int build_tile_tables(shoc_tr_gpu *h, const shoc_tr_geom *g, const std::vector<u
   // column): every column goes the general path
   if (h->O.cross)
     for (int c = 1; c < S; c++) {
-      const int e = in(g->xp1[c]);
-      if (is_wet[c] && is_wet[e] && (east(colof[c]) != colof[e] || g->s2k[c] != g->s2k[e]))
-        h->O.tiled = 0;
+      if ((fl[c] & (CF_WET | FL_XP_WET)) != (CF_WET | FL_XP_WET)) continue;
+      const int e = nb1[c].y;
+      if ((east_of[colof[c]] != colof[e]) || g->s2k[c] != g->s2k[e]) h->O.tiled = 0;
     }
   std::vector<int4> colrec(ncolp, make_int4(0, 0, nz, 0));
   for (int col = 0; col < ncol; col++)
@@ -1616,14 +1634,13 @@ int shoc_tr_gpu_create(const shoc_tr_geom *g, const shoc_tr_opts *o, int ntr, in
   // tiling: tracers per block
   int tw = 8;
   {
-    // tracers (k_vd64) or warps (k_vd32) per column-kernel block: two
-    // blocks per SM at full depth, balanced rounds over the tracers (on
-    // stiff2048 two blocks of 4 warps beat one block of 12: 9.4 against
-    // 11.5 ms for k_vd32)
+    // tracers per k_vd64 block: two blocks per SM at full depth, balanced rounds
+    // over the tracers
     while (tw > 1 && vd_smem(h, g->nz, tw) > 113 * 1024) tw--;
     int nch = (h->nslot + tw - 1) / std::max(tw, 1);
     if (nch > 0) tw = (h->nslot + nch - 1) / nch;
     if (tw < 1) tw = 1;
+    if (f32p) tw = vd32_default_warps(g->nz, h->nslot, h->comp);
   }
   h->tw = tw;
   TRY(build_tile_tables(h, g, cflag, col_bot, col_kb));
@@ -1700,7 +1717,7 @@ int shoc_tr_gpu_create(const shoc_tr_geom *g, const shoc_tr_opts *o, int ntr, in
   h->h_nwarn = (unsigned long long *)((char *)pin + 16);
   h->h_counts = (int *)((char *)pin + 24);
   if (cudaFuncSetAttribute(k_set_dz, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)set_dz_smem(kMaxLayers)) != cudaSuccess ||
+                           (int)set_dz_smem(kMaxLayers, true)) != cudaSuccess ||
       tile64_set_smem_attr() != cudaSuccess ||
       tile32_set_smem_attr() != cudaSuccess)
     TRY(SHOC_TR_ECUDA);
@@ -1782,7 +1799,8 @@ void launch_set_dz(shoc_tr_gpu *h, int what) {
     what |= SD_F32 | (h->comp ? SD_WORK : 0);
   else
     what |= SD_WORK | SD_LU64;
-  k_set_dz<<<h->tl.ncolp / 32, dim3(32, kSetDzWarps), set_dz_smem(h->nz), h->stream>>>(
+  k_set_dz<<<h->tl.ncolp / 32, dim3(32, kSetDzWarps), set_dz_smem(h->nz, (what & SD_F32) != 0),
+             h->stream>>>(
       h->G, h->F, h->W, h->O, h->tl, h->any_vdiff ? 1 : 0, h->d_counts, h->staged ? 1 : 0, what,
       h->colown);
   h->launches++;
@@ -1936,7 +1954,7 @@ int tile64_substep(const shoc_tr_gpu *h, bool last, const SubStep &ss, const Til
   return nl;
 }
 
-// Depth classes of the k_vd32 launches for nw tracers per block: the deepest
+// Depth classes of the k_vd64 launches for nw tracers per block: the deepest
 // tile that still lets 4, 3 and 2 blocks share an SM's shared memory bounds
 // a class; each class is launched with shared memory for its own depth.
 Tile vd_classes(const shoc_tr_gpu *h, int nw) {
@@ -1994,9 +2012,8 @@ int launch_part_b(shoc_tr_gpu *h, const Sched &s, int cur0, const TrSet &T,
         }
         h->launches += h->fu.ntile > 0 ? 1 : 0;
       } else {
-        const Tile tl = vd_classes(h, tw);
         tile32_substep(last, h->O.trasc == SHOC_TR_QUICKEST, h->O.ultimate != 0, st, h->G, h->F,
-                       h->F3, h->W, h->O, T, ss, tl, h->fx2, h->fy2, tin, tout, h->rnd,
+                       h->F3, h->W, h->O, T, ss, h->tl, h->fx2, h->fy2, tin, tout, h->rnd,
                        h->fu.carry, h->fzs64, h->comp ? h->lo[cur] : nullptr,
                        h->comp ? h->lo[cur ^ 1] : nullptr, tw, h->vd_pf ? 1 : 0,
                        h->any_hdiff ? 1 : 0, h->adv_flags, prof ? ev : nullptr);
@@ -2005,8 +2022,7 @@ int launch_part_b(shoc_tr_gpu *h, const Sched &s, int cur0, const TrSet &T,
           h->ev.push_back({1, ev[0], ev[1]});
           h->ev.push_back({2, ev[1], ev[2]});
         }
-        h->launches += (T.ntb > 0 && tl.nwet > 0 ? 1 : 0);
-        for (int k = 0; k < tl.nclass; k++) h->launches += tl.ctile[k + 1] > tl.ctile[k] ? 1 : 0;
+        h->launches += (T.ntb > 0 && h->tl.nwet > 0 ? 1 : 0) + 1;
       }
       int16_t *lo_out = h->comp ? h->lo[cur ^ 1] : nullptr;
       launch_general<float>(h, last, T, ss, tin, tout, c3row, c3_load, lo_out);

@@ -122,7 +122,8 @@ struct Work {
   unsigned long long *dtm_bits;
   unsigned long long *nwarn;
   int *serial_list, *serial_count;
-  // FP32-mixed path: layer thickness and LU factors {dzdt, cm1, 1/div, ud}
+  // FP32-mixed path: layer thickness and the solve's factors {dzdt, cm1, 1/div,
+  // 1/e}: div the diagonal eliminated from the bottom, e from the top
   float *dz32;
   float4 *lu32;
 };
@@ -140,9 +141,9 @@ struct Tile {
   const int *colof;  // [S] 0-based column of each wet cell
   const int *wet;    // [nwet] k_adv32's cells, a lane each: cell, cell | kSegHalo (lends
                      // its west flux only), -1: none
-  const int *vdcol;  // [ncolp] columns in k_vd32 order: whole tiles of 32
+  const int *vdcol;  // [ncolp] columns in the column kernels' order: whole tiles of 32
                      // adjacent columns, shallow tiles first (-1: padding)
-  int nclass;        // k_vd32 depth classes: tiles [ctile[i], ctile[i+1]) have
+  int nclass;        // k_vd64 depth classes: tiles [ctile[i], ctile[i+1]) have
   int ctile[5];      //   no cell below layer cbase[i]
   int cbase[4];
   const int4 *colrec;  // [ncolp] bottom cell, surface-layer cell, bottom layer

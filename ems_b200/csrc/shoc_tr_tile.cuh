@@ -402,7 +402,10 @@ struct ColSums {
 // A0, S0: the column's values and Thomas storage from its bottom layer up, row
 // stride sa; an advected tracer (tbdy) holds its advected values below the
 // surface, any other tracer every layer's old value (A0 is overwritten, so is
-// S0).  L0, C0, D0: LU factors, cells and FP64 thicknesses, row stride 32.
+// S0).  fac: the tridiagonal factors of row j: dzdt, cm1, and the reciprocal
+// diagonals rdiv (eliminated from the bottom: LU) and re (from the top: UL).  C0, D0: cells and
+// FP64 thicknesses, row stride 32; H: the water depth the carry is spread over,
+// the thicknesses from the surface cell's and then the bottom up.
 // RES: an advected tracer's A0 holds every layer's stored advection result
 // and S0 its rounding residual (k_vd32), and the column sums cs.m and cs.dv
 // are taken from them; else they come in cs (k_step32).
@@ -410,13 +413,13 @@ struct ColSums {
 // sets bad for a NaN among what it stores.  The mass bookkeeping sums are
 // plain FP64 sums of at most nz terms: their rounding (a few 1e-16 of the
 // column mass, of either sign) is what the carry may miss per step.
-template <bool LAST, bool RES>
+template <bool LAST, bool RES, class Fac>
 __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const Work &W,
                                               const Opt &O, const TrSet &T, const SubStep &ss,
                                               const TileCol &tc, int col, int n, bool tbdy,
                                               bool adv, bool vdf, float *A0, float *S0, int sa,
-                                              const float4 *L0, const int *C0, const double *D0,
-                                              const float *tr, float *to, double area, double ia,
+                                              const Fac &fac, const int *C0, const double *D0,
+                                              double H, const float *tr, float *to, double area, double ia,
                                               double idt, ColSums cs,
                                               double *carry, bool steady, long long &nwarn,
                                               bool &bad, int16_t *R0 = nullptr,
@@ -441,7 +444,6 @@ __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const
   double mxs = 0.0, mss = 0.0;
   long long nw = 0;
   double vs = ts_old;  // the surface value
-  double H = dzs;      // the water depth the carry is spread over
   // tr_bounds clip and range check (:3278-3293) of the cells below the
   // surface (advected tracers); a < mn and a > mx of a float a, exactly, as
   // float compares
@@ -463,13 +465,12 @@ __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const
   }
   // one pass up the column below the surface: the computed mass (an
   // advected tracer's FP64 values are stored + residual, or come in cs.m),
-  // the clip, the depth and, with a solve, the FP32 forward sweep
+  // the clip and, with a solve, the FP32 forward sweep
   float fwd = 0.f;  // the bottom row's cm1 is 0
   double m = 0.0;
   for (int j = 0; j < nk; ++j) {
     float a = A0[j * sa];
     const double dz = D0[j * 32];
-    H += dz;
     // the row's value - stored: the advection's rounding residual, or the
     // old value's compensation
     double r = 0.0;
@@ -480,15 +481,12 @@ __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const
       mxs += ((double)mnf - ((double)a + r)) * dz;
       a = mnf;
       r = 0.0;
-    }
-    if (R0) R0[j * sa] = lo_bits((float)r);
-    if (tbdy) {
-      nw += (a < mn_up || a > mx_dn);
       A0[j * sa] = a;
     }
+    if (R0) R0[j * sa] = lo_bits((float)r);
+    if (tbdy) nw += (a < mn_up || a > mx_dn);
     if (solve) {
-      const float4 lu = L0[j * 32];
-      fwd = (lu.x * a - lu.y * fwd) * lu.z;
+      fwd = (fac.dzdt(j) * a - fac.cm1(j) * fwd) * fac.rdiv(j);
       S0[j * sa] = fwd;
     }
   }
@@ -552,63 +550,48 @@ __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const
     store(ci.s, (vdf && single) ? vs + dl + F.dt * (0.0 - 0.0) / h : vs + dl, dzs);
   } else {
     // the surface row of the forward sweep
-    {
-      const float4 lu = L0[nk * 32];
-      A0[nk * sa] = (float)vs;
-      fwd = (lu.x * (float)vs - lu.y * fwd) * lu.z;
-      S0[nk * sa] = fwd;
-    }
-    // back substitution (FP32), x(j) replacing s(j), and one row behind it
-    // the FP64 residual of b - A x for A = dz/dt I + the diffusion operator,
+    fwd = (fac.dzdt(nk) * (float)vs - fac.cm1(nk) * fwd) * fac.rdiv(nk);
+    // one pass down: the back substitution (FP32), x(j) replacing s(j), and one
+    // row behind it the FP64 residual of b - A x for A = dz/dt I + the diffusion
+    // operator,
     //   r(j) = dz/dt (a + dl - x) - cm1 (x(j-1) - x) - cp1 (x(j+1) - x)
     // (cp1(j) = cm1(j+1); the bottom row has no cm1 term, the top row no cp1
-    // term), which replaces a(j).  Its diagonal is the FP64 dz / dt, so the
-    // refined solve keeps the column mass the mass diagnostic measures; cm1
-    // is the FP32 factor's (the FP64 one, staged as well, changed neither
-    // the maximum nor the RMS error over 1000 stiff2048 steps, and its
+    // term), whose correction solve's elimination, from the top (UL), follows in
+    // the same pass, g(j) replacing a(j).  The residual's diagonal is the FP64
+    // dz / dt, so the refined solve keeps the column mass the mass diagnostic
+    // measures; cm1 is the FP32 factor's (the FP64 one, staged as well, changed
+    // neither the maximum nor the RMS error over 1000 stiff2048 steps, and its
     // shared memory cost warps).  The FP64 copies of x and of the factors are
     // carried from row to row.
-    float x1 = fwd;
-    float4 l1 = L0[nk * 32];
-    double xd1 = (double)x1, xd2 = 0.0, l2y = 0.0;
+    S0[nk * sa] = fwd;
+    float x1 = fwd, g = 0.f, l2 = 0.f;  // x, cm1 of row j + 1; cm1 of row j + 2
+    float l1 = fac.cm1(nk);
+    double xd1 = (double)x1, xd2 = 0.0;
     double dzdt1 = dzs * idt;
+    double a1 = vs;  // the value before the solve of row j + 1
     for (int j = nk - 1; j >= 0; --j) {
-      const float x = S0[j * sa] - l1.w * x1;
+      const float x = S0[j * sa] - l1 * fac.rdiv(j) * x1;
       S0[j * sa] = x;
-      const double xd = (double)x, l1y = (double)l1.y;
-      const double aj1 =
-          ((j + 1 == nk) ? vs
-                         : (double)A0[(j + 1) * sa] +
-                               (R0 ? (double)lo_val(R0[(j + 1) * sa]) : 0.0)) +
-          dl;
-      double r = dzdt1 * (aj1 - xd1) - l1y * (xd - xd1);
-      if (j + 1 < nk) r = r - l2y * (xd2 - xd1);
-      A0[(j + 1) * sa] = (float)r;
+      const double xd = (double)x;
+      double r = dzdt1 * ((a1 + dl) - xd1) - (double)l1 * (xd - xd1);
+      if (j + 1 < nk) r = r - (double)l2 * (xd2 - xd1);
+      a1 = (double)A0[j * sa] + (R0 ? (double)lo_val(R0[j * sa]) : 0.0);
+      g = ((float)r - l2 * g) * fac.re(j + 1);
+      A0[(j + 1) * sa] = g;
       x1 = x;
       xd2 = xd1;
       xd1 = xd;
-      l2y = l1y;
-      l1 = L0[j * 32];
+      l2 = l1;
+      l1 = fac.cm1(j);
       dzdt1 = D0[j * 32] * idt;
     }
-    {
-      const double a0 =
-          ((nk == 0) ? vs : (double)A0[0] + (R0 ? (double)lo_val(R0[0]) : 0.0)) + dl;
-      double r = dzdt1 * (a0 - xd1);
-      if (nk > 0) r = r - l2y * (xd2 - xd1);
-      A0[0] = (float)r;
-    }
-    // correction solve (FP32 forward and back) and the update in FP64
-    float u = 0.f;
-    for (int j = 0; j <= nk; ++j) {
-      const float4 lu = L0[j * 32];
-      u = (A0[j * sa] - lu.y * u) * lu.z;
-      A0[j * sa] = u;
-    }
-    float d = A0[nk * sa];
-    store(C0[nk * 32], (double)S0[nk * sa] + (double)d, dzs);
-    for (int j = nk - 1; j >= 0; --j) {
-      d = A0[j * sa] - L0[(j + 1) * 32].w * d;
+    double r = dzdt1 * ((a1 + dl) - xd1);
+    if (nk > 0) r = r - (double)l2 * (xd2 - xd1);
+    // up again: the correction's back substitution and the update in FP64
+    float d = ((float)r - l2 * g) * fac.re(0);
+    store(C0[0], (double)S0[0] + (double)d, D0[0]);
+    for (int j = 1; j <= nk; ++j) {
+      d = A0[j * sa] - fac.cm1(j) * fac.re(j) * d;
       store(C0[j * 32], (double)S0[j * sa] + (double)d, D0[j * 32]);
     }
   }
@@ -619,139 +602,200 @@ __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const
 // ---------------------------------------------------------------------------
 // k_vd32
 
-// k_vd32: a block is one tile of 32 columns and nw warps (at most
-// kVd32MaxWarps); the tile's tracer-independent column arrays are staged
-// once and each warp steps its share of the tracers through them (PF: with
-// the next tracer's column staged while the current one is solved).
+// k_vd32: a block is one tile of 32 columns, deepest tiles first; the tile's
+// tracer-independent column arrays are staged once and each warp steps its
+// share of the tracers through them.  Every block has the same shared memory,
+// of which a warp takes as much as the tile is deep: a full-depth tile runs the
+// handle's warps per block, a shallow one more, and one launch serves every
+// depth.
+//
+// What bounds it: latency (shared memory and conversions in each thread's
+// chains along the column) at the 8 to 16 warps an SM holds (128 registers a
+// thread, and the shared memory; vd32_default_warps).  So
+// - the correction solve is eliminated from the top, in the pass that forms the
+//   residual: a tracer takes three passes along the column instead of four;
+// - the factors are arrays of one float a lane, of which a pass reads those it
+//   needs (a float4 a row made 35 shared-memory wavefronts a row of what are now
+//   24), and the water depth is summed once per column;
+// - the warp's lanes stay together: tracers are taken in step, those a column
+//   does not carry being left out.
+// Fetching the next tracer's rows into the current one's as its last pass frees
+// them cost more than it hid (2.90 against 2.57 ms on the first case below).
+// A sub-step (B200), before and now: 1024 x 512 x 50, 24 tracers 2.86 and 2.42 ms;
+// 448 x 300 x 50, 16 tracers, FP32_COMP 0.91 and 0.72; 333 x 217 x 37, 5 tracers
+// 0.128 and 0.080; a batch of 56 447 columns, 60 layers, 4 to 32 tracers 0.93 and
+// 0.69.
+
 constexpr int kVd32MaxWarps = 16;
 // shared memory of k_vd32 (bytes) for columns of at most nd layers:
-// LU float4[nd][32], thicknesses double[nd][32], colC int[nd][32], A, S
-// float[nd][nw][32] (twice with pf: the next tracer's column is staged
+// thicknesses double[nd][32], four factors float[nd][32], cells int[nd][32], A,
+// S float[nd][nw][32] (twice with pf: the next tracer's column is staged
 // while the current one is solved), with comp (FP32_COMP) R, compensations
 // int16[nd][nw][32]
 inline size_t vd32_smem(int nd, int nw, bool pf = false, bool comp = false) {
-  return (size_t)nd * 32 * (16 + 8 + 4) + (size_t)(pf ? 4 : 2) * nd * nw * 32 * 4 +
+  return (size_t)nd * 32 * (8 + 4 * 4 + 4) + (size_t)(pf ? 4 : 2) * nd * nw * 32 * 4 +
          (comp ? (size_t)nd * nw * 32 * 2 : 0);
 }
+// Warps per k_vd32 block at full depth where the caller sets none: the most
+// blocks per SM (up to four) that leave a block three warps, else two blocks,
+// within 196 KB of an SM's memory.  Filling the 227 KB takes the L1 the column's
+// loads go through: 1024 x 512 x 50 (24 tracers) 4 warps 2.42 ms, 5 warps 2.60;
+// 333 x 217 x 37 (5 tracers) three blocks of 3 warps 0.080 ms, of 4 0.091, two of
+// 5 0.108; a batch of 60 layers (32 tracers) two of 2 warps 0.69, of 4 0.86.
+inline int vd32_default_warps(int nz, int nslot, bool comp) {
+  int nw = 1;
+  for (int b = 4; b >= 2; b--) {
+    nw = 1;
+    while (nw < kVd32MaxWarps && b * (vd32_smem(nz, nw + 1, false, comp) + 1024) <= 196 * 1024)
+      nw++;
+    if (nw >= 3) break;
+  }
+  // balanced rounds over the tracers
+  const int rounds = nslot > 0 ? (nslot + nw - 1) / nw : 1;
+  return nslot > 0 ? (nslot + rounds - 1) / rounds : 1;
+}
+// row j of a column's factors in k_vd32's shared memory (p: the column's dzdt
+// at its bottom row, n: floats per factor)
+struct FacSmem {
+  const float *p;
+  int n;
+  __device__ __forceinline__ float dzdt(int j) const { return p[j * 32]; }
+  __device__ __forceinline__ float cm1(int j) const { return p[n + j * 32]; }
+  __device__ __forceinline__ float rdiv(int j) const { return p[2 * n + j * 32]; }
+  __device__ __forceinline__ float re(int j) const { return p[3 * n + j * 32]; }
+};
 
 // COMP: FP32_COMP, each value's 16-bit compensation read from loi and
 // written to loo ([ntr][S] like the values)
 template <bool LAST, bool PF, bool COMP>
-__global__ void __launch_bounds__(kVd32MaxWarps * 32) k_vd32(Geo G, Flow F, Work W, Opt O,
-                                                             TrSet T, SubStep ss, Tile Tl,
-                                                             const float4 *__restrict__ lu32,
-                                                             const float *__restrict__ tri,
-                                                             float *__restrict__ tro,
-                                                             const float *__restrict__ rsi,
-                                                             double *__restrict__ carry,
-                                                             const double *__restrict__ fzs,
-                                                             const int16_t *__restrict__ loi,
-                                                             int16_t *__restrict__ loo,
-                                                             int nw, int tile0, int kbase) {
+__global__ void __launch_bounds__(kVd32MaxWarps * 32)
+    k_vd32(Geo G, Flow F, Work W, Opt O, TrSet T, SubStep ss, Tile Tl,
+           const float4 *__restrict__ lu32, const float *__restrict__ tri,
+           float *__restrict__ tro, const float *__restrict__ rsi, double *__restrict__ carry,
+           const double *__restrict__ fzs, const int16_t *__restrict__ loi,
+           int16_t *__restrict__ loo, int smem_bytes) {
   extern __shared__ __align__(16) unsigned char smem[];
-  // the arrays hold layers kbase .. nz-1 (every column of this launch's
-  // tiles starts at or above kbase), row r = layer - kbase
-  const int nz = G.nz, nd = nz - kbase;
-  float4 *LU = reinterpret_cast<float4 *>(smem);          // [nd][32]
-  double *DZ = reinterpret_cast<double *>(LU + nd * 32);  // [nd][32]
-  int *colC = reinterpret_cast<int *>(DZ + nd * 32);      // [nd][32]
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x, wy = threadIdx.y;
+  const int tile = gridDim.x - 1 - blockIdx.x;  // (the tiles are sorted by depth)
+  const int col = Tl.vdcol[tile * 32 + lane];
+  const TileCol tc = tile_column(G, W, Tl, col);
+  const bool act = tc.act;
+  const int kb = tc.kb, ks = tc.ks, cbot = tc.cbot, c2 = tc.c2;
+  // the arrays hold layers kbase .. nz-1, row r = layer - kbase
+  const int nz = G.nz, kbase = __reduce_min_sync(FULL, act ? kb : nz), nd = nz - kbase;
+  if (nd == 0) return;
+  // warps that step tracers: what the shared memory holds at this depth
+  constexpr int per_row = (PF ? 4 : 2) * 4 + (COMP ? 2 : 0);
+  const int nw = min((int)blockDim.y, (smem_bytes / (nd * 32) - (8 + 4 * 4 + 4)) / per_row);
+  double *DZ = reinterpret_cast<double *>(smem);      // [nd][32]
+  float *LU = reinterpret_cast<float *>(DZ + nd * 32);  // [4][nd][32]
+  int *colC = reinterpret_cast<int *>(LU + 4 * nd * 32);  // [nd][32]
   // per buffer (two with PF): A, S float [nd][nw][32]; then R (COMP)
   float *const bufs = reinterpret_cast<float *>(colC + nd * 32);
-
-  const int lane = threadIdx.x, wy = threadIdx.y;
-  const int tile = tile0 + blockIdx.x;
-  const int col = Tl.vdcol[tile * 32 + lane];
   const int sa = nw * 32;
 
-  const TileCol tc = tile_column(G, W, Tl, col);
-  bool act = tc.act;
-  if (act && tc.kb < kbase) {  // not in this launch's depth class
-    act = false;
-    if (wy == 0) atomicOr(W.status, ST_GEOM);
-  }
-  const int kb = tc.kb, ks = tc.ks, cbot = tc.cbot, c2 = tc.c2;
   // the tile's tracer-independent column arrays, once for every tracer
-  const int kmin = __reduce_min_sync(0xffffffffu, act ? kb : nz);
-  for (int k = kmin + wy; k < nz; k += nw) {
+  for (int k = kbase + wy; k < nz; k += blockDim.y) {
     const int c = (act && k >= kb) ? Tl.cellk[(size_t)k * Tl.ncolp + col] : 0;
     const int r = k - kbase;
     colC[r * 32 + lane] = c;
-    if (LAST && c && k <= ks) cp_async16(&LU[r * 32 + lane], &lu32[c]);
+    if (LAST && c && k <= ks) {
+      const float *lu = reinterpret_cast<const float *>(&lu32[c]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) cp_async4(&LU[(q * nd + r) * 32 + lane], lu + q);
+    }
     if (c && k <= ks) cp_async8(&DZ[r * 32 + lane], &W.dz[c]);
   }
   cp_async_commit();
   cp_async_wait<0>();
   __syncthreads();
-  if (!act) return;
+  if (wy >= nw) return;
 
-  const size_t off = (size_t)wy * 32 + lane + (size_t)(kb - kbase) * sa;
+  const int row0 = act ? kb - kbase : 0;
+  const size_t off = (size_t)wy * 32 + lane + (size_t)row0 * sa;
   auto A0of = [&](int b) { return bufs + (size_t)b * 2 * nd * sa + off; };
   auto S0of = [&](int b) { return bufs + (size_t)b * 2 * nd * sa + (size_t)nd * sa + off; };
   int16_t *const R0 =
       COMP ? reinterpret_cast<int16_t *>(bufs + (size_t)(PF ? 4 : 2) * nd * sa) + off : nullptr;
-  const float4 *const L0 = LU + (kb - kbase) * 32 + lane;
-  const int *const C0 = colC + (kb - kbase) * 32 + lane;
-  const double *const D0 = DZ + (kb - kbase) * 32 + lane;
-  const double area = G.cellarea[c2], ia = 1.0 / area;
-  const bool steady = F.eta[c2] == F.oldeta[c2];
-  const int ntc = G.colntr[col];
-  const int sed = G.zm1[cbot];
+  const FacSmem fac{LU + row0 * 32 + lane, nd * 32};
+  const int *const C0 = colC + row0 * 32 + lane;
+  const double *const D0 = DZ + row0 * 32 + lane;
+  double area = 1.0, ia = 1.0, H = 0.0;
+  bool steady = false;
+  int ntc = 0, sed = 0;
+  if (act) {
+    area = G.cellarea[c2];
+    ia = 1.0 / area;
+    steady = F.eta[c2] == F.oldeta[c2];
+    ntc = G.colntr[col];
+    sed = G.zm1[cbot];
+    H = D0[(ks - kb) * 32];  // the water depth
+    for (int j = 0; j < ks - kb; ++j) H += D0[j * 32];
+  }
+  const int nl = act ? nz - kb : 0;
   // the column's values of slot s into buffer b, one batch of asynchronous
-  // copies: advection results and their rounding residuals (advected
-  // tracers; the residuals go to the Thomas storage until the sweep) or the
-  // old values (the rest)
+  // copies: advection results and their rounding residuals (advected tracers;
+  // the residuals go to the Thomas storage until the sweep) or the old values
+  // (the rest)
   auto stage = [&](int s, int b) {
-    const int n = T.slot_tr[s];
-    const bool tb = (T.trf[n] & TR_TBDY) != 0;
-    const float *src = (tb ? tro : tri) + (size_t)n * G.S;
-    float *const A0 = A0of(b), *const S0 = S0of(b);
-    for (int j = 0; j < nz - kb; ++j) cp_async4(&A0[j * sa], src + C0[j * 32]);
-    if (tb) {
+    if (s < T.nslot) {
+      const int n = T.slot_tr[s];
+      const bool tb = (T.trf[n] & TR_TBDY) != 0;
+      const float *src = (tb ? tro : tri) + (size_t)n * G.S;
       const float *rs = rsi + (size_t)n * G.S;
-      for (int j = 0; j < nz - kb; ++j) cp_async4(&S0[j * sa], rs + C0[j * 32]);
+      float *const A0 = A0of(b), *const S0 = S0of(b);
+      const int rows = n < ntc ? nl : 0;
+      for (int j = 0; j < rows; ++j) {
+        const int c = C0[j * 32];
+        cp_async4(&A0[j * sa], src + c);
+        if (tb) cp_async4(&S0[j * sa], rs + c);
+      }
     }
     cp_async_commit();
   };
-  // warp wy takes the tracers wy, wy + nw, ... the column carries
+  // warp wy takes the tracers wy, wy + nw, ... that a column of the tile carries
+  const int ntmax = __reduce_max_sync(FULL, ntc);
   auto next = [&](int s) {
     for (; s < T.nslot; s += nw)
-      if (T.slot_tr[s] < ntc) return s;
+      if (T.slot_tr[s] < ntmax) return s;
     return T.nslot;
   };
   long long nwarn = 0;
   bool bad = false;  // a NaN among the values this thread stores
   int slot = next(wy), b = 0;
-  if (PF && slot < T.nslot) stage(slot, 0);
+  if (slot < T.nslot) stage(slot, 0);
   while (slot < T.nslot) {
     const int nxt = next(slot + nw);
     if (PF) {  // the next tracer's column is copied while this one is solved
-      if (nxt < T.nslot) {
-        stage(nxt, b ^ 1);
-        cp_async_wait<1>();
-      } else {
-        cp_async_wait<0>();
-      }
+      stage(nxt, b ^ 1);
+      cp_async_wait<1>();
     } else {
-      stage(slot, 0);
+      cp_async_wait<0>();
     }
     const int n = T.slot_tr[slot];
-    const int tf = T.trf[n];
-    const bool tbdy = (tf & TR_TBDY) != 0;
-    const bool adv = tbdy && (tf & TR_ADV);
-    const bool vdf = LAST && (tf & TR_VDIFF);
-    const float *tr = tri + (size_t)n * G.S;
-    float *to = tro + (size_t)n * G.S;
-    to[sed] = tbdy ? tr[cbot] : tr[sed];  // sediment ghost (tracers.c:827-830)
-    const int16_t *li = COMP ? loi + (size_t)n * G.S : nullptr;
-    int16_t *lo = COMP ? loo + (size_t)n * G.S : nullptr;
-    if (COMP) lo[sed] = tbdy ? li[cbot] : li[sed];
-    const ColSums cs{0.0, 0.0, adv ? fzs[(size_t)n * G.ncol + col] : 0.0};
-    if (!PF) cp_async_wait<0>();
-    column_finish<LAST, true>(G, F, W, O, T, ss, tc, col, n, tbdy, adv, vdf, A0of(b), S0of(b),
-                              sa, L0, C0, D0, tr, to, area, ia, 1.0 / F.dt, cs, carry, steady,
-                              nwarn, bad, R0, li, lo);
+    if (n < ntc) {
+      const int tf = T.trf[n];
+      const bool tbdy = (tf & TR_TBDY) != 0;
+      const bool adv = tbdy && (tf & TR_ADV);
+      const bool vdf = LAST && (tf & TR_VDIFF);
+      const float *tr = tri + (size_t)n * G.S;
+      float *to = tro + (size_t)n * G.S;
+      to[sed] = tbdy ? tr[cbot] : tr[sed];  // sediment ghost (tracers.c:827-830)
+      const int16_t *li = COMP ? loi + (size_t)n * G.S : nullptr;
+      int16_t *lo = COMP ? loo + (size_t)n * G.S : nullptr;
+      if (COMP) lo[sed] = tbdy ? li[cbot] : li[sed];
+      const ColSums cs{0.0, 0.0, adv ? fzs[(size_t)n * G.ncol + col] : 0.0};
+      column_finish<LAST, true>(G, F, W, O, T, ss, tc, col, n, tbdy, adv, vdf, A0of(b), S0of(b),
+                                sa, fac, C0, D0, H, tr, to, area, ia, 1.0 / F.dt, cs, carry,
+                                steady, nwarn, bad, R0, li, lo);
+    }
+    __syncwarp();
     slot = nxt;
-    if (PF) b ^= 1;
+    if (PF)
+      b ^= 1;
+    else if (slot < T.nslot)
+      stage(slot, 0);
   }
   if (bad) atomicOr(W.status, ST_NAN);
   if (nwarn) atomicAdd(W.nwarn, (unsigned long long)nwarn);
