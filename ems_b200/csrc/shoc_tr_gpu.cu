@@ -100,7 +100,6 @@ struct shoc_tr_gpu {
     int ntile = 0;
   } ftile[3];
   int fnwb_max = 0;                   // phase-B warps k_step32 may have (0: no k_step32)
-  std::vector<int> vd_depth;          // layers of the k_vd32 tiles, in their (sorted) order
   bool staged = false;                // column-tile fast path
   int cur = 0;
   int *bpt = nullptr, *bin = nullptr;
@@ -971,11 +970,7 @@ __global__ void k_halo_unpack(TR *tra, TR *trb, int S, int ntr, const int *cells
   }
 }
 
-// shared memory of the column kernel of the handle's precision
 cudaError_t tile64_set_smem_attr();
-size_t vd_smem(const shoc_tr_gpu *h, int nd, int nw) {
-  return h->esize == sizeof(float) ? vd32_smem(nd, nw, h->vd_pf, h->comp) : vd64_smem(nd, nw);
-}
 
 // Static tables of the column-tile kernel: the cell of every column at every
 // layer (cells are numbered layer by layer, so a column's cells are found by
@@ -1067,10 +1062,8 @@ int build_tile_tables(shoc_tr_gpu *h, const shoc_tr_geom *g, const std::vector<u
   }
   std::stable_sort(tord.begin(), tord.end(), [&](int a, int b) { return tdepth[a] < tdepth[b]; });
   std::vector<int> vdcol(ncolp, -1);
-  h->vd_depth.resize(ntile);
   for (int i = 0; i < ntile; i++) {
     const int t = tord[i];
-    h->vd_depth[i] = tdepth[t];
     for (int l = 0; l < 32; l++) vdcol[i * 32 + l] = (t * 32 + l < ncol) ? t * 32 + l : -1;
   }
   // k_adv64's segments: columns in order, 32 to a warp.  A column's wet east
@@ -1218,8 +1211,9 @@ int apply_tuning(shoc_tr_gpu *h, const shoc_tr_tuning &t) {
   if (t.tracers_per_block < 1 || t.tracers_per_block > (f32 ? kVd32MaxWarps : 8))
     return SHOC_TR_EUNSUPPORTED;
   if (t.prefetch && !f32) return SHOC_TR_EUNSUPPORTED;
+  // (FP64: two values a row and warp must fit; k_vd64 takes the warps that do)
   const size_t vb = f32 ? vd32_smem(h->nz, t.tracers_per_block, t.prefetch != 0, h->comp)
-                        : vd64_smem(h->nz, t.tracers_per_block);
+                        : (size_t)h->nz * 32 * (4 + 2 * 8 * t.tracers_per_block);
   if (vb > 227 * 1024) return SHOC_TR_EUNSUPPORTED;
   if (t.fused) {
     const int ti = tile_index(t.tile_x);
@@ -1631,17 +1625,9 @@ int shoc_tr_gpu_create(const shoc_tr_geom *g, const shoc_tr_opts *o, int ntr, in
     TRY(dupload<double>(h, &h->fu.carry, nullptr, (size_t)ntr * ncol));
   }
   TRY(dupload<double>(h, &h->fzs64, nullptr, (size_t)ntr * ncol));
-  // tiling: tracers per block
-  int tw = 8;
-  {
-    // tracers per k_vd64 block: two blocks per SM at full depth, balanced rounds
-    // over the tracers
-    while (tw > 1 && vd_smem(h, g->nz, tw) > 113 * 1024) tw--;
-    int nch = (h->nslot + tw - 1) / std::max(tw, 1);
-    if (nch > 0) tw = (h->nslot + nch - 1) / nch;
-    if (tw < 1) tw = 1;
-    if (f32p) tw = vd32_default_warps(g->nz, h->nslot, h->comp);
-  }
+  // tiling: warps per column-kernel block
+  const int tw = f32p ? vd32_default_warps(g->nz, h->nslot, h->comp)
+                      : vd64_default_warps(g->nz, h->nslot);
   h->tw = tw;
   TRY(build_tile_tables(h, g, cflag, col_bot, col_kb));
   {  // face columns of the transport-mode preamble
@@ -1875,7 +1861,7 @@ void launch_general(shoc_tr_gpu *h, bool last, const TrSet &T, const SubStep &ss
 }
 
 // One FP64 transport sub-step over the staged columns: k_adv64, then one
-// k_vd64 launch per depth class.  Returns the kernels launched.
+// k_vd64.  Returns the kernels launched.
 //
 // Layers per warp of k_adv64: a longer climb computes fewer bottom faces twice
 // (one per chunk), a shorter one gives more warps.  The chip holds 148 x 16;
@@ -1934,49 +1920,18 @@ int tile64_substep(const shoc_tr_gpu *h, bool last, const SubStep &ss, const Til
     nl++;
   }
   if (ev) cudaEventRecord(ev[1], st);
-  const int nchunk = (T.nslot + nw - 1) / nw;
-  const dim3 blk(32, nw);
-  for (int i = 0; i < tl.nclass; i++) {
-    const int t0 = tl.ctile[i], nt = tl.ctile[i + 1] - t0, kbase = tl.cbase[i];
-    if (nt <= 0) continue;
-    const size_t smem = vd64_smem(h->nz - kbase, nw);
-    if (last)
-      k_vd64<true><<<nt * nchunk, blk, smem, st>>>(
-          h->G, h->F, h->W, h->O, T, ss, tl, tin, tout, h->fzs64, h->W.vd_dzdt, h->W.vd_cm1,
-          h->W.vd_div, h->W.vd_rdiv, h->W.vd_ud, nw, nchunk, t0, kbase);
-    else
-      k_vd64<false><<<nt * nchunk, blk, smem, st>>>(
-          h->G, h->F, h->W, h->O, T, ss, tl, tin, tout, h->fzs64, h->W.vd_dzdt, h->W.vd_cm1,
-          h->W.vd_div, h->W.vd_rdiv, h->W.vd_ud, nw, nchunk, t0, kbase);
-    nl++;
-  }
+  const int bytes = (int)std::min<size_t>(vd64_smem(h->nz, nw), 227 * 1024);
+  const int blocks = std::max(1, 233472 / (bytes + 1024));
+  const dim3 blk(32, std::min(T.nslot, std::max(nw, kVd64MaxWarps / blocks)));
+  if (last)
+    k_vd64<true><<<tl.ncolp / 32, blk, bytes, st>>>(h->G, h->F, h->W, h->O, T, ss, tl, tin, tout,
+                                                    h->fzs64, bytes);
+  else
+    k_vd64<false><<<tl.ncolp / 32, blk, bytes, st>>>(h->G, h->F, h->W, h->O, T, ss, tl, tin, tout,
+                                                     h->fzs64, bytes);
+  nl++;
   if (ev) cudaEventRecord(ev[2], st);
   return nl;
-}
-
-// Depth classes of the k_vd64 launches for nw tracers per block: the deepest
-// tile that still lets 4, 3 and 2 blocks share an SM's shared memory bounds
-// a class; each class is launched with shared memory for its own depth.
-Tile vd_classes(const shoc_tr_gpu *h, int nw) {
-  Tile t = h->tl;
-  const int ntile = (int)h->vd_depth.size();
-  const size_t per_layer = vd_smem(h, 1, nw);
-  const size_t sm = 233472, rsv = 1024;
-  t.nclass = 0;
-  t.ctile[0] = 0;
-  int start = 0;
-  for (int blocks = 4; blocks >= 1 && start < ntile; blocks--) {
-    int dmax = (int)((sm / blocks - rsv) / per_layer);
-    if (blocks == 1 || dmax >= h->nz) dmax = h->nz;
-    int end = start;
-    while (end < ntile && h->vd_depth[end] <= dmax) end++;
-    if (end == start) continue;
-    t.cbase[t.nclass] = h->nz - h->vd_depth[end - 1];
-    t.ctile[++t.nclass] = end;
-    start = end;
-    if (dmax == h->nz) break;
-  }
-  return t;
 }
 
 // The transport sub-steps of one step for the tracers of T (every tracer, or
@@ -2036,8 +1991,7 @@ int launch_part_b(shoc_tr_gpu *h, const Sched &s, int cur0, const TrSet &T,
       cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
       if (prof)
         for (auto &e : ev) cudaEventCreate(&e);
-      const Tile tl = vd_classes(h, tw);
-      const int nl = tile64_substep(h, last, ss, tl, T, tin, tout, tw, prof ? ev : nullptr);
+      const int nl = tile64_substep(h, last, ss, h->tl, T, tin, tout, tw, prof ? ev : nullptr);
       if (prof) {
         h->ev.push_back({0, ev[0], ev[2]});
         h->ev.push_back({1, ev[0], ev[1]});

@@ -115,7 +115,7 @@ struct Flow {
 struct Work {
   double *dz, *w5, *w9, *dbz, *dfz;     // per step
   double *vd_cm1, *vd_div, *vd_ud, *vd_dzdt;
-  double *vd_rdiv;                      // FP64: 1 / vd_div (0: not for div_known)
+  double *vd_rdiv;                      // FP64: 1 / vd_div (0: not for quot)
   int *sur_t, *nsur_t;                  // [ncol] 0-based column
   ColInfo *col;                         // [ncol]
   int *status;
@@ -143,9 +143,6 @@ struct Tile {
                      // its west flux only), -1: none
   const int *vdcol;  // [ncolp] columns in the column kernels' order: whole tiles of 32
                      // adjacent columns, shallow tiles first (-1: padding)
-  int nclass;        // k_vd64 depth classes: tiles [ctile[i], ctile[i+1]) have
-  int ctile[5];      //   no cell below layer cbase[i]
-  int cbase[4];
   const int4 *colrec;  // [ncolp] bottom cell, surface-layer cell, bottom layer
   // k_adv64's segments of the column order, [nseg][32]: columns, -1: none,
   // with kSegHalo: the column only lends its west flux

@@ -626,6 +626,7 @@ __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const
 // 0.128 and 0.080; a batch of 56 447 columns, 60 layers, 4 to 32 tracers 0.93 and
 // 0.69.
 
+constexpr int kStage = 8;  // layers a warp of a column kernel stages together
 constexpr int kVd32MaxWarps = 16;
 // shared memory of k_vd32 (bytes) for columns of at most nd layers:
 // thicknesses double[nd][32], four factors float[nd][32], cells int[nd][32], A,
@@ -696,16 +697,25 @@ __global__ void __launch_bounds__(kVd32MaxWarps * 32)
   const int sa = nw * 32;
 
   // the tile's tracer-independent column arrays, once for every tracer
-  for (int k = kbase + wy; k < nz; k += blockDim.y) {
-    const int c = (act && k >= kb) ? Tl.cellk[(size_t)k * Tl.ncolp + col] : 0;
-    const int r = k - kbase;
-    colC[r * 32 + lane] = c;
-    if (LAST && c && k <= ks) {
-      const float *lu = reinterpret_cast<const float *>(&lu32[c]);
+  for (int kq = kbase + wy; kq < nz; kq += kStage * blockDim.y) {
+    int cq[kStage];  // the cells first: one latency for all of them
 #pragma unroll
-      for (int q = 0; q < 4; ++q) cp_async4(&LU[(q * nd + r) * 32 + lane], lu + q);
+    for (int i = 0; i < kStage; ++i) {
+      const int k = kq + i * blockDim.y;
+      cq[i] = (act && k >= kb && k < nz) ? Tl.cellk[(size_t)k * Tl.ncolp + col] : 0;
     }
-    if (c && k <= ks) cp_async8(&DZ[r * 32 + lane], &W.dz[c]);
+#pragma unroll
+    for (int i = 0; i < kStage; ++i) {
+      const int k = kq + i * blockDim.y, c = cq[i], r = k - kbase;
+      if (k >= nz) break;
+      colC[r * 32 + lane] = c;
+      if (LAST && c && k <= ks) {
+        const float *lu = reinterpret_cast<const float *>(&lu32[c]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) cp_async4(&LU[(q * nd + r) * 32 + lane], lu + q);
+      }
+      if (c && k <= ks) cp_async8(&DZ[r * 32 + lane], &W.dz[c]);
+    }
   }
   cp_async_commit();
   cp_async_wait<0>();

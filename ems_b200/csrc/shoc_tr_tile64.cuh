@@ -25,12 +25,6 @@
 
 namespace shoc {
 
-// shared memory of k_vd64 (bytes) for columns of at most nd layers:
-// S double[nd][nw][32], colC int[nd][32]
-inline size_t vd64_smem(int nd, int nw) {
-  return (size_t)nd * 32 * 4 + (size_t)nd * nw * 32 * 8;
-}
-
 // ---------------------------------------------------------------------------
 // k_adv64
 //
@@ -81,22 +75,16 @@ template <unsigned LIM>
 __device__ __forceinline__ bool far_out(double x) {
   return ((unsigned)__double2hiint(x) & 0x7fffffffu) - ((1023u - LIM) << 20) >= ((2 * LIM) << 20);
 }
-// a / b for any a and a b the caller keeps y = 1 / b of.  lo: kDivLo where b
-// lies in 2^-200 .. 2^200, so that nothing under- or overflows for |a| in
-// 2^-700 .. 2^700 (div_fast); kDivNever where it does not.  Else the division.
+// Whether quot may form a / b for a b the caller keeps 1 / b of.  lo: kDivLo
+// where b lies in 2^-200 .. 2^200, so that nothing under- or overflows for |a|
+// in 2^-700 .. 2^700; kDivNever where it does not.
 constexpr unsigned kDivLo = (1023u - 700u) << 20, kDivSpan = 1400u << 20;
 constexpr unsigned kDivNever = 0x80000000u;
-__device__ __noinline__ double div_slow(double a, double b) { return a / b; }
 __device__ __forceinline__ unsigned div_range(double b) {
   return far_out<200>(b) ? kDivNever : kDivLo;
 }
 __device__ __forceinline__ bool div_fast(double a, unsigned lo) {
   return ((unsigned)__double2hiint(a) & 0x7fffffffu) - lo < kDivSpan;
-}
-__device__ __forceinline__ double div_known(double a, double b, double y, unsigned lo) {
-  double q = quot(a, b, y);
-  if (!div_fast(a, lo)) q = (a == 0.0 && lo != kDivNever) ? __dmul_rn(a, y) : div_slow(a, b);
-  return q;
 }
 // RN(1 / d) for |d| in 2^-500 .. 2^500: Newton steps from the hardware's
 // approximation (20 bits); the last one starts within an ulp, so it rounds
@@ -528,101 +516,102 @@ __global__ void __launch_bounds__(kAdv64Warps * 32, 16)
 // ---------------------------------------------------------------------------
 // k_vd64
 //
-// One thread per (column, tracer), a warp per 32 columns of one tracer.  What
-// bounds it: the serial chain of the Thomas sweeps (memory is 16 bytes a
+// A block is one tile of 32 columns, deepest tiles first, the tile's
+// tracer-independent arrays (cells, the LU factors and the reciprocal of the
+// divisor) staged once; each warp steps its share of the tracers, a thread per
+// column.  Every block has the same shared memory, of which a warp takes as
+// much as the tile is deep, so one launch serves every depth.
+//
+// What bounds it: the serial chain of the Thomas sweeps (memory is 16 bytes a
 // value).  The forward sweep's IEEE division was most of the chain: the
 // divisor does not depend on the tracer, so k_set_dz stores its reciprocal and
-// div_known takes five dependent operations.  The advected values are copied
-// to shared memory in one batch of asynchronous copies and replaced by the
-// forward sweep's row by row; the back substitution reads them again (from
-// L2), so a warp keeps one array instead of two and twice the warps fit.
+// quot takes five dependent operations; and a row waited for its factors from
+// L2, which a row's branch keeps the compiler from fetching ahead.  The advected
+// values are copied to shared memory in one batch of asynchronous copies and
+// replaced by the forward sweep's row by row; the back substitution reads them
+// again (from L2), so a warp keeps one array instead of two.
+// A sub-step (B200): 384 x 320 x 40, 10 tracers 0.51 ms with divisions and the
+// factors read from L2, 0.37 with reciprocals, 0.23 with the factors in shared
+// memory, a row without branches (a row whose quotient is not quot's to form
+// marks its column, which is swept again) and the tile's cells read eight layers
+// at a time; 64 x 64 x 20, 1 tracer 25 and 18 us.
 // Columns whose surface crosses layer faces during the step run here too: the
 // cells from the lower of the old and new surface cells up to the old one add
 // to the surface balance, and the solve runs up to the new one.
 
+constexpr int kVd64MaxWarps = 16;
+// shared memory (bytes) for columns of at most nd layers: factors dzdt, cm1,
+// div, 1 / div, ud double[5][nd][32], S double[nd][nw][32], cells int[nd][32]
+inline size_t vd64_smem(int nd, int nw) {
+  return (size_t)nd * 32 * (5 * 8 + 4) + (size_t)nd * nw * 32 * 8;
+}
+// Warps per block at full depth where the caller sets none: two blocks per SM
+// within 160 KB of its memory, balanced rounds.  The rest is left to the L1,
+// which the back substitution's values come from: 384 x 320 x 40 (10 tracers)
+// 2 warps 0.23 ms, 4 (194 KB) 0.27; 200 x 180 x 30 (6 tracers) 3 warps 0.055, 6
+// 0.051.
+inline int vd64_default_warps(int nz, int nslot) {
+  int nw = 1;
+  while (nw < kVd64MaxWarps / 2 && 2 * (vd64_smem(nz, nw + 1) + 1024) <= 160 * 1024) nw++;
+  const int rounds = nslot > 0 ? (nslot + nw - 1) / nw : 1;
+  return nslot > 0 ? (nslot + rounds - 1) / rounds : 1;
+}
+
+// What the tracers of one column share: rows nk, nc, no of the cells s (the lower
+// of the old and new surface cells), cs (new) and co (old), nl of the column;
+// surf_conc's elevations and thicknesses (tracers.c:3097-3112)
+struct Col64 {
+  ColInfo ci;
+  int nk, nc, no, nl, cbot, sed;
+  double area, botz, wbot, wb, sub, osub, dz_s, dz_cs;
+};
+
+// One (column, tracer) pair: S0 (row stride sa) the column's shared memory, F0
+// its factors (n1 doubles apart: dzdt, cm1, div, 1 / div, ud), C0 its cells; Fzb:
+// the flux through the bottom of s.
 template <bool LAST>
-__global__ void __launch_bounds__(256) k_vd64(Geo G, Flow F, Work W, Opt O, TrSet T,
-                                              SubStep ss, Tile Tl,
-                                              const double *__restrict__ tri,
-                                              double *__restrict__ tro,
-                                              const double *__restrict__ fzs,
-                                              const double *__restrict__ vdzdt,
-                                              const double *__restrict__ vcm1,
-                                              const double *__restrict__ vdiv,
-                                              const double *__restrict__ vrdiv,
-                                              const double *__restrict__ vud, int nw,
-                                              int nchunk, int tile0, int kbase) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const int nz = G.nz, nd = nz - kbase;
-  double *Sv = reinterpret_cast<double *>(smem);           // [nd][nw][32]
-  int *colC = reinterpret_cast<int *>(Sv + nd * nw * 32);  // [nd][32]
-
-  const int lane = threadIdx.x, wy = threadIdx.y;
-  const int tile = tile0 + blockIdx.x / nchunk, chunk = blockIdx.x % nchunk;
-  const int col = Tl.vdcol[tile * 32 + lane];
-  const int slot = chunk * nw + wy;
-  const int sa = nw * 32;
-
-  const TileCol tc = tile_column(G, W, Tl, col);
-  bool act = tc.act;
-  if (act && tc.kb < kbase) {  // not in this launch's depth class
-    act = false;
-    if (chunk == 0 && wy == 0) atomicOr(W.status, ST_GEOM);
-  }
-  const int kb = tc.kb, ks = tc.ks, cbot = tc.cbot, c2 = tc.c2;
-  const ColInfo ci = tc.ci;
-  const int kmin = __reduce_min_sync(0xffffffffu, act ? kb : nz);
-  for (int k = kmin + wy; k < nz; k += nw)
-    colC[(k - kbase) * 32 + lane] = (act && k >= kb) ? Tl.cellk[(size_t)k * Tl.ncolp + col] : 0;
-  __syncthreads();
-  if (!act || slot >= T.nslot) return;
-
-  const int n = T.slot_tr[slot];
-  if (n >= G.colntr[col]) return;  // tracer not carried in this column
+__device__ __forceinline__ void vd64_column(const Geo &G, const Flow &F, const Work &W,
+                                            const Opt &O, const TrSet &T, const SubStep &ss,
+                                            const Col64 &L, int n, const double *tr, double *to,
+                                            double Fzb, double *S0, int sa, const double *F0,
+                                            int n1, const int *C0, unsigned long long &nwarn,
+                                            int &stat) {
+  const ColInfo &ci = L.ci;
+  const int nk = L.nk, nc = L.nc, no = L.no, nl = L.nl;
   const int tf = T.trf[n];
   const bool tbdy = (tf & TR_TBDY) != 0;
   const bool adv = tbdy && (tf & TR_ADV);
   const bool vdf = LAST && (tf & TR_VDIFF);
   const bool single = (ci.flags & COL_SINGLE) != 0;
   const bool solve = vdf && !single;
-  const double *tr = tri + (size_t)n * G.S;
-  double *to = tro + (size_t)n * G.S;
   // the column: advection results (advected tracers) or the old values
   const double *src = tbdy ? to : tr;
-  double *const S0 = Sv + (kb - kbase) * sa + wy * 32 + lane;
-  const int *const C0 = colC + (kb - kbase) * 32 + lane;
-  const int nk = ks - kb, nl = nz - kb;
   for (int j = 0; j < nl; ++j) cp_async8(&S0[j * sa], src + C0[j * 32]);
   cp_async_commit();
   const double mn = T.mintr[n], mx = T.maxtr[n];
-  {  // sediment ghost (tracers.c:827-830)
-    const int sed = G.zm1[cbot];
-    to[sed] = tbdy ? tr[cbot] : tr[sed];
-  }
-  // s: the lower of the old (co) and new (cs) surface cells
+  to[L.sed] = tbdy ? tr[L.cbot] : tr[L.sed];  // sediment ghost (tracers.c:827-830)
   const int cell_s = ci.s, cs = ci.cs;
-  const int nc = (cs == cell_s) ? nk : G.kof[cs] - kb;        // rows up to the new surface
-  const int no = (ci.co == cell_s) ? nk : G.kof[ci.co] - kb;  // up to the old one
   const double ts_old = tr[cell_s];
-  const double area = G.cellarea[c2];
   cp_async_wait<0>();
 
-  unsigned long long nwarn = 0;
-  int stat = 0;
   double solp = 0.0;
   const bool clip = mn <= kClipEps;
-  // row j of the forward sweep (:4185-4196) for the value a
+  // row j of the forward sweep (:4185-4196) for the value a.  Without a branch,
+  // so that the rows' factors are fetched ahead; bad: a row's quotient is not
+  // quot's to form, and the sweep is run again with the reference's division
+  bool bad = false;
+  auto row_rhs = [&](int j, double a) {
+    const double *f = F0 + j * 32;
+    double rhs = f[0] * a;
+    if (j == 0) return rhs + 0.0;
+    if (j == nc) rhs = rhs - 0.0;
+    return rhs - f[n1] * solp;
+  };
   auto forward = [&](int j, double a) {
-    const int cc = C0[j * 32];
-    const double div = __ldg(&vdiv[cc]), y = __ldg(&vrdiv[cc]);
-    double rhs = __ldg(&vdzdt[cc]) * a;
-    if (j == 0) {
-      rhs = rhs + 0.0;
-    } else {
-      if (j == nc) rhs = rhs - 0.0;
-      rhs = rhs - __ldg(&vcm1[cc]) * solp;
-    }
-    solp = div_known(rhs, div, y, __double2hiint(y) ? kDivLo : kDivNever);
+    const double *f = F0 + j * 32;
+    const double rhs = row_rhs(j, a), y = f[3 * n1];
+    bad = bad || !(div_fast(rhs, kDivLo) || rhs == 0.0) || __double2hiint(y) == 0;
+    solp = quot(rhs, f[2 * n1], y);
     S0[j * sa] = solp;
   };
   double vs = ts_old;
@@ -634,7 +623,7 @@ __global__ void __launch_bounds__(256) k_vd64(Geo G, Flow F, Work W, Opt O, TrSe
       if (isnan(a)) stat |= ST_NAN;
     }
     if (vdf && single) {
-      const double h = W.dz[cs] > O.hmin ? W.dz[cs] : O.hmin;
+      const double h = L.dz_cs > O.hmin ? L.dz_cs : O.hmin;
       const double v = S0[nc * sa];
       to[cs] = v + F.dt * (0.0 - 0.0) / h;
     } else if (solve) {
@@ -646,14 +635,11 @@ __global__ void __launch_bounds__(256) k_vd64(Geo G, Flow F, Work W, Opt O, TrSe
     // the divergences at and above s
     double sv = 0.0;
     if (adv) {
-      const double Fzb = fzs[(size_t)n * G.ncol + col];
+      const double area = L.area;
       const double fcbot = -Fzb * area;
       double surftr = -fcbot;
-      double wbot = (cell_s == cbot) ? G.botz[c2] : G.gridz[cell_s];
-      const double eta = F.eta[c2], oe = F.oldeta[c2];
-      const double sub = oe + ss.subeta_f * (eta - oe);
-      const double osub = ss.first ? oe : oe + ss.osub_f * (eta - oe);
-      const double dzs = sub - wbot;
+      double wbot = L.wbot;
+      const double dzs = L.sub - wbot;
       const double svol = dzs * area;
       double t0 = ts_old;
       int j = nk;
@@ -663,14 +649,13 @@ __global__ void __launch_bounds__(256) k_vd64(Geo G, Flow F, Work W, Opt O, TrSe
         wbot = wtop;
         t0 = tr[C0[(j + 1) * 32]];
       }
-      const double wb = (ci.co == cbot) ? G.botz[c2] : G.gridz[ci.co];
-      surftr += (t0 * area * (osub - wb) - S0[j * sa]);
+      surftr += (t0 * area * (L.osub - L.wb) - S0[j * sa]);
       for (++j; j < nl; ++j) surftr -= (S0[j * sa]);
       if (svol == 0.0 || (surftr < 0.0 && dzs <= O.hmin))
         sv = 0.0;
       else
         sv = surftr / svol;
-      vs = (G.botz[c2] > 0.0 && W.dz[cell_s] < O.hmin) ? ts_old : sv;
+      vs = (L.botz > 0.0 && L.dz_s < O.hmin) ? ts_old : sv;
     }
     double a_below = nk > 0 ? S0[(nk - 1) * sa] : 0.0;
 #pragma unroll 4
@@ -692,48 +677,139 @@ __global__ void __launch_bounds__(256) k_vd64(Geo G, Flow F, Work W, Opt O, TrSe
     if (isnan(vs)) stat |= ST_NAN;
     for (int j = nk; j < nl; ++j) to[C0[j * 32]] = vs;
     if (vdf && single) {
-      const double h = W.dz[cs] > O.hmin ? W.dz[cs] : O.hmin;
+      const double h = L.dz_cs > O.hmin ? L.dz_cs : O.hmin;
       to[cs] = vs + F.dt * (0.0 - 0.0) / h;
     } else if (solve) {
       for (int j = nk; j <= nc; ++j) forward(j, vs);
     }
   }
   if (solve) {
-    // back substitution and update (:4197-4205); a: the value before the solve
+    // the value before the solve
     auto before = [&](int j) {
       if (tbdy && j >= nk) return vs;
       double a = src[C0[j * 32]];
       if (tbdy && clip && a < mn) a = mn;
       return a;
     };
+    if (bad)
+      for (int j = 0; j <= nc; ++j) {
+        solp = row_rhs(j, before(j)) / F0[j * 32 + 2 * n1];
+        S0[j * sa] = solp;
+      }
+    // back substitution and update (:4197-4205)
     double x = S0[nc * sa];
     double a = before(nc);
     double fin = a + (x - a) * 1.0;
     if (isnan(fin)) stat |= ST_NAN;
-    double udp = __ldg(&vud[cs]);
-    // the values of kBack rows are read ahead of the rows they replace
-    constexpr int kBack = 4;
+    double udp = F0[nc * 32 + 4 * n1];
+    // the values are read kBack rows ahead of the rows they replace
+    constexpr int kBack = 8;
     to[cs] = fin;
-    for (int j0 = nc - 1; j0 >= 0; j0 -= kBack) {
-      double av[kBack], uv[kBack];
-      int cv[kBack];
+    double nx[kBack];
 #pragma unroll
-      for (int q = 0; q < kBack; ++q) {
-        const int j = max(j0 - q, 0);
-        cv[q] = C0[j * 32];
-        av[q] = before(j);
-        uv[q] = __ldg(&vud[cv[q]]);
-      }
+    for (int q = 0; q < kBack; ++q) nx[q] = before(max(nc - 1 - q, 0));
+    for (int j0 = nc - 1; j0 >= 0; j0 -= kBack) {
+      double av[kBack];
+#pragma unroll
+      for (int q = 0; q < kBack; ++q) av[q] = nx[q];
+#pragma unroll
+      for (int q = 0; q < kBack; ++q) nx[q] = before(max(j0 - kBack - q, 0));
 #pragma unroll
       for (int q = 0; q < kBack; ++q) {
         if (j0 - q < 0) break;
         x = S0[(j0 - q) * sa] - udp * x;
         const double f = av[q] + (x - av[q]) * 1.0;
-        to[cv[q]] = f;
+        to[C0[(j0 - q) * 32]] = f;
         if (isnan(f)) stat |= ST_NAN;
-        udp = uv[q];
+        udp = F0[(j0 - q) * 32 + 4 * n1];
       }
     }
+  }
+}
+
+template <bool LAST>
+__global__ void __launch_bounds__(kVd64MaxWarps * 32)
+    k_vd64(Geo G, Flow F, Work W, Opt O, TrSet T, SubStep ss, Tile Tl,
+           const double *__restrict__ tri, double *__restrict__ tro,
+           const double *__restrict__ fzs, int smem_bytes) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x, wy = threadIdx.y;
+  const int tile = gridDim.x - 1 - blockIdx.x;  // (the tiles are sorted by depth)
+  const int col = Tl.vdcol[tile * 32 + lane];
+  const TileCol tc = tile_column(G, W, Tl, col);
+  const bool act = tc.act;
+  const int kb = tc.kb, ks = tc.ks, cbot = tc.cbot, c2 = tc.c2;
+  const ColInfo ci = tc.ci;
+  // the arrays hold layers kbase .. nz-1, row r = layer - kbase
+  const int nz = G.nz, kbase = __reduce_min_sync(FULL, act ? kb : nz), nd = nz - kbase;
+  if (nd == 0) return;
+  // warps that step tracers: what the shared memory holds at this depth
+  const int nw = min((int)blockDim.y, (smem_bytes / (nd * 32) - (5 * 8 + 4)) / 8);
+  const int n1 = nd * 32;  // doubles per factor
+  double *const Fc = reinterpret_cast<double *>(smem);  // [5][nd][32]
+  double *const Sv = Fc + 5 * n1;                        // [nd][nw][32]
+  int *const colC = reinterpret_cast<int *>(Sv + nw * n1);  // [nd][32]
+  const int sa = nw * 32;
+  const bool single = (ci.flags & COL_SINGLE) != 0;
+  Col64 L{ci, ks - kb, 0, 0, 0, cbot, 0, 1.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  int ntc = 0;
+  if (act) {
+    L.nc = (ci.cs == ci.s) ? L.nk : G.kof[ci.cs] - kb;
+    L.no = (ci.co == ci.s) ? L.nk : G.kof[ci.co] - kb;
+    L.nl = nz - kb;
+    L.sed = G.zm1[cbot];
+    L.area = G.cellarea[c2];
+    L.botz = G.botz[c2];
+    L.wbot = (ci.s == cbot) ? L.botz : G.gridz[ci.s];
+    L.wb = (ci.co == cbot) ? L.botz : G.gridz[ci.co];
+    L.dz_s = W.dz[ci.s];
+    L.dz_cs = W.dz[ci.cs];
+    const double eta = F.eta[c2], oe = F.oldeta[c2];
+    L.sub = oe + ss.subeta_f * (eta - oe);
+    L.osub = ss.first ? oe : oe + ss.osub_f * (eta - oe);
+    ntc = G.colntr[col];
+  }
+  for (int kq = kbase + wy; kq < nz; kq += kStage * blockDim.y) {
+    int cq[kStage];  // the cells first: one latency for all of them
+#pragma unroll
+    for (int i = 0; i < kStage; ++i) {
+      const int k = kq + i * blockDim.y;
+      cq[i] = (act && k >= kb && k < nz) ? Tl.cellk[(size_t)k * Tl.ncolp + col] : 0;
+    }
+#pragma unroll
+    for (int i = 0; i < kStage; ++i) {
+      const int k = kq + i * blockDim.y, c = cq[i], q = (k - kbase) * 32 + lane;
+      if (k >= nz) break;
+      colC[q] = c;
+      if (LAST && c && !single && k - kb <= L.nc) {
+        cp_async8(&Fc[q], &W.vd_dzdt[c]);
+        cp_async8(&Fc[n1 + q], &W.vd_cm1[c]);
+        cp_async8(&Fc[2 * n1 + q], &W.vd_div[c]);
+        cp_async8(&Fc[3 * n1 + q], &W.vd_rdiv[c]);
+        cp_async8(&Fc[4 * n1 + q], &W.vd_ud[c]);
+      }
+    }
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  if (wy >= nw) return;
+
+  const int row0 = act ? kb - kbase : 0;
+  double *const S0 = Sv + row0 * sa + wy * 32 + lane;
+  const double *const F0 = Fc + row0 * 32 + lane;
+  const int *const C0 = colC + row0 * 32 + lane;
+  const int ntmax = __reduce_max_sync(FULL, ntc);
+  unsigned long long nwarn = 0;
+  int stat = 0;
+  for (int slot = wy; slot < T.nslot; slot += nw) {
+    const int n = T.slot_tr[slot];
+    if (n >= ntmax) continue;  // not carried in this tile
+    if (n < ntc)
+      vd64_column<LAST>(G, F, W, O, T, ss, L, n, tri + (size_t)n * G.S, tro + (size_t)n * G.S,
+                        fzs[(size_t)n * G.ncol + col], S0, sa, F0, n1, C0, nwarn, stat);
+    __syncwarp();
   }
   if (nwarn) atomicAdd(W.nwarn, nwarn);
   if (stat) atomicOr(W.status, stat);
