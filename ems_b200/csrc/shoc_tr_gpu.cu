@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -126,18 +127,26 @@ struct shoc_tr_gpu {
   int prof_n[3] = {0, 0, 0};
   long long launches = 0;
   // pinned readback
-  unsigned long long *h_dtm = nullptr;
-  int *h_status = nullptr;
-  unsigned long long *h_nwarn = nullptr;
-  int *h_counts = nullptr;
+  // (W.dtm_bits, W.nwarn, W.status and d_counts are one device block, so one
+  // copy reads them)
+  struct Readback {
+    unsigned long long dtm, nwarn;
+    int status, pad, counts[2];
+  };
+  Readback *h_rb = nullptr, *d_rb = nullptr;
   int *d_counts = nullptr;  // [0] vcs, [1] vc
   int last_status = 0;
   long long warn_total = 0;
   // pipeline of the drop-in step on host arrays (made on its first use)
   std::vector<int> slot_host;       // slot -> tracer, as T.slot_tr
   cudaStream_t s_up = nullptr, s_dn = nullptr;  // host -> device, device -> host
+  cudaStream_t s_cv = nullptr;      // what an arrived tracer needs on the device
+  double *xup[2] = {nullptr, nullptr};  // FP32-mixed: arriving tracers (FP64)
+  cudaEvent_t ev_in[2] = {nullptr, nullptr}, ev_cv[2] = {nullptr, nullptr};
+  int *h_surf = nullptr;            // page-locked surface vectors, 2 x (ncol + 1)
   std::vector<cudaEvent_t> pev;     // [0] flow sent, then per chunk: sent, stepped
   double *xout = nullptr;           // FP32-mixed: one tracer of FP64 for the way back
+  bool pipe_ready = false;
   uint8_t *c3s = nullptr;           // [kItermax + 2][ncol] k_general cursors between chunks
 };
 
@@ -1384,12 +1393,16 @@ void shoc_tr_gpu_destroy(shoc_tr_gpu *h) {
         if (std::find(done.begin(), done.end(), x) == done.end()) done.push_back(x);
     for (cudaEvent_t x : done) cudaEventDestroy(x);
   }
-  for (cudaStream_t x : {h->s_up, h->s_dn})
+  for (cudaStream_t x : {h->s_up, h->s_cv, h->s_dn})
     if (x) cudaStreamSynchronize(x);
-  for (cudaEvent_t x : h->pev) cudaEventDestroy(x);
+  for (cudaEvent_t x : h->pev)
+    if (x) cudaEventDestroy(x);
+  for (cudaEvent_t x : {h->ev_in[0], h->ev_in[1], h->ev_cv[0], h->ev_cv[1]})
+    if (x) cudaEventDestroy(x);
   for (void *p : h->allocs) cudaFree(p);
-  if (h->h_dtm) cudaFreeHost(h->h_dtm);
-  for (cudaStream_t x : {h->s_up, h->s_dn})
+  if (h->h_rb) cudaFreeHost(h->h_rb);
+  if (h->h_surf) cudaFreeHost(h->h_surf);
+  for (cudaStream_t x : {h->s_up, h->s_cv, h->s_dn})
     if (x) cudaStreamDestroy(x);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
@@ -1576,12 +1589,13 @@ int shoc_tr_gpu_create(const shoc_tr_geom *g, const shoc_tr_opts *o, int ntr, in
   TRY(dupload<int>(h, &W.sur_t, nullptr, ncol));
   TRY(dupload<int>(h, &W.nsur_t, nullptr, ncol));
   TRY(dupload<ColInfo>(h, &W.col, nullptr, ncol));
-  TRY(dupload<int>(h, &W.status, nullptr, 1));
-  TRY(dupload<unsigned long long>(h, &W.dtm_bits, nullptr, 1));
-  TRY(dupload<unsigned long long>(h, &W.nwarn, nullptr, 1));
+  TRY(dupload<shoc_tr_gpu::Readback>(h, &h->d_rb, nullptr, 1));
+  W.status = &h->d_rb->status;
+  W.dtm_bits = &h->d_rb->dtm;
+  W.nwarn = &h->d_rb->nwarn;
+  h->d_counts = h->d_rb->counts;
   TRY(dupload<int>(h, &W.serial_list, nullptr, ncol));
   TRY(dupload<int>(h, &W.serial_count, nullptr, 1));
-  TRY(dupload<int>(h, &h->d_counts, nullptr, 2));
   const bool f32p = precision != SHOC_TR_FP64;
   h->esize = f32p ? sizeof(float) : sizeof(double);
   h->comp = precision == SHOC_TR_FP32_COMP;
@@ -1698,10 +1712,7 @@ int shoc_tr_gpu_create(const shoc_tr_geom *g, const shoc_tr_opts *o, int ntr, in
   // pinned readback words
   void *pin = nullptr;
   if (cudaHostAlloc(&pin, 64, cudaHostAllocDefault) != cudaSuccess) TRY(SHOC_TR_ENOMEM);
-  h->h_dtm = (unsigned long long *)pin;
-  h->h_status = (int *)((char *)pin + 8);
-  h->h_nwarn = (unsigned long long *)((char *)pin + 16);
-  h->h_counts = (int *)((char *)pin + 24);
+  h->h_rb = (shoc_tr_gpu::Readback *)pin;
   if (cudaFuncSetAttribute(k_set_dz, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)set_dz_smem(kMaxLayers, true)) != cudaSuccess ||
       tile64_set_smem_attr() != cudaSuccess ||
@@ -2007,9 +2018,7 @@ int launch_part_b(shoc_tr_gpu *h, const Sched &s, int cur0, const TrSet &T,
 }
 
 int read_status(shoc_tr_gpu *h) {
-  CK(cudaMemcpyAsync(h->h_dtm, h->W.dtm_bits, 8, cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaMemcpyAsync(h->h_status, h->W.status, 4, cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaMemcpyAsync(h->h_counts, h->d_counts, 8, cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaMemcpyAsync(h->h_rb, h->d_rb, sizeof(*h->h_rb), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   return 0;
 }
@@ -2022,13 +2031,13 @@ int probe_schedule(shoc_tr_gpu *h, bool lateral, Sched &s) {
   if (rc) return rc;
   rc = read_status(h);
   if (rc) return rc;
-  int st = *h->h_status;
+  int st = h->h_rb->status;
   if (st & (ST_LASTDRY | ST_GEOM)) {
     h->last_status = map_status(st);
     return h->last_status;
   }
   double dmin;
-  unsigned long long b = *h->h_dtm;
+  unsigned long long b = h->h_rb->dtm;
   memcpy(&dmin, &b, 8);
   if (h->dmin_set > 0.0) dmin = h->dmin_set;  // the basin-wide minimum, given
   rc = make_schedule(h, dmin, s);
@@ -2118,46 +2127,94 @@ int step_async(shoc_tr_gpu *h) {
 // k_general carries from chunk to chunk (c3s); set_dz reads no tracer, so the
 // lateral boundaries of a chunk may follow it.
 
-// slots per chunk: about a twelfth of the tracers, so the first chunk is
-// back on its way while most are still going up and the last chunk's step
-// and copy back (the part nothing overlaps) are short
-int pipe_chunk_slots(const shoc_tr_gpu *h) { return std::max(1, (h->nslot + 11) / 12); }
+// Slots of each chunk.  The first chunk should be back on its way early and the
+// last one's step and copy back, which nothing overlaps, should be short; in
+// between, a chunk's step costs the faces and factors of every cell once more,
+// whatever the number of its tracers.  So the chunks grow from a twelfth of the
+// tracers to a third and shrink again: 300 x 257 x 33, 8 tracers, two sub-steps,
+// FP32-mixed took 4.04 ms a call as eight chunks, 3.53 as five; 256 x 256 x 40, 10
+// tracers, FP64 4.81 and 4.24 (3.39 and 3.87 with the arrived tracers' copies off
+// the link's stream).  A window whose tracers cross the link in tens of
+// microseconds goes as one chunk: the launches of each cost as much (20 x 14 x 6,
+// 3 tracers: 258 us as three, 220 as one).
+std::vector<int> pipe_chunks(const shoc_tr_gpu *h) {
+  const int n = h->nslot;
+  if (n == 0) return {};
+  if ((size_t)n * h->S * sizeof(double) <= (size_t)2 << 20) return {n};
+  std::vector<int> left, right;
+  const int most = std::max(1, n / 3);
+  for (int c = std::max(1, (n + 11) / 12), rest = n; rest > 0; c = std::min(2 * c, most)) {
+    if (rest < 2 * c) {  // the middle
+      left.push_back(rest);
+      break;
+    }
+    left.push_back(c);
+    right.push_back(c);
+    rest -= 2 * c;
+  }
+  left.insert(left.end(), right.rbegin(), right.rend());
+  return left;
+}
 
 int pipe_init(shoc_tr_gpu *h) {
-  if (h->s_up) return 0;
-  CK(cudaStreamCreateWithFlags(&h->s_up, cudaStreamNonBlocking));
-  CK(cudaStreamCreateWithFlags(&h->s_dn, cudaStreamNonBlocking));
+  if (h->pipe_ready) return 0;
+  for (cudaStream_t *x : {&h->s_up, &h->s_cv, &h->s_dn})
+    if (!*x) CK(cudaStreamCreateWithFlags(x, cudaStreamNonBlocking));
+  int rc = 0;
   if (h->esize == sizeof(float)) {
-    int rc = dalloc(h, &h->xout, (size_t)h->S);
-    if (rc) return rc;
+    if (!h->xout && (rc = dalloc(h, &h->xout, (size_t)h->S))) return rc;
+    h->xup[0] = h->xfer;
+    if (!h->xup[1] && (rc = dalloc(h, &h->xup[1], (size_t)h->S))) return rc;
   }
-  int rc = dalloc(h, &h->c3s, (size_t)(kItermax + 2) * h->ncol);
-  if (rc) return rc;
-  h->pev.assign(1 + 2 * (size_t)h->nslot, nullptr);
-  for (auto &e : h->pev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  if (!h->c3s && (rc = dalloc(h, &h->c3s, (size_t)(kItermax + 2) * h->ncol))) return rc;
+  if (!h->h_surf &&
+      cudaHostAlloc((void **)&h->h_surf, 2 * ((size_t)h->ncol + 1) * sizeof(int),
+                    cudaHostAllocDefault) != cudaSuccess) {
+    cudaGetLastError();
+    h->h_surf = nullptr;
+    return SHOC_TR_ENOMEM;
+  }
+  h->pev.resize(1 + 2 * (size_t)h->nslot, nullptr);
+  for (auto &e : h->pev)
+    if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  for (cudaEvent_t *e : {&h->ev_in[0], &h->ev_in[1], &h->ev_cv[0], &h->ev_cv[1]})
+    if (!*e) CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+  h->pipe_ready = true;
   return 0;
 }
 
 // wait for every copy that may still touch the caller's host arrays
 void pipe_drain(shoc_tr_gpu *h) {
   cudaStreamSynchronize(h->s_up);
+  cudaStreamSynchronize(h->s_cv);
   cudaStreamSynchronize(h->s_dn);
   cudaStreamSynchronize(h->stream);
 }
 
-int up_tracer(shoc_tr_gpu *h, int cur, int n, const double *src) {
-  cudaStream_t s = h->s_up;
+// Tracer n, the i-th of the call, up the link on s_up; what it needs on the
+// device then (the copy into the other ping-pong buffer, the conversion) runs on
+// s_cv, so that the link does not wait for it (FP32-mixed: two buffers for the
+// arriving FP64 values).
+int up_tracer(shoc_tr_gpu *h, int cur, int i, int n, const double *src) {
   const size_t S = (size_t)h->S;
+  const int b = i & 1;
   if (h->esize == sizeof(double)) {
-    double *a = (double *)h->tr[cur] + n * S, *b = (double *)h->tr[cur ^ 1] + n * S;
-    CK(cudaMemcpyAsync(a, src, S * sizeof(double), cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(b, a, S * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    double *p = (double *)h->tr[cur] + n * S, *q = (double *)h->tr[cur ^ 1] + n * S;
+    CK(cudaMemcpyAsync(p, src, S * sizeof(double), cudaMemcpyHostToDevice, h->s_up));
+    CK(cudaEventRecord(h->ev_in[b], h->s_up));
+    CK(cudaStreamWaitEvent(h->s_cv, h->ev_in[b], 0));
+    CK(cudaMemcpyAsync(q, p, S * sizeof(double), cudaMemcpyDeviceToDevice, h->s_cv));
   } else {
-    float *a = (float *)h->tr[cur] + n * S, *b = (float *)h->tr[cur ^ 1] + n * S;
-    CK(cudaMemcpyAsync(h->xfer, src, S * sizeof(double), cudaMemcpyHostToDevice, s));
-    k_to_f32x2<<<592, 256, 0, s>>>(h->xfer, a, b, S, h->comp ? h->lo[cur] + n * S : nullptr,
-                                   h->comp ? h->lo[cur ^ 1] + n * S : nullptr);
+    float *p = (float *)h->tr[cur] + n * S, *q = (float *)h->tr[cur ^ 1] + n * S;
+    if (i >= 2) CK(cudaStreamWaitEvent(h->s_up, h->ev_cv[b], 0));
+    CK(cudaMemcpyAsync(h->xup[b], src, S * sizeof(double), cudaMemcpyHostToDevice, h->s_up));
+    CK(cudaEventRecord(h->ev_in[b], h->s_up));
+    CK(cudaStreamWaitEvent(h->s_cv, h->ev_in[b], 0));
+    k_to_f32x2<<<592, 256, 0, h->s_cv>>>(h->xup[b], p, q, S,
+                                         h->comp ? h->lo[cur] + n * S : nullptr,
+                                         h->comp ? h->lo[cur ^ 1] + n * S : nullptr);
     h->launches++;
+    CK(cudaEventRecord(h->ev_cv[b], h->s_cv));
   }
   return 0;
 }
@@ -2180,24 +2237,36 @@ int down_tracer(shoc_tr_gpu *h, int buf, int n, double *dst) {
 int step_pipelined(shoc_tr_gpu *h, shoc_tr_state *st) {
   int rc = pipe_init(h);
   if (rc) return rc;
-  rc = shoc_tr_gpu_set_flow(h, st);
+  // the surface vectors go through page-locked memory (the caller's copies of
+  // them are rarely registered)
+  shoc_tr_state fl = *st;
+  if (st->sur_t && st->nsur_t) {
+    const size_t nb = ((size_t)h->ncol + 1) * sizeof(int);
+    memcpy(h->h_surf, st->sur_t, nb);
+    memcpy(h->h_surf + h->ncol + 1, st->nsur_t, nb);
+    fl.sur_t = h->h_surf;
+    fl.nsur_t = h->h_surf + h->ncol + 1;
+  }
+  rc = shoc_tr_gpu_set_flow(h, &fl);
   if (rc) return rc;
-  const int cur = h->cur, csl = pipe_chunk_slots(h);
-  const int nch = (h->nslot + csl - 1) / csl;
+  const int cur = h->cur;
+  const std::vector<int> chunk = pipe_chunks(h);
+  const int nch = (int)chunk.size();
   cudaEvent_t *ev = h->pev.data();  // [0] flow sent, [1 + 2j] chunk j sent, [2 + 2j] stepped
   // the tracers follow the flow fields up the link
   CK(cudaEventRecord(ev[0], h->stream));
   CK(cudaStreamWaitEvent(h->s_up, ev[0], 0));
-  for (int j = 0; j < nch; j++) {
-    for (int sl = j * csl; sl < std::min(h->nslot, (j + 1) * csl); sl++) {
+  int up = 0;
+  for (int j = 0, sl = 0; j < nch; j++) {
+    for (const int end = sl + chunk[j]; sl < end; sl++) {
       const int n = h->slot_host[sl];
-      rc = up_tracer(h, cur, n, st->tr_wc[n]);
+      rc = up_tracer(h, cur, up++, n, st->tr_wc[n]);
       if (rc) {
         pipe_drain(h);
         return rc;
       }
     }
-    CK(cudaEventRecord(ev[1 + 2 * j], h->s_up));
+    CK(cudaEventRecord(ev[1 + 2 * j], h->s_cv));
   }
   // the schedule from this step's flow, while the tracers travel
   Sched s;
@@ -2208,8 +2277,8 @@ int step_pipelined(shoc_tr_gpu *h, shoc_tr_state *st) {
     return rc;
   }
   const int fin = cur ^ (int)(s.sub.size() & 1);  // the buffer the step ends in
-  for (int j = 0; j < nch; j++) {
-    const int s0 = j * csl, ns = std::min(h->nslot - s0, csl);
+  for (int j = 0, s0 = 0; j < nch; s0 += chunk[j++]) {
+    const int ns = chunk[j];
     TrSet Tc = h->T;
     Tc.slot_tr = h->T.slot_tr + s0;
     Tc.nslot = ns;
@@ -2534,21 +2603,20 @@ int shoc_tr_gpu_run(shoc_tr_gpu *h, int nsteps) {
 int shoc_tr_gpu_sync(shoc_tr_gpu *h, shoc_tr_diag *diag) {
   if (!h) return SHOC_TR_EARG;
   DeviceScope dev_(h->device);
-  CK(cudaMemcpyAsync(h->h_status, h->W.status, 4, cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaMemcpyAsync(h->h_nwarn, h->W.nwarn, 8, cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaMemcpyAsync(h->h_counts, h->d_counts, 8, cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaMemsetAsync(h->W.status, 0, 4, h->stream));
-  CK(cudaMemsetAsync(h->W.nwarn, 0, 8, h->stream));
+  CK(cudaMemcpyAsync(h->h_rb, h->d_rb, sizeof(*h->h_rb), cudaMemcpyDeviceToHost, h->stream));
+  // nwarn and, beside it, the status
+  CK(cudaMemsetAsync(&h->d_rb->nwarn, 0, offsetof(shoc_tr_gpu::Readback, pad) -
+                     offsetof(shoc_tr_gpu::Readback, nwarn), h->stream));
   CK(cudaStreamSynchronize(h->stream));
-  int rc = map_status(*h->h_status);
+  int rc = map_status(h->h_rb->status);
   if (!rc) rc = h->last_status;
   h->last_status = 0;
   if (diag) {
     diag->nsub = (int)h->sched.sub.size();
     diag->dtm = h->sched.dtm;
-    diag->nwarn = (long long)*h->h_nwarn;
-    diag->vcs = h->h_counts[0];
-    diag->vc = h->h_counts[1];
+    diag->nwarn = (long long)h->h_rb->nwarn;
+    diag->vcs = h->h_rb->counts[0];
+    diag->vc = h->h_rb->counts[1];
   }
   if (h->profile) {
     std::vector<cudaEvent_t> done;
@@ -2576,9 +2644,14 @@ int shoc_tr_gpu_step(shoc_tr_gpu *h, shoc_tr_state *st, shoc_tr_diag *diag) {
     shoc_tr_gpu_sync(h, nullptr);
     return rc;
   }
+  // the surface vectors come back with the status
+  const size_t nb = (size_t)h->ncol * sizeof(int);
+  int *const sur = h->h_surf + 1, *const nsur = sur + h->ncol + 1;
+  if (st->sur_t) CK(cudaMemcpyAsync(sur, h->W.sur_t, nb, cudaMemcpyDeviceToHost, h->stream));
+  if (st->nsur_t) CK(cudaMemcpyAsync(nsur, h->W.nsur_t, nb, cudaMemcpyDeviceToHost, h->stream));
   rc = shoc_tr_gpu_sync(h, diag);
-  int rc2 = shoc_tr_gpu_get_surface(h, st->sur_t, st->nsur_t);
-  if (!rc) rc = rc2;
+  if (st->sur_t) memcpy(st->sur_t + 1, sur, nb);
+  if (st->nsur_t) memcpy(st->nsur_t + 1, nsur, nb);
   return rc;
 }
 
@@ -2794,10 +2867,10 @@ static int cols_buffer(shoc_tr_gpu *h) {
 }
 
 static int cols_status(shoc_tr_gpu *h) {
-  CK(cudaMemcpyAsync(h->h_status, h->W.status, 4, cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaMemcpyAsync(&h->h_rb->status, h->W.status, 4, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaMemsetAsync(h->W.status, 0, 4, h->stream));
   CK(cudaStreamSynchronize(h->stream));
-  return map_status(*h->h_status);
+  return map_status(h->h_rb->status);
 }
 
 int shoc_tr_gpu_tridiag(shoc_tr_gpu *h, const double *C, const double *Cm1, const double *Cp1,
@@ -2990,9 +3063,9 @@ int shoc_tr_gpu_substep_min(shoc_tr_gpu *h, double *dmin) {
   h->launches++;
   launch_set_dz(h, SD_PROBE | SD_SEARCH);
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(h->h_dtm, h->W.dtm_bits, 8, cudaMemcpyDeviceToHost, st));
+  CK(cudaMemcpyAsync(&h->h_rb->dtm, h->W.dtm_bits, 8, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  unsigned long long b = *h->h_dtm;
+  unsigned long long b = h->h_rb->dtm;
   memcpy(dmin, &b, 8);
   return SHOC_TR_OK;
 }
