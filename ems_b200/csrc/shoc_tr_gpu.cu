@@ -263,7 +263,9 @@ __device__ __forceinline__ void atomic_min_pos(unsigned long long *p, double v) 
 // layer the thicknesses, the work arrays, the sub-step search and the rows of
 // the tridiagonal matrix (their divisions included); (2) one warp runs the
 // recurrence div(j) = C(j) - cm1(j) cp1(j-1) / div(j-1) from shared memory;
-// (3) all warps write the factors.  Every value is the reference's expression
+// (3) all warps write the factors.  (In shared memory a row is 28 bytes: four
+// blocks an SM at 50 layers, where a column for each value made three.)  Every
+// value is the reference's expression
 // on the reference's operands; the sub-step minimum does not depend on the
 // order the cells are visited in.
 //
@@ -280,9 +282,9 @@ constexpr int SD_WORK = 8;    // w5, w9, dbz, dfz of the tile kernels' columns
 constexpr int SD_LU64 = 16;   // FP64 LU factors of the tile kernels' columns
                               // (the general path's columns get all of them)
 constexpr int kSetDzWarps = 8;
-// bytes: FP64 faces (then ud), rows cm1 and dz/dt (then div; for SD_F32 once
-// more, then the UL diagonal) and the cells of nz layers of 32 columns
-inline size_t set_dz_smem(int nz, bool f32) { return (size_t)nz * 32 * ((f32 ? 4 : 3) * 8 + 4); }
+// bytes: FP64 faces (SD_F32: then the diagonal eliminated from the top), rows cm1
+// and dz/dt (then div) and the cells of nz layers of 32 columns
+inline size_t set_dz_smem(int nz) { return (size_t)nz * 32 * (3 * 8 + 4); }
 
 __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
     k_set_dz(Geo G, Flow F, Work W, Opt O, Tile Tl, int any_vdiff, int *counts, int list_all,
@@ -290,13 +292,11 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr unsigned FULL = 0xffffffffu;
   const int nz = G.nz, lane = threadIdx.x, wy = threadIdx.y;
-  double *const sZ = reinterpret_cast<double *>(smem) + lane;  // bottom face z, then ud
+  double *const sZ = reinterpret_cast<double *>(smem) + lane;  // bottom face z, then sE
   double *const sCm = sZ + nz * 32;                            // cm1
   double *const sDv = sCm + nz * 32;                           // dz / dt, then div
-  double *const sE = sDv + nz * 32;                            // dz / dt, then e (SD_F32)
-  int *const sC = reinterpret_cast<int *>(reinterpret_cast<double *>(smem) +
-                                          ((what & SD_F32) ? 4 : 3) * nz * 32) +
-                  lane;
+  double *const sE = sZ;                                       // dz / dt, then e (SD_F32)
+  int *const sC = reinterpret_cast<int *>(reinterpret_cast<double *>(smem) + 3 * nz * 32) + lane;
   __shared__ int sJa[32];        // highest layer <= jn of zero thickness
   __shared__ double sMin[kSetDzWarps];
   const int col = blockIdx.x * 32 + lane;
@@ -376,7 +376,6 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
     if (j <= jn && !dzc) atomicMax(&sJa[lane], j);
     if (any_vdiff) {  // rows of the implicit solve (:3841-3889)
       sDv[k * 32] = dzc / dt;
-      if (what & SD_F32) sE[k * 32] = dzc / dt;
       sCm[k * 32] = -__ldg(&F.Kz[cc]) / (0.5 * (dzm + dzc));
     }
     if (search && j <= js) {
@@ -403,6 +402,13 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
   for (int o = 16; o > 0; o >>= 1) dtmin = fmin(dtmin, __shfl_xor_sync(FULL, dtmin, o));
   if (lane == 0) sMin[wy] = dtmin;
   __syncthreads();
+
+  // the faces are done with: the second elimination's rows take their place
+  if ((what & SD_F32) && any_vdiff) {
+    for (int k = wy; k < nz; k += kSetDzWarps)
+      if (on && k >= kb) sE[k * 32] = sDv[k * 32];
+    __syncthreads();
+  }
 
   // (2) flags and the solve's range, in every warp alike; warp 0 runs the LU
   int flags = 0, cbs = 0, jb = 0, stat = 0;
@@ -450,7 +456,6 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
       double div = sDv[k * 32] - bp1;
       sCm[k * 32] = 0.0;
       sDv[k * 32] = div;
-      sZ[k * 32] = 0.0;
       const int kt = kb + jn - 1;
 #pragma unroll 2
       for (++k; k <= kt; ++k) {
@@ -461,7 +466,6 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
         div = C - cm1 * ud;
         if (div == 0.0) stat |= ST_PIVOT;
         sDv[k * 32] = div;
-        sZ[k * 32] = ud;
         bp1 = cp1;
       }
     }
@@ -505,7 +509,7 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
   __syncthreads();
 
   // (3) the factors (and the work arrays of a column the tile kernels turned
-  // out not to handle, whose faces the ud have overwritten: from W.dz)
+  // out not to handle, whose faces may be overwritten: from W.dz)
   const bool lu64 = (what & SD_LU64) || !staged;
   const bool late = on && pre_staged && !staged && !(what & SD_WORK);
   if (!solve && !late) return;
@@ -514,8 +518,11 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
     const int j = k - kb + 1, cc = sC[k * 32];
     const double dzc = W.dz[cc];
     if (solve && j >= jb && j <= jn) {
-      const double dzdt = dzc / dt, cm1 = sCm[k * 32], div = sDv[k * 32], ud = sZ[k * 32];
+      const double dzdt = dzc / dt, cm1 = sCm[k * 32], div = sDv[k * 32];
       if (lu64) {
+        // the elimination factor, as the recurrence formed it (cm1 is the upper
+        // diagonal of the row below)
+        const double ud = j > jb ? cm1 / sDv[(k - 1) * 32] : 0.0;
         W.vd_cm1[cc] = cm1;
         W.vd_div[cc] = div;
         W.vd_ud[cc] = ud;
@@ -1714,7 +1721,7 @@ int shoc_tr_gpu_create(const shoc_tr_geom *g, const shoc_tr_opts *o, int ntr, in
   if (cudaHostAlloc(&pin, 64, cudaHostAllocDefault) != cudaSuccess) TRY(SHOC_TR_ENOMEM);
   h->h_rb = (shoc_tr_gpu::Readback *)pin;
   if (cudaFuncSetAttribute(k_set_dz, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)set_dz_smem(kMaxLayers, true)) != cudaSuccess ||
+                           (int)set_dz_smem(kMaxLayers)) != cudaSuccess ||
       tile64_set_smem_attr() != cudaSuccess ||
       tile32_set_smem_attr() != cudaSuccess)
     TRY(SHOC_TR_ECUDA);
@@ -1796,8 +1803,7 @@ void launch_set_dz(shoc_tr_gpu *h, int what) {
     what |= SD_F32 | (h->comp ? SD_WORK : 0);
   else
     what |= SD_WORK | SD_LU64;
-  k_set_dz<<<h->tl.ncolp / 32, dim3(32, kSetDzWarps), set_dz_smem(h->nz, (what & SD_F32) != 0),
-             h->stream>>>(
+  k_set_dz<<<h->tl.ncolp / 32, dim3(32, kSetDzWarps), set_dz_smem(h->nz), h->stream>>>(
       h->G, h->F, h->W, h->O, h->tl, h->any_vdiff ? 1 : 0, h->d_counts, h->staged ? 1 : 0, what,
       h->colown);
   h->launches++;
