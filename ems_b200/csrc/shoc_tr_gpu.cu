@@ -282,8 +282,9 @@ constexpr int SD_WORK = 8;    // w5, w9, dbz, dfz of the tile kernels' columns
 constexpr int SD_LU64 = 16;   // FP64 LU factors of the tile kernels' columns
                               // (the general path's columns get all of them)
 constexpr int kSetDzWarps = 8;
-// bytes: FP64 faces (SD_F32: then the diagonal eliminated from the top), rows cm1
-// and dz/dt (then div) and the cells of nz layers of 32 columns
+// bytes: FP64 faces (then the diagonal eliminated from the top with SD_F32, else
+// the elimination factors), rows cm1 and dz/dt (then div) and the cells of nz
+// layers of 32 columns
 inline size_t set_dz_smem(int nz) { return (size_t)nz * 32 * (3 * 8 + 4); }
 
 __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
@@ -466,6 +467,7 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
         div = C - cm1 * ud;
         if (div == 0.0) stat |= ST_PIVOT;
         sDv[k * 32] = div;
+        if (!(what & SD_F32)) sZ[k * 32] = ud;
         bp1 = cp1;
       }
     }
@@ -521,8 +523,11 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
       const double dzdt = dzc / dt, cm1 = sCm[k * 32], div = sDv[k * 32];
       if (lu64) {
         // the elimination factor, as the recurrence formed it (cm1 is the upper
-        // diagonal of the row below)
-        const double ud = j > jb ? cm1 / sDv[(k - 1) * 32] : 0.0;
+        // diagonal of the row below); where the second elimination has the
+        // faces' place it is formed again, for the few general-path columns
+        const double ud = j <= jb           ? 0.0
+                          : (what & SD_F32) ? cm1 / sDv[(k - 1) * 32]
+                                            : sZ[k * 32];
         W.vd_cm1[cc] = cm1;
         W.vd_div[cc] = div;
         W.vd_ud[cc] = ud;
