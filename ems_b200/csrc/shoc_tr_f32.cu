@@ -57,20 +57,15 @@ void tile32_substep(bool last, bool quick, bool ult, cudaStream_t st, const Geo 
                     double *carry, double *fzs, const int16_t *lo_in, int16_t *lo_out,
                     int vd_nw, int vd_pf, int any_hd, int adv_flags, cudaEvent_t *ev) {
   if (ev) cudaEventRecord(ev[0], st);
-  if (T.ntb > 0 && Tl.nwet > 0) {
+  // kMaxTracers a launch: the kernel lists its tracers in shared memory
+  for (int s0 = 0; s0 < T.ntb && Tl.nwet > 0; s0 += kMaxTracers) {
     const int grid = (Tl.nwet + kAdv32Block - 1) / kAdv32Block;
-    if (quick && ult)
-      adv_mode<true, true>(adv_flags, grid, st, G, F3, W, T, ss, Tl, fx2, fy2, tin, tout, rnd,
-                           fzs, any_hd, lo_in);
-    else if (quick)
-      adv_mode<true, false>(adv_flags, grid, st, G, F3, W, T, ss, Tl, fx2, fy2, tin, tout, rnd,
-                            fzs, any_hd, lo_in);
-    else if (ult)
-      adv_mode<false, true>(adv_flags, grid, st, G, F3, W, T, ss, Tl, fx2, fy2, tin, tout, rnd,
-                            fzs, any_hd, lo_in);
-    else
-      adv_mode<false, false>(adv_flags, grid, st, G, F3, W, T, ss, Tl, fx2, fy2, tin, tout, rnd,
-                             fzs, any_hd, lo_in);
+    TrSet Tc = T;
+    Tc.slot_tr += s0;
+    Tc.ntb = std::min(T.ntb - s0, kMaxTracers);
+    auto adv = quick ? (ult ? adv_mode<true, true> : adv_mode<true, false>)
+                     : (ult ? adv_mode<false, true> : adv_mode<false, false>);
+    adv(adv_flags, grid, st, G, F3, W, Tc, ss, Tl, fx2, fy2, tin, tout, rnd, fzs, any_hd, lo_in);
   }
   if (ev) cudaEventRecord(ev[1], st);
   // one launch for every depth: blocks of the shared memory vd_nw warps need at

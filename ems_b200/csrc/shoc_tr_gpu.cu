@@ -1999,7 +1999,7 @@ int launch_part_b(shoc_tr_gpu *h, const Sched &s, int cur0, const TrSet &T,
           h->ev.push_back({1, ev[0], ev[1]});
           h->ev.push_back({2, ev[1], ev[2]});
         }
-        h->launches += (T.ntb > 0 && h->tl.nwet > 0 ? 1 : 0) + 1;
+        h->launches += (h->tl.nwet > 0 ? (T.ntb + kMaxTracers - 1) / kMaxTracers : 0) + 1;
       }
       int16_t *lo_out = h->comp ? h->lo[cur ^ 1] : nullptr;
       launch_general<float>(h, last, T, ss, tin, tout, c3row, c3_load, lo_out);

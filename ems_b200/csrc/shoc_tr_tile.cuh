@@ -164,7 +164,8 @@ constexpr int kAdv32Block = 128, kAdv32MinBlocks = 5;
 constexpr int kAdvValues = 11;     // stencil values of a cell and tracer
 // dynamic shared memory of k_adv32: the double-buffered stencil values
 constexpr size_t kAdvSmem = (size_t)2 * kAdvValues * kAdv32Block * sizeof(float);
-constexpr int kMaxTracers = 256;   // tracers a handle of the FP32-mixed path may carry
+constexpr int kMaxTracers = 256;   // tracers a launch of k_adv32 lists (a handle without
+                                   // the compensated store may carry)
 
 namespace f32 {
 
