@@ -67,3 +67,63 @@ def test_extreme_values(scale):
     case.tr[2, c] = np.where(c % 5 < 2, -case.tr[2, c], case.tr[2, c])
     case.tr[3, c] = scale * (c % 2)
     check(case)
+
+
+def test_open_floor():
+    """Water through the floor: those columns go the general path."""
+    case = window(50, 14, 8, 3)
+    bots = case.win.bot_t[1:case.win.ncol + 1]
+    case.w[bots[::3]] = 2e-6
+    check(case)
+
+
+def test_maps_that_do_not_stack():
+    """East neighbours of one layer swapped between two rows: no column is a tile's."""
+    case = window(20, 12, 6, 2, land_frac=0.0, depth=(28.0, 29.0))
+    w = case.win
+    wet = np.zeros(w.sgsiz, bool)
+    wet[w.wet_cells()] = True
+    a = next(c for c in w.wet_cells() if w.s2k[c] == 3 and w.s2i[c] == 9 and w.s2j[c] == 4)
+    b = w.yp1[a]
+    ea, eb = int(w.xp1[a]), int(w.xp1[b])
+    assert wet[[a, b, ea, eb]].all()
+    w.xp1[a], w.xp1[b], w.xm1[ea], w.xm1[eb] = eb, ea, b, a
+    check(case)
+
+
+@pytest.mark.parametrize("ntr", [12, 13, 31])
+def test_dropin_chunks(ntr):
+    """More than 2 MB of tracers cross the link in chunks: crossing surfaces and
+    the thin-surface cursor, which runs through the tracers of a column."""
+    layers = np.array([-30.0, -22.0, -14.0, -8.0, -3.0, -1.0, 0.6, 2.5])
+    case = window(80, 60, 7, ntr, layers=layers, depth=(4.0, 29.0), eta_offset=(1.9, -1.7),
+                  hmin=1.2, dt=1500.0)
+    case.maxtr[:] = np.quantile(case.tr[0, case.win.wet_cells()], 0.6)
+    assert case.tr.nbytes > 2 << 20
+    tr, sur, nsur = case.copy_state()
+    t = gpu.TracerStep(case)
+    nsub = [t.step(tr, sur, nsur).nsub for _ in range(2)]
+    t.close()
+    assert max(nsub) > 1
+    rc, ref, rsur, rnsur, _ = oracle.run_oracle(case, 2)
+    assert rc == 0
+    np.testing.assert_array_equal(tr[:, 1:], ref[:, 1:])
+    np.testing.assert_array_equal(sur, rsur)
+    np.testing.assert_array_equal(nsur, rnsur)
+
+
+def test_more_tracers_than_an_fp32_launch_lists():
+    """Compensated FP32: a tracer's values do not depend on how many there are."""
+    def last(case, keep):
+        t = gpu.TracerStep(case, precision=gpu.FP32_COMP)
+        t.start()
+        t.run(2)
+        t.sync()
+        tr = t.download()[keep]
+        t.close()
+        return tr[:, case.win.wet_cells()]
+    many = window(33, 9, 7, 259)
+    few = window(33, 9, 7, 4)
+    keep = [0, 255, 256, 258]
+    few.tr[:] = many.tr[keep]
+    np.testing.assert_array_equal(last(many, keep), last(few, [0, 1, 2, 3]))
