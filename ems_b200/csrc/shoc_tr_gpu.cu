@@ -1072,7 +1072,7 @@ int build_tile_tables(shoc_tr_gpu *h, const shoc_tr_geom *g, const std::vector<u
   }
   // k_vd32 column order: tiles of 32 adjacent columns (a warp's lanes at one
   // layer are adjacent cells: coalesced loads and stores), the tiles sorted
-  // by depth so launches per depth class size shared memory to their tiles
+  // by depth so that blocks running at the same time are alike
   const int ntile = ncolp / 32;
   std::vector<int> tdepth(ntile, 0), tord(ntile);
   for (int t = 0; t < ntile; t++) {
@@ -2139,22 +2139,32 @@ int step_async(shoc_tr_gpu *h) {
 // lateral boundaries of a chunk may follow it.
 
 // Slots of each chunk.  The first chunk should be back on its way early and the
-// last one's step and copy back, which nothing overlaps, should be short; in
-// between, a chunk's step costs the faces and factors of every cell once more,
-// whatever the number of its tracers.  So the chunks grow from a twelfth of the
-// tracers to a third and shrink again: 300 x 257 x 33, 8 tracers, two sub-steps,
-// FP32-mixed took 4.04 ms a call as eight chunks, 3.53 as five; 256 x 256 x 40, 10
-// tracers, FP64 4.81 and 4.24 (3.39 and 3.87 with the arrived tracers' copies off
-// the link's stream).  A window whose tracers cross the link in tens of
-// microseconds goes as one chunk: the launches of each cost as much (20 x 14 x 6,
-// 3 tracers: 258 us as three, 220 as one).
+// last one's step and copy back, which nothing overlaps, should be short: a 24th
+// of the tracers.  In between, a chunk's step costs the faces and factors of
+// every cell once more, whatever the number of its tracers, which the link hides
+// from two tracers on; a chunk larger than that, or than a twelfth, only keeps
+// the way back waiting.  But launching a chunk costs the host as much as some MB
+// on the link, so where the tracers are small it takes more of them, up to a
+// third.  The chunks double from the first size to that one, and shrink again.
+// A call (B200), by the middle chunks: 256 x 256 x 40, 10 tracers, FP64 one
+// tracer 5.55 ms, two 4.69, four 5.00; 400 x 400 x 40, 12, FP64 one 13.6, two 11.8;
+// 1024 x 512 x 50, 24, FP32-mixed two 76.4, twelve 92.2 (first chunk two 76.8);
+// 160 x 150 x 30, 24, FP64 (3 MB each) two 2.88, six 3.30; 100 x 90 x 30, 24, FP64
+// (1.3 MB) two 1.47, four 1.42, eight 1.58.
+// Twelfths throughout, with the arrived tracers' copies on the link's stream,
+// took 6.13, 14.0, 76.8, 3.55 and 1.92 ms.  A window whose tracers cross the link
+// in tens of microseconds goes as one chunk: the launches of each cost as much
+// (20 x 14 x 6, 3 tracers: 258 us as three, 220 as one).
+constexpr size_t kChunkGrow = (size_t)4 << 20;
 std::vector<int> pipe_chunks(const shoc_tr_gpu *h) {
   const int n = h->nslot;
   if (n == 0) return {};
-  if ((size_t)n * h->S * sizeof(double) <= (size_t)2 << 20) return {n};
+  const size_t bytes = (size_t)h->S * sizeof(double);
+  if (n * bytes <= (size_t)2 << 20) return {n};
   std::vector<int> left, right;
-  const int most = std::max(1, n / 3);
-  for (int c = std::max(1, (n + 11) / 12), rest = n; rest > 0; c = std::min(2 * c, most)) {
+  const int most = std::max({2, (n + 11) / 12,
+                             std::min(n / 3, (int)((kChunkGrow + bytes - 1) / bytes))});
+  for (int c = (n + 23) / 24, rest = n; rest > 0; c = std::min(2 * c, most)) {
     if (rest < 2 * c) {  // the middle
       left.push_back(rest);
       break;
@@ -3275,13 +3285,13 @@ int shoc_tr_gpu_autotune_ex(shoc_tr_gpu *h, int steps, int use_cache, shoc_tr_tu
     if (from_cache) *from_cache = 1;
     return SHOC_TR_OK;
   }
-  // candidates: tracers per column-kernel block for the two-kernel sub-step;
+  // candidates: warps per column-kernel block for the two-kernel sub-step;
   // tile widths and phase-B warps for the fused one (FP32-mixed, where it fits)
   std::vector<shoc_tr_tuning> cand;
   shoc_tr_tuning base = current_tuning(h);
   const std::vector<int> tws = h->esize == sizeof(float)
                                    ? std::vector<int>{2, 3, 4, 5, 6, 8, 12, 16}
-                                   : std::vector<int>{2, 3, 4, 5, 6, 8};
+                                   : std::vector<int>{1, 2, 3, 4, 5, 6, 8};
   for (int pf : {0, 1}) {
     if (pf && h->esize != sizeof(float)) continue;
     for (int tw : tws) {
