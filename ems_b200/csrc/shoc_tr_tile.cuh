@@ -27,10 +27,9 @@
 //           vertical diffusion (implicit_vdiff_tr, :4067-4214) as an FP32
 //           Thomas sweep, an FP64 residual and one FP32 correction solve,
 //           with the column's FP64 mass carry (column_finish).  A block owns
-//           32 columns of similar depth (a static depth-sorted column order)
-//           so its lanes loop over similar layer ranges; the columns' values,
-//           residuals, LU factors and FP64 thicknesses are staged into shared
-//           memory in one batch of asynchronous copies.
+//           32 neighbouring columns, the blocks in order of depth; the
+//           columns' values, residuals, LU factors and FP64 thicknesses are
+//           staged into shared memory by asynchronous copies.
 //
 // Mass carry.  Storing FP32 values loses mass at every rounding (and the
 // FP32 solve conserves the column mass only to its residual).  Per (tracer,

@@ -374,8 +374,9 @@ class TracerStep:
 
     def autotune(self, steps=2):
         """Pick the fastest launch configuration (`steps` trial steps per
-        candidate from the current state, which is put back); returns the
-        tracers per block (shoc_tr_gpu_autotune, no cache)."""
+        candidate from the current state, which is put back); returns
+        tracers_per_block, the column kernel's warps per block
+        (shoc_tr_gpu_autotune, no cache)."""
         tw = C.c_int()
         _check("autotune", self.L.shoc_tr_gpu_autotune(self.h, int(steps), C.byref(tw)))
         return tw.value

@@ -127,3 +127,25 @@ def test_more_tracers_than_an_fp32_launch_lists():
     keep = [0, 255, 256, 258]
     few.tr[:] = many.tr[keep]
     np.testing.assert_array_equal(last(many, keep), last(few, [0, 1, 2, 3]))
+
+
+@pytest.mark.parametrize("nz", [3, 8, 9, 17, 33])
+def test_preamble_depths(nz):
+    """Columns shorter than, as long as and longer than a batch of cells, with
+    surfaces that cross layer faces between the steps."""
+    case = window(14, 11, nz, 2, eta_offset=(1.9, -1.7),
+                  layers=np.concatenate([np.linspace(-5.0 * nz, -1.5, nz), [2.5]]))
+    detadt = (case.eta - case.oldeta) / case.dt
+    t = gpu.TracerStep(case)
+    t.start()
+    t.set_preamble(True, detadt)
+    sur, nsur = case.sur_t.copy(), case.nsur_t.copy()
+    for _ in range(2):
+        want = oracle.preamble(case, detadt, sur, nsur)
+        t.run(1)
+        t.sync()
+        got = t.get_flow()
+        for k in ("w", "u1flux3d", "u2flux3d", "dzu1", "dzu2"):
+            np.testing.assert_array_equal(got[k], want[k], err_msg=k)
+        sur, nsur = t.surface()
+    t.close()
