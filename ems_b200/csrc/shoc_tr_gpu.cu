@@ -1277,9 +1277,8 @@ int apply_tuning(shoc_tr_gpu *h, const shoc_tr_tuning &t) {
   if (t.tracers_per_block < 1 || t.tracers_per_block > (f32 ? kVd32MaxWarps : 8))
     return SHOC_TR_EUNSUPPORTED;
   if (t.prefetch && !f32) return SHOC_TR_EUNSUPPORTED;
-  // (FP64: two values a row and warp must fit; k_vd64 takes the warps that do)
   const size_t vb = f32 ? vd32_smem(h->nz, t.tracers_per_block, t.prefetch != 0, h->comp)
-                        : (size_t)h->nz * 32 * (4 + 2 * 8 * t.tracers_per_block);
+                        : vd64_tuned(h->nz, t.tracers_per_block);
   if (vb > 227 * 1024) return SHOC_TR_EUNSUPPORTED;
   if (t.fused) {
     const int ti = tile_index(t.tile_x);

@@ -545,14 +545,27 @@ constexpr int kVd64MaxWarps = 16;
 inline size_t vd64_smem(int nd, int nw) {
   return (size_t)nd * 32 * (5 * 8 + 4) + (size_t)nd * nw * 32 * 8;
 }
+// what a setting of nw warps is held to (a launch takes the warps that do fit)
+inline size_t vd64_tuned(int nz, int nw) { return (size_t)nz * 32 * (4 + 2 * 8 * nw); }
 // Warps per block at full depth where the caller sets none: two blocks per SM
 // within 160 KB of its memory, balanced rounds.  The rest is left to the L1,
 // which the back substitution's values come from: 384 x 320 x 40 (10 tracers)
 // 2 warps 0.23 ms, 4 (194 KB) 0.27; 200 x 180 x 30 (6 tracers) 3 warps 0.055, 6
-// 0.051.
+// 0.051.  Deeper columns, where that is a single warp, take two, while two such
+// blocks fit (512 x 256 x 50, 24 tracers: 1 warp 1.32 ms, 2 0.94, 3 0.88, 4 1.13);
+// still deeper ones what a block has within 200 KB (448 x 300 x 60, 16 tracers: 1
+// warp 1.21 ms, 2 0.91, 3 1.15, 6 0.89; 400 x 300 x 80, 12 tracers: 1 warp 1.69, 2
+// 1.24, 4 0.95, 5 1.05).
 inline int vd64_default_warps(int nz, int nslot) {
   int nw = 1;
   while (nw < kVd64MaxWarps / 2 && 2 * (vd64_smem(nz, nw + 1) + 1024) <= 160 * 1024) nw++;
+  if (nw == 1) {
+    nw = 2;
+    if (2 * (vd64_smem(nz, nw) + 1024) > 227 * 1024)
+      while (nw < kVd64MaxWarps / 2 && vd64_smem(nz, nw + 1) <= 200 * 1024 &&
+             vd64_tuned(nz, nw + 1) <= 227 * 1024)
+        nw++;
+  }
   const int rounds = nslot > 0 ? (nslot + nw - 1) / nw : 1;
   return nslot > 0 ? (nslot + rounds - 1) / rounds : 1;
 }
