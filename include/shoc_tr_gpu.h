@@ -248,8 +248,9 @@ int shoc_tr_gpu_set_substep_min(shoc_tr_gpu *h, double dmin);
 /* cudaStream_t of the handle, for event timing by the caller. */
 void *shoc_tr_gpu_stream(shoc_tr_gpu *h);
 
-/* Launch tuning: columns per block (32; 0 keeps it) and tracers per block
- * of the column kernel (0 keeps it).  Takes effect at the next step. */
+/* Launch tuning: columns per block (32; 0 keeps it) and warps per block of
+ * the column kernel (0 keeps it; tracers_per_block of shoc_tr_tuning below).
+ * Takes effect at the next step. */
 int shoc_tr_gpu_set_tiling(shoc_tr_gpu *h, int cols_per_block, int tracers_per_block);
 
 /* The transport kernels' launch configuration.  No reference counterpart
@@ -257,8 +258,9 @@ int shoc_tr_gpu_set_tiling(shoc_tr_gpu *h, int cols_per_block, int tracers_per_b
 typedef struct {
   int fused;             /* FP32-mixed: 1 one fused launch per sub-step (k_step32),
                             0 the advection + column kernel pair */
-  int tracers_per_block; /* column kernel: tracers per k_vd64 block (1..8), or warps per
-                            k_vd32 block, each stepping its share of the tracers (1..16) */
+  int tracers_per_block; /* column kernel: warps per k_vd64 block (1..8) or k_vd32 block
+                            (1..16), each stepping its share of the tracers; its shared
+                            memory is sized for them at full depth */
   int tile_x;            /* k_step32: tile width along i (8, 16, 32; 32 / tile_x
                             columns along j) */
   int phase_b_warps;     /* k_step32: warps of its column phase */
@@ -277,9 +279,10 @@ int shoc_tr_gpu_set_tuning(shoc_tr_gpu *h, const shoc_tr_tuning *t);
  * candidate configuration, times the transport kernels with CUDA events,
  * puts the state back (a device copy taken before the trials: the tracers,
  * surface vectors and mass carry are as they were) and keeps the fastest.
- * Candidates: 2..8 tracers per k_vd64 block, or 2..16 warps per k_vd32
- * block with and without its prefetch; for FP32-mixed also the fused sub-step with tile widths 8, 16, 32 and the most and half
- * the most phase-B warps its shared memory allows.  With use_cache != 0 the
+ * Candidates: 1..8 warps per k_vd64 block, or 2..16 warps per k_vd32
+ * block with and without its prefetch; for FP32-mixed also the fused sub-step
+ * with tile widths 8, 16, 32 and the most and half the most phase-B warps its
+ * shared memory allows.  With use_cache != 0 the
  * choice is looked up in and saved to a file keyed by the GPU model and the
  * window's configuration (sizes, tracers, precision, scheme, diffusion),
  * named by the environment variable SHOC_TR_TUNE_CACHE (default
@@ -289,22 +292,21 @@ int shoc_tr_gpu_set_tuning(shoc_tr_gpu *h, const shoc_tr_tuning *t);
  * The device copy holds one tracer buffer (ntr x S values, plus their
  * compensations with SHOC_TR_FP32_COMP); without room for it the call
  * returns SHOC_TR_ENOMEM and changes nothing.
- * shoc_tr_gpu_autotune is autotune_ex without the cache, returning the
- * tracers per block. */
+ * shoc_tr_gpu_autotune is autotune_ex without the cache, returning
+ * tracers_per_block. */
 int shoc_tr_gpu_autotune_ex(shoc_tr_gpu *h, int steps, int use_cache, shoc_tr_tuning *best,
                             int *from_cache);
 int shoc_tr_gpu_autotune(shoc_tr_gpu *h, int steps, int *tracers_per_block);
 
 /* Time of the transport of a step's last sub-step (the transport kernels
- * of the precision: one launch for SHOC_TR_FP64, the advection and the column
- * kernel for SHOC_TR_FP32_MIXED), averaged over the steps since the last call
+ * of the precision: the advection and the column kernel, or the fused one),
+ * averaged over the steps since the last call
  * (CUDA events on the handle's stream; enabled by shoc_tr_gpu_profile(h, 1)).
  * No reference counterpart: measurement hooks of this library. */
 int shoc_tr_gpu_profile(shoc_tr_gpu *h, int enable);
 int shoc_tr_gpu_kernel_time(shoc_tr_gpu *h, double *ms_per_launch, int *launches);
 /* The same for one part: 0 the whole transport (as above), 1 the advection
- * kernel, 2 the column kernel (tr_bounds, surf_conc, vertical diffusion) of
- * SHOC_TR_FP32_MIXED. */
+ * kernel, 2 the column kernel (tr_bounds, surf_conc, vertical diffusion). */
 int shoc_tr_gpu_kernel_time_part(shoc_tr_gpu *h, int part, double *ms_per_launch,
                                  int *launches);
 
