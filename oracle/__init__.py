@@ -4,7 +4,7 @@ Only tests/, __graft_entry__.smoke() and bench.py's CPU-baseline / reference
 arm may import this package, and only as the thing results are checked
 against or timed beside -- never as part of the product path.
 
-  run_oracle(case, nsteps, ...)  the C restatement (oracle/shoc_oracle.c)
+  run_oracle(case, nsteps, ...)  the C restatement (oracle/shoc_oracle.c), every scheme
   run_ref(case, nsteps, ...)     the reference's own tracers.c, compiled
                                  unmodified (oracle/_ref, built by
                                  oracle/build.py where the reference exists)

@@ -235,6 +235,69 @@ static void van_leer(oracle_ctx *o, const shoc_tr_geom *g, const shoc_tr_state *
   van_leer_do(o->Fz, tr, st->w, o->w8, 1, o->vc, o->s1, g->zp1, g->zm1);
 }
 
+/* Face value of the centred, fourth-order, uniform-grid QUICKEST and
+ * second-order upwind schemes (order2_do, tracers.c:1690-1709; order4_do,
+ * :1757-1776; quickest_uniform, :1944-2031; order2_upwind_do, :3008-3036) from
+ * the values at i-2 .. i+1; d: the centred weight (d3, d4 or w5). */
+static double other_face(int trasc, double d, double vel, double cn, double tm2, double tm1,
+                         double t0, double tp1) {
+  if (trasc == SHOC_TR_ORDER2) return d * (t0 - tm1) + tm1;
+  if (trasc == SHOC_TR_ORDER4) return (7.0 * (tm1 + t0) - (tp1 + tm2)) / 12.0;
+  if (trasc == SHOC_TR_QUICKEST_CO) {
+    double face = 0.5 * (t0 + tm1), grad = t0 - tm1, curv = 0.0;
+    if (cn > 0.0)
+      curv = t0 - 2.0 * tm1 + tm2;
+    else if (cn < 0.0)
+      curv = tp1 - 2.0 * t0 + tm1;
+    return face - 0.5 * cn * grad - (1.0 - cn * cn) * curv / 6.0;
+  }
+  if (vel > 0.0) return 0.5 * (3.0 - cn) * tm1 - 0.5 * (1.0 - cn) * tm2;
+  if (vel < 0.0) return 0.5 * (3.0 - cn) * t0 - 0.5 * (1.0 - cn) * tp1;
+  return 0.0;
+}
+
+/* Their face values: horizontal ones on the interior faces, QUICKEST_CO's on
+ * every wet cell's. */
+static void other_schemes(oracle_ctx *o, const shoc_tr_geom *g, const shoc_tr_state *st, int trasc,
+                          const double *tr) {
+  const int co = trasc == SHOC_TR_QUICKEST_CO;
+  const int nx = co ? g->a3_t : g->v3_e1, ny = co ? g->a3_t : g->v3_e2;
+  const int *lx = co ? g->w3_t : g->w3_e1, *ly = co ? g->w3_t : g->w3_e2;
+  for (int cc = 1; cc <= nx; cc++) {
+    int c = lx[cc], m = g->xm1[c];
+    o->Fx[c] = other_face(trasc, o->d3[g->m2d[c]], st->u1[c], o->w6[c], tr[g->xm1[m]], tr[m],
+                          tr[c], tr[g->xp1[c]]);
+  }
+  for (int cc = 1; cc <= ny; cc++) {
+    int c = ly[cc], m = g->ym1[c];
+    o->Fy[c] = other_face(trasc, o->d4[g->m2d[c]], st->u2[c], o->w7[c], tr[g->ym1[m]], tr[m],
+                          tr[c], tr[g->yp1[c]]);
+  }
+  for (int cc = 1; cc <= o->vc; cc++) {
+    int c = o->s1[cc], m = g->zm1[c];
+    o->Fz[c] = other_face(trasc, o->w5[c], st->w[c], o->w8[c], tr[g->zm1[m]], tr[m], tr[c],
+                          tr[g->zp1[c]]);
+  }
+}
+
+/* First-order upwind fluxes (order1, tracers.c:1584-1617), ghost cells' faces
+ * among them; no limiter. */
+static double upwind(double U, double tm1, double t0) {
+  return 0.5 * (U + fabs(U)) * tm1 + 0.5 * (U - fabs(U)) * t0;
+}
+static void order1(oracle_ctx *o, const shoc_tr_geom *g, const shoc_tr_state *st,
+                   const double *tr, double dtu) {
+  for (int cc = 1; cc <= g->n3_t; cc++) {
+    int c = g->w3_t[cc];
+    o->Fx[c] = upwind(st->u1flux3d[c], tr[g->xm1[c]], tr[c]);
+    o->Fy[c] = upwind(st->u2flux3d[c], tr[g->ym1[c]], tr[c]);
+  }
+  for (int cc = 1; cc <= o->vc; cc++) {
+    int c = o->s1[cc];
+    o->Fz[c] = dtu * upwind(st->w[c], tr[g->zm1[c]], tr[c]);
+  }
+}
+
 /* ULTIMATE universal limiter (ulimate_filter, tracers.c:3501-3557). */
 static void ultimate(const double *cr, double *Fx, const double *F, const int *ctp,
                      int vs, int ve, const int *mapm, const int *mapp) {
@@ -273,10 +336,16 @@ static void ultimate(const double *cr, double *Fx, const double *F, const int *c
 /* Face fluxes: scheme, limiter, times volume flux (advect, tracers.c:1487-1576) */
 static void advect(oracle_ctx *o, const shoc_tr_geom *g, const shoc_tr_state *st,
                    const shoc_tr_opts *op, const double *tr, double dtu) {
+  if (op->trasc == SHOC_TR_ORDER1) {
+    order1(o, g, st, tr, dtu);
+    return;
+  }
   if (op->trasc == SHOC_TR_QUICKEST)
     quickest(o, g, tr);
-  else
+  else if (op->trasc == SHOC_TR_VANLEER)
     van_leer(o, g, st, tr);
+  else
+    other_schemes(o, g, st, op->trasc, tr);
   if (op->ultimate) {
     ultimate(o->w6, o->Fx, tr, g->w3_e1, 1, g->v3_e1, g->xm1, g->xp1);
     ultimate(o->w6, o->Fx, tr, g->w3_t, g->v3_t + 1, g->a3_t, g->xm1, g->xp1);
@@ -390,7 +459,7 @@ static long long tr_bounds(oracle_ctx *o, const shoc_tr_geom *g, shoc_tr_state *
 }
 
 /* Advection + horizontal diffusion with sub-stepping
- * (advect_diffuse, tracers.c:401-1054; QUICKEST/VANLEER branches). */
+ * (advect_diffuse, tracers.c:401-1054). */
 static int advect_diffuse(oracle_ctx *o, const shoc_tr_geom *g, shoc_tr_state *st,
                           const shoc_tr_opts *op, shoc_tr_diag *diag) {
   const int *zm1m = g->zm1;
@@ -637,8 +706,11 @@ static int vert_diffuse_3d(oracle_ctx *o, const shoc_tr_geom *g, shoc_tr_state *
 int oracle_step(oracle_ctx *o, const shoc_tr_geom *g, shoc_tr_state *st,
                 const shoc_tr_opts *op, shoc_tr_diag *diag) {
   if (!o || !g || !st || !op) return SHOC_TR_EARG;
-  if (op->trasc != SHOC_TR_QUICKEST && op->trasc != SHOC_TR_VANLEER)
-    return SHOC_TR_EUNSUPPORTED;
+  switch (op->trasc) {
+    case SHOC_TR_QUICKEST: case SHOC_TR_VANLEER: case SHOC_TR_ORDER1: case SHOC_TR_ORDER2:
+    case SHOC_TR_ORDER4: case SHOC_TR_QUICKEST_CO: case SHOC_TR_ORDER2_UW: break;
+    default: return SHOC_TR_EUNSUPPORTED;
+  }
   if (diag) memset(diag, 0, sizeof(*diag));
   lateral_bc(g, st);
   set_dz(o, g, st, op);
