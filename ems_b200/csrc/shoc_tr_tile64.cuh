@@ -48,7 +48,8 @@ namespace shoc {
 //    one straight line of code the compiler interleaves; one check of the
 //    exponents of the cell's stencil values decides whether quotients may be
 //    formed this way, and a cell that fails it (values below 2^-400 or above
-//    2^490, NaN) computes its faces by the reference's divisions;
+//    2^490, NaN), or has a divisor recip does not round, computes its faces by
+//    the reference's divisions;
 //  - the faces' factors live in shared memory, written when a layer is set up
 //    (in registers they left 12 warps on an SM), and a tracer's stencil values
 //    are loaded while the one before it is computed, of the two values beyond a
@@ -88,7 +89,9 @@ __device__ __forceinline__ bool div_fast(double a, unsigned lo) {
 }
 // RN(1 / d) for |d| in 2^-500 .. 2^500: Newton steps from the hardware's
 // approximation (20 bits); the last one starts within an ulp, so it rounds
-// correctly (Markstein)
+// correctly (Markstein) unless d's significand is all ones: there it meets a
+// tie (2 - 2^-52: 0.5, not 0.5 + 2^-53) that quot does not make good.  unsafe:
+// d may be such a divisor (its low word decides, one comparison)
 __device__ __forceinline__ double recip(double d) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
@@ -96,6 +99,7 @@ __device__ __forceinline__ double recip(double d) {
   y = __fma_rn(__fma_rn(-d, y, 1.0), y, y);
   return __fma_rn(__fma_rn(-d, y, 1.0), y, y);
 }
+__device__ __forceinline__ bool recip_unsafe(double d) { return __double2loint(d) == -1; }
 
 // One face, set up once per cell for every tracer, in the warp's shared memory
 // (a row of 32 doubles each): the Courant number, the scheme's factors for its
@@ -177,16 +181,20 @@ __device__ __noinline__ double face_ref64(const double *f, int bits, double tu, 
 // them, tu (i-2 for a positive Courant number, i+1 for a negative one; tm2 and
 // tp1, both of them, for ORDER4) (advect: quickest :1870-1884, van_leer_do
 // :2102-2117, the other schemes, then ulimate_filter), without horizontal
-// diffusion, for values in the checked range
+// diffusion, for values in the checked range; redo is set where a divisor is not
+// recip's and face_ref64 has to be asked
 template <int SCH, bool ULT>
 __device__ __forceinline__ double face_flux64(const double *f, int bits, double tu, double tm1,
-                                              double t0, double tm2, double tp1) {
+                                              double t0, double tm2, double tp1, bool &redo) {
   if (SCH == SHOC_TR_ORDER1) return order1_flux(f[FC_U * 32], tm1, t0);
   const bool pos = (bits & F64_POS) != 0, val = (bits & F64_VAL) != 0;
   const double tc = pos ? tm1 : t0, td = pos ? t0 : tm1;
   const double diff = td - tu, c = tc - tu, cr = f[FC_CR * 32];
   double y = 0.0;
-  if (ULT || SCH == SHOC_TR_VANLEER) y = recip(diff);
+  if (ULT || SCH == SHOC_TR_VANLEER) {
+    y = recip(diff);
+    redo = redo || recip_unsafe(diff);
+  }
   double v;
   if (SCH == SHOC_TR_QUICKEST) {
     const double grad = t0 - tm1;
@@ -326,12 +334,13 @@ __global__ void __launch_bounds__(kAdv64Warps * 32, 16)
         ec.add(tu);
         ec.add(tm1);
         ec.add(t0);
-        if (SCH == SHOC_TR_ORDER1)
+        if (SCH == SHOC_TR_ORDER1) {
           Fz = order1_z(ft[FC_U * 32], tm1, t0);
-        else if (ec.bad() || (bits & F64_REF))
-          Fz = face_ref64<SCH, ULT>(ft, bits, tu, tm1, t0, tm2, tp1);
-        else
-          Fz = face_flux64<SCH, ULT>(ft, bits, tu, tm1, t0, tm2, tp1);
+        } else {
+          bool redo = ec.bad() || (bits & F64_REF);
+          Fz = face_flux64<SCH, ULT>(ft, bits, tu, tm1, t0, tm2, tp1, redo);
+          if (redo) Fz = face_ref64<SCH, ULT>(ft, bits, tu, tm1, t0, tm2, tp1);
+        }
       }
       sF[(s - sl0) * 32] = Fz;
     }
@@ -434,11 +443,12 @@ __global__ void __launch_bounds__(kAdv64Warps * 32, 16)
       if (adv) {
         // (faces a lane does not have hold whatever their factors give: they
         // are not used)
-        Fxw = face_flux64<SCH, ULT>(fw, bw, tuw, txm1, t0, txm2, txp1);
-        Fys = face_flux64<SCH, ULT>(fs, bs, tus, tym1, t0, tym2, typ1);
-        Fyn = face_flux64<SCH, ULT>(fn, bn, tun, t0, typ1, tym1, typ2);
+        bool redo = refs != 0;
+        Fxw = face_flux64<SCH, ULT>(fw, bw, tuw, txm1, t0, txm2, txp1, redo);
+        Fys = face_flux64<SCH, ULT>(fs, bs, tus, tym1, t0, tym2, typ1, redo);
+        Fyn = face_flux64<SCH, ULT>(fn, bn, tun, t0, typ1, tym1, typ2, redo);
         Fzt = SCH == SHOC_TR_ORDER1 ? order1_z(ft[FC_U * 32], t0, tp1)
-                                    : face_flux64<SCH, ULT>(ft, bt, tut, t0, tp1, tm1, tp2);
+                                    : face_flux64<SCH, ULT>(ft, bt, tut, t0, tp1, tm1, tp2, redo);
         if (SCH != SHOC_TR_ORDER1) {
           ExpCheck ec;
           ec.add(t0);
@@ -458,7 +468,7 @@ __global__ void __launch_bounds__(kAdv64Warps * 32, 16)
             ec.add(tm1);
             ec.add(tp2);
           }
-          if (ec.bad() || refs) {
+          if (ec.bad() || redo) {
 #pragma unroll 1
             for (int q = 0; q < 4; ++q) {  // (one call: four would cost registers)
               const bool w = q == 0, y = q == 1, z = q == 3;
