@@ -65,11 +65,18 @@ namespace shoc {
 // 34, 1990: with y the correctly rounded reciprocal, q within an ulp of a / b
 // and r = a - b q exact, RN(q + r y) is RN(a / b); the first correction brings
 // RN(a y) within an ulp) where neither a, b nor a / b are near the ends of the
-// range, or a is 0
+// range, or a is 0.  A zero quotient may have the other sign (a = -0 over b > 0);
+// with a residual of the opposite sign, which costs the same, it has a's.
 __device__ __forceinline__ double quot(double a, double b, double y) {
   double q = __dmul_rn(a, y);
   q = __fma_rn(__fma_rn(-b, q, a), y, q);
   return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+// the same for b > 0, of a zero too
+__device__ __forceinline__ double quot_pos(double a, double b, double y) {
+  double q = __dmul_rn(a, y);
+  q = __fma_rn(-__fma_rn(b, q, -a), y, q);
+  return __fma_rn(-__fma_rn(b, q, -a), y, q);
 }
 // |x| outside 2^-lim .. 2^lim (a zero too)
 template <unsigned LIM>
@@ -202,22 +209,22 @@ __device__ __forceinline__ double face_flux64(const double *f, int bits, double 
     // (2 tc is exact, so its fused subtraction rounds as the separate one)
     const double curv =
         __fma_rn(-2.0, tc, f[FC_DB * 32] * (f[FC_P * 32] * td + f[FC_Q * 32] * tu));
-    const double q = v - 0.5 * cr * grad - quot(f[FC_E * 32] * curv, 6.0, 1.0 / 6.0);
+    const double q = v - 0.5 * cr * grad - quot_pos(f[FC_E * 32] * curv, 6.0, 1.0 / 6.0);
     v = (bits & F64_MOVE) ? q : v;
   } else if (SCH == SHOC_TR_QUICKEST_CO) {
     const double curv = pos ? t0 - 2.0 * tm1 + tu : tu - 2.0 * t0 + tm1;
     const double w = (bits & F64_MOVE) ? f[FC_E * 32] * curv : 0.0;
-    v = 0.5 * (t0 + tm1) - 0.5 * cr * (t0 - tm1) - quot(w, 6.0, 1.0 / 6.0);
+    v = 0.5 * (t0 + tm1) - 0.5 * cr * (t0 - tm1) - quot_pos(w, 6.0, 1.0 / 6.0);
   } else if (SCH == SHOC_TR_VANLEER) {
     // with the flow negative the reference's differences, and their quotient,
-    // have the opposite signs, and the value is t0 minus the term
+    // have the opposite signs (a zero too), and the value is t0 minus the term
     const double p = c * (td - tc);
-    const double s = p > 0.0 ? quot(2.0 * p, diff, y) : 0.0;
+    const double s = p > 0.0 ? quot(2.0 * p, diff, y) : pos ? 0.0 : -0.0;
     v = val ? tc + f[FC_E * 32] * s : 0.0;
   } else if (SCH == SHOC_TR_ORDER2) {
     v = val ? order2_face(f[FC_D * 32], tm1, t0) : 0.0;
   } else if (SCH == SHOC_TR_ORDER4) {
-    v = val ? quot(7.0 * (tm1 + t0) - (tp1 + tm2), 12.0, 1.0 / 12.0) : 0.0;
+    v = val ? quot_pos(7.0 * (tm1 + t0) - (tp1 + tm2), 12.0, 1.0 / 12.0) : 0.0;
   } else {  // ORDER2_UW
     v = val ? 0.5 * (3.0 - cr) * tc - 0.5 * (1.0 - cr) * tu : 0.0;
   }
@@ -225,8 +232,8 @@ __device__ __forceinline__ double face_flux64(const double *f, int bits, double 
     const double nc = quot(c, diff, y), nu = quot(v - tu, diff, y), acr = fabs(cr);
     const double ya = f[FC_Y * 32], p = nc * diff;
     const bool in = nc >= 0.0 && nc <= 1.0;
-    const bool cap = nu > quot(nc, acr, ya);
-    const double up = tu + p, upc = tu + quot(p, acr, ya);
+    const bool cap = nu > quot_pos(nc, acr, ya);
+    const double up = tu + p, upc = tu + quot_pos(p, acr, ya);
     double l = cap ? upc : v;
     l = nu < nc ? up : l;
     l = nu > 1.0 ? td : l;
@@ -234,6 +241,20 @@ __device__ __forceinline__ double face_flux64(const double *f, int bits, double 
     v = (diff != 0.0 && (bits & F64_LIM)) ? l : v;
   }
   return v * f[FC_U * 32];
+}
+
+// What the reference has for a floor that lets nothing through (w = 0): 0 times the
+// face value between the ghost below, which holds t0, t0 and tp1 above.  It
+// matters where t0 is a zero whose sign it may decide (the schemes of
+// kFloorZero64: the others' is +0 then), or not finite.
+template <int SCH>
+constexpr bool kFloorZero64 = SCH == SHOC_TR_ORDER1 || SCH == SHOC_TR_ORDER4 ||
+                              SCH == SHOC_TR_QUICKEST_CO;
+template <int SCH>
+__device__ __forceinline__ double floor_flux64(double t0, double tp1) {
+  if (SCH == SHOC_TR_VANLEER || SCH == SHOC_TR_ORDER2_UW) return 0.0;
+  if (SCH == SHOC_TR_ORDER4) return 0.0 * order4_face(t0, t0, t0, tp1);
+  return 0.0 * (kFloorZero64<SCH> ? t0 : 0.0 + t0);
 }
 
 // Whether every value of a list lies in 2^-400 .. 2^490 or is 0: differences
@@ -469,6 +490,7 @@ __global__ void __launch_bounds__(kAdv64Warps * 32, 16)
             ec.add(tp2);
           }
           if (ec.bad() || redo) {
+            if (k == kb) sF[(s - sl0) * 32] = floor_flux64<SCH>(t0, tp1);
 #pragma unroll 1
             for (int q = 0; q < 4; ++q) {  // (one call: four would cost registers)
               const bool w = q == 0, y = q == 1, z = q == 3;
@@ -506,12 +528,13 @@ __global__ void __launch_bounds__(kAdv64Warps * 32, 16)
       const double dtr = (Fxe - Fxw + Fyn - Fys) * dtu;
       double val = dtr;
       if (k <= ks) {
-        const double Fzb = sF[(s - sl0) * 32];
+        const double Fzb = kFloorZero64<SCH> && k == kb ? floor_flux64<SCH>(t0, tp1)
+                                                          : sF[(s - sl0) * 32];
         if (below) {
           sF[(s - sl0) * 32] = Fzt;
           // interior cell (tracers.c:912-925); Ds = Hn1 = 1 in z coordinates
-          const double net = quot(dtr, area, yarea) + (Fzt - Fzb);
-          val = t0 - quot(net, dzc, ydz);
+          const double net = quot_pos(dtr, area, yarea) + (Fzt - Fzb);
+          val = t0 - quot_pos(net, dzc, ydz);
           if (!((div_fast(dtr, rng) || dtr == 0.0) && (div_fast(net, rng) || net == 0.0)))
             val = t0 - (dtr / area + (Fzt - Fzb)) / dzc;
         } else {
