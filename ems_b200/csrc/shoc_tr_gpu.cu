@@ -443,10 +443,7 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
   ci.cbs = cbs;
   ci.flags = flags;
   ci.ks = kb + js - 1;
-  // (k_adv64 takes floors as closed: a column whose floor lets water through
-  // goes the general path)
-  const bool staged = on && O.tiled && staged_column(ci, bot, O.cross != 0) &&
-                      !(O.cross && F.w[bot] != 0.0);
+  const bool staged = on && O.tiled && staged_column(ci, bot, O.cross != 0);
   if (staged) ci.flags |= COL_STAGED;
   if (wy == 0) {
     if (solve) {

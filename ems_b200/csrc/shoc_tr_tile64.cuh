@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(kAdv64Warps * 32, 16)
   const bool own = sc >= 0 && !(sc & kSegHalo);
   const int col = sc >= 0 ? (sc & ~kSegHalo) : -1;
   int kb = G.nz, ks = -1, c2 = 0, ntc = 0;
-  bool staged = false;
+  bool staged = false, open = false;  // open: water goes through the floor, in this chunk
   if (col >= 0) {
     const int4 r = __ldg(&Tl.colrec[col]);
     kb = r.z;
@@ -312,6 +312,7 @@ __global__ void __launch_bounds__(kAdv64Warps * 32, 16)
     staged = own && (ci.flags & COL_STAGED);
     ks = ci.ks;
     ntc = __ldg(&G.colntr[col]);
+    if (staged && kb >= k0 && kb < k1) open = __double_as_longlong(__ldg(&F.w[r.x])) != 0;
   }
   if (!__any_sync(FULL, staged)) return;
   const double dtu = ss.dtu;
@@ -332,18 +333,20 @@ __global__ void __launch_bounds__(kAdv64Warps * 32, 16)
     return dtu * (0.5 * (w + fabs(w)) * tm1 + 0.5 * (w - fabs(w)) * t0);
   };
 
-  // the flux through the bottom of the chunk's first layer, for every tracer
+  // the flux through the bottom of the chunk's first layer, or through an open
+  // floor in the chunk, for every tracer (a closed floor's is 0)
   {
-    const int c = (staged && k0 >= kb && k0 <= ks) ? __ldg(&Tl.cellk[(size_t)k0 * Tl.ncolp + col])
-                                                   : 0;
+    const int kk = open ? kb : k0;
+    const int c = (staged && (open || k0 > kb) && kk <= ks)
+                      ? __ldg(&Tl.cellk[(size_t)kk * Tl.ncolp + col]) : 0;
     int4 nzv = make_int4(0, 0, 0, 0);
     int bits = 0;
-    const bool flow = c && k0 > kb;  // (a column's floor is closed)
+    const bool flow = c != 0;
     if (flow) {
       nzv = __ldg(&Tl.nbz[c]);
       bits = zset(ft, c, nzv.x, nzv.z);
     }
-    const int vm1 = nzv.x, vm2 = (k0 - 2 >= kb) ? nzv.y : vm1;
+    const int vm1 = (kk - 1 >= kb) ? nzv.x : c, vm2 = (kk - 2 >= kb) ? nzv.y : vm1;
     for (int s = sl0; s < sl1; ++s) {
       double Fz = 0.0;
       const int n = __ldg(&T.slot_tr[s]);
@@ -490,7 +493,7 @@ __global__ void __launch_bounds__(kAdv64Warps * 32, 16)
             ec.add(tp2);
           }
           if (ec.bad() || redo) {
-            if (k == kb) sF[(s - sl0) * 32] = floor_flux64<SCH>(t0, tp1);
+            if (k == kb && !open) sF[(s - sl0) * 32] = floor_flux64<SCH>(t0, tp1);
 #pragma unroll 1
             for (int q = 0; q < 4; ++q) {  // (one call: four would cost registers)
               const bool w = q == 0, y = q == 1, z = q == 3;
@@ -528,7 +531,7 @@ __global__ void __launch_bounds__(kAdv64Warps * 32, 16)
       const double dtr = (Fxe - Fxw + Fyn - Fys) * dtu;
       double val = dtr;
       if (k <= ks) {
-        const double Fzb = kFloorZero64<SCH> && k == kb ? floor_flux64<SCH>(t0, tp1)
+        const double Fzb = kFloorZero64<SCH> && k == kb && !open ? floor_flux64<SCH>(t0, tp1)
                                                           : sF[(s - sl0) * 32];
         if (below) {
           sF[(s - sl0) * 32] = Fzt;
