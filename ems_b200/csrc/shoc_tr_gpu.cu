@@ -1150,13 +1150,14 @@ int build_tile_tables(shoc_tr_gpu *h, const shoc_tr_geom *g, const std::vector<u
     if (e >= 0 && e != col + 1) seg.push_back(e | kSegHalo);
   }
   while (seg.size() & 31) seg.push_back(-1);
-  // maps that do not stack (a cell's east neighbour outside its column's east
-  // column): every column goes the general path
+  // cells whose wet east neighbour is not in their column's east column (maps that
+  // do not stack): k_adv64_apart's
+  std::vector<int> apart;
   if (h->O.cross)
     for (int c = 1; c < S; c++) {
       if ((fl[c] & (CF_WET | FL_XP_WET)) != (CF_WET | FL_XP_WET)) continue;
       const int e = nb1[c].y;
-      if ((east_of[colof[c]] != colof[e]) || g->s2k[c] != g->s2k[e]) h->O.tiled = 0;
+      if (east_of[colof[c]] != colof[e] || g->s2k[c] != g->s2k[e]) apart.push_back(c);
     }
   std::vector<int4> colrec(ncolp, make_int4(0, 0, nz, 0));
   for (int col = 0; col < ncol; col++)
@@ -1193,6 +1194,11 @@ int build_tile_tables(shoc_tr_gpu *h, const shoc_tr_geom *g, const std::vector<u
   if ((rc = dupload(h, &ip, seg.data(), seg.size()))) return rc;
   T.seg = ip;
   T.nseg = (int)(seg.size() / 32);
+  if (!apart.empty()) {
+    if ((rc = dupload(h, &ip, apart.data(), apart.size()))) return rc;
+    T.apart = ip;
+    T.napart = (int)apart.size();
+  }
   return 0;
 }
 
@@ -1982,6 +1988,12 @@ int tile64_substep(const shoc_tr_gpu *h, bool last, const SubStep &ss, const Til
       case SHOC_TR_ORDER2_UW: adv64_ult<SHOC_TR_ORDER2_UW>(h, ss, tl, T, tin, tout); break;
     }
     nl++;
+    if (tl.napart > 0) {
+      const int blocks = (int)std::min<long long>(((long long)tl.napart * T.ntb + 127) / 128,
+                                                  kGeneralBlocks);
+      k_adv64_apart<<<blocks, 128, 0, st>>>(h->G, h->F, h->W, h->O, T, ss, tl, tin, tout);
+      nl++;
+    }
   }
   if (ev) cudaEventRecord(ev[1], st);
   const int bytes = (int)std::min<size_t>(vd64_smem(h->nz, nw), 227 * 1024);

@@ -148,6 +148,8 @@ struct Tile {
   // with kSegHalo: the column only lends its west flux
   const int *seg;
   int nseg;
+  const int *apart;  // [napart] cells whose wet east neighbour is not the next lane's
+  int napart;
   int ncolp;         // columns rounded up to whole tiles
   int nwet;
 };

@@ -384,7 +384,8 @@ __global__ void __launch_bounds__(kAdv64Warps * 32, 16)
       me = __ldg(&Tl.m2e[c]);
       fl = __ldg(&Tl.fl[c]);
     }
-    // a wet east neighbour is the next lane's cell (the segments see to it)
+    // a wet east neighbour is the next lane's cell (the segments see to it; where
+    // it is not, k_adv64_apart does the cell again)
     const bool ewet = (fl & FL_XP_WET) != 0;
     const bool nwet = (fl & FL_YP_WET) != 0;
     const bool below = k < ks;  // interior cell: its top face is in the water
@@ -546,6 +547,55 @@ __global__ void __launch_bounds__(kAdv64Warps * 32, 16)
       }
       tro[(size_t)n * G.S + c] = val;
     }
+  }
+}
+
+// The cells of maps that do not stack: k_adv64 gave them another cell's flux for
+// their east one.  A thread per (cell, tracer) forms their value again from the
+// same operands.  (An east face of its own in k_adv64's loop cost every window:
+// 384 x 320 x 40, 10 tracers 5.45 -> 6.25 ms for 4 steps.  Their columns on the
+// general path cost 0.33 ms a step at 200 x 180 x 30, however few they were.)
+__global__ void __launch_bounds__(128)
+    k_adv64_apart(Geo G, Flow F, Work W, Opt O, TrSet T, SubStep ss, Tile Tl,
+                  const double *__restrict__ tri, double *__restrict__ tro) {
+  const double dtu = ss.dtu;
+  const long long tot = (long long)Tl.napart * T.ntb;
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < tot;
+       q += (long long)gridDim.x * blockDim.x) {
+    const int c = Tl.apart[q % Tl.napart], n = T.slot_tr[q / Tl.napart];
+    const TileCol tc = tile_column(G, W, Tl, Tl.colof[c]);
+    if (!tc.act || n >= G.colntr[Tl.colof[c]]) continue;
+    const int tf = T.trf[n], k = Tl.kof[c], fl = Tl.fl[c];
+    const bool adv = (tf & TR_ADV) != 0, hd = (tf & TR_HDIFF) != 0;
+    const int4 n1 = Tl.nb1[c], n2 = Tl.nb2[c], nzv = Tl.nbz[c];
+    const int2 me = Tl.m2e[c];
+    const double *tr = tri + (size_t)n * G.S;
+    const double t0 = tr[c], txm1 = tr[n1.x], txp1 = tr[n1.y], tym1 = tr[n1.z], typ1 = tr[n1.w];
+    double Fxw = 0.0, Fys = 0.0, Fxe = 0.0, Fyn = 0.0;
+    if (adv || hd) {
+      Fxw = flux_x(G, F, W, O, fl, adv, hd, c, tc.c2, tr[n2.x], txm1, t0, txp1, dtu);
+      Fys = flux_y(G, F, W, O, fl, adv, hd, c, tc.c2, tr[n2.z], tym1, t0, typ1, dtu);
+      Fxe = flux_x(G, F, W, O, (fl & FL_XP_E1) ? CF_E1 : 0, adv, hd, n1.y, me.x, txm1, t0, txp1,
+                   tr[n2.y], dtu);
+      if (fl & FL_YP_WET)
+        Fyn = flux_y(G, F, W, O, (fl & FL_YP_E2) ? CF_E2 : 0, adv, hd, n1.w, me.y, tym1, t0,
+                     typ1, tr[n2.w], dtu);
+      else if (adv && O.trasc == SHOC_TR_ORDER1)
+        Fyn = order1_flux(F.u2flux3d[n1.w], t0, typ1);
+    }
+    const double dtr = (Fxe - Fxw + Fyn - Fys) * dtu;
+    double val = dtr;
+    if (k < tc.ks) {
+      double Fzb = 0.0, Fzt = 0.0;
+      if (adv) {
+        const double tm1 = k > tc.kb ? tr[nzv.x] : t0, tm2 = k - 1 > tc.kb ? tr[nzv.y] : tm1;
+        const double tp1 = tr[nzv.z], w9c = W.w9[c], w9p = W.w9[nzv.z];
+        Fzb = flux_z(F, W, O, c, W.w9[nzv.x], w9c, w9p, tm2, tm1, t0, tp1, dtu);
+        Fzt = flux_z(F, W, O, nzv.z, w9c, w9p, W.w9[nzv.w], tm1, t0, tp1, tr[nzv.w], dtu);
+      }
+      val = t0 - (dtr / G.cellarea[tc.c2] + (Fzt - Fzb)) / W.dz[c];
+    }
+    tro[(size_t)n * G.S + c] = val;
   }
 }
 
