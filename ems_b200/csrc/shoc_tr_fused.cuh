@@ -60,9 +60,9 @@ struct Fused {
 // row j of a column's tridiagonal factors in k_step32's shared memory
 struct FacVec {
   const float4 *l;
-  __device__ __forceinline__ float dzdt(int j) const { return l[j * 32].x; }
-  __device__ __forceinline__ float cm1(int j) const { return l[j * 32].y; }
-  __device__ __forceinline__ float rdiv(int j) const { return l[j * 32].z; }
+  __device__ __forceinline__ float cm1(int j) const { return l[j * 32].x; }
+  __device__ __forceinline__ float rdiv(int j) const { return l[j * 32].y; }
+  __device__ __forceinline__ float ud(int j) const { return l[j * 32].z; }
   __device__ __forceinline__ float re(int j) const { return l[j * 32].w; }
 };
 

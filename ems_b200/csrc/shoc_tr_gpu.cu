@@ -472,15 +472,16 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
   }
   if (wy == 1 && solve && (what & SD_F32)) {
     // the same matrix eliminated from the top (the FP32-mixed correction
-    // solve): e(j) = C(j) - cm1(j+1) cm1(j+1) / e(j+1)
+    // solve): e(j) = C(j) - cm1(j+1) cm1(j+1) / e(j+1); row j keeps 1 / e(j)
     const int kt = kb + jn - 1, kl = kb + jb - 1;
-    double up = sCm[kt * 32], e = sE[kt * 32] - up;
-    sE[kt * 32] = e;
-    for (int k = kt - 1; k >= kl; --k) {
-      const double cm1 = k > kl ? sCm[k * 32] : 0.0;
-      e = (sE[k * 32] - cm1 - up) - up * (up / e);
-      sE[k * 32] = e;
-      up = cm1;
+    double cm1 = sCm[kt * 32], e = sE[kt * 32] - cm1;
+    for (int k = kt; k >= kl; --k) {
+      const double re = 1.0 / e;
+      sE[k * 32] = re;
+      if (k == kl) break;
+      const double up = cm1;
+      cm1 = k - 1 > kl ? sCm[(k - 1) * 32] : 0.0;
+      e = (sE[(k - 1) * 32] - cm1 - up) - up * (up * re);
     }
   }
   if (wy == 0) {
@@ -517,23 +518,23 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
     const int j = k - kb + 1, cc = sC[k * 32];
     const double dzc = W.dz[cc];
     if (solve && j >= jb && j <= jn) {
-      const double dzdt = dzc / dt, cm1 = sCm[k * 32], div = sDv[k * 32];
+      const double cm1 = sCm[k * 32], div = sDv[k * 32];
+      // the elimination factor, as the recurrence formed it (cm1 is the upper
+      // diagonal of the row below); where the second elimination has the faces'
+      // place it is formed again
+      const double ud = j <= jb           ? 0.0
+                        : (what & SD_F32) ? cm1 / sDv[(k - 1) * 32]
+                                          : sZ[k * 32];
       if (lu64) {
-        // the elimination factor, as the recurrence formed it (cm1 is the upper
-        // diagonal of the row below); where the second elimination has the
-        // faces' place it is formed again, for the few general-path columns
-        const double ud = j <= jb           ? 0.0
-                          : (what & SD_F32) ? cm1 / sDv[(k - 1) * 32]
-                                            : sZ[k * 32];
         W.vd_cm1[cc] = cm1;
         W.vd_div[cc] = div;
         W.vd_ud[cc] = ud;
-        W.vd_dzdt[cc] = dzdt;
+        W.vd_dzdt[cc] = dzc / dt;
         if (what & SD_LU64) W.vd_rdiv[cc] = div_range(div) == kDivLo ? 1.0 / div : 0.0;
       }
       if (what & SD_F32)
         W.lu32[cc] =
-            make_float4((float)dzdt, (float)cm1, (float)(1.0 / div), (float)(1.0 / sE[k * 32]));
+            make_float4((float)cm1, (float)(1.0 / div), (float)ud, (float)sE[k * 32]);
     }
     if (late) {
       const double dzm = j > 1 ? W.dz[sC[(k - 1) * 32]] : dzsed;

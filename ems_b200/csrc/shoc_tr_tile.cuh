@@ -402,8 +402,9 @@ struct ColSums {
 // A0, S0: the column's values and Thomas storage from its bottom layer up, row
 // stride sa; an advected tracer (tbdy) holds its advected values below the
 // surface, any other tracer every layer's old value (A0 is overwritten, so is
-// S0).  fac: the tridiagonal factors of row j: dzdt, cm1, and the reciprocal
-// diagonals rdiv (eliminated from the bottom: LU) and re (from the top: UL).  C0, D0: cells and
+// S0).  fac: the tridiagonal factors of row j: cm1, the reciprocal diagonals rdiv
+// (eliminated from the bottom: LU) and re (from the top: UL) and the elimination
+// factor ud of LU (0 in the bottom row).  C0, D0: cells and
 // FP64 thicknesses, row stride 32; H: the water depth the carry is spread over,
 // the thicknesses from the surface cell's and then the bottom up.
 // RES: an advected tracer's A0 holds every layer's stored advection result
@@ -466,7 +467,7 @@ __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const
   // one pass up the column below the surface: the computed mass (an
   // advected tracer's FP64 values are stored + residual, or come in cs.m),
   // the clip and, with a solve, the FP32 forward sweep
-  float fwd = 0.f;  // the bottom row's cm1 is 0
+  float z = 0.f;  // the sweep's right side, before the division by the diagonal
   double m = 0.0;
   for (int j = 0; j < nk; ++j) {
     float a = A0[j * sa];
@@ -486,8 +487,8 @@ __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const
     if (R0) R0[j * sa] = lo_bits((float)r);
     if (tbdy) nw += (a < mn_up || a > mx_dn);
     if (solve) {
-      fwd = (fac.dzdt(j) * a - fac.cm1(j) * fwd) * fac.rdiv(j);
-      S0[j * sa] = fwd;
+      z = (float)(dz * idt) * a - fac.ud(j) * z;
+      S0[j * sa] = z * fac.rdiv(j);
     }
   }
   mxs += (tbdy && !RES) ? cs.m : m;
@@ -550,39 +551,43 @@ __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const
     store(ci.s, (vdf && single) ? vs + dl + F.dt * (0.0 - 0.0) / h : vs + dl, dzs);
   } else {
     // the surface row of the forward sweep
-    fwd = (fac.dzdt(nk) * (float)vs - fac.cm1(nk) * fwd) * fac.rdiv(nk);
+    double dzdt1 = dzs * idt;
+    z = (float)dzdt1 * (float)vs - fac.ud(nk) * z;
     // one pass down: the back substitution (FP32), x(j) replacing s(j), and one
     // row behind it the FP64 residual of b - A x for A = dz/dt I + the diffusion
     // operator,
     //   r(j) = dz/dt (a + dl - x) - cm1 (x(j-1) - x) - cp1 (x(j+1) - x)
     // (cp1(j) = cm1(j+1); the bottom row has no cm1 term, the top row no cp1
     // term), whose correction solve's elimination, from the top (UL), follows in
-    // the same pass, g(j) replacing a(j).  The residual's diagonal is the FP64
+    // the same pass, its right side h(j) replacing a(j).  No factor is a
+    // product of rounded ones: the FP32 solves' operands are FP64 values rounded once.  The residual's diagonal is the FP64
     // dz / dt, so the refined solve keeps the column mass the mass diagnostic
     // measures; cm1 is the FP32 factor's (the FP64 one, staged as well, changed
     // neither the maximum nor the RMS error over 1000 stiff2048 steps, and its
     // shared memory cost warps).  The FP64 copies of x and of the factors are
     // carried from row to row.
-    S0[nk * sa] = fwd;
-    float x1 = fwd, g = 0.f, l2 = 0.f;  // x, cm1 of row j + 1; cm1 of row j + 2
-    float l1 = fac.cm1(nk);
+    float x1 = z * fac.rdiv(nk);  // x of row j + 1
+    S0[nk * sa] = x1;
+    float l1 = fac.cm1(nk), u1 = fac.ud(nk);  // factors of row j + 1
+    float g = 0.f, l2 = 0.f;  // of row j + 2: the elimination's right side over e, cm1
     double xd1 = (double)x1, xd2 = 0.0;
-    double dzdt1 = dzs * idt;
     double a1 = vs;  // the value before the solve of row j + 1
     for (int j = nk - 1; j >= 0; --j) {
-      const float x = S0[j * sa] - l1 * fac.rdiv(j) * x1;
+      const float x = S0[j * sa] - u1 * x1;
       S0[j * sa] = x;
       const double xd = (double)x;
       double r = dzdt1 * ((a1 + dl) - xd1) - (double)l1 * (xd - xd1);
       if (j + 1 < nk) r = r - (double)l2 * (xd2 - xd1);
       a1 = (double)A0[j * sa] + (R0 ? (double)lo_val(R0[j * sa]) : 0.0);
-      g = ((float)r - l2 * g) * fac.re(j + 1);
-      A0[(j + 1) * sa] = g;
+      const float h1 = (float)r - l2 * g;
+      A0[(j + 1) * sa] = h1;
+      g = h1 * fac.re(j + 1);
       x1 = x;
       xd2 = xd1;
       xd1 = xd;
       l2 = l1;
       l1 = fac.cm1(j);
+      u1 = fac.ud(j);
       dzdt1 = D0[j * 32] * idt;
     }
     double r = dzdt1 * ((a1 + dl) - xd1);
@@ -591,7 +596,7 @@ __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const
     float d = ((float)r - l2 * g) * fac.re(0);
     store(C0[0], (double)S0[0] + (double)d, D0[0]);
     for (int j = 1; j <= nk; ++j) {
-      d = A0[j * sa] - fac.cm1(j) * fac.re(j) * d;
+      d = (A0[j * sa] - fac.cm1(j) * d) * fac.re(j);
       store(C0[j * 32], (double)S0[j * sa] + (double)d, D0[j * 32]);
     }
   }
@@ -633,8 +638,9 @@ constexpr int kVd32MaxWarps = 16;
 // S float[nd][nw][32] (twice with pf: the next tracer's column is staged
 // while the current one is solved), with comp (FP32_COMP) R, compensations
 // int16[nd][nw][32]
+constexpr int kVd32Row = 8 + 4 * 4 + 4;
 inline size_t vd32_smem(int nd, int nw, bool pf = false, bool comp = false) {
-  return (size_t)nd * 32 * (8 + 4 * 4 + 4) + (size_t)(pf ? 4 : 2) * nd * nw * 32 * 4 +
+  return (size_t)nd * 32 * kVd32Row + (size_t)(pf ? 4 : 2) * nd * nw * 32 * 4 +
          (comp ? (size_t)nd * nw * 32 * 2 : 0);
 }
 // Warps per k_vd32 block at full depth where the caller sets none: the most
@@ -655,14 +661,14 @@ inline int vd32_default_warps(int nz, int nslot, bool comp) {
   const int rounds = nslot > 0 ? (nslot + nw - 1) / nw : 1;
   return nslot > 0 ? (nslot + rounds - 1) / rounds : 1;
 }
-// row j of a column's factors in k_vd32's shared memory (p: the column's dzdt
+// row j of a column's factors in k_vd32's shared memory (p: the column's cm1
 // at its bottom row, n: floats per factor)
 struct FacSmem {
   const float *p;
   int n;
-  __device__ __forceinline__ float dzdt(int j) const { return p[j * 32]; }
-  __device__ __forceinline__ float cm1(int j) const { return p[n + j * 32]; }
-  __device__ __forceinline__ float rdiv(int j) const { return p[2 * n + j * 32]; }
+  __device__ __forceinline__ float cm1(int j) const { return p[j * 32]; }
+  __device__ __forceinline__ float rdiv(int j) const { return p[n + j * 32]; }
+  __device__ __forceinline__ float ud(int j) const { return p[2 * n + j * 32]; }
   __device__ __forceinline__ float re(int j) const { return p[3 * n + j * 32]; }
 };
 
@@ -688,7 +694,7 @@ __global__ void __launch_bounds__(kVd32MaxWarps * 32)
   if (nd == 0) return;
   // warps that step tracers: what the shared memory holds at this depth
   constexpr int per_row = (PF ? 4 : 2) * 4 + (COMP ? 2 : 0);
-  const int nw = min((int)blockDim.y, (smem_bytes / (nd * 32) - (8 + 4 * 4 + 4)) / per_row);
+  const int nw = min((int)blockDim.y, (smem_bytes / (nd * 32) - kVd32Row) / per_row);
   double *DZ = reinterpret_cast<double *>(smem);      // [nd][32]
   float *LU = reinterpret_cast<float *>(DZ + nd * 32);  // [4][nd][32]
   int *colC = reinterpret_cast<int *>(LU + 4 * nd * 32);  // [nd][32]
