@@ -5,6 +5,7 @@
 
 Each library is rebuilt only when a source is newer than it.
 """
+import hashlib
 import os
 import subprocess
 import sys
@@ -66,11 +67,12 @@ def gpu_lib(force=False, verbose=False):
     if force or _stale(out, deps):
         objs = []
         log = ""
+        build_id = sources_id()
         for (name, fmad), src in zip(GPU_SRC, srcs):
             obj = os.path.join(LIBDIR, os.path.splitext(name)[0] + ".o")
             cmd = [_nvcc()] + NVCC_ARCH + [
                 "-O3", "-lineinfo", "-std=c++17", "--fmad=%s" % ("true" if fmad else "false"),
-                "-Xcompiler", "-fPIC", "-I", INCLUDE, "-I", CSRC, "-c", "-o", obj, src]
+                "-DSHOC_TR_BUILD_ID=\"%s\"" % build_id, "-Xcompiler", "-fPIC", "-I", INCLUDE, "-I", CSRC, "-c", "-o", obj, src]
             if verbose:
                 cmd.insert(1, "-Xptxas=-v")
             log += _run(cmd)
@@ -81,6 +83,16 @@ def gpu_lib(force=False, verbose=False):
         if verbose:
             sys.stdout.write(log)
     return out
+
+
+def sources_id():
+    """Short hash of the CUDA library's sources: names the build in the autotuner's
+    cache, whose measurements hold for these kernels alone."""
+    h = hashlib.sha256()
+    for name in [s for s, _ in GPU_SRC] + GPU_HDR:
+        with open(os.path.join(CSRC, name), "rb") as f:
+            h.update(f.read())
+    return h.hexdigest()[:12]
 
 
 def build_all(force=False):

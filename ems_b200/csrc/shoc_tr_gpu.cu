@@ -3203,14 +3203,19 @@ std::string tune_cache_path() {
   return std::string(home) + "/.cache/shoc_tr_gpu/tuning.txt";
 }
 
+// The key names the build: a choice measured on other kernels, or under another
+// meaning of a field, is not found.
+#ifndef SHOC_TR_BUILD_ID  // the hash of the sources (ems_b200/_build.py)
+#define SHOC_TR_BUILD_ID __DATE__ "_" __TIME__
+#endif
 std::string tune_key(const shoc_tr_gpu *h) {
   cudaDeviceProp p;
   if (cudaGetDeviceProperties(&p, h->device) != cudaSuccess) return std::string();
-  std::string name = p.name;
+  std::string name = std::string(SHOC_TR_BUILD_ID "|") + p.name;
   for (char &c : name)
     if (c == ' ' || c == '\t') c = '_';
   char buf[512];
-  snprintf(buf, sizeof buf, "v2|%s|sm%d%d|S%d|C%d|Z%d|N%d|B%d|P%d|A%d|U%d|F%d|H%d|V%d",
+  snprintf(buf, sizeof buf, "v3|%s|sm%d%d|S%d|C%d|Z%d|N%d|B%d|P%d|A%d|U%d|F%d|H%d|V%d",
            name.c_str(), p.major, p.minor, h->S, h->ncol, h->nz, h->ntr, h->T.ntb, h->precision,
            h->O.trasc, h->O.ultimate, h->adv_flags, h->any_hdiff ? 1 : 0, h->any_vdiff ? 1 : 0);
   return std::string(buf);

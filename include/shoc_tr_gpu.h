@@ -283,8 +283,9 @@ int shoc_tr_gpu_set_tuning(shoc_tr_gpu *h, const shoc_tr_tuning *t);
  * block with and without its prefetch; for FP32-mixed also the fused sub-step
  * with tile widths 8, 16, 32 and the most and half the most phase-B warps its
  * shared memory allows.  With use_cache != 0 the
- * choice is looked up in and saved to a file keyed by the GPU model and the
- * window's configuration (sizes, tracers, precision, scheme, diffusion),
+ * choice is looked up in and saved to a file keyed by the library's build, the
+ * GPU model and the window's configuration (sizes, tracers, precision, scheme,
+ * diffusion),
  * named by the environment variable SHOC_TR_TUNE_CACHE (default
  * $HOME/.cache/shoc_tr_gpu/tuning.txt, "off" for none): a cached choice is
  * applied without trial steps and *from_cache set to 1.  best / from_cache

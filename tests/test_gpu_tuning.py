@@ -1,0 +1,29 @@
+"""The autotuner's cache and candidates."""
+import pytest
+
+from ems_b200 import gpu, synth
+
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("need_gpu")]
+
+
+def test_cache_of_another_build_is_not_used(tmp_path, monkeypatch):
+    """A line of the same window and GPU whose key has another build's name, or
+    none as older libraries wrote it, is not taken."""
+    path = tmp_path / "tuning.txt"
+    monkeypatch.setenv("SHOC_TR_TUNE_CACHE", str(path))
+    case = synth.make("small")
+
+    def tuned():
+        t = gpu.TracerStep(case)
+        t.start()
+        best, cached = t.autotune_ex(1)
+        t.close()
+        return cached
+
+    assert not tuned()
+    assert tuned()
+    key, values = path.read_text().split(None, 1)
+    window = key.split("|")[-13:]  # GPU model and window configuration
+    path.write_text("".join("%s %s" % ("|".join(head + window), values)
+                            for head in (["v2"], ["v3", "0" * 12])))
+    assert not tuned()
