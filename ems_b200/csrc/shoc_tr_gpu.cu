@@ -2522,11 +2522,14 @@ int shoc_tr_gpu_set_preamble(shoc_tr_gpu *h, int on) {
   if (on && !h->pre.ok) return SHOC_TR_EUNSUPPORTED;
   DeviceScope dev_(h->device);
   if (on) {
+    // only what is made here is filled on the default stream and waited for: the
+    // call must not wait for the caller's own work there every step
+    const bool made = !h->F.dzu1 || !h->F.dzu2 || !h->pre.detadt;
     int rc = 0;
     if (!rc && !h->F.dzu1) rc = dupload<double>(h, (double **)&h->F.dzu1, nullptr, (size_t)h->S);
     if (!rc && !h->F.dzu2) rc = dupload<double>(h, (double **)&h->F.dzu2, nullptr, (size_t)h->S);
     if (!rc && !h->pre.detadt) rc = dupload<double>(h, &h->pre.detadt, nullptr, (size_t)h->S2);
-    if (!rc) rc = default_stream_done();
+    if (!rc && made) rc = default_stream_done();
     if (rc) return rc;
   }
   if (h->pre.on != (on != 0)) {
