@@ -2317,9 +2317,9 @@ int step_pipelined(shoc_tr_gpu *h, shoc_tr_state *st) {
   // them are rarely registered)
   shoc_tr_state fl = *st;
   if (st->sur_t && st->nsur_t) {
-    const size_t nb = ((size_t)h->ncol + 1) * sizeof(int);
-    memcpy(h->h_surf, st->sur_t, nb);
-    memcpy(h->h_surf + h->ncol + 1, st->nsur_t, nb);
+    const size_t nb = (size_t)h->ncol * sizeof(int);  // elements 1 to ncol
+    memcpy(h->h_surf + 1, st->sur_t + 1, nb);
+    memcpy(h->h_surf + 1 + h->ncol + 1, st->nsur_t + 1, nb);
     fl.sur_t = h->h_surf;
     fl.nsur_t = h->h_surf + h->ncol + 1;
   }
