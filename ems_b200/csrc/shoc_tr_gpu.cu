@@ -247,7 +247,7 @@ __device__ __forceinline__ void atomic_min_pos(unsigned long long *p, double v) 
   atomicMin(p, (unsigned long long)__double_as_longlong(v));
 }
 
-// The step's set-up, a block of kSetDzWarps warps per tile of 32 columns (lane =
+// The step's set-up, a block of up to kSetDzWarps warps per tile of 32 columns (lane =
 // column): set_dz (tracers.c:5731-5848), the scheme work arrays w5/w9 (:561-567)
 // and their 2/(w9+w9) factors, the sub-step search (:591-668) as a
 // min-reduction, the column flags and the tracer-independent LU factors of
@@ -281,7 +281,11 @@ constexpr int SD_F32 = 4;     // also the FP32 thickness and LU factors
 constexpr int SD_WORK = 8;    // w5, w9, dbz, dfz of the tile kernels' columns
 constexpr int SD_LU64 = 16;   // FP64 LU factors of the tile kernels' columns
                               // (the general path's columns get all of them)
+// Warps of a block: one per layer up to eight (a window of few layers has nothing
+// for more: 1000 x 800 x 2, 3 tracers, FP32-mixed 0.58 ms a step with eight, 0.43
+// so), and two at least, of which the second eliminates from the top.
 constexpr int kSetDzWarps = 8;
+inline int set_dz_warps(int nz) { return std::max(2, std::min(nz, kSetDzWarps)); }
 // bytes: FP64 faces (then the diagonal eliminated from the top with SD_F32, else
 // the elimination factors), rows cm1 and dz/dt (then div) and the cells of nz
 // layers of 32 columns
@@ -292,7 +296,7 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
              int what, const int *own) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr unsigned FULL = 0xffffffffu;
-  const int nz = G.nz, lane = threadIdx.x, wy = threadIdx.y;
+  const int nz = G.nz, lane = threadIdx.x, wy = threadIdx.y, nwarp = blockDim.y;
   double *const sZ = reinterpret_cast<double *>(smem) + lane;  // bottom face z, then sE
   double *const sCm = sZ + nz * 32;                            // cm1
   double *const sDv = sCm + nz * 32;                           // dz / dt, then div
@@ -309,7 +313,7 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
   if (wy == 0) sJa[lane] = 0;
   const int sur = on ? W.nsur_t[col] : 0;
   const int sed = on ? __ldg(&G.zm1[bot]) : 0;
-  for (int k = wy; k < nz; k += kSetDzWarps)
+  for (int k = wy; k < nz; k += nwarp)
     if (on && k >= kb) {
       const int c = __ldg(&Tl.cellk[(size_t)k * Tl.ncolp + col]);
       sC[k * 32] = c;
@@ -367,7 +371,7 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
   double dtmin = __longlong_as_double(0x7ff0000000000000ll);
   const bool search = (what & SD_SEARCH) && O.substep != 0 && wet && (!own || own[col]);
   const bool all_work = (what & SD_WORK) || !pre_staged;
-  for (int k = nz - 1 - wy; k >= 0; k -= kSetDzWarps) {
+  for (int k = nz - 1 - wy; k >= 0; k -= nwarp) {
     if (!on || k < kb) continue;
     const int j = k - kb + 1, cc = sC[k * 32];
     const double dzc = dzof(j), dzm = dzof(j - 1);
@@ -406,7 +410,7 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
 
   // the faces are done with: the second elimination's rows take their place
   if ((what & SD_F32) && any_vdiff) {
-    for (int k = wy; k < nz; k += kSetDzWarps)
+    for (int k = wy; k < nz; k += nwarp)
       if (on && k >= kb) sE[k * 32] = sDv[k * 32];
     __syncthreads();
   }
@@ -502,7 +506,7 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
       if (wc) atomicAdd(&counts[0], wc);
       if (wn) atomicAdd(&counts[1], wn);
       double v = sMin[0];
-      for (int i = 1; i < kSetDzWarps; ++i) v = fmin(v, sMin[i]);
+      for (int i = 1; i < nwarp; ++i) v = fmin(v, sMin[i]);
       if (v < __longlong_as_double(0x7ff0000000000000ll)) atomic_min_pos(W.dtm_bits, v);
     }
   }
@@ -513,7 +517,7 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
   const bool lu64 = (what & SD_LU64) || !staged;
   const bool late = on && pre_staged && !staged && !(what & SD_WORK);
   if (!solve && !late) return;
-  for (int k = wy; k < nz; k += kSetDzWarps) {
+  for (int k = wy; k < nz; k += nwarp) {
     if (k < kb) continue;
     const int j = k - kb + 1, cc = sC[k * 32];
     const double dzc = W.dz[cc];
@@ -1856,7 +1860,7 @@ void launch_set_dz(shoc_tr_gpu *h, int what) {
     what |= SD_F32 | (h->comp ? SD_WORK : 0);
   else
     what |= SD_WORK | SD_LU64;
-  k_set_dz<<<h->tl.ncolp / 32, dim3(32, kSetDzWarps), set_dz_smem(h->nz), h->stream>>>(
+  k_set_dz<<<h->tl.ncolp / 32, dim3(32, set_dz_warps(h->nz)), set_dz_smem(h->nz), h->stream>>>(
       h->G, h->F, h->W, h->O, h->tl, h->any_vdiff ? 1 : 0, h->d_counts, h->staged ? 1 : 0, what,
       h->colown);
   h->launches++;
