@@ -649,11 +649,19 @@ inline size_t vd32_smem(int nd, int nw, bool pf = false, bool comp = false) {
 // loads go through: 1024 x 512 x 50 (24 tracers) 4 warps 2.42 ms, 5 warps 2.60;
 // 333 x 217 x 37 (5 tracers) three blocks of 3 warps 0.080 ms, of 4 0.091, two of
 // 5 0.108; a batch of 60 layers (32 tracers) two of 2 warps 0.69, of 4 0.86.
+// Shallow columns leave memory for any number; blocks of four warps, or of the
+// tracers where they are five at most, still let one block copy its column arrays
+// while others solve, and fill the 16 warps the registers allow (col_warps; the
+// column kernel, FP32-mixed and FP64: 500 x 400 x 4, 16 tracers 0.186 and 0.170 ms,
+// 16 and 8 warps 0.325 and 0.212; 400 x 300 x 8, 16 tracers 0.142 and 0.131, 0.223
+// and 0.152; 300 x 300 x 20, 24 tracers 0.235 and 0.221, 6 and 8 warps 0.291 and 0.232).
+inline int col_warps(int nslot) { return nslot <= 5 ? 5 : 4; }
 inline int vd32_default_warps(int nz, int nslot, bool comp) {
   int nw = 1;
   for (int b = 4; b >= 2; b--) {
     nw = 1;
-    while (nw < kVd32MaxWarps && b * (vd32_smem(nz, nw + 1, false, comp) + 1024) <= 196 * 1024)
+    const int most = b == 4 ? col_warps(nslot) : kVd32MaxWarps / b;
+    while (nw < most && b * (vd32_smem(nz, nw + 1, false, comp) + 1024) <= 196 * 1024)
       nw++;
     if (nw >= 3) break;
   }

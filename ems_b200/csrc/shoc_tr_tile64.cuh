@@ -635,7 +635,9 @@ inline size_t vd64_smem(int nd, int nw) {
 inline size_t vd64_tuned(int nz, int nw) { return (size_t)nz * 32 * (4 + 2 * 8 * nw); }
 // Warps per block at full depth where the caller sets none: two blocks per SM
 // within 160 KB of its memory, balanced rounds.  The rest is left to the L1,
-// which the back substitution's values come from: 384 x 320 x 40 (10 tracers)
+// which the back substitution's values come from.  Where four blocks of four
+// warps fit (22 layers), col_warps as in k_vd32; deeper, 192 x 160 x 24 (6 tracers)
+// 6 warps 42.6 us, 3 45.1: 384 x 320 x 40 (10 tracers)
 // 2 warps 0.23 ms, 4 (194 KB) 0.27; 200 x 180 x 30 (6 tracers) 3 warps 0.055, 6
 // 0.051.  Deeper columns, where that is a single warp, take two, while two such
 // blocks fit (512 x 256 x 50, 24 tracers: 1 warp 1.32 ms, 2 0.94, 3 0.88, 4 1.13);
@@ -644,7 +646,9 @@ inline size_t vd64_tuned(int nz, int nw) { return (size_t)nz * 32 * (4 + 2 * 8 *
 // 1.24, 4 0.95, 5 1.05).
 inline int vd64_default_warps(int nz, int nslot) {
   int nw = 1;
-  while (nw < kVd64MaxWarps / 2 && 2 * (vd64_smem(nz, nw + 1) + 1024) <= 160 * 1024) nw++;
+  const bool shallow = 4 * (vd64_smem(nz, 4) + 1024) <= 227 * 1024;
+  const int most = shallow ? col_warps(nslot) : kVd64MaxWarps / 2;
+  while (nw < most && 2 * (vd64_smem(nz, nw + 1) + 1024) <= 160 * 1024) nw++;
   if (nw == 1) {
     nw = 2;
     if (2 * (vd64_smem(nz, nw) + 1024) > 227 * 1024)

@@ -48,3 +48,31 @@ def test_set_up_of_few_layers(precision):
     a block has eight warps whatever the layers)."""
     step, adv, col = times(window(1000, 800, 2, 3), precision)
     assert step - adv - col < 0.35 * (adv + col)
+
+
+@pytest.mark.parametrize("precision", [gpu.FP32_MIXED, gpu.FP32_COMP, gpu.FP64])
+@pytest.mark.parametrize("nz", [4, 8])
+def test_column_kernel_default_in_shallow_columns(precision, nz):
+    """The default number of warps per block is within 15 % of the best (it was 1.3
+    to 1.8 times as slow where a block had as many as its memory holds)."""
+    case = window(400, 300, nz, 16)
+    t = gpu.TracerStep(case, precision=precision)
+    t.start()
+    t.run(3)
+    t.sync()
+
+    def col(warps):
+        t.set_tiling(tracers=warps)
+        best = np.inf
+        for _ in range(3):
+            t.profile(True)
+            t.run(4)
+            t.sync()
+            best = min(best, t.kernel_time(2)[0])
+        t.profile(False)
+        return best
+
+    default = col(t.get_tuning()["tracers_per_block"])
+    rest = [col(w) for w in (2, 4, 8)]
+    t.close()
+    assert default <= 1.15 * min(rest)
