@@ -55,7 +55,7 @@ void tile32_substep(bool last, bool quick, bool ult, cudaStream_t st, const Geo 
                     const TrSet &T, const SubStep &ss, const Tile &Tl, const f32::Face2 *fx2,
                     const f32::Face2 *fy2, const float *tin, float *tout, float *rnd,
                     double *carry, double *fzs, const int16_t *lo_in, int16_t *lo_out,
-                    int vd_nw, int vd_pf, int any_hd, int adv_flags, cudaEvent_t *ev) {
+                    const ColLaunch *launch, int nlaunch, int vd_pf, int any_hd, int adv_flags, cudaEvent_t *ev) {
   if (ev) cudaEventRecord(ev[0], st);
   // kMaxTracers a launch: the kernel lists its tracers in shared memory
   for (int s0 = 0; s0 < T.ntb && Tl.nwet > 0; s0 += kMaxTracers) {
@@ -68,19 +68,17 @@ void tile32_substep(bool last, bool quick, bool ult, cudaStream_t st, const Geo 
     adv(adv_flags, grid, st, G, F3, W, Tc, ss, Tl, fx2, fy2, tin, tout, rnd, fzs, any_hd, lo_in);
   }
   if (ev) cudaEventRecord(ev[1], st);
-  // one launch for every depth: blocks of the shared memory vd_nw warps need at
-  // full depth, and as many warps, for the shallow tiles to use it up, as the
-  // registers allow those blocks (16 warps an SM)
   const bool comp = lo_out != nullptr;
-  const int bytes = (int)vd32_smem(G.nz, vd_nw, vd_pf != 0, comp);
-  const int blocks = std::max(1, 233472 / (bytes + 1024));
-  const dim3 blk(32, std::min(T.nslot, std::max(vd_nw, kVd32MaxWarps / blocks)));
   auto kern = comp ? (last ? (vd_pf ? k_vd32<true, true, true> : k_vd32<true, false, true>)
                            : (vd_pf ? k_vd32<false, true, true> : k_vd32<false, false, true>))
                    : (last ? (vd_pf ? k_vd32<true, true, false> : k_vd32<true, false, false>)
                            : (vd_pf ? k_vd32<false, true, false> : k_vd32<false, false, false>));
-  kern<<<Tl.ncolp / 32, blk, bytes, st>>>(G, F, W, O, T, ss, Tl, W.lu32, tin, tout, rnd, carry,
-                                          fzs, lo_in, lo_out, bytes);
+  for (int i = 0; i < nlaunch; i++) {
+    const ColLaunch &l = launch[i];
+    kern<<<l.ntile, dim3(32, l.warps), l.bytes, st>>>(G, F, W, O, T, ss, Tl, W.lu32, tin, tout,
+                                                      rnd, carry, fzs, lo_in, lo_out, l.bytes,
+                                                      l.tile0);
+  }
   if (ev) cudaEventRecord(ev[2], st);
 }
 

@@ -101,6 +101,7 @@ struct shoc_tr_gpu {
     int ntile = 0;
   } ftile[3];
   int fnwb_max = 0;                   // phase-B warps k_step32 may have (0: no k_step32)
+  std::vector<int> vd_depth;          // layers of the column kernels' tiles, ascending
   bool staged = false;                // column-tile fast path
   int cur = 0;
   int *bpt = nullptr, *bin = nullptr;
@@ -114,7 +115,7 @@ struct shoc_tr_gpu {
   long long graph_launches[2] = {0, 0};
   int graph_nsub = -1;
   // tiling
-  int tw = 8;
+  int tw = 8, tw_default = 8;
   bool vd_pf = false;  // k_vd32 stages the next tracer's column during the solve
   // profiling
   bool profile = false;
@@ -1130,8 +1131,10 @@ int build_tile_tables(shoc_tr_gpu *h, const shoc_tr_geom *g, const std::vector<u
   }
   std::stable_sort(tord.begin(), tord.end(), [&](int a, int b) { return tdepth[a] < tdepth[b]; });
   std::vector<int> vdcol(ncolp, -1);
+  h->vd_depth.resize(ntile);
   for (int i = 0; i < ntile; i++) {
     const int t = tord[i];
+    h->vd_depth[i] = tdepth[t];
     for (int l = 0; l < 32; l++) vdcol[i * 32 + l] = (t * 32 + l < ncol) ? t * 32 + l : -1;
   }
   // k_adv64's segments: columns in order, 32 to a warp.  A column's wet east
@@ -1285,9 +1288,14 @@ int apply_tuning(shoc_tr_gpu *h, const shoc_tr_tuning &t) {
   if (t.tracers_per_block < 1 || t.tracers_per_block > (f32 ? kVd32MaxWarps : 8))
     return SHOC_TR_EUNSUPPORTED;
   if (t.prefetch && !f32) return SHOC_TR_EUNSUPPORTED;
-  const size_t vb = f32 ? vd32_smem(h->nz, t.tracers_per_block, t.prefetch != 0, h->comp)
-                        : vd64_tuned(h->nz, t.tracers_per_block);
-  if (vb > 227 * 1024) return SHOC_TR_EUNSUPPORTED;
+  // the window's layers decide, but for what the default needs in columns that do
+  // not have them all
+  auto fits = [&](int nd) {
+    return (f32 ? vd32_smem(nd, t.tracers_per_block, t.prefetch != 0, h->comp)
+                : vd64_tuned(nd, t.tracers_per_block)) <= 227 * 1024;
+  };
+  if (!fits(t.tracers_per_block > h->tw_default ? h->nz : std::max(1, h->vd_depth.back())))
+    return SHOC_TR_EUNSUPPORTED;
   if (t.fused) {
     const int ti = tile_index(t.tile_x);
     if (!f32 || h->comp || !h->fnwb_max || ti < 0 || !h->ftile[ti].tcol) return SHOC_TR_EUNSUPPORTED;
@@ -1703,11 +1711,11 @@ int shoc_tr_gpu_create(const shoc_tr_geom *g, const shoc_tr_opts *o, int ntr, in
     TRY(dupload<double>(h, &h->fu.carry, nullptr, (size_t)ntr * ncol));
   }
   TRY(dupload<double>(h, &h->fzs64, nullptr, (size_t)ntr * ncol));
-  // tiling: warps per column-kernel block
-  const int tw = f32p ? vd32_default_warps(g->nz, h->nslot, h->comp)
-                      : vd64_default_warps(g->nz, h->nslot);
-  h->tw = tw;
   TRY(build_tile_tables(h, g, cflag, col_bot, col_kb));
+  // tiling: warps per column-kernel block
+  const int nd = std::max(1, h->vd_depth.back());
+  h->tw = f32p ? vd32_default_warps(nd, h->nslot, h->comp) : vd64_default_warps(nd, h->nslot);
+  h->tw_default = h->tw;
   {  // face columns of the transport-mode preamble
     std::vector<int2> fc;
     std::vector<double> bz;
@@ -1935,8 +1943,56 @@ void launch_general(shoc_tr_gpu *h, bool last, const TrSet &T, const SubStep &ss
   h->launches++;
 }
 
-// One FP64 transport sub-step over the staged columns: k_adv64, then one
-// k_vd64.  Returns the kernels launched.
+// The launches of the column kernel for nslot tracers and nw warps a block: one,
+// with the shared memory the window's deepest tile needs, whose shallower tiles use
+// theirs up with more warps.  Where the tracers are too few for that and an SM
+// would hold four warps or less of its 16, the shallower tiles are launched by
+// themselves, if that doubles the warps an SM and they make up more than a round of
+// the deep launch (148 SMs).  (From six warps on the deep tiles' time alone, which
+// shallow ones no longer fill, cost more: 400 x 300 x 60, half of it 18 layers at
+// most, 3 tracers FP32-mixed 432 us in one launch, 460 in two.)
+// 400 x 300, 60 layers of which the columns have 8 at most, 1 tracer: the kernel
+// takes 25 us FP32-mixed and 27 FP64, 70 and 93 with memory for 60 layers; 300 x
+// 200, 128 layers on 3 % of the columns and 18 at most on the others 167 and 168 us,
+// 279 and 275 in one launch.
+constexpr int kColLaunches = 4;
+int col_launches(const shoc_tr_gpu *h, int nslot, int nw, ColLaunch *out) {
+  const bool f32 = h->esize == sizeof(float);
+  const int full = kVd32MaxWarps;
+  static_assert(kVd32MaxWarps == kVd64MaxWarps, "one rule for both column kernels");
+  auto config = [&](int depth, int &blocks) {
+    ColLaunch l{};
+    const size_t need = f32 ? vd32_smem(depth, nw, h->vd_pf, h->comp) : vd64_smem(depth, nw);
+    l.bytes = (int)std::min<size_t>(need, 227 * 1024);
+    blocks = std::max(1, 233472 / (l.bytes + 1024));
+    l.warps = std::max(1, std::min(nslot, std::max(nw, full / blocks)));
+    return l;
+  };
+  const std::vector<int> &depth = h->vd_depth;
+  int n = 0, hi = (int)depth.size();
+  while (hi > 0) {
+    int blocks, b;
+    ColLaunch l = config(std::max(1, depth[hi - 1]), blocks);
+    int lo = 0;
+    if (n + 1 < kColLaunches)
+      for (int d = depth[hi - 1] - 1; d >= 1 && !lo; d--) {
+        if (blocks * l.warps > 4) break;
+        const ColLaunch s = config(d, b);
+        if (std::min(full, b * s.warps) < 2 * std::min(full, blocks * l.warps)) continue;
+        lo = (int)(std::upper_bound(depth.begin(), depth.begin() + hi, d) - depth.begin());
+        if (lo <= 148 * blocks) lo = 0;
+        break;
+      }
+    l.tile0 = lo;
+    l.ntile = hi - lo;
+    out[n++] = l;
+    hi = lo;
+  }
+  return n;
+}
+
+// One FP64 transport sub-step over the staged columns: k_adv64, then k_vd64.
+// Returns the kernels launched.
 //
 // Layers per warp of k_adv64: a longer climb computes fewer bottom faces twice
 // (one per chunk), a shorter one gives more warps.  The chip holds 148 x 16;
@@ -2001,16 +2057,14 @@ int tile64_substep(const shoc_tr_gpu *h, bool last, const SubStep &ss, const Til
     }
   }
   if (ev) cudaEventRecord(ev[1], st);
-  const int bytes = (int)std::min<size_t>(vd64_smem(h->nz, nw), 227 * 1024);
-  const int blocks = std::max(1, 233472 / (bytes + 1024));
-  const dim3 blk(32, std::min(T.nslot, std::max(nw, kVd64MaxWarps / blocks)));
-  if (last)
-    k_vd64<true><<<tl.ncolp / 32, blk, bytes, st>>>(h->G, h->F, h->W, h->O, T, ss, tl, tin, tout,
-                                                    h->fzs64, bytes);
-  else
-    k_vd64<false><<<tl.ncolp / 32, blk, bytes, st>>>(h->G, h->F, h->W, h->O, T, ss, tl, tin, tout,
-                                                     h->fzs64, bytes);
-  nl++;
+  ColLaunch cl[kColLaunches];
+  const int ncl = col_launches(h, T.nslot, nw, cl);
+  for (int i = 0; i < ncl; i++) {
+    auto kern = last ? k_vd64<true> : k_vd64<false>;
+    kern<<<cl[i].ntile, dim3(32, cl[i].warps), cl[i].bytes, st>>>(
+        h->G, h->F, h->W, h->O, T, ss, tl, tin, tout, h->fzs64, cl[i].bytes, cl[i].tile0);
+  }
+  nl += ncl;
   if (ev) cudaEventRecord(ev[2], st);
   return nl;
 }
@@ -2048,17 +2102,19 @@ int launch_part_b(shoc_tr_gpu *h, const Sched &s, int cur0, const TrSet &T,
         }
         h->launches += h->fu.ntile > 0 ? 1 : 0;
       } else {
+        ColLaunch cl[kColLaunches];
+        const int ncl = col_launches(h, T.nslot, tw, cl);
         tile32_substep(last, h->O.trasc == SHOC_TR_QUICKEST, h->O.ultimate != 0, st, h->G, h->F,
                        h->F3, h->W, h->O, T, ss, h->tl, h->fx2, h->fy2, tin, tout, h->rnd,
                        h->fu.carry, h->fzs64, h->comp ? h->lo[cur] : nullptr,
-                       h->comp ? h->lo[cur ^ 1] : nullptr, tw, h->vd_pf ? 1 : 0,
+                       h->comp ? h->lo[cur ^ 1] : nullptr, cl, ncl, h->vd_pf ? 1 : 0,
                        h->any_hdiff ? 1 : 0, h->adv_flags, prof ? ev : nullptr);
         if (prof) {  // pairs share events; sync destroys each event once
           h->ev.push_back({0, ev[0], ev[2]});
           h->ev.push_back({1, ev[0], ev[1]});
           h->ev.push_back({2, ev[1], ev[2]});
         }
-        h->launches += (h->tl.nwet > 0 ? (T.ntb + kMaxTracers - 1) / kMaxTracers : 0) + 1;
+        h->launches += (h->tl.nwet > 0 ? (T.ntb + kMaxTracers - 1) / kMaxTracers : 0) + ncl;
       }
       int16_t *lo_out = h->comp ? h->lo[cur ^ 1] : nullptr;
       launch_general<float>(h, last, T, ss, tin, tout, c3row, c3_load, lo_out);

@@ -609,10 +609,10 @@ __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const
 
 // k_vd32: a block is one tile of 32 columns, deepest tiles first; the tile's
 // tracer-independent column arrays are staged once and each warp steps its
-// share of the tracers through them.  Every block has the same shared memory,
-// of which a warp takes as much as the tile is deep: a full-depth tile runs the
-// handle's warps per block, a shallow one more, and one launch serves every
-// depth.
+// share of the tracers through them.  Every block of a launch has the same shared
+// memory, of which a warp takes as much as the tile is deep: the deepest tile runs
+// the handle's warps per block, a shallow one more, and one launch serves every
+// depth, unless there are too few tracers for that (col_launches).
 //
 // What bounds it: latency (shared memory and conversions in each thread's
 // chains along the column) at the 8 to 16 warps an SM holds (128 registers a
@@ -688,11 +688,11 @@ __global__ void __launch_bounds__(kVd32MaxWarps * 32)
            const float4 *__restrict__ lu32, const float *__restrict__ tri,
            float *__restrict__ tro, const float *__restrict__ rsi, double *__restrict__ carry,
            const double *__restrict__ fzs, const int16_t *__restrict__ loi,
-           int16_t *__restrict__ loo, int smem_bytes) {
+           int16_t *__restrict__ loo, int smem_bytes, int tile0) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x, wy = threadIdx.y;
-  const int tile = gridDim.x - 1 - blockIdx.x;  // (the tiles are sorted by depth)
+  const int tile = tile0 + gridDim.x - 1 - blockIdx.x;  // (the tiles are sorted by depth)
   const int col = Tl.vdcol[tile * 32 + lane];
   const TileCol tc = tile_column(G, W, Tl, col);
   const bool act = tc.act;

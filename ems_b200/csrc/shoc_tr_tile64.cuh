@@ -605,8 +605,9 @@ __global__ void __launch_bounds__(128)
 // A block is one tile of 32 columns, deepest tiles first, the tile's
 // tracer-independent arrays (cells, the LU factors and the reciprocal of the
 // divisor) staged once; each warp steps its share of the tracers, a thread per
-// column.  Every block has the same shared memory, of which a warp takes as
-// much as the tile is deep, so one launch serves every depth.
+// column.  Every block of a launch has the same shared memory, of which a warp
+// takes as much as the tile is deep, so one launch serves every depth unless there
+// are too few tracers for that (col_launches).
 //
 // What bounds it: the serial chain of the Thomas sweeps (memory is 16 bytes a
 // value).  The forward sweep's IEEE division was most of the chain: the
@@ -834,11 +835,11 @@ template <bool LAST>
 __global__ void __launch_bounds__(kVd64MaxWarps * 32)
     k_vd64(Geo G, Flow F, Work W, Opt O, TrSet T, SubStep ss, Tile Tl,
            const double *__restrict__ tri, double *__restrict__ tro,
-           const double *__restrict__ fzs, int smem_bytes) {
+           const double *__restrict__ fzs, int smem_bytes, int tile0) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x, wy = threadIdx.y;
-  const int tile = gridDim.x - 1 - blockIdx.x;  // (the tiles are sorted by depth)
+  const int tile = tile0 + gridDim.x - 1 - blockIdx.x;  // (the tiles are sorted by depth)
   const int col = Tl.vdcol[tile * 32 + lane];
   const TileCol tc = tile_column(G, W, Tl, col);
   const bool act = tc.act;

@@ -76,3 +76,28 @@ def test_column_kernel_default_in_shallow_columns(precision, nz):
     rest = [col(w) for w in (2, 4, 8)]
     t.close()
     assert default <= 1.15 * min(rest)
+
+
+@pytest.mark.parametrize("precision", [gpu.FP32_MIXED, gpu.FP32_COMP, gpu.FP64])
+def test_column_kernel_where_no_column_has_all_layers(precision):
+    """60 layers, columns of 8 at most, one tracer: the column kernel takes what it
+    takes in a window of 8 layers (2.5 to 3.5 times that where its shared memory
+    is sized for 60)."""
+    shallow = times(window(400, 300, 60, 1, depth=(3.0, 39.0)), precision)
+    few = times(window(400, 300, 8, 1, depth=(3.0, 39.0)), precision)
+    assert shallow[2] < 1.5 * few[2]
+
+
+@pytest.mark.parametrize("precision", [gpu.FP32_MIXED, gpu.FP32_COMP, gpu.FP64])
+def test_column_kernel_with_a_trench(precision):
+    """128 layers on a few columns, 18 at most on the others, one tracer: the
+    column kernel takes four times what it takes without them (6.7 where the
+    shallow tiles run at the deep ones' few blocks an SM)."""
+    layers = synth.uniform_layers(128, 640.0)
+    r = np.random.default_rng(5)
+    bathy = -5.0 * r.uniform(2.0, 18.0, (200, 300))
+    land = np.zeros((200, 300), np.uint8)
+    flat = window(300, 200, 128, 1, bathy_land=(synth._snap_bathy(bathy, layers), land))
+    bathy[:, :9] = -639.0
+    trench = window(300, 200, 128, 1, bathy_land=(synth._snap_bathy(bathy, layers), land))
+    assert times(trench, precision)[2] < 5.2 * times(flat, precision)[2]
