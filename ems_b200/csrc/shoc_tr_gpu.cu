@@ -289,20 +289,24 @@ constexpr int kSetDzWarps = 8;
 inline int set_dz_warps(int nz) { return std::max(2, std::min(nz, kSetDzWarps)); }
 // bytes: FP64 faces (then the diagonal eliminated from the top with SD_F32, else
 // the elimination factors), rows cm1 and dz/dt (then div) and the cells of nz
-// layers of 32 columns
-inline size_t set_dz_smem(int nz) { return (size_t)nz * 32 * (3 * 8 + 4); }
+// layers of 32 columns: those of the window's deepest column (300 x 200, 128 layers
+// of which the columns have 20 at most, 1 tracer, FP32-mixed: 61 us a step beside the transport
+// with rows for 128 layers, 27 so)
+inline size_t set_dz_smem(int nd) { return (size_t)nd * 32 * (3 * 8 + 4); }
 
 __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
     k_set_dz(Geo G, Flow F, Work W, Opt O, Tile Tl, int any_vdiff, int *counts, int list_all,
-             int what, const int *own) {
+             int what, const int *own, int nd) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr unsigned FULL = 0xffffffffu;
   const int nz = G.nz, lane = threadIdx.x, wy = threadIdx.y, nwarp = blockDim.y;
-  double *const sZ = reinterpret_cast<double *>(smem) + lane;  // bottom face z, then sE
-  double *const sCm = sZ + nz * 32;                            // cm1
-  double *const sDv = sCm + nz * 32;                           // dz / dt, then div
-  double *const sE = sZ;                                       // dz / dt, then e (SD_F32)
-  int *const sC = reinterpret_cast<int *>(reinterpret_cast<double *>(smem) + 3 * nz * 32) + lane;
+  // row k of each array is layer k, of which no column has one below k0
+  const int k0 = nz - nd, r0 = lane - k0 * 32;
+  double *const sZ = reinterpret_cast<double *>(smem) + r0;  // bottom face z, then sE
+  double *const sCm = sZ + nd * 32;                          // cm1
+  double *const sDv = sCm + nd * 32;                         // dz / dt, then div
+  double *const sE = sZ;                                     // dz / dt, then e (SD_F32)
+  int *const sC = reinterpret_cast<int *>(reinterpret_cast<double *>(smem) + 3 * nd * 32) + r0;
   __shared__ int sJa[32];        // highest layer <= jn of zero thickness
   __shared__ double sMin[kSetDzWarps];
   const int col = blockIdx.x * 32 + lane;
@@ -314,7 +318,7 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
   if (wy == 0) sJa[lane] = 0;
   const int sur = on ? W.nsur_t[col] : 0;
   const int sed = on ? __ldg(&G.zm1[bot]) : 0;
-  for (int k = wy; k < nz; k += nwarp)
+  for (int k = k0 + wy; k < nz; k += nwarp)
     if (on && k >= kb) {
       const int c = __ldg(&Tl.cellk[(size_t)k * Tl.ncolp + col]);
       sC[k * 32] = c;
@@ -372,7 +376,7 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
   double dtmin = __longlong_as_double(0x7ff0000000000000ll);
   const bool search = (what & SD_SEARCH) && O.substep != 0 && wet && (!own || own[col]);
   const bool all_work = (what & SD_WORK) || !pre_staged;
-  for (int k = nz - 1 - wy; k >= 0; k -= nwarp) {
+  for (int k = nz - 1 - wy; k >= k0; k -= nwarp) {
     if (!on || k < kb) continue;
     const int j = k - kb + 1, cc = sC[k * 32];
     const double dzc = dzof(j), dzm = dzof(j - 1);
@@ -411,7 +415,7 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
 
   // the faces are done with: the second elimination's rows take their place
   if ((what & SD_F32) && any_vdiff) {
-    for (int k = wy; k < nz; k += nwarp)
+    for (int k = k0 + wy; k < nz; k += nwarp)
       if (on && k >= kb) sE[k * 32] = sDv[k * 32];
     __syncthreads();
   }
@@ -518,7 +522,7 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
   const bool lu64 = (what & SD_LU64) || !staged;
   const bool late = on && pre_staged && !staged && !(what & SD_WORK);
   if (!solve && !late) return;
-  for (int k = wy; k < nz; k += nwarp) {
+  for (int k = k0 + wy; k < nz; k += nwarp) {
     if (k < kb) continue;
     const int j = k - kb + 1, cc = sC[k * 32];
     const double dzc = W.dz[cc];
@@ -1868,9 +1872,10 @@ void launch_set_dz(shoc_tr_gpu *h, int what) {
     what |= SD_F32 | (h->comp ? SD_WORK : 0);
   else
     what |= SD_WORK | SD_LU64;
-  k_set_dz<<<h->tl.ncolp / 32, dim3(32, set_dz_warps(h->nz)), set_dz_smem(h->nz), h->stream>>>(
+  const int nd = std::max(1, h->vd_depth.back());
+  k_set_dz<<<h->tl.ncolp / 32, dim3(32, set_dz_warps(nd)), set_dz_smem(nd), h->stream>>>(
       h->G, h->F, h->W, h->O, h->tl, h->any_vdiff ? 1 : 0, h->d_counts, h->staged ? 1 : 0, what,
-      h->colown);
+      h->colown, nd);
   h->launches++;
 }
 

@@ -101,3 +101,12 @@ def test_column_kernel_with_a_trench(precision):
     bathy[:, :9] = -639.0
     trench = window(300, 200, 128, 1, bathy_land=(synth._snap_bathy(bathy, layers), land))
     assert times(trench, precision)[2] < 5.2 * times(flat, precision)[2]
+
+
+@pytest.mark.parametrize("precision", [gpu.FP32_MIXED, gpu.FP64])
+def test_set_up_where_no_column_has_all_layers(precision):
+    """128 layers, columns of 20 at most: the step beside its transport kernels takes
+    about what it takes in a window of 20 layers (twice that with shared memory
+    for 128)."""
+    a, b = (times(window(300, 200, nz, 1, depth=(3.0, 99.0)), precision) for nz in (128, 20))
+    assert a[0] - a[1] - a[2] < 1.5 * (b[0] - b[1] - b[2])
