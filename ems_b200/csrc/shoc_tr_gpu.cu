@@ -101,6 +101,11 @@ struct shoc_tr_gpu {
     int ntile = 0;
   } ftile[3];
   int fnwb_max = 0;                   // phase-B warps k_step32 may have (0: no k_step32)
+  struct AdvItems {                   // k_adv64's list for a number of tracer groups
+    int lmax = 0, n = 0;
+    int2 *d = nullptr;
+  };
+  std::vector<AdvItems> adv_items;
   std::vector<int> vd_depth;          // layers of the column kernels' tiles, ascending
   bool staged = false;                // column-tile fast path
   int cur = 0;
@@ -1205,6 +1210,47 @@ int build_tile_tables(shoc_tr_gpu *h, const shoc_tr_geom *g, const std::vector<u
   T.vdcol = ip;
   if ((rc = dupload(h, &ip, seg.data(), seg.size()))) return rc;
   T.seg = ip;
+  // k_adv64's work: the layers of each segment in chunks, a warp each.  A longer
+  // climb computes fewer bottom faces twice (one per chunk), a shorter one gives more
+  // warps: the chunks are the longest that still make about six rounds of the warps
+  // the chip holds.  The layers are those the segments' columns have: counted and
+  // cut over the window's layers, chunks were too long and many of them empty (384 x
+  // 320 x 40, 2 to 40 layers deep, 10 tracers, 4 steps 5.44 ms, 4.69 so; 400 x 300, 60
+  // layers of which the columns have 8 at most, 1 tracer, k_adv64 0.155 and 0.093).
+  if (h->O.cross) {
+    const int nseg = (int)(seg.size() / 32);
+    std::vector<int> kmin(nseg, nz);
+    long long layers = 0;
+    for (int i = 0; i < nseg; i++) {
+      for (int l = 0; l < 32; l++) {
+        const int e = seg[i * 32 + l];
+        if (e >= 0 && !(e & kSegHalo)) kmin[i] = std::min(kmin[i], col_kb[e]);
+      }
+      layers += nz - kmin[i];
+    }
+    const int groups = (h->T.ntb + kAdv64Group - 1) / kAdv64Group;
+    const long long resident = 148LL * std::min<long long>(
+        16, 233472 / (adv64_smem(std::min(std::max(h->T.ntb, 1), kAdv64Group)) + 1024));
+    for (int q = 1; q <= groups; q++) {
+      shoc_tr_gpu::AdvItems it;
+      it.lmax = (int)std::max<long long>(1, layers * q / (resident * 6));
+      if (q > 1 && h->adv_items.back().lmax == it.lmax) {
+        h->adv_items.push_back(h->adv_items.back());
+        continue;
+      }
+      std::vector<int2> list;
+      for (int i = 0; i < nseg; i++) {
+        const int d = nz - kmin[i], n = (d + it.lmax - 1) / it.lmax;
+        for (int j = 0; j < n; j++) {
+          const int k0 = kmin[i] + j * ((d + n - 1) / n), k1 = std::min(nz, k0 + (d + n - 1) / n);
+          if (k0 < k1) list.push_back(make_int2(i, k0 | k1 << 16));
+        }
+      }
+      it.n = (int)list.size();
+      if ((rc = dupload(h, &it.d, list.data(), list.size()))) return rc;
+      h->adv_items.push_back(it);
+    }
+  }
   T.nseg = (int)(seg.size() / 32);
   if (!apart.empty()) {
     if ((rc = dupload(h, &ip, apart.data(), apart.size()))) return rc;
@@ -1999,25 +2045,19 @@ int col_launches(const shoc_tr_gpu *h, int nslot, int nw, ColLaunch *out) {
 // One FP64 transport sub-step over the staged columns: k_adv64, then k_vd64.
 // Returns the kernels launched.
 //
-// Layers per warp of k_adv64: a longer climb computes fewer bottom faces twice
-// (one per chunk), a shorter one gives more warps.  The chip holds 148 x 16;
-// the chunks are the longest that still make about six rounds of them.
 template <int SCH, bool U>
 void adv64(const shoc_tr_gpu *h, const SubStep &ss, const Tile &tl, const TrSet &T,
            const double *tin, double *tout) {
-  const long long want = 148LL * 16 * 6;
   const int ng = std::min(T.ntb, kAdv64Group), groups = (T.ntb + ng - 1) / ng;
-  const int lmax = (int)std::max<long long>(1, (long long)tl.nseg * h->nz * groups / want);
-  const int nch = (h->nz + std::min(lmax, h->nz) - 1) / std::min(lmax, h->nz);
-  const int L = (h->nz + nch - 1) / nch;
-  const dim3 grid((tl.nseg + kAdv64Warps - 1) / kAdv64Warps * nch, groups);
+  const shoc_tr_gpu::AdvItems &it = h->adv_items[groups - 1];
+  const dim3 grid((it.n + kAdv64Warps - 1) / kAdv64Warps, groups);
   const size_t smem = adv64_smem(ng);
   if (h->adv_flags == 1)
     k_adv64<SCH, U, true><<<grid, kAdv64Warps * 32, smem, h->stream>>>(
-        h->G, h->F, h->W, T, ss, tl, tin, tout, h->fzs64, nch, L, ng);
+        h->G, h->F, h->W, T, ss, tl, tin, tout, h->fzs64, it.d, it.n, ng);
   else
     k_adv64<SCH, U, false><<<grid, kAdv64Warps * 32, smem, h->stream>>>(
-        h->G, h->F, h->W, T, ss, tl, tin, tout, h->fzs64, nch, L, ng);
+        h->G, h->F, h->W, T, ss, tl, tin, tout, h->fzs64, it.d, it.n, ng);
 }
 template <int SCH>
 void adv64_ult(const shoc_tr_gpu *h, const SubStep &ss, const Tile &tl, const TrSet &T,

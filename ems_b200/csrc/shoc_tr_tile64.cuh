@@ -281,19 +281,21 @@ inline size_t adv64_smem(int ng) {
 }
 
 // PLAIN: every advected tracer is advected without horizontal diffusion.
-// Block b: segments kAdv64Warps (b / nch) .., layers [ch L, ch L + L) of chunk
-// ch = b % nch; blockIdx.y: groups of ng tracers.
+// A warp's work is item kAdv64Warps blockIdx.x + its number of the list: a segment
+// (x) and layers k0 to below k1 of it (y: k0 | k1 << 16); blockIdx.y: groups of ng
+// tracers.
 template <int SCH, bool ULT, bool PLAIN>
 __global__ void __launch_bounds__(kAdv64Warps * 32, 16)
     k_adv64(Geo G, Flow F, Work W, TrSet T, SubStep ss, Tile Tl,
             const double *__restrict__ tri, double *__restrict__ tro, double *__restrict__ fzs,
-            int nch, int L, int ng) {
+            const int2 *__restrict__ items, int nitem, int ng) {
   extern __shared__ double sAdv[];  // per warp: [kAdv64Faces][FC_N][32], [ng][32]
   constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
-  const int seg = (blockIdx.x / nch) * kAdv64Warps + wy;
-  if (seg >= Tl.nseg) return;
-  const int k0 = (blockIdx.x % nch) * L, k1 = min(G.nz, k0 + L);
+  const int item = blockIdx.x * kAdv64Warps + wy;
+  if (item >= nitem) return;
+  const int2 it = __ldg(&items[item]);
+  const int seg = it.x, k0 = it.y & 0xffff, k1 = it.y >> 16;
   const int sl0 = blockIdx.y * ng, sl1 = min(T.ntb, sl0 + ng);
   double *const fw = sAdv + (size_t)wy * (kAdv64Faces * FC_N + ng) * 32 + lane;
   double *const fs = fw + FC_N * 32, *const fn = fs + FC_N * 32, *const ft = fn + FC_N * 32;

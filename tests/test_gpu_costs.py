@@ -110,3 +110,11 @@ def test_set_up_where_no_column_has_all_layers(precision):
     for 128)."""
     a, b = (times(window(300, 200, nz, 1, depth=(3.0, 99.0)), precision) for nz in (128, 20))
     assert a[0] - a[1] - a[2] < 1.5 * (b[0] - b[1] - b[2])
+
+
+def test_fp64_advection_where_no_column_has_all_layers():
+    """60 layers, columns of 8 at most: the FP64 advection kernel takes what it takes
+    in a window of 8 layers (1.4 times that where its chunks of layers are counted
+    over 60)."""
+    a, b = (times(window(400, 300, nz, 1, depth=(3.0, 39.0)), gpu.FP64) for nz in (60, 8))
+    assert a[1] < 1.2 * b[1]
