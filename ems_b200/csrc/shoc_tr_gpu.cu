@@ -107,6 +107,7 @@ struct shoc_tr_gpu {
   };
   std::vector<AdvItems> adv_items;
   std::vector<int> vd_depth;          // layers of the column kernels' tiles, ascending
+  std::vector<long long> vd_layers;   // of the first i of them together
   bool staged = false;                // column-tile fast path
   int cur = 0;
   int *bpt = nullptr, *bin = nullptr;
@@ -1141,9 +1142,11 @@ int build_tile_tables(shoc_tr_gpu *h, const shoc_tr_geom *g, const std::vector<u
   std::stable_sort(tord.begin(), tord.end(), [&](int a, int b) { return tdepth[a] < tdepth[b]; });
   std::vector<int> vdcol(ncolp, -1);
   h->vd_depth.resize(ntile);
+  h->vd_layers.assign(ntile + 1, 0);
   for (int i = 0; i < ntile; i++) {
     const int t = tord[i];
     h->vd_depth[i] = tdepth[t];
+    h->vd_layers[i + 1] = h->vd_layers[i] + tdepth[t];
     for (int l = 0; l < 32; l++) vdcol[i * 32 + l] = (t * 32 + l < ncol) ? t * 32 + l : -1;
   }
   // k_adv64's segments: columns in order, 32 to a warp.  A column's wet east
@@ -1997,11 +2000,15 @@ void launch_general(shoc_tr_gpu *h, bool last, const TrSet &T, const SubStep &ss
 // The launches of the column kernel for nslot tracers and nw warps a block: one,
 // with the shared memory the window's deepest tile needs, whose shallower tiles use
 // theirs up with more warps.  Where the tracers are too few for that and an SM
-// would hold four warps or less of its 16, the shallower tiles are launched by
-// themselves, if that doubles the warps an SM and they make up more than a round of
-// the deep launch (148 SMs).  (From six warps on the deep tiles' time alone, which
-// shallow ones no longer fill, cost more: 400 x 300 x 60, half of it 18 layers at
-// most, 3 tracers FP32-mixed 432 us in one launch, 460 in two.)
+// would hold four warps or less of its 16, the shallower tiles may be launched by
+// themselves, with twice the warps an SM.  That gains the time they take off the
+// deep launch, and loses what they filled beside its last deep tiles, about half a
+// deep tile's time: in units of a layer's time, the tiles' layers over 148 SMs times
+// the rounds of tracers per resident block, before less after, against half the
+// deepest tile's layers and rounds.  (150 x 120 x 128 of any depth, 3 tracers
+// FP32-mixed: 326 us a step in one launch, 405 in three.  From six warps an SM on the
+// shallow launch gained nothing: 400 x 300 x 60, half of it 18 layers at most, 3
+// tracers 432 and 460.)
 // 400 x 300, 60 layers of which the columns have 8 at most, 1 tracer: the kernel
 // takes 25 us FP32-mixed and 27 FP64, 70 and 93 with memory for 60 layers; 300 x
 // 200, 128 layers on 3 % of the columns and 18 at most on the others 167 and 168 us,
@@ -2031,7 +2038,12 @@ int col_launches(const shoc_tr_gpu *h, int nslot, int nw, ColLaunch *out) {
         const ColLaunch s = config(d, b);
         if (std::min(full, b * s.warps) < 2 * std::min(full, blocks * l.warps)) continue;
         lo = (int)(std::upper_bound(depth.begin(), depth.begin() + hi, d) - depth.begin());
-        if (lo <= 148 * blocks) lo = 0;
+        if (lo == 0) break;
+        const ColLaunch t = config(std::max(1, depth[lo - 1]), b);
+        auto rounds = [&](int w) { return (nslot + w - 1) / w; };
+        const double gain = h->vd_layers[lo] / 148.0 * ((double)rounds(l.warps) / blocks -
+                                            (double)rounds(t.warps) / b);
+        if (gain <= 0.5 * depth[hi - 1] * rounds(std::max(nw, 1))) lo = 0;
         break;
       }
     l.tile0 = lo;

@@ -118,3 +118,18 @@ def test_fp64_advection_where_no_column_has_all_layers():
     over 60)."""
     a, b = (times(window(400, 300, nz, 1, depth=(3.0, 39.0)), gpu.FP64) for nz in (60, 8))
     assert a[1] < 1.2 * b[1]
+
+
+def test_column_kernel_of_any_depth_stays_one_launch():
+    """128 layers, columns of any depth, three tracers: too few tiles for more
+    launches than one (three took 1.4 times as long as one).  Launches are counted:
+    k_adv32, k_vd32 and k_general of a sub-step, k_lateral and k_set_dz."""
+    t = gpu.TracerStep(window(150, 120, 128, 3), precision=gpu.FP32_MIXED)
+    t.start()
+    t.run(3)
+    t.sync()
+    n = t.launches()
+    t.run(4)
+    t.sync()
+    assert t.launches() - n == 4 * 5
+    t.close()
