@@ -3471,7 +3471,7 @@ int shoc_tr_gpu_autotune_ex(shoc_tr_gpu *h, int steps, int use_cache, shoc_tr_tu
   shoc_tr_tuning base = current_tuning(h);
   const std::vector<int> tws = h->esize == sizeof(float)
                                    ? std::vector<int>{2, 3, 4, 5, 6, 8, 12, 16}
-                                   : std::vector<int>{1, 2, 3, 4, 5, 6, 8};
+                                   : std::vector<int>{2, 3, 4, 5, 6, 8};
   for (int pf : {0, 1}) {
     if (pf && h->esize != sizeof(float)) continue;
     for (int tw : tws) {
@@ -3505,8 +3505,19 @@ int shoc_tr_gpu_autotune_ex(shoc_tr_gpu *h, int steps, int use_cache, shoc_tr_tu
   const bool prof0 = h->profile;
   shoc_tr_tuning win = base;
   double best_ms = 1e300;
+  // numbers of warps that make the same launches (more than the tracers, or than the
+  // shared memory holds) are tried once
+  std::vector<std::vector<int>> tried;
   for (const auto &c : cand) {
     if (apply_tuning(h, c) != SHOC_TR_OK) continue;
+    if (!c.fused) {
+      ColLaunch cl[kColLaunches];
+      const int n = col_launches(h, h->nslot, std::max(1, std::min(h->tw, h->nslot)), cl);
+      std::vector<int> key = {c.prefetch};
+      for (int i = 0; i < n; i++) key.insert(key.end(), {cl[i].tile0, cl[i].bytes, cl[i].warps});
+      if (std::find(tried.begin(), tried.end(), key) != tried.end()) continue;
+      tried.push_back(key);
+    }
     shoc_tr_gpu_profile(h, 1);
     rc = shoc_tr_gpu_run(h, steps);
     if (!rc) rc = shoc_tr_gpu_sync(h, nullptr);

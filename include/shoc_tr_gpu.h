@@ -279,7 +279,7 @@ int shoc_tr_gpu_set_tuning(shoc_tr_gpu *h, const shoc_tr_tuning *t);
  * candidate configuration, times the transport kernels with CUDA events,
  * puts the state back (a device copy taken before the trials: the tracers,
  * surface vectors and mass carry are as they were) and keeps the fastest.
- * Candidates: 1..8 warps per k_vd64 block, or 2..16 warps per k_vd32
+ * Candidates: 2..8 warps per k_vd64 block, or 2..16 warps per k_vd32
  * block with and without its prefetch; for FP32-mixed also the fused sub-step
  * with tile widths 8, 16, 32 and the most and half the most phase-B warps its
  * shared memory allows.  With use_cache != 0 the

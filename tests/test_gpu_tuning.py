@@ -27,3 +27,23 @@ def test_cache_of_another_build_is_not_used(tmp_path, monkeypatch):
     path.write_text("".join("%s %s" % ("|".join(head + window), values)
                             for head in (["v2"], ["v3", "0" * 12])))
     assert not tuned()
+
+
+@pytest.mark.parametrize("precision", [gpu.FP64, gpu.FP32_MIXED])
+def test_launches_that_are_the_same_are_tried_once(precision):
+    """Two tracers: two warps per block, whatever more is asked for; FP32-mixed with
+    and without the prefetch (the fused kernel does not take so many layers)."""
+    case = synth.build_case("tune", 40, 30, synth.uniform_layers(120, 600.0), seed=9, ntr=2,
+                            depth=(500.0, 599.0))
+    t = gpu.TracerStep(case, precision=precision)
+    t.start()
+    t.run(3)
+    t.sync()
+    n = t.launches()
+    t.run(1)
+    t.sync()
+    step, n = t.launches() - n, t.launches()
+    t.autotune(1)
+    most = {gpu.FP64: 1, gpu.FP32_MIXED: 2}[precision]
+    assert t.launches() - n <= most * step
+    t.close()
