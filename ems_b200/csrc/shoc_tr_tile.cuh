@@ -412,8 +412,11 @@ struct ColSums {
 // are taken from them; else they come in cs (k_step32).
 // carry: [ntr][ncol] (null: none).  Adds the values it flags to nwarn and
 // sets bad for a NaN among what it stores.  The mass bookkeeping sums are
-// plain FP64 sums of at most nz terms: their rounding (a few 1e-16 of the
-// column mass, of either sign) is what the carry may miss per step.
+// FP64 sums of at most nz terms: their rounding (a few 1e-16 of the column mass, of
+// either sign) is what the carry may miss per step.  The stored mass is summed from
+// the bottom up, thick layers first, and keeps its rounding errors: without them
+// the 24-bit values of the thin layers on top end on ties, which lean one way
+// (512 x 256 x 50 stiff layers, 1000 steps: a drift of -7e-16 of the mass against 5e-17).
 template <bool LAST, bool RES, class Fac>
 __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const Work &W,
                                               const Opt &O, const TrSet &T, const SubStep &ss,
@@ -441,8 +444,8 @@ __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const
   const double ts_old = (double)tr[ci.s] + (li ? lo_dec(li[ci.s], tr[ci.s]) : 0.0);
   const double dzs = D0[nk * 32];
   // FP64 mass bookkeeping per unit area: what the step computed (mxs) and
-  // what is stored (mss)
-  double mxs = 0.0, mss = 0.0;
+  // what is stored (mss + msc)
+  double mxs = 0.0, mss = 0.0, msc = 0.0;
   long long nw = 0;
   double vs = ts_old;  // the surface value
   // tr_bounds clip and range check (:3278-3293) of the cells below the
@@ -540,7 +543,9 @@ __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const
       lout[c] = lo_round(v, fin, dec);
       st += dec;
     }
-    mss += st * dz;
+    const double t = __fma_rn(st, dz, mss);
+    msc += __fma_rn(st, dz, mss - t);  // what the sum's rounding left out
+    mss = t;
   };
   if (!solve) {
     // the values as they are, plus the carry's shift (tr_bounds has run)
@@ -600,7 +605,7 @@ __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const
       store(C0[j * 32], (double)S0[j * sa] + (double)d, D0[j * 32]);
     }
   }
-  if (carry && steady) carry[(size_t)n * G.ncol + col] = (mxs - mss) * area;
+  if (carry && steady) carry[(size_t)n * G.ncol + col] = ((mxs - mss) - msc) * area;
   nwarn += nw;
 }
 
@@ -626,10 +631,10 @@ __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const
 //   does not carry being left out.
 // Fetching the next tracer's rows into the current one's as its last pass frees
 // them cost more than it hid (2.90 against 2.57 ms on the first case below).
-// A sub-step (B200), before and now: 1024 x 512 x 50, 24 tracers 2.86 and 2.42 ms;
-// 448 x 300 x 50, 16 tracers, FP32_COMP 0.91 and 0.72; 333 x 217 x 37, 5 tracers
-// 0.128 and 0.080; a batch of 56 447 columns, 60 layers, 4 to 32 tracers 0.93 and
-// 0.69.
+// A sub-step (B200) with four passes, and now: 1024 x 512 x 50, 24 tracers 2.86 and
+// 2.38 ms; 448 x 300 x 50, 16 tracers, FP32_COMP 0.91 and 0.70; 333 x 217 x 37, 5
+// tracers 0.128 and 0.074; a batch of 56 447 columns, 60 layers, 4 to 32 tracers 0.93
+// and 0.68.
 
 constexpr int kStage = 8;  // layers a warp of a column kernel stages together
 constexpr int kVd32MaxWarps = 16;
@@ -646,9 +651,9 @@ inline size_t vd32_smem(int nd, int nw, bool pf = false, bool comp = false) {
 // Warps per k_vd32 block at full depth where the caller sets none: the most
 // blocks per SM (up to four) that leave a block three warps, else two blocks,
 // within 196 KB of an SM's memory.  Filling the 227 KB takes the L1 the column's
-// loads go through: 1024 x 512 x 50 (24 tracers) 4 warps 2.42 ms, 5 warps 2.60;
-// 333 x 217 x 37 (5 tracers) three blocks of 3 warps 0.080 ms, of 4 0.091, two of
-// 5 0.108; a batch of 60 layers (32 tracers) two of 2 warps 0.69, of 4 0.86.
+// loads go through: 1024 x 512 x 50 (24 tracers) 4 warps 2.4 ms, 5 warps 2.6;
+// 333 x 217 x 37 (5 tracers) three blocks of 3 warps 0.074 ms, of 4 0.085, two of
+// 5 0.098; a batch of 60 layers (32 tracers) two of 2 warps 0.67, of 4 0.84.
 // Shallow columns leave memory for any number; blocks of four warps, or of the
 // tracers where they are five at most, still let one block copy its column arrays
 // while others solve, and fill the 16 warps the registers allow (col_warps; the
