@@ -12,12 +12,15 @@
 //   per sub-step:
 //     k_adv32 + k_vd32 (FP32-mixed, shoc_tr_tile.cuh; or the one fused
 //                 k_step32 of shoc_tr_fused.cuh, SHOC_TR_GPU_KERNELS=fused)
-//                 or k_adv64 + k_vd64 (FP64, shoc_tr_tile64.cuh): the
-//                 columns whose surface cell stays in its layer, one thread
-//                 per cell, then one per (column, tracer)
-//     k_general   the other columns (surface crossing a layer face, thin-
-//                 surface fix coupling tracers, degenerate solve range), one
-//                 thread per (column, tracer): column_pass
+//                 or k_adv64 + k_vd64 (FP64, shoc_tr_tile64.cuh): advection,
+//                 one thread per cell (k_adv32) or a warp per segment of
+//                 columns and chunk of layers (k_adv64), then one thread per
+//                 (column, tracer).  FP32-mixed: QUICKEST and Van Leer, columns
+//                 whose surface cell stays in its layer
+//     k_general   the other columns (thin-surface fix coupling tracers,
+//                 degenerate solve range; FP32-mixed: surface crossing a layer
+//                 face, other schemes), one thread per (column, tracer):
+//                 column_pass
 // Tracers ping-pong between two buffers; a step is captured in a CUDA graph
 // once its sub-step schedule is known.
 #include <cuda_runtime.h>

@@ -58,7 +58,8 @@ namespace shoc {
 // cell and the reference's divisions; climbing, 2.35 ms with the limiter's
 // cases as branches, 1.15 ms as selections, 1.08 ms with upwind loads alone,
 // 1.00 ms with loads a tracer ahead and one-warp blocks (four-warp blocks wait
-// for their deepest column: 1.04).  A warp per face with the fluxes meeting in
+// for their deepest column: 1.04), 0.81 with chunks of the layers the columns have
+// (build_tile_tables).  A warp per face with the fluxes meeting in
 // shared memory took 1.25 ms: more warps, but a quarter more instructions.
 
 // Correctly rounded a / b from y = RN(1 / b) (P. Markstein, IBM J. Res. Dev.
@@ -641,8 +642,8 @@ inline size_t vd64_tuned(int nz, int nw) { return (size_t)nz * 32 * (4 + 2 * 8 *
 // which the back substitution's values come from.  Where four blocks of four
 // warps fit (22 layers), col_warps as in k_vd32; deeper, 192 x 160 x 24 (6 tracers)
 // 6 warps 42.6 us, 3 45.1: 384 x 320 x 40 (10 tracers)
-// 2 warps 0.23 ms, 4 (194 KB) 0.27; 200 x 180 x 30 (6 tracers) 3 warps 0.055, 6
-// 0.051.  Deeper columns, where that is a single warp, take two, while two such
+// 2 warps 0.23 ms, 4 (194 KB) 0.27; 200 x 180 x 30 (6 tracers) 3 warps 0.051, 6
+// 0.049.  Deeper columns, where that is a single warp, take two, while two such
 // blocks fit (512 x 256 x 50, 24 tracers: 1 warp 1.32 ms, 2 0.94, 3 0.88, 4 1.13);
 // still deeper ones what a block has within 200 KB (448 x 300 x 60, 16 tracers: 1
 // warp 1.21 ms, 2 0.91, 3 1.15, 6 0.89; 400 x 300 x 80, 12 tracers: 1 warp 1.69, 2
