@@ -1770,7 +1770,9 @@ int shoc_tr_gpu_create(const shoc_tr_geom *g, const shoc_tr_opts *o, int ntr, in
   TRY(build_tile_tables(h, g, cflag, col_bot, col_kb));
   // tiling: warps per column-kernel block
   const int nd = std::max(1, h->vd_depth.back());
-  h->tw = f32p ? vd32_default_warps(nd, h->nslot, h->comp) : vd64_default_warps(nd, h->nslot);
+  const int ntile = h->tl.ncolp / 32;
+  h->tw = f32p ? vd32_default_warps(nd, h->nslot, h->comp, ntile)
+               : vd64_default_warps(nd, h->nslot, ntile);
   h->tw_default = h->tw;
   {  // face columns of the transport-mode preamble
     std::vector<int2> fc;

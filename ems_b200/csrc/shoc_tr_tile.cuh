@@ -661,9 +661,16 @@ inline size_t vd32_smem(int nd, int nw, bool pf = false, bool comp = false) {
 // 16 and 8 warps 0.325 and 0.212; 400 x 300 x 8, 16 tracers 0.142 and 0.131, 0.223
 // and 0.152; 300 x 300 x 20, 24 tracers 0.235 and 0.221, 6 and 8 warps 0.291 and 0.232).
 inline int col_warps(int nslot) { return nslot <= 5 ? 5 : 4; }
-inline int vd32_default_warps(int nz, int nslot, bool comp) {
+// A window with few tiles has no more blocks for an SM (148 of them), and those take
+// as many warps as there are tracers, up to 16 an SM: 46 x 139 x 9 (140 tiles, 24
+// tracers, FP32_COMP) 12 warps 25 us, 4 45; 152 x 20 x 35 (5 tracers) 5 warps 24, 3 34.
+inline int col_blocks(int ntile) {
+  return ntile > 3 * 148 ? 4 : ntile > 0 ? (ntile + 147) / 148 : 1;
+}
+inline int vd32_default_warps(int nz, int nslot, bool comp, int ntile) {
   int nw = 1;
-  for (int b = 4; b >= 2; b--) {
+  const int b0 = col_blocks(ntile);
+  for (int b = b0; b >= (b0 < 2 ? b0 : 2); b--) {
     nw = 1;
     const int most = b == 4 ? col_warps(nslot) : kVd32MaxWarps / b;
     while (nw < most && b * (vd32_smem(nz, nw + 1, false, comp) + 1024) <= 196 * 1024)

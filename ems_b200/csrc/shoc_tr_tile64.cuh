@@ -648,11 +648,17 @@ inline size_t vd64_tuned(int nz, int nw) { return (size_t)nz * 32 * (4 + 2 * 8 *
 // still deeper ones what a block has within 200 KB (448 x 300 x 60, 16 tracers: 1
 // warp 1.21 ms, 2 0.91, 3 1.15, 6 0.89; 400 x 300 x 80, 12 tracers: 1 warp 1.69, 2
 // 1.24, 4 0.95, 5 1.05).
-inline int vd64_default_warps(int nz, int nslot) {
+inline int vd64_default_warps(int nz, int nslot, int ntile) {
   int nw = 1;
-  const bool shallow = 4 * (vd64_smem(nz, 4) + 1024) <= 227 * 1024;
+  const int b0 = col_blocks(ntile);  // (few tiles: as many warps as a block may have)
+  const bool shallow = b0 > 2 && 4 * (vd64_smem(nz, 4) + 1024) <= 227 * 1024;
   const int most = shallow ? col_warps(nslot) : kVd64MaxWarps / 2;
-  while (nw < most && 2 * (vd64_smem(nz, nw + 1) + 1024) <= 160 * 1024) nw++;
+  if (b0 > 1)
+    while (nw < most && 2 * (vd64_smem(nz, nw + 1) + 1024) <= 160 * 1024) nw++;
+  else
+    while (nw < most && vd64_smem(nz, nw + 1) <= 200 * 1024 &&
+           vd64_tuned(nz, nw + 1) <= 227 * 1024)
+      nw++;
   if (nw == 1) {
     nw = 2;
     if (2 * (vd64_smem(nz, nw) + 1024) > 227 * 1024)
