@@ -60,9 +60,9 @@ struct Fused {
 // row j of a column's tridiagonal factors in k_step32's shared memory
 struct FacVec {
   const float4 *l;
-  __device__ __forceinline__ float cm1(int j) const { return l[j * 32].x; }
-  __device__ __forceinline__ float rdiv(int j) const { return l[j * 32].y; }
-  __device__ __forceinline__ float ud(int j) const { return l[j * 32].z; }
+  __device__ __forceinline__ float x(int j) const { return l[j * 32].x; }
+  __device__ __forceinline__ float cm1(int j) const { return l[j * 32].y; }
+  __device__ __forceinline__ float rdiv(int j) const { return l[j * 32].z; }
   __device__ __forceinline__ float re(int j) const { return l[j * 32].w; }
 };
 
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(kFusedThreads, 2)
                        adv ? accF[slot * 32 + lane] : 0.0};
       bool bad = false;
       cp_async_wait<0>();
-      column_finish<LAST, false>(G, F, W, O, T, ss, tc, col, n, tbdy, adv, vdf, A0, S0, 32, fac,
+      column_finish<LAST, false, false>(G, F, W, O, T, ss, tc, col, n, tbdy, adv, vdf, A0, S0, 32, fac,
                                  C0, D0, H, tr, to, area, ia, idt, cs, Fu.carry,
                                  steady, nwarn, bad);
       if (bad) nstat |= ST_NAN;

@@ -289,6 +289,7 @@ constexpr int SD_PROBE = 1;   // leave the surface vectors as they are
 constexpr int SD_SEARCH = 2;  // the sub-step minimum into W.dtm_bits
 constexpr int SD_F32 = 4;     // also the FP32 thickness and LU factors
 constexpr int SD_WORK = 8;    // w5, w9, dbz, dfz of the tile kernels' columns
+constexpr int SD_UD = 32;     // FP32_COMP: ud in place of dz / dt
 constexpr int SD_LU64 = 16;   // FP64 LU factors of the tile kernels' columns
                               // (the general path's columns get all of them)
 // Warps of a block: one per layer up to eight (a window of few layers has nothing
@@ -490,16 +491,15 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
   }
   if (wy == 1 && solve && (what & SD_F32)) {
     // the same matrix eliminated from the top (the FP32-mixed correction
-    // solve): e(j) = C(j) - cm1(j+1) cm1(j+1) / e(j+1); row j keeps 1 / e(j)
+    // solve): e(j) = C(j) - cm1(j+1) cm1(j+1) / e(j+1)
     const int kt = kb + jn - 1, kl = kb + jb - 1;
-    double cm1 = sCm[kt * 32], e = sE[kt * 32] - cm1;
-    for (int k = kt; k >= kl; --k) {
-      const double re = 1.0 / e;
-      sE[k * 32] = re;
-      if (k == kl) break;
-      const double up = cm1;
-      cm1 = k - 1 > kl ? sCm[(k - 1) * 32] : 0.0;
-      e = (sE[(k - 1) * 32] - cm1 - up) - up * (up * re);
+    double up = sCm[kt * 32], e = sE[kt * 32] - up;
+    sE[kt * 32] = e;
+    for (int k = kt - 1; k >= kl; --k) {
+      const double cm1 = k > kl ? sCm[k * 32] : 0.0;
+      e = (sE[k * 32] - cm1 - up) - up * (up / e);
+      sE[k * 32] = e;
+      up = cm1;
     }
   }
   if (wy == 0) {
@@ -540,19 +540,20 @@ __global__ void __launch_bounds__(kSetDzWarps * 32, 4)
       // the elimination factor, as the recurrence formed it (cm1 is the upper
       // diagonal of the row below); where the second elimination has the faces'
       // place it is formed again
-      const double ud = j <= jb           ? 0.0
-                        : (what & SD_F32) ? cm1 / sDv[(k - 1) * 32]
-                                          : sZ[k * 32];
+      double ud = 0.0;
+      if (j > jb && (lu64 || (what & SD_UD)))
+        ud = (what & SD_F32) ? cm1 / sDv[(k - 1) * 32] : sZ[k * 32];
+      const double dzdt = dzc / dt;
       if (lu64) {
         W.vd_cm1[cc] = cm1;
         W.vd_div[cc] = div;
         W.vd_ud[cc] = ud;
-        W.vd_dzdt[cc] = dzc / dt;
+        W.vd_dzdt[cc] = dzdt;
         if (what & SD_LU64) W.vd_rdiv[cc] = div_range(div) == kDivLo ? 1.0 / div : 0.0;
       }
       if (what & SD_F32)
-        W.lu32[cc] =
-            make_float4((float)cm1, (float)(1.0 / div), (float)ud, (float)sE[k * 32]);
+        W.lu32[cc] = make_float4((float)((what & SD_UD) ? ud : dzdt), (float)cm1,
+                                 (float)(1.0 / div), (float)(1.0 / sE[k * 32]));
     }
     if (late) {
       const double dzm = j > 1 ? W.dz[sC[(k - 1) * 32]] : dzsed;
@@ -1923,7 +1924,7 @@ void launch_lateral(shoc_tr_gpu *h, int cur, const TrSet &T, bool reset) {
 // follow from the precision)
 void launch_set_dz(shoc_tr_gpu *h, int what) {
   if (h->esize == sizeof(float))
-    what |= SD_F32 | (h->comp ? SD_WORK : 0);
+    what |= SD_F32 | (h->comp ? SD_WORK | SD_UD : 0);
   else
     what |= SD_WORK | SD_LU64;
   const int nd = std::max(1, h->vd_depth.back());

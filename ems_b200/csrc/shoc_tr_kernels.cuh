@@ -122,9 +122,10 @@ struct Work {
   unsigned long long *dtm_bits;
   unsigned long long *nwarn;
   int *serial_list, *serial_count;
-  // FP32-mixed path: layer thickness and the solve's factors {cm1, 1/div, ud, 1/e},
-  // each formed in FP64 and rounded once: div the diagonal eliminated from the
-  // bottom, ud(j) = cm1(j) / div(j-1), e the diagonal eliminated from the top
+  // FP32-mixed path: layer thickness and the solve's factors {dz/dt, or with
+  // FP32_COMP ud; cm1; 1/div; 1/e}, each formed in FP64 and rounded once: div the
+  // diagonal eliminated from the bottom, ud(j) = cm1(j) / div(j-1), e the diagonal
+  // eliminated from the top
   float *dz32;
   float4 *lu32;
 };

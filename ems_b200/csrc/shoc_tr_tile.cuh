@@ -403,8 +403,8 @@ struct ColSums {
 // stride sa; an advected tracer (tbdy) holds its advected values below the
 // surface, any other tracer every layer's old value (A0 is overwritten, so is
 // S0).  fac: the tridiagonal factors of row j: cm1, the reciprocal diagonals rdiv
-// (eliminated from the bottom: LU) and re (from the top: UL) and the elimination
-// factor ud of LU (0 in the bottom row).  C0, D0: cells and
+// (eliminated from the bottom: LU) and re (from the top: UL), and dzdt or, with UD,
+// the elimination factor ud of LU (0 in the bottom row).  C0, D0: cells and
 // FP64 thicknesses, row stride 32; H: the water depth the carry is spread over,
 // the thicknesses from the surface cell's and then the bottom up.
 // RES: an advected tracer's A0 holds every layer's stored advection result
@@ -417,7 +417,7 @@ struct ColSums {
 // the bottom up, thick layers first, and keeps its rounding errors: without them
 // the 24-bit values of the thin layers on top end on ties, which lean one way
 // (512 x 256 x 50 stiff layers, 1000 steps: a drift of -7e-16 of the mass against 5e-17).
-template <bool LAST, bool RES, class Fac>
+template <bool LAST, bool RES, bool UD, class Fac>
 __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const Work &W,
                                               const Opt &O, const TrSet &T, const SubStep &ss,
                                               const TileCol &tc, int col, int n, bool tbdy,
@@ -470,7 +470,15 @@ __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const
   // one pass up the column below the surface: the computed mass (an
   // advected tracer's FP64 values are stored + residual, or come in cs.m),
   // the clip and, with a solve, the FP32 forward sweep
-  float z = 0.f;  // the sweep's right side, before the division by the diagonal
+  float z = 0.f;  // UD: the sweep's right side, else that over the diagonal
+  auto sweep = [&](int j, double dzdt, float a) {
+    if constexpr (UD) {
+      z = (float)dzdt * a - fac.x(j) * z;
+      return z * fac.rdiv(j);
+    }
+    z = (fac.x(j) * a - fac.cm1(j) * z) * fac.rdiv(j);
+    return z;
+  };
   double m = 0.0;
   for (int j = 0; j < nk; ++j) {
     float a = A0[j * sa];
@@ -490,8 +498,7 @@ __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const
     if (R0) R0[j * sa] = lo_bits((float)r);
     if (tbdy) nw += (a < mn_up || a > mx_dn);
     if (solve) {
-      z = (float)(dz * idt) * a - fac.ud(j) * z;
-      S0[j * sa] = z * fac.rdiv(j);
+      S0[j * sa] = sweep(j, dz * idt, a);
     }
   }
   mxs += (tbdy && !RES) ? cs.m : m;
@@ -557,42 +564,45 @@ __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const
   } else {
     // the surface row of the forward sweep
     double dzdt1 = dzs * idt;
-    z = (float)dzdt1 * (float)vs - fac.ud(nk) * z;
     // one pass down: the back substitution (FP32), x(j) replacing s(j), and one
     // row behind it the FP64 residual of b - A x for A = dz/dt I + the diffusion
     // operator,
     //   r(j) = dz/dt (a + dl - x) - cm1 (x(j-1) - x) - cp1 (x(j+1) - x)
     // (cp1(j) = cm1(j+1); the bottom row has no cm1 term, the top row no cp1
     // term), whose correction solve's elimination, from the top (UL), follows in
-    // the same pass, its right side h(j) replacing a(j).  No factor is a
-    // product of rounded ones: the FP32 solves' operands are FP64 values rounded once.  The residual's diagonal is the FP64
+    // the same pass, its right side h(j) (UD) or h(j) / e(j) replacing a(j).
+    // With UD, which FP32_COMP takes, the FP32 solves' operands are FP64 values rounded
+    // once.  Else the elimination factors are FP32 products, cm1 / div and cm1 / e of
+    // rounded cm1, 1 / div and 1 / e: the first solve is up to 1.2 times as far off in
+    // stiff columns (RMS), the corrected one the same to three digits, as what is left is
+    // cm1's own rounding; plain FP32 storage shows neither.  The residual's diagonal is the FP64
     // dz / dt, so the refined solve keeps the column mass the mass diagnostic
     // measures; cm1 is the FP32 factor's (the FP64 one, staged as well, changed
     // neither the maximum nor the RMS error over 1000 stiff2048 steps, and its
     // shared memory cost warps).  The FP64 copies of x and of the factors are
     // carried from row to row.
-    float x1 = z * fac.rdiv(nk);  // x of row j + 1
+    float x1 = sweep(nk, dzdt1, (float)vs);  // x of row j + 1
     S0[nk * sa] = x1;
-    float l1 = fac.cm1(nk), u1 = fac.ud(nk);  // factors of row j + 1
+    float l1 = fac.cm1(nk), u1 = fac.x(nk);  // factors of row j + 1
     float g = 0.f, l2 = 0.f;  // of row j + 2: the elimination's right side over e, cm1
     double xd1 = (double)x1, xd2 = 0.0;
     double a1 = vs;  // the value before the solve of row j + 1
     for (int j = nk - 1; j >= 0; --j) {
-      const float x = S0[j * sa] - u1 * x1;
+      const float x = S0[j * sa] - (UD ? u1 : l1 * fac.rdiv(j)) * x1;
       S0[j * sa] = x;
       const double xd = (double)x;
       double r = dzdt1 * ((a1 + dl) - xd1) - (double)l1 * (xd - xd1);
       if (j + 1 < nk) r = r - (double)l2 * (xd2 - xd1);
       a1 = (double)A0[j * sa] + (R0 ? (double)lo_val(R0[j * sa]) : 0.0);
       const float h1 = (float)r - l2 * g;
-      A0[(j + 1) * sa] = h1;
       g = h1 * fac.re(j + 1);
+      A0[(j + 1) * sa] = UD ? h1 : g;
       x1 = x;
       xd2 = xd1;
       xd1 = xd;
       l2 = l1;
       l1 = fac.cm1(j);
-      u1 = fac.ud(j);
+      u1 = fac.x(j);
       dzdt1 = D0[j * 32] * idt;
     }
     double r = dzdt1 * ((a1 + dl) - xd1);
@@ -601,7 +611,8 @@ __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const
     float d = ((float)r - l2 * g) * fac.re(0);
     store(C0[0], (double)S0[0] + (double)d, D0[0]);
     for (int j = 1; j <= nk; ++j) {
-      d = (A0[j * sa] - fac.cm1(j) * d) * fac.re(j);
+      d = UD ? (A0[j * sa] - fac.cm1(j) * d) * fac.re(j)
+             : A0[j * sa] - fac.cm1(j) * fac.re(j) * d;
       store(C0[j * 32], (double)S0[j * sa] + (double)d, D0[j * 32]);
     }
   }
@@ -681,14 +692,14 @@ inline int vd32_default_warps(int nz, int nslot, bool comp, int ntile) {
   const int rounds = nslot > 0 ? (nslot + nw - 1) / nw : 1;
   return nslot > 0 ? (nslot + rounds - 1) / rounds : 1;
 }
-// row j of a column's factors in k_vd32's shared memory (p: the column's cm1
-// at its bottom row, n: floats per factor)
+// row j of a column's factors in k_vd32's shared memory (p: the column's dz/dt
+// or ud at its bottom row, n: floats per factor)
 struct FacSmem {
   const float *p;
   int n;
-  __device__ __forceinline__ float cm1(int j) const { return p[j * 32]; }
-  __device__ __forceinline__ float rdiv(int j) const { return p[n + j * 32]; }
-  __device__ __forceinline__ float ud(int j) const { return p[2 * n + j * 32]; }
+  __device__ __forceinline__ float x(int j) const { return p[j * 32]; }
+  __device__ __forceinline__ float cm1(int j) const { return p[n + j * 32]; }
+  __device__ __forceinline__ float rdiv(int j) const { return p[2 * n + j * 32]; }
   __device__ __forceinline__ float re(int j) const { return p[3 * n + j * 32]; }
 };
 
@@ -822,7 +833,7 @@ __global__ void __launch_bounds__(kVd32MaxWarps * 32)
       int16_t *lo = COMP ? loo + (size_t)n * G.S : nullptr;
       if (COMP) lo[sed] = tbdy ? li[cbot] : li[sed];
       const ColSums cs{0.0, 0.0, adv ? fzs[(size_t)n * G.ncol + col] : 0.0};
-      column_finish<LAST, true>(G, F, W, O, T, ss, tc, col, n, tbdy, adv, vdf, A0of(b), S0of(b),
+      column_finish<LAST, true, COMP>(G, F, W, O, T, ss, tc, col, n, tbdy, adv, vdf, A0of(b), S0of(b),
                                 sa, fac, C0, D0, H, tr, to, area, ia, 1.0 / F.dt, cs, carry,
                                 steady, nwarn, bad, R0, li, lo);
     }

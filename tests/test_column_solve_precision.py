@@ -1,5 +1,5 @@
-"""The FP32 column solve's arithmetic (column_finish, shoc_tr_tile.cuh), restated in
-numpy: its first solve is no further from the 64-bit one than the Thomas solve with
+"""The FP32 column solve's arithmetic (column_finish, shoc_tr_tile.cuh) as FP32_COMP
+takes it, restated in numpy: its first solve is no further from the 64-bit one than the Thomas solve with
 FP64 factors rounded once (the lower diagonal, 1 / div and the elimination factor
 cm1 / div), where a factor made of two rounded ones is; after the FP64 residual and
 the correction, eliminated from the top, the error is that of the FP32 diffusivity.
