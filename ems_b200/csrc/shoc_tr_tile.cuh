@@ -643,8 +643,8 @@ __device__ __forceinline__ void column_finish(const Geo &G, const Flow &F, const
 // Fetching the next tracer's rows into the current one's as its last pass frees
 // them cost more than it hid (2.90 against 2.57 ms on the first case below).
 // A sub-step (B200) with four passes, and now: 1024 x 512 x 50, 24 tracers 2.86 and
-// 2.38 ms; 448 x 300 x 50, 16 tracers, FP32_COMP 0.91 and 0.70; 333 x 217 x 37, 5
-// tracers 0.128 and 0.074; a batch of 56 447 columns, 60 layers, 4 to 32 tracers 0.93
+// 2.41 ms; 448 x 300 x 50, 16 tracers, FP32_COMP 0.91 and 0.70; 333 x 217 x 37, 5
+// tracers 0.128 and 0.076; a batch of 56 447 columns, 60 layers, 4 to 32 tracers 0.93
 // and 0.68.
 
 constexpr int kStage = 8;  // layers a warp of a column kernel stages together
